@@ -155,6 +155,8 @@ B200MOE_API int b200moe_router_topk(const void* x, int x_dtype, const float* w, 
  * b200moe_router_select: adds the partials in index order and applies the scoring,
  * group-limited selection and weight normalisation exactly as b200moe_router_topk, over
  * the first E columns of rows that are partials_row_stride floats apart (the padded count). */
+/* K splits with which b200moe_router_logits_bf16x3 should run for T tokens and E padded expert rows. */
+B200MOE_API int b200moe_router_ksplits(int64_t T, int64_t H, int E);
 B200MOE_API int b200moe_router_logits_bf16x3(const void* x_bf16, const void* w3_bf16, float* partials,
                                  int64_t T, int64_t H, int E, int ksplits, void* stream);
 B200MOE_API int b200moe_router_select(const float* partials, int nsplit, int64_t partials_row_stride,
@@ -433,6 +435,37 @@ B200MOE_API int b200moe_marlin_expand_f16(const void* packed, const void* scales
  * permuted column order (blocks of 64 columns, or of 32 when groupsize == -1). */
 B200MOE_API int b200moe_marlin_pack(const int32_t* q, void* packed_i32, const void* scales_f16,
                         void* scales_out_f16, int64_t K, int64_t N, int64_t groupsize, void* stream);
+
+/* ======================= one pass of a single-rank layer ================== */
+/* DeepseekV3MoE.forward (moe/all2all_moe.py:167-184) at ep_size 1 as one host call: router, permutation
+ * metadata, permute (+ quantize), the two grouped GEMMs, weighted un-permute and, when shared_inter != 0, the
+ * shared experts (:161-165, 182-183).  Same kernels, same order and same results as the separate calls. */
+enum { B200MOE_LAYER_FP8 = 0, B200MOE_LAYER_W4A16 = 1, B200MOE_LAYER_W4A8 = 2 };
+typedef struct b200moe_layer {
+  int32_t struct_bytes;              /* sizeof(b200moe_layer) */
+  int32_t method;                    /* B200MOE_LAYER_*: which grouped GEMM pair, hence which weight layout */
+  int32_t act;                       /* 0 = SiLU, 1 = tanh-GELU */
+  int32_t experts, top_k, n_group, topk_group, scoring, norm_topk_prob;
+  float scaling;
+  int32_t router_rows;               /* rows of router_w3: experts rounded up to a multiple of 128 */
+  int32_t reserved;
+  int64_t hidden, inter;
+  const void* router_w3;             /* as in b200moe_router_logits_bf16x3 */
+  const float* router_bias;          /* [experts] or NULL */
+  const void *w13, *w13_scale, *w13_pairs;   /* e4m3 + f32 scales | packed + pairs | packed + f32 scales + pairs */
+  const void *w2, *w2_scale, *w2_pairs;
+  int64_t shared_inter;              /* width of the shared experts, 0 = none */
+  const void *shared_w13, *shared_w2;        /* bf16 [2*shared_inter, hidden], [hidden, shared_inter] */
+  void *side_stream, *fork_event, *join_event;   /* cudaStream_t / cudaEvent_t of the caller (shared experts only) */
+  int32_t* status;                   /* device status word of the GEMMs, may be NULL */
+} b200moe_layer;
+/* Bytes of workspace a pass of T tokens needs (256-byte aligned); -1 for a bad descriptor. */
+B200MOE_API int64_t b200moe_layer_workspace_bytes(const b200moe_layer* layer, int64_t T);
+/* Where a pass of T tokens leaves its permuted rows and its group table (byte offsets into the workspace). */
+B200MOE_API int b200moe_layer_workspace_layout(const b200moe_layer* layer, int64_t T, int64_t* send, int64_t* seg);
+/* x, y: bf16 [T, hidden], contiguous. */
+B200MOE_API int b200moe_layer_forward(const b200moe_layer* layer, const void* x, void* y, int64_t T,
+                        void* workspace, int64_t workspace_bytes, void* stream);
 
 /* ============ expert-parallel exchange folded into the kernels ============= */
 /* Replaces the two all_to_all_single calls and the host-side split lists of

@@ -67,6 +67,10 @@ SIGNATURES = {
     "b200moe_weight_dequant_int8": (_i, [_p, _p, _p, _i, _i64, _i64, _p]),
     "b200moe_weight_quant_w4a8": (_i, [_p, _i, _p, _p, _p, _p, _i64, _i64, _p]),
     "b200moe_weight_quant_w4a16": (_i, [_p, _i, _p, _p, _p, _i64, _i64, _p]),
+    "b200moe_router_ksplits": (_i, [_i64, _i64, _i]),
+    "b200moe_layer_workspace_bytes": (_i64, [_p, _i64]),
+    "b200moe_layer_workspace_layout": (_i, [_p, _i64, _p, _p]),
+    "b200moe_layer_forward": (_i, [_p, _p, _p, _i64, _p, _i64, _p]),
     "b200moe_pack_bits": (_i, [_p, _p, _i64, _i64, _i, _i, _i, _p]),
     "b200moe_unpack_bits": (_i, [_p, _p, _i64, _i64, _i, _i, _i, _p]),
 }
@@ -74,6 +78,19 @@ SIGNATURES = {
 class GemmOpts(C.Structure):
     """b200moe_gemm_opts: per-call launch options of the grouped GEMMs."""
     _fields_ = [("max_ctas", C.c_int32), ("pair_mode", C.c_int32)]
+
+
+class Layer(C.Structure):
+    """b200moe_layer: everything of a single-rank layer that stays the same from pass to pass."""
+    _fields_ = ([(n, C.c_int32) for n in ("struct_bytes", "method", "act", "experts", "top_k", "n_group", "topk_group",
+                                          "scoring", "norm_topk_prob")]
+                + [("scaling", C.c_float), ("router_rows", C.c_int32), ("reserved", C.c_int32),
+                   ("hidden", C.c_int64), ("inter", C.c_int64)]
+                + [(n, C.c_void_p) for n in ("router_w3", "router_bias", "w13", "w13_scale", "w13_pairs", "w2",
+                                             "w2_scale", "w2_pairs")]
+                + [("shared_inter", C.c_int64)]
+                + [(n, C.c_void_p) for n in ("shared_w13", "shared_w2", "side_stream", "fork_event", "join_event",
+                                             "status")])
 
 
 _lib = None
@@ -127,8 +144,12 @@ def ptr(t) -> int:
     return 0 if t is None else t.data_ptr()
 
 
+# The raw handle of the current stream without building a torch.cuda.Stream around it (0.2 us instead of 2 us).
+_raw_stream, _current_device = torch._C._cuda_getCurrentRawStream, torch._C._cuda_getDevice
+
+
 def stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(_current_device())
 
 
 def require_cuda(*tensors) -> None:
@@ -143,6 +164,7 @@ def require_cuda(*tensors) -> None:
             raise RuntimeError("b200moe operators run on CUDA tensors only (no CPU path)")
         if cur is None:
             cur = torch.cuda.current_device()
-        if t.device.index != cur:
-            raise RuntimeError(f"tensor on cuda:{t.device.index} but the current device is cuda:{cur}: make the "
+        index = t.device.index
+        if index != cur:
+            raise RuntimeError(f"tensor on cuda:{index} but the current device is cuda:{cur}: make the "
                                "tensor's device current before calling (torch.cuda.set_device or torch.cuda.device)")

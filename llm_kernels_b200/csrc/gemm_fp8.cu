@@ -28,6 +28,7 @@
 // writes B200MOE_DEVICE_TIMEOUT to the status word and returns.
 #include <cuda.h>
 
+#include <algorithm>
 #include <type_traits>
 
 #include "common.cuh"
@@ -761,7 +762,8 @@ extern "C" int b200moe_grouped_gemm_fp8(const void* a, int64_t a_row_stride_byte
 static int check_grouped_common(const char* who, const void* a, const void* b, const void* c,
                                 const int64_t* seg, int64_t a_stride, int64_t kbytes, int64_t M_total,
                                 int64_t N, int num_groups, int num_weights) {
-  B200MOE_REQUIRE(a && b && c && seg, B200MOE_BAD_ARG, "%s: null pointer", who);
+  // one group over all rows needs no table
+  B200MOE_REQUIRE(a && b && c && (seg || num_groups == 1), B200MOE_BAD_ARG, "%s: null pointer", who);
   B200MOE_REQUIRE(M_total >= 0 && M_total < (int64_t(1) << 31) && N > 0 && N % 128 == 0 && kbytes > 0 && kbytes % 128 == 0,
                   B200MOE_BAD_SHAPE, "%s: M=%lld N=%lld (N must be a multiple of 128, K of 128 bytes)", who,
                   (long long)M_total, (long long)N);
@@ -846,6 +848,19 @@ extern "C" int b200moe_grouped_gemm_f16(const void* a, int64_t a_row_stride_byte
 // w3 [E, 3H].  The products x*part are exact in f32, the three partial dot products accumulate
 // in the same TMEM accumulator.  The K loop (3H) is split over `ksplits` CTAs per tile whose
 // partial sums land in partials[ks] and are added in index order by b200moe_router_select.
+//
+// The splits spread a decode batch (one m-tile) over the SMs and bound the length of one tensor-core accumulation
+// (about 16 K blocks of 64): the f32 accumulator of the MMA truncates, and the error of a long chain reaches the
+// routing weights (measured 5e-5 relative for 4096-term dot products in two splits, below 1e-5 with short chains);
+// the partial sums are added with IEEE roundings by the selection kernel.
+extern "C" int b200moe_router_ksplits(int64_t T, int64_t H, int E) {
+  const int64_t tiles = std::max<int64_t>(1, ((T + BM - 1) / BM) * ((E + BN - 1) / BN));
+  const int64_t kb = std::max<int64_t>(1, 3 * H / 64);
+  int64_t ks = std::max<int64_t>(1, std::min<int64_t>(16, std::max<int64_t>(148 / tiles, (kb + 15) / 16)));
+  while (ks > 1 && (kb + ks - 1) / ks * (ks - 1) >= kb) --ks;
+  return static_cast<int>(ks);
+}
+
 extern "C" int b200moe_router_logits_bf16x3(const void* x_bf16, const void* w3_bf16, float* partials,
                                             int64_t T, int64_t H, int E, int ksplits, void* stream) {
   B200MOE_REQUIRE(x_bf16 && w3_bf16 && partials, B200MOE_BAD_ARG, "router_logits_bf16x3: null pointer");

@@ -23,6 +23,7 @@ Experts are sharded as in the reference (:130-147): rank r owns experts
 grouped path (moe/sglang_moe_all_gather_all_reduce.py:208-264): w13 [E_l, 2I, H] =
 [gate ; up], w2 [E_l, H, I], both e4m3 with f32 128x128 block scales.
 """
+import ctypes as C
 import math
 from typing import Optional
 
@@ -134,15 +135,7 @@ class MoEGate(nn.Module):
             # many SMs (a decode batch is one m-tile)
             w3 = self._split_weight(w)
             Ep = w3.shape[0]
-            tiles = ((T + 127) // 128) * ((Ep + 255) // 256)
-            kb = 3 * h // 64
-            # Splits also bound the length of one tensor-core accumulation (about 16 K blocks of 64): the f32
-            # accumulator of the MMA truncates, and the error of a long chain reaches the routing weights (measured
-            # 5e-5 relative for 4096-term dot products in two splits, below 1e-5 with short chains); the partial sums
-            # are added with IEEE roundings by the selection kernel.
-            ks = max(1, min(16, max(148 // tiles, -(-kb // 16))))
-            while ks > 1 and -(-kb // ks) * (ks - 1) >= kb:
-                ks -= 1
+            ks = N.lib().b200moe_router_ksplits(T, h, Ep)
             part = self._scratch(ks * T * Ep)
             N.check(N.lib().b200moe_router_logits_bf16x3(N.ptr(x), N.ptr(w3), N.ptr(part), T, h, Ep, ks, N.stream()))
             N.check(N.lib().b200moe_router_select(
@@ -294,6 +287,9 @@ class DeepseekV3MoE(nn.Module):
         self._buffers_cache = {}
         self._status = torch.zeros(1, dtype=torch.int32, device=dev)
         self._last_recv_rows = None
+        self._last, self._last_tokens = None, 0
+        self._native = None               # (key, structure, its address, what it points to) of _describe
+        self._workspace = None
         # Optional per-stage timing: set to a list and every forward appends
         # (stage name, CUDA event recorded when the stage's launches were queued).
         self.stage_events = None
@@ -379,6 +375,10 @@ class DeepseekV3MoE(nn.Module):
     # ---- forward ---------------------------------------------------------------------
     @torch.no_grad()
     def forward(self, hidden_states):
+        if self.ep_size == 1 and self.stage_events is None:
+            y = self._forward_native(hidden_states)
+            if y is not None:
+                return y
         orig_shape = hidden_states.shape
         self._mark("start")
         topk_idx, topk_weight = self.gate(hidden_states)
@@ -391,6 +391,91 @@ class DeepseekV3MoE(nn.Module):
         if self.n_shared:
             self._shared_finish(fork, y)
         return y.view(*orig_shape)
+
+    def _describe(self):
+        """The layer as the C structure of b200moe_layer_forward, or None where that call does not apply.  Rebuilt when
+        a weight, the router or a setting changed since the last pass: `key` is everything the structure was made from."""
+        gate, bufs, cfg = self.gate, self._buffers, self.config
+        w, bias = gate.weight, gate.e_score_correction_bias
+        tensors = [w, bias]
+        tensors += [t for n, t in bufs.items() if t is not None]
+        key = [v for t in tensors for v in (t.data_ptr(), t._version)]
+        key += [self.method, self._gelu, gate.scoring_func, gate.topk_method, gate.top_k, gate.n_group, gate.topk_group,
+                gate.norm_topk_prob, gate.routed_scaling_factor]
+        if self._native is not None and self._native[0] == key:
+            return self._native[1]
+        self._native = None
+        if (gate.scoring_func not in ("sigmoid", "softmax") or gate.topk_method != "noaux_tc" or type(gate) is not MoEGate
+                or w.dtype != torch.float32 or bias.dtype != torch.float32 or gate.top_k != cfg.num_experts_per_tok):
+            return None
+        N.require_cuda(*tensors)
+        assert all(t.is_contiguous() for t in tensors)
+        w3 = gate._split_weight(w)
+        d = N.Layer(struct_bytes=C.sizeof(N.Layer), act=int(self._gelu), experts=cfg.n_routed_experts, top_k=gate.top_k,
+                    n_group=gate.n_group, topk_group=gate.topk_group, scoring=0 if gate.scoring_func == "sigmoid" else 1,
+                    norm_topk_prob=1 if gate.norm_topk_prob else 0, scaling=float(gate.routed_scaling_factor),
+                    router_rows=w3.shape[0], hidden=cfg.hidden_size, inter=cfg.moe_intermediate_size,
+                    router_w3=N.ptr(w3), router_bias=N.ptr(bias), status=N.ptr(self._status))
+        for n in ("w13", "w2"):
+            if self.method == "fp8_block":
+                d.method, parts = 0, (bufs[n + "_weight"], bufs[n + "_weight_scale"], None)
+            elif self.method == "w4a16":
+                d.method, parts = 1, (bufs[n + "_qweight"], None, self._pairs(n, "_scale", "_zero"))
+            else:
+                if not self._raw_nibbles_ok(n):
+                    return None
+                d.method, parts = 2, (bufs[n + "_qweight"], bufs[n + "_weight_scale"], self._pairs(n))
+            for suffix, t in zip(("", "_scale", "_pairs"), parts):
+                setattr(d, n + suffix, N.ptr(t))
+        keep = [w3]
+        if self.n_shared:
+            if self._shared_stream is None:
+                self._shared_stream = torch.cuda.Stream(device=self._dev)
+            ev = [torch.cuda.Event(), torch.cuda.Event()]
+            for e in ev:
+                e.record()                      # creates the handle
+            d.shared_inter = bufs["shared_w2"].shape[2]
+            d.shared_w13, d.shared_w2 = N.ptr(bufs["shared_w13"]), N.ptr(bufs["shared_w2"])
+            d.side_stream, d.fork_event, d.join_event = self._shared_stream.cuda_stream, ev[0].cuda_event, ev[1].cuda_event
+            keep += ev
+        self._native = (key, d, C.addressof(d), keep)
+        return d
+
+    def _forward_native(self, hidden_states):
+        """One pass of a single-rank layer as one host call (b200moe_layer_forward); None where the layer's state needs
+        the separate calls (stages that expand the int4 weights first)."""
+        H = self.config.hidden_size
+        x = hidden_states if hidden_states.is_contiguous() else hidden_states.contiguous()
+        T = x.numel() // H
+        if x.dtype != torch.bfloat16 or T == 0 or x.shape[-1] != H or (
+                self.method != "fp8_block" and
+                T * self.num_experts_per_tok > self.w4_fused_rows_per_group * self.experts_per_rank):
+            return None
+        assert not self.gate.training
+        N.require_cuda(x)
+        if self._describe() is None:
+            return None
+        lib, desc = N.lib(), self._native[2]
+        need = lib.b200moe_layer_workspace_bytes(desc, T)
+        ws = self._workspace
+        if ws is None or ws.numel() < need:
+            ws = self._workspace = torch.empty(need, dtype=torch.uint8, device=self._dev)
+        y = torch.empty_like(x)
+        N.check(lib.b200moe_layer_forward(desc, x.data_ptr(), y.data_ptr(), T, ws.data_ptr(), ws.numel(), N.stream()))
+        self._last_recv_rows, self._last = T * self.num_experts_per_tok, None
+        self._last_tokens = T
+        return y
+
+    def _last_rows(self):
+        """(permuted rows, row count, group table, weight indices) of the last forward."""
+        if self._last is None and self._last_tokens:
+            send, seg = C.c_int64(), C.c_int64()
+            H, S, E = self.config.hidden_size, self._last_recv_rows, self.config.n_routed_experts
+            N.check(N.lib().b200moe_layer_workspace_layout(self._native[2], self._last_tokens, C.byref(send), C.byref(seg)))
+            ws, rec = self._workspace, self._record_bytes(H)
+            self._last = (ws[send.value:send.value + S * rec].view(S, rec), S,
+                          ws[seg.value:seg.value + 8 * (E + 1)].view(torch.int64), None)
+        return self._last
 
     def make_graphed(self, example: torch.Tensor, warmup: int = 2):
         """Captures one forward pass for inputs of `example`'s shape and dtype into a CUDA graph and
@@ -419,6 +504,7 @@ class DeepseekV3MoE(nn.Module):
             graph.replay()
             return static_out
         run.graph, run.static_input, run.static_output = graph, static_in, static_out
+        run.workspace = self._workspace     # the graph's kernels keep using it, whatever later passes allocate
         return run
 
     # the reference's unfused entry point routes to the same pipeline
@@ -816,7 +902,7 @@ class DeepseekV3MoE(nn.Module):
         """Re-launches the two grouped GEMMs of the last forward on its resident inputs (all
         groups, current stream) and returns their average durations in ms, timed with CUDA
         events: (gemm1_ms, gemm2_ms, rows).  fp8_block only."""
-        assert self.method == "fp8_block" and getattr(self, "_last", None) is not None
+        assert self.method == "fp8_block" and self._last_rows() is not None
         buf, rows, seg, widx = self._last
         H, I = self.config.hidden_size, self.config.moe_intermediate_size
         a_q, a_s = buf[:, :H], buf[:, H:H + (H // 128) * 4].view(torch.float32)
