@@ -1,4 +1,7 @@
 // Status strings and the per-thread last-error message of the C ABI.
+#include <mutex>
+#include <vector>
+
 #include "common.cuh"
 
 namespace b200moe {
@@ -17,6 +20,21 @@ int check_launch(const char* what) {
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess)
     return fail(B200MOE_LAUNCH_FAILED, "%s: %s", what, cudaGetErrorString(e));
+  return B200MOE_OK;
+}
+
+int set_dynamic_smem(const void* kernel, size_t bytes) {
+  struct Entry { const void* kernel; int dev; size_t bytes; };
+  static std::mutex mu;
+  static std::vector<Entry> done;
+  int dev = -1;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lock(mu);
+  for (const Entry& e : done)
+    if (e.kernel == kernel && e.dev == dev && e.bytes >= bytes) return B200MOE_OK;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+  if (e != cudaSuccess) return fail(B200MOE_LAUNCH_FAILED, "%zu bytes of shared memory: %s", bytes, cudaGetErrorString(e));
+  done.push_back({kernel, dev, bytes});
   return B200MOE_OK;
 }
 

@@ -22,6 +22,9 @@ inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s
 // Returns B200MOE_OK or records the CUDA launch error.
 int check_launch(const char* what);
 
+// Opts a kernel in to `bytes` of dynamic shared memory on the current device, once per kernel and device.
+int set_dynamic_smem(const void* kernel, size_t bytes);
+
 #define B200MOE_REQUIRE(cond, status, ...)                 \
   do {                                                     \
     if (!(cond)) return ::b200moe::fail((status), __VA_ARGS__); \

@@ -33,6 +33,7 @@
 
 #include "common.cuh"
 #include "epilogue.cuh"
+#include "gemm_rows.cuh"
 #include "ptx.cuh"
 #include "tma_host.cuh"
 
@@ -590,8 +591,7 @@ gemm_block_kernel(const __grid_constant__ RowMaps tmap_a,
 // ---- host side ---------------------------------------------------------------------------
 template <int KIND, bool PAIR>
 static int launch_gemm_as(const RowMaps& ma, const CUtensorMap& mb, const GemmParams& p, int grid, cudaStream_t st) {
-  cudaFuncSetAttribute(gemm_block_kernel<KIND, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       static_cast<int>(kSmemBytes));
+  if (int rc = set_dynamic_smem(reinterpret_cast<const void*>(gemm_block_kernel<KIND, PAIR>), kSmemBytes)) return rc;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(grid));
   cfg.blockDim = dim3(kThreads);
@@ -683,6 +683,15 @@ __global__ void __launch_bounds__(256) sum_splits_kernel(const float* __restrict
     }
   }
 }
+
+static int sum_splits(const float* partials, int ksplits, int64_t n, void* c, int c_dtype, cudaStream_t st) {
+  const unsigned grid = static_cast<unsigned>(std::min<int64_t>((n / 4 + 255) / 256, 148 * 8));
+  if (c_dtype == B200MOE_F32) sum_splits_kernel<float><<<grid, 256, 0, st>>>(partials, ksplits, n, static_cast<float*>(c));
+  else if (c_dtype == B200MOE_BF16) sum_splits_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(partials, ksplits, n, static_cast<__nv_bfloat16*>(c));
+  else sum_splits_kernel<__half><<<grid, 256, 0, st>>>(partials, ksplits, n, static_cast<__half*>(c));
+  return check_launch("sum_splits");
+}
+
 }  // namespace b200moe
 
 extern "C" int b200moe_gemm_fp8_block_splitk(const void* a, const float* a_s, const void* b, const float* b_s,
@@ -706,15 +715,8 @@ extern "C" int b200moe_gemm_fp8_block_splitk(const void* a, const float* a_s, co
   GemmParams p{a_s, K / 128, b_s, partials, N * 4, nullptr, 0, nullptr, nullptr, M,
                static_cast<int>(N), static_cast<int>(K), 1, 1, B200MOE_F32, 0, nullptr, ksplits, M * N * 4, 0,
                nullptr, nullptr, 0, 0};
-  const int64_t tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN) * ksplits;
-  if (int rc = launch_gemm<kFp8>(a, K, b, p, tiles, as_stream(stream))) return rc;
-  const int64_t n = M * N;
-  const unsigned grid = static_cast<unsigned>(std::min<int64_t>((n / 4 + 255) / 256, 148 * 8));
-  cudaStream_t st = as_stream(stream);
-  if (c_dtype == B200MOE_F32) sum_splits_kernel<float><<<grid, 256, 0, st>>>(partials, ksplits, n, static_cast<float*>(c));
-  else if (c_dtype == B200MOE_BF16) sum_splits_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(partials, ksplits, n, static_cast<__nv_bfloat16*>(c));
-  else sum_splits_kernel<__half><<<grid, 256, 0, st>>>(partials, ksplits, n, static_cast<__half*>(c));
-  return check_launch("sum_splits");
+  if (int rc = launch_gemm<kFp8>(a, K, b, p, ((M + BM - 1) / BM) * ((N + BN - 1) / BN) * ksplits, as_stream(stream))) return rc;
+  return sum_splits(partials, ksplits, M * N, c, c_dtype, as_stream(stream));
 }
 
 extern "C" int b200moe_grouped_gemm_fp8(const void* a, int64_t a_row_stride_bytes, const float* a_s,
@@ -751,6 +753,10 @@ extern "C" int b200moe_grouped_gemm_fp8(const void* a, int64_t a_row_stride_byte
     B200MOE_REQUIRE(c_row_stride_bytes >= N * (c_dtype == B200MOE_F32 ? 4 : 2), B200MOE_BAD_ARG, "grouped_gemm_fp8: c row stride too small");
   }
   if (M_total == 0) return B200MOE_OK;
+  if (!opts && !c_row_map && !c_row_addr && M_total <= rows::kMaxRowsPerGroup * num_groups)
+    return rows::launch_fp8(a, a_row_stride_bytes, a_s, a_s_row_stride, b, b_s, c, c_dtype, c_row_stride_bytes, c_s, c_s_row_stride,
+                            M_total, N, K, num_groups, num_weights, seg_indptr, weight_indices, epilogue != 0 ? 1 : 0,
+                            epilogue == 4 ? 1 : 0, status_word, as_stream(stream));
   GemmParams p{a_s, a_s_row_stride, b_s, c, c_row_stride_bytes, c_s, c_s_row_stride, seg_indptr,
                weight_indices, M_total, static_cast<int>(N), static_cast<int>(K), num_groups,
                num_weights, c_dtype, epilogue == 4 ? 1 : epilogue, status_word, 1, 0, 0, c_row_map, c_row_addr, 0,

@@ -364,7 +364,7 @@ extern "C" int b200moe_grouped_gemm_w4a16(const void* a, int64_t a_row_stride_by
   w4::Params16 p{static_cast<const uint32_t*>(scale_zero_t), c, c_row_stride_bytes, seg_indptr, weight_indices, M_total,
                  static_cast<int>(N), static_cast<int>(K), num_groups, c_dtype, epilogue != 0 ? 1 : 0,
                  epilogue == 5 ? 1 : 0, status_word};
-  cudaFuncSetAttribute(w4::gemm_w4a16_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(w4::kSmem16));
+  if (int rc = set_dynamic_smem(reinterpret_cast<const void*>(w4::gemm_w4a16_kernel), w4::kSmem16)) return rc;
   w4::gemm_w4a16_kernel<<<sms, w4::kThreads, w4::kSmem16, as_stream(stream)>>>(ma, mp, p);
   return check_launch("gemm_w4a16_kernel");
 }

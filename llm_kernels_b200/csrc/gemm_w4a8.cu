@@ -119,15 +119,6 @@ __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volati
   return __all_sync(0xffffffffu, ptx::mbar_wait(bar, parity, abort_flag));
 }
 
-__device__ __forceinline__ void tmem_ld_wait16(uint32_t (&a)[16], uint32_t (&b)[16]) {
-  asm volatile("tcgen05.wait::ld.sync.aligned;"
-               : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]), "+r"(a[4]), "+r"(a[5]), "+r"(a[6]), "+r"(a[7]),
-                 "+r"(a[8]), "+r"(a[9]), "+r"(a[10]), "+r"(a[11]), "+r"(a[12]), "+r"(a[13]), "+r"(a[14]), "+r"(a[15]),
-                 "+r"(b[0]), "+r"(b[1]), "+r"(b[2]), "+r"(b[3]), "+r"(b[4]), "+r"(b[5]), "+r"(b[6]), "+r"(b[7]),
-                 "+r"(b[8]), "+r"(b[9]), "+r"(b[10]), "+r"(b[11]), "+r"(b[12]), "+r"(b[13]), "+r"(b[14]), "+r"(b[15])
-               :: "memory");
-}
-
 __global__ void __launch_bounds__(kThreads8, 1)
 gemm_w4a8_kernel(const __grid_constant__ RowMaps tmap_a, const __grid_constant__ CUtensorMap tmap_p, const Params8 p) {
   extern __shared__ uint8_t smem_raw[];
@@ -431,7 +422,7 @@ gemm_w4a8_kernel(const __grid_constant__ RowMaps tmap_a, const __grid_constant__
             float4 tq[8];
 #pragma unroll
             for (int j4 = 0; j4 < 4; ++j4) { rq[j4] = rsp[mb * 4 + j4]; tq[2 * j4] = tsp[mb * 8 + j4 * 2]; tq[2 * j4 + 1] = tsp[mb * 8 + j4 * 2 + 1]; }
-            tmem_ld_wait16(d0, d1);
+            ptx::tmem_ld_wait16(d0, d1);
             // exact integers: sum_k a_k (q_k - z) s = s (a.q - z sum_k a_k)
 #pragma unroll
             for (int j4 = 0; j4 < 4; ++j4) {
@@ -597,7 +588,7 @@ extern "C" int b200moe_grouped_gemm_w4a8(const void* a, int64_t a_row_stride_byt
   w4::Params8 p{a_s, a_s_row_stride, b_s, static_cast<const uint16_t*>(s4z4_t), c, c_row_stride_bytes, c_s, c_s_row_stride,
                 seg_indptr, weight_indices, M_total, static_cast<int>(N), static_cast<int>(K), num_groups, c_dtype,
                 epilogue != 0 ? 1 : 0, epilogue == 4 ? 1 : 0, status_word};
-  cudaFuncSetAttribute(w4::gemm_w4a8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(w4::kSmem8));
+  if (int rc = set_dynamic_smem(reinterpret_cast<const void*>(w4::gemm_w4a8_kernel), w4::kSmem8)) return rc;
   w4::gemm_w4a8_kernel<<<sms, w4::kThreads8, w4::kSmem8, as_stream(stream)>>>(ma, mp, p);
   return check_launch("gemm_w4a8_kernel");
 }

@@ -285,6 +285,15 @@ __device__ __forceinline__ void tmem_ld_wait32(uint32_t (&r)[32]) {
       :
       : "memory");
 }
+// The same for two 16-column loads.
+__device__ __forceinline__ void tmem_ld_wait16(uint32_t (&a)[16], uint32_t (&b)[16]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]), "+r"(a[4]), "+r"(a[5]), "+r"(a[6]), "+r"(a[7]),
+                 "+r"(a[8]), "+r"(a[9]), "+r"(a[10]), "+r"(a[11]), "+r"(a[12]), "+r"(a[13]), "+r"(a[14]), "+r"(a[15]),
+                 "+r"(b[0]), "+r"(b[1]), "+r"(b[2]), "+r"(b[3]), "+r"(b[4]), "+r"(b[5]), "+r"(b[6]), "+r"(b[7]),
+                 "+r"(b[8]), "+r"(b[9]), "+r"(b[10]), "+r"(b[11]), "+r"(b[12]), "+r"(b[13]), "+r"(b[14]), "+r"(b[15])
+               :: "memory");
+}
 // Two IEEE f32 fused multiply-adds in one instruction: (d0, d1) += (a0, a1) * (s.x, s.y), where `s2`
 // holds the two multipliers packed in 64 bits (pack_f32x2).  Per lane identical to fmaf().
 __device__ __forceinline__ uint64_t pack_f32x2(float lo, float hi) {

@@ -52,7 +52,16 @@ def weight_dequant(x: torch.Tensor, s: torch.Tensor, block_size: int = 128) -> t
     return y
 
 
-_partials = {}
+_workspaces = {}
+
+
+def _workspace(device, nbytes: int) -> torch.Tensor:
+    """One scratch buffer per device and stream."""
+    key = (device, N.stream())
+    ws = _workspaces.get(key)
+    if ws is None or ws.numel() < nbytes:
+        ws = _workspaces[key] = torch.empty(nbytes, dtype=torch.uint8, device=device)
+    return ws
 
 
 def _split_k(M: int, Nn: int, K: int) -> int:
@@ -84,13 +93,10 @@ def fp8_gemm(a: torch.Tensor, a_s: torch.Tensor, b: torch.Tensor, b_s: torch.Ten
     c = a.new_empty(*a.size()[:-1], Nn, dtype=out_dtype or torch.get_default_dtype())
     ks = _split_k(M, Nn, K) if ksplits is None else int(ksplits)
     if ks > 1 and M > 0:
-        key = (a.device, torch.cuda.current_stream(a.device).cuda_stream)
-        part = _partials.get(key)
-        if part is None or part.numel() < ks * M * Nn:
-            part = _partials[key] = torch.empty(ks * M * Nn, dtype=torch.float32, device=a.device)
+        part = _workspace(a.device, ks * M * Nn * 4)
         N.check(N.lib().b200moe_gemm_fp8_block_splitk(N.ptr(a), N.ptr(a_s), N.ptr(b), N.ptr(b_s), N.ptr(c),
                                                       N.dtype_code(c.dtype), M, Nn, K, ks, N.ptr(part),
-                                                      part.numel() * 4, N.stream()))
+                                                      part.numel(), N.stream()))
         return c
     N.check(N.lib().b200moe_gemm_fp8_block(N.ptr(a), N.ptr(a_s), N.ptr(b), N.ptr(b_s), N.ptr(c),
                                            N.dtype_code(c.dtype), M, Nn, K, N.stream()))
