@@ -1,19 +1,28 @@
-// Grouped w4a16 GEMM (asymmetric group-128 int4 weights, bf16 activations) with the dequantization fused into the
-// operand path (no expanded copy of the weights).
+// Grouped w4a16 GEMM (asymmetric group-128 int4 weights, w = bf16((q - zero) * scale), bf16 activations, f32 accumulation) with
+// the dequantization fused into the operand path (no expanded copy of the weights).
 //
-// One persistent CTA per SM, 512 threads:
-//   warp 0       TMA producer of the PACKED weights (+ the K group's (scale, zero) pairs as bulk copies), 6-slot ring
-//   warp 2       TMA producer of the bf16 activation tile (box of 16/32/64/128 rows x 128 B), 3-slot ring
-//   warps 12-15  converters: one packed word (8 consecutive k of one output channel, quantization/bitpack.py:38-67)
-//                becomes one 16-byte chunk of a bf16 operand row, w = bf16((q - zero) * scale) as
-//                b200moe_w4a16_expand_bf16 (the zero-point extension of
-//                fast_dequant/simple_marlin/marlin_w4a16_gemm.cu:44-64), written in the 128-byte-swizzled layout the
-//                tensor core reads (2 slots); fence.proxy.async, arrive
-//   warp 1       owns TMEM; 4 x tcgen05.mma.kind::f16 (M128 N256 K16) per K block; there are no block scales, so the
-//                whole K loop accumulates in TMEM (one stage per tile, the epilogue of tile i overlaps tile i + 1)
-//   warps 4-11   tile epilogue (plain, or act(gate) * up); warps whose 32 rows lie beyond the group's rows skip it
-// Each weight tile is converted once per (m-tile, n-tile): the kernel is for groups of about one m-tile (decode);
-// callers with many rows per expert expand once instead.
+// What bounds it: the conversion of every packed weight to bf16 by the CUDA cores, once per chunk of tokens, then the packed
+// bytes themselves.  The weights are the M = 128 side of the MMA and their operand lives in TENSOR MEMORY: lane = output
+// channel, column = two consecutive k.  A converter thread owns one channel, reads its packed words (eight consecutive k each,
+// quantization/bitpack.py:38-67) from the TMA ring and stores bf16 pairs with tcgen05.st; the converted weights never touch
+// shared memory, whose traffic (write the 32 KB tile, read it and a 128-row token tile for the MMA) bounded a version with
+// the tokens on the M side.  The tokens are the N = 16..CHUNK columns, so few rows cost little tensor-core time.
+//
+// Measured on 8 experts of a Mixtral layer (gate/up N 28672 K 4096, then down N 4096 K 14336; us; tokens on the M side and
+// weights through shared memory -> here): 1-16 rows per expert 436 + 219 -> 205 + 108, 64 rows 440 + 221 -> 213 + 111,
+// 128 rows 451 + 225 -> 287 + 121, 256 rows 821 + 438 -> 524 + 228.  A 64-k block of 256 channels takes 910 cycles: 1000 for
+// the conversion by each of the two converter groups (they alternate), 150 for the issue of the MMAs.  The roles that are one
+// thread are entered through elect.sync: under `lane == 0` every tcgen05 instruction took about 90 cycles to issue (1340
+// cycles per block).
+//
+// One persistent CTA per SM, 768 threads:
+//   warp 0       TMA producer of the packed words: two boxes of 128 channels x 128 B (256 k) and their (scale, zero)
+//                pairs as bulk copies, 4 slots of 34 KB
+//   warp 2       TMA producer of the token rows: box of 16/32/64/128 rows x 64 k, 64 KB ring
+//   warps 8-23   converters: warp w serves TMEM lanes 32 (w % 4).. of channel half (w / 4) % 2 and every other 64-k block
+//   warp 1       owns TMEM: 4 operand stages x 2 halves x 32 columns, 256 columns of accumulators; per 64-k block 2 x 4
+//                tcgen05.mma.kind::f16 (M128, N = tokens, K16); the whole K loop accumulates in TMEM
+//   warps 4-7    tile epilogue (plain, or act(gate) * up); with CHUNK = 64 it overlaps the next tile
 //
 // Every wait is a bounded mbarrier wait; on expiry the kernel drains its copies, frees TMEM, writes
 // B200MOE_DEVICE_TIMEOUT to the status word and returns.
@@ -26,41 +35,66 @@
 #include "w4_common.cuh"
 
 namespace b200moe {
-namespace w4 {
+namespace w4a16 {
 
-constexpr int BM = 128, BN = 256, BK = 128;
-constexpr int kAStages = 3, kBStages = 2, kAccStages = 2;
-constexpr uint32_t kABytes = BM * BK, kBBytes = BN * BK;
-constexpr int kThreads = 512;
-constexpr int kFirstEpiWarp = 4, kEpiWarps = 8, kFirstConvWarp = 12, kConvWarps = 4;
+constexpr int kWStages = 4, kOpStages = 4;
+constexpr uint32_t kWBytes = 2 * 128 * 128;            // two halves of 128 channels x 32 words (256 k)
+constexpr uint32_t kPairBytes = 128 * 4;               // (scale, zero) of one half and one 128-k group
+constexpr uint32_t kWSlot = kWBytes + 4 * kPairBytes;  // [group][half][128] pairs behind the words
+constexpr uint32_t kTRing = 65536;                     // token ring: 8 slots of 64 rows or 4 of 128 rows, 128 B each
+constexpr int kMaxTStages = 8;
+constexpr int kThreads = 768, kEpiWarp0 = 4, kEpiWarps = 4, kConvWarp0 = 8, kConvWarps = 16;
+constexpr uint32_t kAccCol = 256;                      // first accumulator column
+static_assert(kWSlot % 1024 == 0, "the 128-byte swizzle needs 1 KB aligned slots");
 
-struct Tile { int m0, m_end, expert, nt; };
-
-constexpr int kQStages = 6;                              // packed ring: 256 rows x 8 words = 8 KB per K block
-constexpr uint32_t kQBytes = 256 * 8 * 4;
-constexpr uint32_t kQPair = 128 * 4;                     // (scale, zero) of the 128 channels of one half
-constexpr uint32_t kQSlot = kQBytes + 2 * kQPair;
-struct Tail16 {
-  uint64_t a_full[kAStages], a_empty[kAStages];
-  uint64_t p_full[kQStages], p_empty[kQStages];
-  uint64_t b_full[kBStages], b_empty[kBStages];
-  uint64_t tmem_full[kAccStages], tmem_empty[kAccStages];
+struct Tail {
+  uint64_t w_full[kWStages], w_empty[kWStages];
+  uint64_t t_full[kMaxTStages], t_empty[kMaxTStages];
+  uint64_t op_full[kOpStages], op_empty[kOpStages];
+  uint64_t acc_full[2], acc_empty[2];
   uint32_t tmem_base;
   int abort_flag;
-  int32_t seg[kMaxGroups + 1];
-  int32_t pref[kMaxGroups + 1];
+  int32_t seg[w4::kMaxGroups + 1];
+  int32_t pref[w4::kMaxGroups + 1];                    // exclusive prefix of token chunks per group
 };
-constexpr size_t kRing16 = size_t(kAStages) * kABytes + size_t(kBStages) * kBBytes + size_t(kQStages) * kQSlot;
-constexpr size_t kSmem16 = 1024 + kRing16 + sizeof(Tail16);
+constexpr size_t kSmem = 1024 + size_t(kWStages) * kWSlot + kTRing + sizeof(Tail);
+static_assert(kSmem <= 232448, "shared memory of one CTA");
 
-struct Params16 {
-  const uint32_t* sz_t;           // [W, K/128, N]: (scale, zero) bf16 pairs (scale in the low half), one group's pairs contiguous
+struct Params {
+  const uint32_t* sz_t;           // [W, K/128, N]: (scale, zero) bf16 pairs (scale in the low half)
   void* c; int64_t c_stride;      // bytes
   const int64_t* seg; const int64_t* widx;
-  int64_t M_total;
-  int N, K, num_groups, c_dtype, fused, act;    // K in elements; fused: 0 plain, 1 act(gate)*up -> bf16
+  int N, K, num_groups, c_dtype, fused, act;
   int32_t* status;
 };
+
+struct Tile { int m0, rows, tn, expert, ct; };
+
+template <int CHUNK>
+__device__ __forceinline__ Tile decode(const Tail* sh, const Params& p, int t, int num_ct) {
+  // chunks of one group and channel tile are neighbours: they run at the same time and share the weights in L2
+  int lo = 0, hi = p.num_groups;                       // last g with pref[g] * num_ct <= t
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (sh->pref[mid] * num_ct <= t) lo = mid; else hi = mid;
+  }
+  const int chunks = sh->pref[lo + 1] - sh->pref[lo];
+  const int rem = t - sh->pref[lo] * num_ct;
+  Tile tl;
+  tl.ct = rem / chunks;
+  tl.m0 = sh->seg[lo] + (rem - tl.ct * chunks) * CHUNK;
+  tl.rows = min(CHUNK, sh->seg[lo + 1] - tl.m0);
+  tl.tn = (tl.rows + 15) & ~15;
+  tl.expert = p.widx ? static_cast<int>(p.widx[lo]) : lo;
+  return tl;
+}
+
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  return __all_sync(0xffffffffu, ptx::mbar_wait(bar, parity, abort_flag));
+}
+
+__device__ __forceinline__ uint32_t bf2_bits(__nv_bfloat162 v) { return *reinterpret_cast<const uint32_t*>(&v); }
+__device__ __forceinline__ __nv_bfloat162 bits_bf2(uint32_t v) { return *reinterpret_cast<const __nv_bfloat162*>(&v); }
 
 // One packed word (nibble i = k 8c + i) -> eight bf16 values (q - zero) * scale as four bf16x2 registers in k order.
 // 0x4300 | q is the bf16 number 128 + q; the two subtractions are exact and the product is rounded once, which is
@@ -84,41 +118,54 @@ __device__ __forceinline__ uint4 dequant_word_bf16(uint32_t w, uint32_t scale_ze
   return make_uint4(r[0], r[1], r[2], r[3]);
 }
 
-__device__ __forceinline__ Tile decode_tile16(const Tail16* sh, const Params16& p, int t, int num_n_tiles) {
-  const int mt = t / num_n_tiles;
-  int lo = 0, hi = p.num_groups;
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (sh->pref[mid] <= mt) lo = mid; else hi = mid;
+// One channel's (scale, zero) of a 128-k group, prepared for convert_word: v = (x - c) * s on bf16 pairs, where x holds
+// 128 + q of an even k and 128 + 8 q of the odd k after it.
+struct Affine { uint32_t c, s; bool whole; };
+__device__ __forceinline__ Affine make_affine(uint32_t scale_zero) {
+  const uint32_t sb = scale_zero & 0xFFFFu;
+  const float z = __uint_as_float(scale_zero & 0xFFFF0000u), s = __uint_as_float(sb << 16);
+  Affine a;
+  // 128 + z and 128 + 8 z are bf16 numbers when z is a whole number of 0..15, and s / 8 is exact unless it underflows:
+  // then the one subtraction gives q - z (8 (q - z)) exactly and the product rounds the same real number as
+  // (q - z) * s.  Zero points or scales outside take the general form.
+  a.whole = z >= 0.f && z <= 15.f && z == truncf(z) && ((sb & 0x7F80u) >= (4u << 7) || (sb & 0x7FFFu) == 0u);
+  a.c = bf2_bits(__floats2bfloat162_rn(128.f + z, 128.f + 8.f * z));
+  a.s = bf2_bits(__floats2bfloat162_rn(s, s * 0.125f));
+  return a;
+}
+// Eight nibbles (nibble i = k 8c + i) -> four bf16 pairs in k order: 17 instructions.
+__device__ __forceinline__ void convert_word(uint32_t w, const Affine& a, uint32_t* r) {
+  const uint32_t w1 = w >> 1;
+#pragma unroll
+  for (int b = 0; b < 4; ++b) {
+    // byte b holds nibbles 2b (bits 0-3) and 2b + 1 (bits 3-6 after the shift): 0x4300 | q is 128 + q in bf16
+    const uint32_t x = (__byte_perm(w, w1, b | (b << 4) | ((4 + b) << 8) | ((4 + b) << 12)) & 0x0078000Fu) | 0x43004300u;
+    r[b] = bf2_bits(__hmul2(__hsub2(bits_bf2(x), bits_bf2(a.c)), bits_bf2(a.s)));
   }
-  Tile tl;
-  tl.m0 = sh->seg[lo] + (mt - sh->pref[lo]) * BM;
-  tl.m_end = sh->seg[lo + 1];
-  tl.expert = p.widx ? static_cast<int>(p.widx[lo]) : lo;
-  tl.nt = t - mt * num_n_tiles;
-  return tl;
 }
 
-
+template <int CHUNK>
 __global__ void __launch_bounds__(kThreads, 1)
-gemm_w4a16_kernel(const __grid_constant__ RowMaps tmap_a, const __grid_constant__ CUtensorMap tmap_p, const Params16 p) {
+gemm_w4a16_kernel(const __grid_constant__ w4::RowMaps tmap_a, const __grid_constant__ CUtensorMap tmap_p,
+                  const __grid_constant__ Params p) {
+  constexpr int kTStages = static_cast<int>(kTRing / (CHUNK * 128));
+  constexpr int kAccStages = 128 / CHUNK;              // CHUNK = 64: two, CHUNK = 128: one
+  static_assert(kTStages <= kMaxTStages && kAccStages >= 1, "");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* smem_a = smem;
-  uint8_t* smem_b = smem_a + size_t(kAStages) * kABytes;
-  uint8_t* smem_p = smem_b + size_t(kBStages) * kBBytes;         // kQStages x ([256 rows][8 words] + pairs)
-  Tail16* sh = reinterpret_cast<Tail16*>(smem_p + size_t(kQStages) * kQSlot);
+  uint8_t* smem_t = smem + size_t(kWStages) * kWSlot;
+  Tail* sh = reinterpret_cast<Tail*>(smem_t + kTRing);
   volatile int* abort_flag = &sh->abort_flag;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int KB = p.K / 64;                                        // 64 bf16 = 128 bytes per K block
-  const int KG = p.K / 128;                                       // scale groups along K
-  const int num_n_tiles = p.fused ? (p.N / 2) / 128 : (p.N + BN - 1) / BN;
+  const int KS = p.K / 64;                             // 64-k blocks; even, since K is a multiple of 128
+  const int KW = (KS + 3) / 4;                         // 256-k slots of packed words, the last one maybe half
+  const int num_ct = p.fused ? p.N / 256 : (p.N + 255) / 256;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kAStages; ++s) { ptx::mbar_init(&sh->a_full[s], 1); ptx::mbar_init(&sh->a_empty[s], 1); }
-    for (int s = 0; s < kQStages; ++s) { ptx::mbar_init(&sh->p_full[s], 1); ptx::mbar_init(&sh->p_empty[s], kConvWarps); }
-    for (int s = 0; s < kBStages; ++s) { ptx::mbar_init(&sh->b_full[s], kConvWarps); ptx::mbar_init(&sh->b_empty[s], 1); }
-    for (int s = 0; s < kAccStages; ++s) { ptx::mbar_init(&sh->tmem_full[s], 1); ptx::mbar_init(&sh->tmem_empty[s], kEpiWarps); }
+    for (int s = 0; s < kWStages; ++s) { ptx::mbar_init(&sh->w_full[s], 1); ptx::mbar_init(&sh->w_empty[s], kConvWarps); }
+    for (int s = 0; s < kTStages; ++s) { ptx::mbar_init(&sh->t_full[s], 1); ptx::mbar_init(&sh->t_empty[s], 1); }
+    for (int s = 0; s < kOpStages; ++s) { ptx::mbar_init(&sh->op_full[s], kConvWarps / 2); ptx::mbar_init(&sh->op_empty[s], 1); }
+    for (int s = 0; s < kAccStages; ++s) { ptx::mbar_init(&sh->acc_full[s], 1); ptx::mbar_init(&sh->acc_empty[s], kEpiWarps); }
     sh->abort_flag = 0;
     ptx::fence_barrier_init();
     ptx::fence_proxy_async();
@@ -127,7 +174,7 @@ gemm_w4a16_kernel(const __grid_constant__ RowMaps tmap_a, const __grid_constant_
     ptx::prefetch_tensormap(&tmap_p);
   }
   if (warp == 1) {
-    ptx::tmem_alloc<1>(&sh->tmem_base, kTmemCols);
+    ptx::tmem_alloc<1>(&sh->tmem_base, w4::kTmemCols);
     ptx::tmem_relinquish<1>();
   }
   for (int g = threadIdx.x; g <= p.num_groups; g += kThreads) sh->seg[g] = static_cast<int32_t>(p.seg[g]);
@@ -139,7 +186,7 @@ gemm_w4a16_kernel(const __grid_constant__ RowMaps tmap_a, const __grid_constant_
     for (int g0 = 0; g0 < p.num_groups; g0 += 32) {
       const int g = g0 + lane;
       int v = 0;
-      if (g < p.num_groups) { const int m = sh->seg[g + 1] - sh->seg[g]; v = m > 0 ? (m + BM - 1) / BM : 0; }
+      if (g < p.num_groups) { const int m = sh->seg[g + 1] - sh->seg[g]; v = m > 0 ? (m + CHUNK - 1) / CHUNK : 0; }
       int incl = v;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) { const int u = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += u; }
@@ -150,178 +197,224 @@ gemm_w4a16_kernel(const __grid_constant__ RowMaps tmap_a, const __grid_constant_
   }
   __syncthreads();
   const uint32_t tmem_base = sh->tmem_base;
-  const int total_tiles = sh->pref[p.num_groups] * num_n_tiles;
-  const int first = static_cast<int>(blockIdx.x), step = static_cast<int>(gridDim.x);
-  auto half_rows = [&](const Tile& tl, int& row0, int& row1) {   // first weight row of the tile's two 128-row halves
-    row0 = tl.expert * p.N + (p.fused ? tl.nt * 128 : tl.nt * BN);
-    row1 = p.fused ? tl.expert * p.N + p.N / 2 + tl.nt * 128 : row0 + 128;
+  const int total = sh->pref[p.num_groups] * num_ct, first = static_cast<int>(blockIdx.x), step = static_cast<int>(gridDim.x);
+  // first output channel of the tile's two halves (within the expert's N channels)
+  auto half_ch = [&](const Tile& tl, int& n0, int& n1) {
+    n0 = p.fused ? tl.ct * 128 : tl.ct * 256;
+    n1 = p.fused ? p.N / 2 + tl.ct * 128 : n0 + 128;
   };
 
-  if (warp < kFirstEpiWarp) {
-    ptx::setmaxnreg_dec<48>();
-    if (warp == 0 && lane == 0) {
-      // packed weights: two boxes of 128 rows x 8 words per K block
-      int stage = 0; uint32_t phase = 0;
-      Armed armed;
-      bool ok = true;
-      for (int t = first; ok && t < total_tiles; t += step) {
-        const Tile tl = decode_tile16(sh, p, t, num_n_tiles);
-        int row0, row1;
-        half_rows(tl, row0, row1);
-        const int n0 = row0 - tl.expert * p.N, n1 = row1 - tl.expert * p.N;
-        const bool second = n1 < p.N;
-        for (int kb = 0; kb < KB; ++kb) {
-          if (!ptx::mbar_wait(&sh->p_empty[stage], phase ^ 1u, abort_flag)) { ok = false; break; }
-          uint8_t* sp = smem_p + size_t(stage) * kQSlot;
-          const uint32_t* sz = p.sz_t + (static_cast<int64_t>(tl.expert) * KG + (kb >> 1)) * p.N;   // a group spans 2 K blocks
-          ptx::mbar_arrive_expect_tx(&sh->p_full[stage], kQBytes + kQPair + (second ? kQPair : 0u));
-          armed.arm(stage, phase);
-          ptx::tma_load_2d(sp, &tmap_p, &sh->p_full[stage], kb * 8, row0);
-          ptx::tma_load_2d(sp + kQBytes / 2, &tmap_p, &sh->p_full[stage], kb * 8, row1);
-          ptx::bulk_load(sp + kQBytes, sz + n0, kQPair, &sh->p_full[stage]);
-          if (second) ptx::bulk_load(sp + kQBytes + kQPair, sz + n1, kQPair, &sh->p_full[stage]);
-          if (++stage == kQStages) { stage = 0; phase ^= 1u; }
+  if (warp == 0 && ptx::elect_one()) {
+    // ---- packed words and their (scale, zero) pairs ----------------------------------------------------------------
+    int stage = 0; uint32_t phase = 0;
+    w4::Armed armed;
+    bool ok = true;
+    for (int t = first; ok && t < total; t += step) {
+      const Tile tl = decode<CHUNK>(sh, p, t, num_ct);
+      int n0, n1;
+      half_ch(tl, n0, n1);
+      const bool second = n1 < p.N;
+      const int row0 = tl.expert * p.N + n0, row1 = tl.expert * p.N + n1;
+      const uint32_t* sz = p.sz_t + static_cast<int64_t>(tl.expert) * (p.K / 128) * p.N;
+      for (int kw = 0; kw < KW; ++kw) {
+        if (!ptx::mbar_wait(&sh->w_empty[stage], phase ^ 1u, abort_flag)) { ok = false; break; }
+        uint8_t* sw = smem + size_t(stage) * kWSlot;
+        const bool two = kw * 4 + 2 < KS;              // the slot's second 128-k group exists
+        ptx::mbar_arrive_expect_tx(&sh->w_full[stage], (kWBytes / 2 + kPairBytes * (two ? 2u : 1u)) * (second ? 2u : 1u));
+        armed.arm(stage, phase);
+        ptx::tma_load_2d(sw, &tmap_p, &sh->w_full[stage], kw * 32, row0);          // words past K: zero fill
+        const uint32_t* szk = sz + static_cast<int64_t>(kw) * 2 * p.N;
+        ptx::bulk_load(sw + kWBytes, szk + n0, kPairBytes, &sh->w_full[stage]);
+        if (two) ptx::bulk_load(sw + kWBytes + 2 * kPairBytes, szk + p.N + n0, kPairBytes, &sh->w_full[stage]);
+        if (second) {
+          ptx::tma_load_2d(sw + kWBytes / 2, &tmap_p, &sh->w_full[stage], kw * 32, row1);
+          ptx::bulk_load(sw + kWBytes + kPairBytes, szk + n1, kPairBytes, &sh->w_full[stage]);
+          if (two) ptx::bulk_load(sw + kWBytes + 3 * kPairBytes, szk + p.N + n1, kPairBytes, &sh->w_full[stage]);
         }
+        if (++stage == kWStages) { stage = 0; phase ^= 1u; }
       }
-      if (!ok) armed.drain(sh->p_full, kQStages);
-    } else if (warp == 2 && lane == 0) {
-      int stage = 0; uint32_t phase = 0;
-      Armed armed;
-      bool ok = true;
-      auto box_sel = [](int rows) { return rows <= 16 ? 0 : (rows <= 32 ? 1 : (rows <= 64 ? 2 : 3)); };
-      for (int t = first; ok && t < total_tiles; t += step) {
-        const Tile tl = decode_tile16(sh, p, t, num_n_tiles);
-        const int sel = box_sel(min(BM, tl.m_end - tl.m0));
-        const uint32_t bytes = (16u << sel) * BK;
-        for (int kb = 0; kb < KB; ++kb) {
-          if (!ptx::mbar_wait(&sh->a_empty[stage], phase ^ 1u, abort_flag)) { ok = false; break; }
-          ptx::mbar_arrive_expect_tx(&sh->a_full[stage], bytes);
-          armed.arm(stage, phase);
-          ptx::tma_load_2d(smem_a + size_t(stage) * kABytes, &tmap_a.m[sel], &sh->a_full[stage], kb * BK, tl.m0);
-          if (++stage == kAStages) { stage = 0; phase ^= 1u; }
-        }
+    }
+    if (!ok) armed.drain(sh->w_full, kWStages);
+  } else if (warp == 2 && ptx::elect_one()) {
+    // ---- token rows ------------------------------------------------------------------------------------------------
+    int stage = 0; uint32_t phase = 0;
+    w4::Armed armed;
+    bool ok = true;
+    for (int t = first; ok && t < total; t += step) {
+      const Tile tl = decode<CHUNK>(sh, p, t, num_ct);
+      const int sel = tl.tn <= 16 ? 0 : (tl.tn <= 32 ? 1 : (tl.tn <= 64 ? 2 : 3));
+      for (int ks = 0; ks < KS; ++ks) {
+        if (!ptx::mbar_wait(&sh->t_empty[stage], phase ^ 1u, abort_flag)) { ok = false; break; }
+        ptx::mbar_arrive_expect_tx(&sh->t_full[stage], (16u << sel) * 128u);
+        armed.arm(stage, phase);
+        ptx::tma_load_2d(smem_t + size_t(stage) * (CHUNK * 128), &tmap_a.m[sel], &sh->t_full[stage], ks * 128, tl.m0);
+        if (++stage == kTStages) { stage = 0; phase ^= 1u; }
       }
-      if (!ok) armed.drain(sh->a_full, kAStages);
-    } else if (warp == 1 && lane == 0) {
-      constexpr uint32_t idesc = ptx::umma_idesc(1, 1, 1, BM, BN);     // D f32, A and B bf16
-      int sa = 0, sb = 0, as = 0;
-      uint32_t pa = 0, pb = 0, pacc = 0;
-      bool ok = true;
-      for (int t = first; ok && t < total_tiles; t += step) {
-        if (!ptx::mbar_wait(&sh->tmem_empty[as], pacc ^ 1u, abort_flag)) break;     // the stage's previous tile has been read
-        const uint32_t d = tmem_base + static_cast<uint32_t>(as) * BN;
-        for (int kb = 0; kb < KB; ++kb) {
-          if (!ptx::mbar_wait(&sh->a_full[sa], pa, abort_flag) || !ptx::mbar_wait(&sh->b_full[sb], pb, abort_flag)) { ok = false; break; }
-          ptx::tc_fence_after_sync();
-          const uint64_t adesc = ptx::umma_desc_sw128(ptx::smem_u32(smem_a + size_t(sa) * kABytes));
-          const uint64_t bdesc = ptx::umma_desc_sw128(ptx::smem_u32(smem_b + size_t(sb) * kBBytes));
+    }
+    if (!ok) armed.drain(sh->t_full, kTStages);
+  } else if (warp == 1 && ptx::elect_one()) {
+    // ---- MMA issuer: channels (tensor memory) are the M = 128 rows, tokens (shared memory) the N columns -----------
+    int so = 0, st = 0, as = 0;
+    uint32_t po = 0, pt = 0, pacc = 0;
+    bool ok = true;
+    for (int t = first; ok && t < total; t += step) {
+      const Tile tl = decode<CHUNK>(sh, p, t, num_ct);
+      const uint32_t idesc = ptx::umma_idesc(1, 1, 1, 128, static_cast<uint32_t>(tl.tn));    // D f32, A and B bf16
+      if (!ptx::mbar_wait(&sh->acc_empty[as], pacc ^ 1u, abort_flag)) break;     // the stage's previous tile has been read
+      const uint32_t d = tmem_base + kAccCol + static_cast<uint32_t>(as) * (2 * CHUNK);
+      for (int ks = 0; ks < KS; ++ks) {
+        if (!ptx::mbar_wait(&sh->t_full[st], pt, abort_flag) || !ptx::mbar_wait(&sh->op_full[so], po, abort_flag)) { ok = false; break; }
+        ptx::tc_fence_after_sync();
+        const uint32_t a = tmem_base + static_cast<uint32_t>(so) * 64u;
+        const uint64_t tdesc = ptx::umma_desc_sw128(ptx::smem_u32(smem_t + size_t(st) * (CHUNK * 128)));
 #pragma unroll
-          for (int k = 0; k < BK / 32; ++k) ptx::umma_f16<1>(d, adesc + 2 * k, bdesc + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
-          ptx::umma_commit(&sh->a_empty[sa]);
-          ptx::umma_commit(&sh->b_empty[sb]);
-          if (++sa == kAStages) { sa = 0; pa ^= 1u; }
-          if (++sb == kBStages) { sb = 0; pb ^= 1u; }
+        for (int k = 0; k < 4; ++k) {      // halves alternate: an instruction does not wait for the one that feeds its accumulator
+          ptx::umma_f16_ts(d, a + 8u * k, tdesc + 2 * k, idesc, (ks > 0 || k > 0) ? 1u : 0u);
+          ptx::umma_f16_ts(d + CHUNK, a + 32u + 8u * k, tdesc + 2 * k, idesc, (ks > 0 || k > 0) ? 1u : 0u);
+        }
+        ptx::umma_commit(&sh->op_empty[so]);
+        ptx::umma_commit(&sh->t_empty[st]);
+        if (++so == kOpStages) { so = 0; po ^= 1u; }
+        if (++st == kTStages) { st = 0; pt ^= 1u; }
+      }
+      if (!ok) break;
+      ptx::umma_commit(&sh->acc_full[as]);               // the tile's accumulators are complete
+      if (++as == kAccStages) { as = 0; pacc ^= 1u; }
+    }
+  } else if (warp >= kConvWarp0) {
+    // ---- converters: thread = output channel, one 64-k block (eight packed words) at a time --------------------------
+    const int cw = warp - kConvWarp0;
+    const int q = cw & 3, half = (cw >> 2) & 1, par = cw >> 3;   // kConvWarp0 % 4 == 0: TMEM lane quarter = warp % 4
+    const int row = q * 32 + lane;                                // channel within the half = TMEM lane
+    const uint8_t* my_w = smem + half * (kWBytes / 2) + row * 128;
+    const uint8_t* my_sz = smem + kWBytes + half * kPairBytes + row * 4;
+    const uint32_t my_t = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(half) * 32u;
+    int sw = 0, so = par;
+    uint32_t pw = 0, po = 0;
+    bool ok = true;
+    for (int t = first; ok && t < total; t += step) {
+      for (int kw = 0; ok && kw < KW; ++kw) {
+        if (!warp_wait(&sh->w_full[sw], pw, abort_flag)) { ok = false; break; }
+#pragma unroll 1
+        for (int s = par; s < 4; s += 2) {                        // this warp's 64-k blocks of the slot
+          if (kw * 4 + s >= KS) break;
+          const uint8_t* src = my_w + size_t(sw) * kWSlot;
+          const uint4 wa = *reinterpret_cast<const uint4*>(src + (((2 * s) ^ (row & 7)) << 4));
+          const uint4 wb = *reinterpret_cast<const uint4*>(src + (((2 * s + 1) ^ (row & 7)) << 4));
+          const uint32_t sz = *reinterpret_cast<const uint32_t*>(my_sz + size_t(sw) * kWSlot + (s >> 1) * (2 * kPairBytes));
+          const uint32_t wd[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
+          const Affine a = make_affine(sz);
+          uint32_t r[32];
+          if (__all_sync(0xffffffffu, a.whole)) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) convert_word(wd[i], a, r + 4 * i);
+          } else {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const uint4 v = dequant_word_bf16(wd[i], sz);
+              r[4 * i] = v.x; r[4 * i + 1] = v.y; r[4 * i + 2] = v.z; r[4 * i + 3] = v.w;
+            }
+          }
+          if (!warp_wait(&sh->op_empty[so], po ^ 1u, abort_flag)) { ok = false; break; }
+          ptx::tc_fence_after_sync();
+          ptx::tmem_st32(my_t + static_cast<uint32_t>(so) * 64u, r);
+          ptx::tmem_st_wait();
+          ptx::tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive(&sh->op_full[so]);
+          so += 2;
+          if (so >= kOpStages) { so = par; po ^= 1u; }
         }
         if (!ok) break;
-        ptx::umma_commit(&sh->tmem_full[as]);        // the tile's accumulators are complete
-        if (++as == kAccStages) { as = 0; pacc ^= 1u; }
+        if (lane == 0) ptx::mbar_arrive(&sh->w_empty[sw]);       // after the __syncwarp of the last block: every lane has read
+        if (++sw == kWStages) { sw = 0; pw ^= 1u; }
       }
     }
-  } else if (warp >= kFirstConvWarp) {
-    // converters: thread t owns operand rows t and t + 128 of the tile (all 8 words = 64 k of each)
-    ptx::setmaxnreg_dec<96>();
-    const int ct = threadIdx.x - kFirstConvWarp * 32;       // 0..127
-    int sp = 0, sb = 0;
-    uint32_t pp = 0, pb = 0;
-    bool ok = true;
-    for (int t = first; ok && t < total_tiles; t += step) {
-      const Tile tl = decode_tile16(sh, p, t, num_n_tiles);
-      const bool second = (p.fused ? p.N / 2 + tl.nt * 128 : tl.nt * BN + 128) < p.N;
-      for (int kb = 0; kb < KB; ++kb) {
-        if (!__all_sync(0xffffffffu, ptx::mbar_wait(&sh->p_full[sp], pp, abort_flag)) ||
-            !__all_sync(0xffffffffu, ptx::mbar_wait(&sh->b_empty[sb], pb ^ 1u, abort_flag))) { ok = false; break; }
-        const uint4* src = reinterpret_cast<const uint4*>(smem_p + size_t(sp) * kQSlot);
-        const uint32_t* pz = reinterpret_cast<const uint32_t*>(smem_p + size_t(sp) * kQSlot + kQBytes);
-        const uint32_t sz0 = pz[ct], sz1 = second ? pz[128 + ct] : 0u;
-        uint8_t* dst = smem_b + size_t(sb) * kBBytes;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int n = ct + h * 128;                        // operand row
-          const uint4 w0 = src[n * 2], w1 = src[n * 2 + 1];
-          const uint32_t wd[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
-          const uint32_t sz = h ? sz1 : sz0;
-#pragma unroll
-          for (int c = 0; c < 8; ++c)
-            *reinterpret_cast<uint4*>(dst + static_cast<uint32_t>(n) * 128u + ((static_cast<uint32_t>(c) ^ (n & 7u)) << 4)) =
-                dequant_word_bf16(wd[c], sz);
-        }
-        ptx::fence_proxy_async();
-        __syncwarp();
-        if (lane == 0) { ptx::mbar_arrive(&sh->b_full[sb]); ptx::mbar_arrive(&sh->p_empty[sp]); }
-        if (++sp == kQStages) { sp = 0; pp ^= 1u; }
-        if (++sb == kBStages) { sb = 0; pb ^= 1u; }
-      }
-    }
-  } else {
-    // epilogue warps: one TMEM read-back per tile
-    ptx::setmaxnreg_inc<184>();
-    const int e = warp - kFirstEpiWarp, q = warp & 3, hsel = e >> 2;
-    const int r_in_tile = q * 32 + lane;
+  } else if (warp >= kEpiWarp0) {
+    // ---- epilogue: thread = output channel (one of each half) --------------------------------------------------------
+    const int q = warp & 3, c = q * 32 + lane;
     const uint32_t lane_base = static_cast<uint32_t>(q * 32) << 16;
-    int as = 0; uint32_t pacc = 0;
-    bool ok = true;
-    for (int t = first; ok && t < total_tiles; t += step) {
-      const Tile tl = decode_tile16(sh, p, t, num_n_tiles);
-      const bool live = q * 32 < min(BM, tl.m_end - tl.m0);
-      const int row = tl.m0 + r_in_tile;
-      if (!__all_sync(0xffffffffu, ptx::mbar_wait(&sh->tmem_full[as], pacc, abort_flag))) { ok = false; break; }
+    int as = 0;
+    uint32_t pacc = 0;
+    for (int t = first; t < total; t += step) {
+      const Tile tl = decode<CHUNK>(sh, p, t, num_ct);
+      int n0, n1;
+      half_ch(tl, n0, n1);
+      const bool second = n1 < p.N;
+      if (!warp_wait(&sh->acc_full[as], pacc, abort_flag)) break;
       ptx::tc_fence_after_sync();
-      float acc[128];
-      if (live) {
-        const uint32_t tcol = tmem_base + lane_base + static_cast<uint32_t>(as) * BN + static_cast<uint32_t>(hsel) * 64;
+      const uint32_t tcol = tmem_base + lane_base + kAccCol + static_cast<uint32_t>(as) * (2 * CHUNK);
+      uint8_t* out = static_cast<uint8_t*>(p.c) + static_cast<int64_t>(tl.m0) * p.c_stride;
+#pragma unroll 1
+      for (int mb = 0; mb < tl.tn; mb += 16) {
+        uint32_t d0[16], d1[16];
+        ptx::tmem_ld16(tcol + mb, d0);
+        ptx::tmem_ld16(tcol + CHUNK + mb, d1);
+        ptx::tmem_ld_wait16(d0, d1);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          uint32_t r[32];
-          ptx::tmem_ld32(tcol + (c >> 1) * 128 + (c & 1) * 32, r);
-          ptx::tmem_ld_wait32(r);
-#pragma unroll
-          for (int j = 0; j < 32; ++j) acc[c * 32 + j] = __uint_as_float(r[j]);
+        for (int m = 0; m < 16; ++m) {
+          if (mb + m >= tl.rows) break;
+          const float v0 = __uint_as_float(d0[m]), v1 = __uint_as_float(d1[m]);
+          uint8_t* dst = out + static_cast<int64_t>(mb + m) * p.c_stride;
+          if (p.fused) {
+            reinterpret_cast<__nv_bfloat16*>(dst)[tl.ct * 128 + c] = __float2bfloat16_rn(bf16r(gate_act(bf16r(v0), p.act)) * bf16r(v1));
+          } else if (p.c_dtype == B200MOE_F32) {
+            reinterpret_cast<float*>(dst)[n0 + c] = v0;
+            if (second) reinterpret_cast<float*>(dst)[n1 + c] = v1;
+          } else if (p.c_dtype == B200MOE_BF16) {
+            reinterpret_cast<__nv_bfloat16*>(dst)[n0 + c] = __float2bfloat16_rn(v0);
+            if (second) reinterpret_cast<__nv_bfloat16*>(dst)[n1 + c] = __float2bfloat16_rn(v1);
+          } else {
+            reinterpret_cast<__half*>(dst)[n0 + c] = __float2half_rn(v0);
+            if (second) reinterpret_cast<__half*>(dst)[n1 + c] = __float2half_rn(v1);
+          }
         }
       }
       ptx::tc_fence_before_sync();
       __syncwarp();
-      if (lane == 0) ptx::mbar_arrive(&sh->tmem_empty[as]);
+      if (lane == 0) ptx::mbar_arrive(&sh->acc_empty[as]);
       if (++as == kAccStages) { as = 0; pacc ^= 1u; }
-      if (!live || row >= tl.m_end) continue;
-      uint8_t* dst = static_cast<uint8_t*>(p.c) + static_cast<int64_t>(row) * p.c_stride;
-      if (!p.fused) {
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          const int col0 = tl.nt * BN + half * 128 + hsel * 64;
-          if (col0 >= p.N) continue;
-          if (p.c_dtype == B200MOE_F32) store_row64(reinterpret_cast<float*>(dst) + col0, acc + half * 64);
-          else if (p.c_dtype == B200MOE_BF16) store_row64(reinterpret_cast<__nv_bfloat16*>(dst) + col0, acc + half * 64);
-          else store_row64(reinterpret_cast<__half*>(dst) + col0, acc + half * 64);
-        }
-      } else {
-#pragma unroll
-        for (int j = 0; j < 64; ++j) {
-          const float g = bf16r(acc[j]);
-          const float u = bf16r(acc[64 + j]);
-          acc[j] = bf16r(gate_act(g, p.act)) * u;
-        }
-        store_row64(reinterpret_cast<__nv_bfloat16*>(dst) + tl.nt * 128 + hsel * 64, acc);
-      }
     }
   }
 
+  // ---- teardown ------------------------------------------------------------------------------------------------
   ptx::tc_fence_before_sync();
   __syncthreads();
-  if (warp == 1) ptx::tmem_dealloc<1>(tmem_base, kTmemCols);
+  if (warp == 1) ptx::tmem_dealloc<1>(tmem_base, w4::kTmemCols);
   if (threadIdx.x == 0 && sh->abort_flag && p.status) *p.status = B200MOE_DEVICE_TIMEOUT;
 }
 
-}  // namespace w4
+// Average rows per group above which a tile takes 128 tokens (one set of accumulators) instead of 64 (two sets, the epilogue
+// overlaps).  Gate/up above, us: 64 rows per group 213 with chunks of 64; 96 rows 262 with chunks of 128, where two chunks of
+// 64 would be 2 x 210.  Groups are ragged, so the line is below 64: from about 48 on average some need a second chunk of 64.
+constexpr int kWideChunkRows = 48;
+
+template <int CHUNK>
+static int launch_chunk(const w4::RowMaps& ma, const CUtensorMap& mp, const Params& p, int sms, cudaStream_t st) {
+  if (int rc = set_dynamic_smem(reinterpret_cast<const void*>(gemm_w4a16_kernel<CHUNK>), kSmem)) return rc;
+  gemm_w4a16_kernel<CHUNK><<<sms, kThreads, kSmem, st>>>(ma, mp, p);
+  return check_launch("gemm_w4a16_kernel");
+}
+
+static int launch(const void* a, int64_t a_stride, const void* b_packed, const void* scale_zero_t, void* c, int c_dtype,
+                  int64_t c_stride, int64_t M_total, int64_t N, int64_t K, int num_groups, int num_weights, const int64_t* seg,
+                  const int64_t* widx, int fused, int act, int32_t* status, cudaStream_t st) {
+  int sms = 0;
+  if (int rc = require_sm100(&sms)) return rc;
+  w4::RowMaps ma;
+  CUtensorMap mp;
+  for (int i = 0; i < 4; ++i)
+    if (int rc = cached_tensor_map_u8(&ma.m[i], a, static_cast<uint64_t>(M_total), static_cast<uint64_t>(2 * K),
+                                      static_cast<uint64_t>(a_stride), 16u << i)) return rc;
+  if (int rc = make_tensor_map_i32_plain(&mp, b_packed, static_cast<uint64_t>(num_weights) * N, static_cast<uint64_t>(K / 8),
+                                         static_cast<uint64_t>(K / 8) * 4, 32, 128, true)) return rc;
+  const Params p{static_cast<const uint32_t*>(scale_zero_t), c, c_stride, seg, widx, static_cast<int>(N), static_cast<int>(K),
+                 num_groups, c_dtype, fused, act, status};
+  return M_total <= kWideChunkRows * static_cast<int64_t>(num_groups) ? launch_chunk<64>(ma, mp, p, sms, st)
+                                                                      : launch_chunk<128>(ma, mp, p, sms, st);
+}
+
+}  // namespace w4a16
 }  // namespace b200moe
 
 using namespace b200moe;
@@ -340,7 +433,7 @@ extern "C" int b200moe_grouped_gemm_w4a16(const void* a, int64_t a_row_stride_by
   B200MOE_REQUIRE(num_groups >= 1 && num_groups <= w4::kMaxGroups && num_weights >= 1 &&
                   static_cast<int64_t>(num_weights) * N < (int64_t(1) << 31), B200MOE_BAD_SHAPE,
                   "grouped_gemm_w4a16: num_groups=%d (max %d) num_weights=%d", num_groups, w4::kMaxGroups, num_weights);
-  B200MOE_REQUIRE(aligned(a, 16) && aligned(b_packed, 16) && aligned(scale_zero_t, 4) && aligned(c, 16) &&
+  B200MOE_REQUIRE(aligned(a, 16) && aligned(b_packed, 16) && aligned(scale_zero_t, 16) && aligned(c, 16) &&
                   a_row_stride_bytes % 16 == 0 && a_row_stride_bytes >= 2 * K && c_row_stride_bytes % 16 == 0,
                   B200MOE_BAD_ALIGN, "grouped_gemm_w4a16: pointers and row strides must be 16-byte aligned");
   if (epilogue != 0) {
@@ -352,19 +445,7 @@ extern "C" int b200moe_grouped_gemm_w4a16(const void* a, int64_t a_row_stride_by
     B200MOE_REQUIRE(c_row_stride_bytes >= N * (c_dtype == B200MOE_F32 ? 4 : 2), B200MOE_BAD_ARG, "grouped_gemm_w4a16: c row stride too small");
   }
   if (M_total == 0) return B200MOE_OK;
-  int sms = 0;
-  if (int rc = require_sm100(&sms)) return rc;
-  w4::RowMaps ma;
-  CUtensorMap mp;
-  for (int i = 0; i < 4; ++i)
-    if (int rc = cached_tensor_map_u8(&ma.m[i], a, static_cast<uint64_t>(M_total), static_cast<uint64_t>(2 * K),
-                                      static_cast<uint64_t>(a_row_stride_bytes), 16u << i)) return rc;
-  if (int rc = make_tensor_map_i32_plain(&mp, b_packed, static_cast<uint64_t>(num_weights) * N, static_cast<uint64_t>(K / 8),
-                                         static_cast<uint64_t>(K / 8) * 4, 8, 128)) return rc;
-  w4::Params16 p{static_cast<const uint32_t*>(scale_zero_t), c, c_row_stride_bytes, seg_indptr, weight_indices, M_total,
-                 static_cast<int>(N), static_cast<int>(K), num_groups, c_dtype, epilogue != 0 ? 1 : 0,
-                 epilogue == 5 ? 1 : 0, status_word};
-  if (int rc = set_dynamic_smem(reinterpret_cast<const void*>(w4::gemm_w4a16_kernel), w4::kSmem16)) return rc;
-  w4::gemm_w4a16_kernel<<<sms, w4::kThreads, w4::kSmem16, as_stream(stream)>>>(ma, mp, p);
-  return check_launch("gemm_w4a16_kernel");
+  return w4a16::launch(a, a_row_stride_bytes, b_packed, scale_zero_t, c, c_dtype, c_row_stride_bytes, M_total, N, K, num_groups,
+                       num_weights, seg_indptr, weight_indices, epilogue != 0 ? 1 : 0, epilogue == 5 ? 1 : 0, status_word,
+                       as_stream(stream));
 }

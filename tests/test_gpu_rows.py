@@ -1,5 +1,5 @@
-"""The GEMMs for few rows per group (csrc/gemm_fp8_rows.cu) against the 128-token tiles of csrc/gemm_fp8.cu, which the
-other test files compare with the oracle."""
+"""The GEMMs for few rows per group (csrc/gemm_fp8_rows.cu, csrc/gemm_w4a16.cu) against the 128-token tiles of
+csrc/gemm_fp8.cu, which the other test files compare with the oracle."""
 import pytest
 import torch
 
@@ -46,3 +46,36 @@ def test_rows_kernel_fused_is_bit_identical(N, K, epilogue):
     with G.gemm_options():
         G.grouped_gemm_fp8(a, a_s, b, b_s, seg, widx, *out[1], epilogue=epilogue)
     assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("whole_zeros", [True, False])
+@pytest.mark.parametrize("rows", [ROWS, [0, 129, 64, 200, 128, 17, 127, 0]])
+@pytest.mark.parametrize("N,K", [(128, 128), (384, 640), (512, 1024)])
+def test_w4a16_kernel_is_bit_identical(N, K, rows, whole_zeros):
+    """Both token-chunk widths, K with and without a half-filled 256-k slot, whole zero points (one subtraction per pair)
+    and others (the general conversion): the same bf16 weights and the same K order, so the same bits as expanding the
+    weights first."""
+    from llm_kernels_b200.moe import group_gemm_kernel as G
+    from llm_kernels_b200.quantization import w4a16_kernel
+    dev = torch.device("cuda:0")
+    g = torch.Generator(device=dev).manual_seed(3)
+    W, M = len(rows), sum(rows)
+    packed = torch.randint(-2 ** 31, 2 ** 31, (W, N, K // 8), generator=g, device=dev, dtype=torch.int64).to(torch.int32)
+    sc = (torch.rand(W, N, K // 128, generator=g, device=dev) * 0.02 + 1e-3).to(torch.bfloat16)
+    zp = torch.randint(0, 16, (W, N, K // 128), generator=g, device=dev).to(torch.bfloat16)
+    if not whole_zeros:
+        zp[:, ::3] += 0.375
+        zp[:, 1::7] = -21.0
+        sc[:, 2::5] = 2.0 ** -124
+    a = torch.randn(M, K, generator=g, device=dev).to(torch.bfloat16)
+    seg = torch.tensor([0] + torch.tensor(rows).cumsum(0).tolist(), dtype=torch.int64, device=dev)
+    widx = torch.randperm(W, generator=g, device=dev)
+    pairs, full = G.pair_scales_t(sc, zp), w4a16_kernel.expand_bf16(packed, sc, zp)
+    for epi, cols, dt in ((0, N, torch.float32), (0, N, torch.float16), (2, N // 2, torch.bfloat16), (5, N // 2, torch.bfloat16)):
+        if epi and N % 256:
+            continue
+        c, want = (torch.full((M, cols), float("nan"), dtype=dt, device=dev) for _ in range(2))
+        G.grouped_gemm_w4a16(a, packed, pairs, seg, widx, c, epilogue=epi)
+        G.grouped_gemm_bf16(a, full, seg, widx, want, epilogue=epi) if dt != torch.float16 else \
+            want.copy_(G.grouped_gemm_bf16(a, full, seg, widx, torch.empty(M, cols, dtype=torch.float32, device=dev)))
+        assert torch.equal(c, want)
