@@ -22,7 +22,9 @@
 //               64 staging registers, so that two 32-column TMEM loads are always in
 //               flight (setmaxnreg: 56 registers for warpgroup 0, 224 for the other two)
 // Tiles are (group, m-tile, n-tile) with n fastest, so CTAs running together
-// share an A tile and walk one expert's weights once through L2.
+// share an A tile and walk one expert's weights once through L2.  Weights too large for that are walked in bands of 8
+// n-tiles, each down all m-tiles of the group: otherwise they came from HBM once per 1.3 m-tiles (8 experts x 2048 rows,
+// bf16, N 28672 K 4096, 235 MB per expert: 4950 us that way, 3440 us in bands).
 //
 // Every wait is a bounded mbarrier wait; on expiry the kernel drains, frees TMEM,
 // writes B200MOE_DEVICE_TIMEOUT to the status word and returns.
@@ -52,6 +54,13 @@ constexpr uint32_t kBBytes = BN * BK;
 constexpr uint32_t kStageBytes = kABytes + kBBytes;
 constexpr int kMaxGroups = 1024;
 constexpr uint32_t kTmemCols = 512;
+// n-tiles per band of the tile order.  148 tiles that run together are then about 8 n-tiles x 18 m-tiles (2048 weight rows,
+// 2304 tokens): near the square that touches the fewest bytes, and small enough that the weights of a band (17 MB for a
+// K of 8 KB) stay in L2 while the band walks down the group.  Weights that L2 holds next to the tokens are walked as
+// before, all n-tiles of an m-tile first: bands gain nothing there (fp8 layer of 4096 tokens, 29 MB per expert: 1 % slower).
+constexpr int kBand = 8;
+constexpr int64_t kBandMinBytes = 48 << 20;
+constexpr int kPairRowsPerGroup = 768;   // see launch_gemm
 
 struct SharedTail {
   uint64_t full[kMaxStages];
@@ -96,6 +105,7 @@ struct GemmParams {
   int accumulate;
   // fused gate/up epilogues (swiglu != 0): 0 = SiLU, 1 = tanh-GELU
   int act;
+  int band;                           // columns per band of the tile order, set by launch_gemm
 };
 
 struct Tile { int m0, m_end, expert, nt, ks; };
@@ -116,13 +126,21 @@ __device__ __forceinline__ Tile decode_tile(const SharedTail* sh, const GemmPara
     const int mid = (lo + hi) >> 1;
     if (sh->pref[mid] <= mt) lo = mid; else hi = mid;
   }
+  // inside a group: bands of p.band columns, every band down all m-tiles of the group; split-K launches keep whole rows,
+  // from which the MMA issuer derives its split
+  const int m_tiles = sh->pref[lo + 1] - sh->pref[lo];
+  const int rem = t - sh->pref[lo] * per;
+  const int band_cols = min(p.band, per);
+  const int band = rem / (m_tiles * band_cols);
+  const int in_band = rem - band * (m_tiles * band_cols);
+  const int cols = min(band_cols, per - band * band_cols);
+  const int m = in_band / cols, col = band * band_cols + in_band - m * cols;
   Tile tl;
-  tl.m0 = sh->seg[lo] + (mt - sh->pref[lo]) * bmt + m_off;
+  tl.m0 = sh->seg[lo] + m * bmt + m_off;
   tl.m_end = sh->seg[lo + 1];
   tl.expert = p.widx ? static_cast<int>(p.widx[lo]) : lo;
-  const int rem = t - mt * per;
-  tl.nt = rem / p.ksplits;
-  tl.ks = rem - tl.nt * p.ksplits;
+  tl.nt = col / p.ksplits;
+  tl.ks = col - tl.nt * p.ksplits;
   return tl;
 }
 
@@ -242,7 +260,7 @@ gemm_block_kernel(const __grid_constant__ RowMaps tmap_a,
     ptx::setmaxnreg_dec<56>();
   if (warp == 0) {
     // ================================ TMA producer ================================
-    if (lane == 0) {
+    if (ptx::elect_one()) {
       int stage = 0; uint32_t phase = 0;
       uint32_t armed = 0, armed_parity = 0;
       bool ok = true;
@@ -307,7 +325,7 @@ gemm_block_kernel(const __grid_constant__ RowMaps tmap_a,
     }
   } else if (warp == 1) {
     // ================================ MMA issuer ==================================
-    if (lane == 0 && leader) {
+    if (leader && ptx::elect_one()) {
       // D f32 (1) / s32 (2); operand formats: e4m3 = 0, signed int8 = 1, bf16 = 1
       constexpr uint32_t idesc = KIND == kFp8 ? ptx::umma_idesc(1, 0, 0, BMT, BN)
                                  : (KIND == kI8 ? ptx::umma_idesc(2, 1, 1, BMT, BN)
@@ -627,11 +645,17 @@ static int launch_gemm(const void* a, int64_t a_stride, const void* b, GemmParam
                                     static_cast<uint64_t>(a_stride), 16u << i)) return rc;
   if (int rc = cached_tensor_map_u8(&mb, b, static_cast<uint64_t>(p.num_weights) * p.N, static_cast<uint64_t>(p.K),
                                   static_cast<uint64_t>(p.K), 128)) return rc;
+  p.band = p.ksplits == 1 && static_cast<int64_t>(p.N) * p.K > kBandMinBytes ? kBand : INT32_MAX;
   int grid = sms;
   if (max_ctas > 0 && max_ctas < grid) grid = max_ctas;
   if (tiles_hint > 0 && tiles_hint < grid) grid = static_cast<int>(tiles_hint);
   // N must cover both halves of a pair's tile; split-K launches stay single.
-  bool pair = pair_mode == 1;
+  // Without options, 16-bit operands with many rows per group run in pairs: a pair moves a third less from L2 to its SMs,
+  // which at the power cap is time.  Rows per group, us single -> pair (8 groups, gate/up N 28672 K 4096, then down N 4096
+  // K 14336): 300 656-685 -> 724 and 365 -> 431 (256-row tiles pad more), 1024 1711-1828 -> 1577 and 770-838 -> 718,
+  // 2048 3440-3626 -> 2764 and 1698-1757 -> 1597.  The block-scaled kinds are bound by their promotion: no gain.
+  constexpr bool k16bit = KIND == kBf16 || KIND == kF16;
+  bool pair = pair_mode == 1 || (k16bit && !opts && p.M_total >= kPairRowsPerGroup * static_cast<int64_t>(p.num_groups));
   if (p.ksplits > 1 || grid < 2 || (!p.swiglu && p.N % BN != 0)) pair = false;
   if (pair) return launch_gemm_as<KIND, true>(ma, mb, p, grid & ~1, st);
   return launch_gemm_as<KIND, false>(ma, mb, p, grid, st);

@@ -121,3 +121,29 @@ def test_i8_and_16bit_pairs_equal_single(dev, modes, counts):
         assert torch.equal(s, p) and not torch.isnan(p).any()
         ref = R.grouped_gemm_plain(a.to(dt), b.to(dt), seg, torch.arange(W))
         assert R.rel_fro(p.cpu().float(), ref.float()) < 3e-3
+
+
+@pytest.mark.parametrize("counts,N,K,epilogue", [([900, 0, 1300, 131], 2688, 9600, 0),     # bands, half a last n-tile: single CTAs
+                                                 ([1025, 2, 1500], 2816, 9472, 0),         # bands of 8 + 3 n-tiles: pairs
+                                                 ([1025, 2, 1500], 5632, 9472, 2)])        # the same, gate/up tiles
+def test_bf16_default_order_and_pairs(counts, N, K, epilogue):
+    """Without options, large 16-bit weights are walked in bands and many rows per group run in pairs: the same bits as one
+    call per group with few rows (single CTAs, no second m-tile for a band to walk down)."""
+    from llm_kernels_b200.moe import group_gemm_kernel as G
+    dev = torch.device("cuda:0")
+    g = torch.Generator(device=dev).manual_seed(11)
+    M, W = sum(counts), len(counts)
+    a = torch.randn(M, K, generator=g, device=dev).to(torch.bfloat16)
+    b = (torch.randn(W, N, K, generator=g, device=dev) * 0.02).to(torch.bfloat16)
+    seg = torch.tensor([0] + torch.tensor(counts).cumsum(0).tolist(), dtype=torch.int64, device=dev)
+    cols = N if epilogue == 0 else N // 2
+    c, want = (torch.full((M, cols), float("nan"), dtype=torch.bfloat16, device=dev) for _ in range(2))
+    G.grouped_gemm_bf16(a, b, seg, None, c, epilogue=epilogue)
+    m0 = 0
+    for i, n in enumerate(counts):
+        for r in range(m0, m0 + n, 128):
+            rows = min(128, m0 + n - r)
+            one = torch.tensor([0, rows], dtype=torch.int64, device=dev)
+            G.grouped_gemm_bf16(a[r:r + rows], b[i:i + 1], one, None, want[r:r + rows], epilogue=epilogue)
+        m0 += n
+    assert torch.equal(c, want)
