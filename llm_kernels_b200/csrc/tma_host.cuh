@@ -97,6 +97,22 @@ inline int make_tensor_map_i32_plain(CUtensorMap* m, const void* base, uint64_t 
   return B200MOE_OK;
 }
 
+// int32 matrix rows x cols seen as [cols / 32][rows][32]: one box is box_rows rows x 128 columns, which land in shared memory
+// as four [box_rows][32 words] tiles with the 128-byte swizzle.
+inline int make_tensor_map_i32_kgroups(CUtensorMap* m, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows) {
+  EncodeFn enc = get_tensor_map_encoder();
+  if (!enc) return fail(B200MOE_UNSUPPORTED_DEVICE, "cuTensorMapEncodeTiled is not available from this driver");
+  const cuuint64_t dims[3] = {32, rows, cols / 32};
+  const cuuint64_t strides[2] = {cols * 4, 128};
+  const cuuint32_t box[3] = {32, box_rows, 4};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  const CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_INT32, 3, const_cast<void*>(base), dims, strides, box, estr,
+                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(B200MOE_BAD_ARG, "cuTensorMapEncodeTiled (k groups) failed with %d", (int)r);
+  return B200MOE_OK;
+}
+
 inline int require_sm100(int* sms) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return fail(B200MOE_UNSUPPORTED_DEVICE, "no CUDA device");
