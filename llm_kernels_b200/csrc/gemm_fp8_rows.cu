@@ -200,7 +200,7 @@ gemm_fp8_rows_kernel(const __grid_constant__ w4::RowMaps tmap_a, const __grid_co
     n1 = p.fused ? p.N / 2 + tl.ct * 128 : n0 + 128;
   };
 
-  if (warp == 0 && lane == 0) {
+  if (warp == 0 && ptx::elect_one()) {
     // ---- weights and token rows ------------------------------------------------------------------------------------
     int stage = 0; uint32_t phase = 0;
     w4::Armed armed;
@@ -225,7 +225,7 @@ gemm_fp8_rows_kernel(const __grid_constant__ w4::RowMaps tmap_a, const __grid_co
       }
     }
     if (!ok) armed.drain(sh->full, kStages);
-  } else if (warp == 1 && lane == 0) {
+  } else if (warp == 1 && ptx::elect_one()) {
     // ---- MMA issuer: channels are the M = 128 rows, tokens the N columns -------------------------------------------
     int st = 0, as = 0;
     uint32_t ph = 0, pacc = 0;
