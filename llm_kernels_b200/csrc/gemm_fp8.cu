@@ -716,31 +716,43 @@ static int sum_splits(const float* partials, int ksplits, int64_t n, void* c, in
   return check_launch("sum_splits");
 }
 
+template <int KIND>
+static int gemm_splitk(const char* who, const void* a, const float* a_s, const void* b, const float* b_s, void* c, int c_dtype,
+                       int64_t M, int64_t N, int64_t K, int ksplits, float* partials, int64_t partials_bytes, void* stream) {
+  B200MOE_REQUIRE(a && a_s && b && b_s && c && partials, B200MOE_BAD_ARG, "%s: null pointer", who);
+  B200MOE_REQUIRE(M >= 0 && M < (int64_t(1) << 31) && N > 0 && K > 0 && K % 128 == 0 && N % 128 == 0 && N * K < (int64_t(1) << 40),
+                  B200MOE_BAD_SHAPE, "%s: M=%lld N=%lld K=%lld (N and K must be multiples of 128)",
+                  who, (long long)M, (long long)N, (long long)K);
+  const int64_t KB = K / 128;
+  const int64_t per = ksplits > 0 ? (KB + ksplits - 1) / ksplits : 0;
+  B200MOE_REQUIRE(ksplits >= 1 && ksplits <= 16 && per * (ksplits - 1) < KB, B200MOE_BAD_ARG,
+                  "%s: %d splits of %lld K blocks (every split needs at least one)", who, ksplits, (long long)KB);
+  B200MOE_REQUIRE(c_dtype == B200MOE_F32 || c_dtype == B200MOE_F16 || c_dtype == B200MOE_BF16, B200MOE_BAD_DTYPE,
+                  "%s: c dtype %d", who, c_dtype);
+  B200MOE_REQUIRE(aligned(a, 16) && aligned(b, 16) && aligned(c, 16) && aligned(partials, 16), B200MOE_BAD_ALIGN,
+                  "%s: Input tensors must be 16-byte aligned", who);
+  B200MOE_REQUIRE(partials_bytes >= static_cast<int64_t>(ksplits) * M * N * 4, B200MOE_WORKSPACE_TOO_SMALL,
+                  "%s: partials need %lld bytes", who, (long long)(static_cast<int64_t>(ksplits) * M * N * 4));
+  if (M == 0) return B200MOE_OK;
+  GemmParams p{a_s, K / 128, b_s, partials, N * 4, nullptr, 0, nullptr, nullptr, M,
+               static_cast<int>(N), static_cast<int>(K), 1, 1, B200MOE_F32, 0, nullptr, ksplits, M * N * 4, 0,
+               nullptr, nullptr, 0, 0};
+  if (int rc = launch_gemm<KIND>(a, K, b, p, ((M + BM - 1) / BM) * ((N + BN - 1) / BN) * ksplits, as_stream(stream))) return rc;
+  return sum_splits(partials, ksplits, M * N, c, c_dtype, as_stream(stream));
+}
+
 }  // namespace b200moe
 
 extern "C" int b200moe_gemm_fp8_block_splitk(const void* a, const float* a_s, const void* b, const float* b_s,
                                              void* c, int c_dtype, int64_t M, int64_t N, int64_t K, int ksplits,
                                              float* partials, int64_t partials_bytes, void* stream) {
-  B200MOE_REQUIRE(a && a_s && b && b_s && c && partials, B200MOE_BAD_ARG, "gemm_fp8_block_splitk: null pointer");
-  B200MOE_REQUIRE(M >= 0 && M < (int64_t(1) << 31) && N > 0 && K > 0 && K % 128 == 0 && N % 128 == 0 && N * K < (int64_t(1) << 40),
-                  B200MOE_BAD_SHAPE, "gemm_fp8_block_splitk: M=%lld N=%lld K=%lld (N and K must be multiples of 128)",
-                  (long long)M, (long long)N, (long long)K);
-  const int64_t KB = K / 128;
-  const int64_t per = ksplits > 0 ? (KB + ksplits - 1) / ksplits : 0;
-  B200MOE_REQUIRE(ksplits >= 1 && ksplits <= 16 && per * (ksplits - 1) < KB, B200MOE_BAD_ARG,
-                  "gemm_fp8_block_splitk: %d splits of %lld K blocks (every split needs at least one)", ksplits, (long long)KB);
-  B200MOE_REQUIRE(c_dtype == B200MOE_F32 || c_dtype == B200MOE_F16 || c_dtype == B200MOE_BF16, B200MOE_BAD_DTYPE,
-                  "gemm_fp8_block_splitk: c dtype %d", c_dtype);
-  B200MOE_REQUIRE(aligned(a, 16) && aligned(b, 16) && aligned(c, 16) && aligned(partials, 16), B200MOE_BAD_ALIGN,
-                  "gemm_fp8_block_splitk: Input tensors must be 16-byte aligned");
-  B200MOE_REQUIRE(partials_bytes >= static_cast<int64_t>(ksplits) * M * N * 4, B200MOE_WORKSPACE_TOO_SMALL,
-                  "gemm_fp8_block_splitk: partials need %lld bytes", (long long)(static_cast<int64_t>(ksplits) * M * N * 4));
-  if (M == 0) return B200MOE_OK;
-  GemmParams p{a_s, K / 128, b_s, partials, N * 4, nullptr, 0, nullptr, nullptr, M,
-               static_cast<int>(N), static_cast<int>(K), 1, 1, B200MOE_F32, 0, nullptr, ksplits, M * N * 4, 0,
-               nullptr, nullptr, 0, 0};
-  if (int rc = launch_gemm<kFp8>(a, K, b, p, ((M + BM - 1) / BM) * ((N + BN - 1) / BN) * ksplits, as_stream(stream))) return rc;
-  return sum_splits(partials, ksplits, M * N, c, c_dtype, as_stream(stream));
+  return gemm_splitk<kFp8>("gemm_fp8_block_splitk", a, a_s, b, b_s, c, c_dtype, M, N, K, ksplits, partials, partials_bytes, stream);
+}
+
+extern "C" int b200moe_gemm_i8_block_splitk(const void* a, const float* a_s, const void* b, const float* b_s,
+                                            void* c, int c_dtype, int64_t M, int64_t N, int64_t K, int ksplits,
+                                            float* partials, int64_t partials_bytes, void* stream) {
+  return gemm_splitk<kI8>("gemm_i8_block_splitk", a, a_s, b, b_s, c, c_dtype, M, N, K, ksplits, partials, partials_bytes, stream);
 }
 
 extern "C" int b200moe_grouped_gemm_fp8(const void* a, int64_t a_row_stride_bytes, const float* a_s,

@@ -66,8 +66,10 @@ def act_quant(x: torch.Tensor, block_size: int = 128) -> Tuple[torch.Tensor, tor
 def w4a8_gemm(a: torch.Tensor, a_s: torch.Tensor, b: torch.Tensor, b_s: torch.Tensor, b_s4: torch.Tensor,
               b_z4: torch.Tensor, GROUP_SIZE_INT4: int = 128, elements_per_sample: int = 8,
               pack_direction: str = "row", out_dtype: torch.dtype = None) -> torch.Tensor:
-    """c[..., N] = a[..., K] (int8) . dequant(b)^T with per-K-block scales (reference :406-448)."""
-    from ..moe.group_gemm_kernel import grouped_gemm_i8
+    """c[..., N] = a[..., K] (int8) . dequant(b)^T with per-K-block scales (reference :406-448).  Few rows (M <= 128) split
+    the K loop over all SMs as fp8_gemm does: one m-tile alone kept N / 256 of them busy (M = 24, N = 4096, K = 7168)."""
+    from ..moe.group_gemm_kernel import _opts, grouped_gemm_i8
+    from .fp8_kernel import _split_k, _workspace
     assert a.is_contiguous() and b.is_contiguous(), 'Input tensors must be contiguous'
     assert a_s.is_contiguous() and b_s.is_contiguous(), 'Scaling factor tensors must be contiguous'
     assert b_s4.is_contiguous() and b_z4.is_contiguous(), 'Scaling factor and zero point tensors must be contiguous'
@@ -77,7 +79,16 @@ def w4a8_gemm(a: torch.Tensor, a_s: torch.Tensor, b: torch.Tensor, b_s: torch.Te
     w8 = expand_int8(b, b_s4, b_z4)
     Nn = w8.shape[0]
     c = a.new_empty(*a.size()[:-1], Nn, dtype=out_dtype or torch.get_default_dtype())
-    seg = torch.tensor([0, M], dtype=torch.int64, device=a.device)
-    grouped_gemm_i8(a.view(M, K), a_s.reshape(M, -1).float(), w8.unsqueeze(0), b_s.float().unsqueeze(0), seg, None,
+    ks = _split_k(M, Nn, K)
+    if ks > 1 and M > 0 and _opts() is None:
+        N.require_cuda(a, a_s, b_s)
+        assert a.dtype == torch.int8
+        a_s, b_s = a_s.reshape(M, -1).float(), b_s.float()
+        part = _workspace(a.device, ks * M * Nn * 4)
+        N.check(N.lib().b200moe_gemm_i8_block_splitk(N.ptr(a), N.ptr(a_s), N.ptr(w8), N.ptr(b_s), N.ptr(c),
+                                                     N.dtype_code(c.dtype), M, Nn, K, ks, N.ptr(part), part.numel(),
+                                                     N.stream()))
+        return c
+    grouped_gemm_i8(a.view(M, K), a_s.reshape(M, -1).float(), w8.unsqueeze(0), b_s.float().unsqueeze(0), None, None,
                     c.view(M, Nn))
     return c
