@@ -325,6 +325,11 @@ B200MOE_API int b200moe_grouped_gemm_fp8(const void* a, int64_t a_row_stride_byt
 B200MOE_API int b200moe_w4a8_expand_int8(const void* packed, const int8_t* s4, const int8_t* z4, void* out,
                              int64_t W, int64_t N, int64_t K, void* stream);
 
+/* Writes 0 to *ok (device, the caller sets it to 1) if (q - z4) * s4 leaves int8 for a nibble that a weight of the stack
+ * holds: such a weight cannot go through b200moe_grouped_gemm_w4a8.  Layouts as for b200moe_w4a8_expand_int8. */
+B200MOE_API int b200moe_w4a8_range_check(const void* packed, const int8_t* s4, const int8_t* z4, int64_t W, int64_t N,
+                             int64_t K, int32_t* ok, void* stream);
+
 /* Asymmetric group-128 int4 -> bf16: w = (q - zero) * scale rounded once to bf16.
  * Extends the symmetric dequantization of the reference's w4a16 kernel
  * (fast_dequant/simple_marlin/marlin_w4a16_gemm.cu:44-64, utils.py:98-136) with a

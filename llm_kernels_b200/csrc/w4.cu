@@ -41,6 +41,27 @@ __global__ void __launch_bounds__(256) w4a8_expand_kernel(const uint32_t* __rest
   }
 }
 
+// Clears *ok where (q - z4) * s4 leaves int8 for a nibble that the weight holds.  One thread: 8 channels of one packed row and
+// one 128-k group.  The packed words are only read where nibbles 0 and 15, the ends of the range, do not both stay inside
+// (the product is linear in q): for weights from the quantizer the pass reads s4 and z4 alone.
+__global__ void __launch_bounds__(256) w4a8_range_kernel(const uint32_t* __restrict__ packed, const int8_t* __restrict__ s4,
+                                                         const int8_t* __restrict__ z4, int64_t rows8, int64_t K,
+                                                         int32_t* __restrict__ ok) {
+  const int64_t kg = K / 128, total = rows8 * kg;
+  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
+       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    const int64_t r = i / kg, g = i - r * kg;
+    auto inside = [](int v) { return v >= -128 && v <= 127; };
+    for (int c = 0; c < 8; ++c) {
+      const int s = s4[(r * 8 + c) * kg + g], z = z4[(r * 8 + c) * kg + g];
+      if (inside(-z * s) && inside((15 - z) * s)) continue;
+      bool good = true;
+      for (int j = 0; j < 128; ++j) good &= inside((static_cast<int>((packed[r * K + g * 128 + j] >> (4 * c)) & 0xF) - z) * s);
+      if (!good) *ok = 0;
+    }
+  }
+}
+
 // one thread: one packed word = 8 consecutive k of one row -> 8 bf16
 __global__ void __launch_bounds__(256) w4a16_expand_kernel(const uint32_t* __restrict__ packed,
                                                            const __nv_bfloat16* __restrict__ scale,
@@ -126,6 +147,18 @@ extern "C" int b200moe_w4a8_expand_int8(const void* packed, const int8_t* s4, co
   w4a8_expand_kernel<<<grid, 256, 0, as_stream(stream)>>>(static_cast<const uint32_t*>(packed), s4, z4,
                                                           static_cast<int8_t*>(out), W, N, K);
   return check_launch("w4a8_expand_int8");
+}
+
+extern "C" int b200moe_w4a8_range_check(const void* packed, const int8_t* s4, const int8_t* z4, int64_t W, int64_t N,
+                                        int64_t K, int32_t* ok, void* stream) {
+  B200MOE_REQUIRE(packed && s4 && z4 && ok, B200MOE_BAD_ARG, "w4a8_range_check: null pointer");
+  B200MOE_REQUIRE(W >= 0 && N > 0 && K > 0 && N % 8 == 0 && K % 128 == 0, B200MOE_BAD_SHAPE,
+                  "w4a8_range_check: N=%lld must be a multiple of 8 and K=%lld of 128", (long long)N, (long long)K);
+  if (W == 0) return B200MOE_OK;
+  const int64_t rows8 = W * (N / 8), total = rows8 * (K / 128);
+  const unsigned grid = static_cast<unsigned>(std::min<int64_t>((total + 255) / 256, 148 * 32));
+  w4a8_range_kernel<<<grid, 256, 0, as_stream(stream)>>>(static_cast<const uint32_t*>(packed), s4, z4, rows8, K, ok);
+  return check_launch("w4a8_range_check");
 }
 
 extern "C" int b200moe_w4a16_expand_bf16(const void* packed, const void* scale_bf16, const void* zero_bf16,

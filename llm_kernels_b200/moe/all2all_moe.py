@@ -281,9 +281,10 @@ class DeepseekV3MoE(nn.Module):
             self._shared_stream = None
         # int4 methods: up to this many rows per expert group on average the dequantization runs inside the GEMMs
         # (every tile converts its weights once); above it the weights are expanded once per forward instead
-        # (measured break-even: 64 rows for w4a8, whose tiles hold 64 tokens; 256 for w4a16, whose tiles hold 128)
+        # Whole w4a8 layer (256 experts, hidden 7168), us expanded -> inside the GEMMs: 47 rows 7785 -> 2509, 94 rows 8019 -> 4755,
+        # 128 rows 8901 -> 6215, 192 rows 10528 -> 8967, 256 rows 11871 -> 11467.
         self.w4_fused_rows_per_group = int(getattr(config, "w4_fused_rows_per_group",
-                                                   256 if self.method == "w4a16" else 64))
+                                                   256 if self.method == "w4a16" else 192))
         self._buffers_cache = {}
         self._status = torch.zeros(1, dtype=torch.int32, device=dev)
         self._last_recv_rows = None
@@ -840,25 +841,24 @@ class DeepseekV3MoE(nn.Module):
         """The fused w4a8 GEMM multiplies the raw nibbles and applies (q - z4) * s4 to the dot product, which equals
         the reference's int8 product (quantization/w4a8_kernel.py:362-380, where the product is cast to int8) only
         while (q - z4) * s4 stays inside int8 for every nibble the weight holds.  The reference's quantizer keeps it
-        there (:228-262); any weight is checked once here (smallest and largest nibble of every scale group), and one
-        that fails is expanded to int8 instead."""
+        there (:228-262); any weight is checked once here (b200moe_w4a8_range_check), and one that fails is expanded to
+        int8 instead."""
         packed, s4, z4 = getattr(self, name + "_qweight"), getattr(self, name + "_s4"), getattr(self, name + "_z4")
         key = (packed.data_ptr(), packed._version, s4.data_ptr(), s4._version, z4.data_ptr(), z4._version)
         hit = self._buffers_cache.get(("raw_ok", name))
         if hit is None or hit[0] != key:
             W, R8, K = packed.shape                      # nibble i of a word: output row 8 r + i
-            ok = True
-            for e in range(W):                           # one expert at a time keeps the scratch small
-                lo = torch.empty(R8, 8, K // 128, dtype=torch.int32, device=packed.device)
-                hi = torch.empty_like(lo)
-                for i in range(8):
-                    q = ((packed[e] >> (4 * i)) & 15).view(R8, K // 128, 128)
-                    lo[:, i], hi[:, i] = q.amin(-1), q.amax(-1)
-                s, zz = s4[e].to(torch.int32).view(R8, 8, -1), z4[e].to(torch.int32).view(R8, 8, -1)
-                a, b = (lo - zz) * s, (hi - zz) * s
-                ok = ok and bool((torch.minimum(a, b).min() >= -128) & (torch.maximum(a, b).max() <= 127))
-                if not ok:
-                    break
+            if packed.is_cuda:
+                assert packed.is_contiguous() and s4.is_contiguous() and z4.is_contiguous()
+                flag = torch.ones(1, dtype=torch.int32, device=packed.device)
+                N.check(N.lib().b200moe_w4a8_range_check(N.ptr(packed), N.ptr(s4), N.ptr(z4), W, 8 * R8, K, N.ptr(flag),
+                                                         N.stream()))
+                ok = bool(flag.item())
+            else:                                        # the same from the smallest and largest nibble of every group
+                q = torch.stack([(packed >> (4 * i)) & 15 for i in range(8)], dim=2).view(W, 8 * R8, K // 128, 128)
+                s, zz = s4.to(torch.int32), z4.to(torch.int32)
+                a, b = (q.amin(-1) - zz) * s, (q.amax(-1) - zz) * s
+                ok = bool((torch.minimum(a, b).min() >= -128) & (torch.maximum(a, b).max() <= 127))
             hit = (key, ok)
             self._buffers_cache[("raw_ok", name)] = hit
         return hit[1]

@@ -79,3 +79,52 @@ def test_w4a16_kernel_is_bit_identical(N, K, rows, whole_zeros):
         G.grouped_gemm_bf16(a, full, seg, widx, want, epilogue=epi) if dt != torch.float16 else \
             want.copy_(G.grouped_gemm_bf16(a, full, seg, widx, torch.empty(M, cols, dtype=torch.float32, device=dev)))
         assert torch.equal(c, want)
+
+
+@pytest.mark.parametrize("rows", [ROWS, [128, 0, 129, 95, 1, 32]])
+@pytest.mark.parametrize("N,K", [(128, 128), (384, 640), (512, 1152)])
+def test_w4a8_kernel_is_bit_identical(N, K, rows):
+    """Raw nibbles with the zero point taken off the dot product in exact f32 arithmetic against weights expanded to int8:
+    the same bits, with scales and zero points up to the ends of what keeps (q - z) * s inside int8."""
+    from llm_kernels_b200.moe import group_gemm_kernel as G
+    from llm_kernels_b200.quantization import w4a8_kernel
+    dev = torch.device("cuda:0")
+    g = torch.Generator(device=dev).manual_seed(4)
+    W, M = len(rows), sum(rows)
+    packed = torch.randint(-2 ** 31, 2 ** 31, (W, N // 8, K), generator=g, device=dev, dtype=torch.int64).to(torch.int32)
+    s4 = torch.randint(-8, 9, (W, N, K // 128), generator=g, device=dev).to(torch.int8)
+    z4 = torch.randint(0, 16, (W, N, K // 128), generator=g, device=dev).to(torch.int8)
+    s4[:, ::5], z4[:, ::5] = 1, -112                        # 112 .. 127
+    s4[:, 1::5], z4[:, 1::5] = 1, 127                       # -127 .. -112
+    s4[:, 2::5], z4[:, 2::5] = -1, -112                     # -127 .. -112
+    a = torch.randint(-128, 128, (M, K), generator=g, device=dev).to(torch.int8)
+    a[::3] = -128                                           # the largest sums
+    a_s = torch.rand(M, K // 128, generator=g, device=dev) * 0.01 + 1e-3
+    b_s = torch.rand(W, N // 128, K // 128, generator=g, device=dev) * 0.01 + 1e-3
+    seg = torch.tensor([0] + torch.tensor(rows).cumsum(0).tolist(), dtype=torch.int64, device=dev)
+    widx = torch.randperm(W, generator=g, device=dev)
+    for dt in (torch.float32, torch.bfloat16, torch.float16):
+        c, want = (torch.full((M, N), float("nan"), dtype=dt, device=dev) for _ in range(2))
+        G.grouped_gemm_w4a8(a, a_s, packed, G.pair_scales_t(s4, z4), b_s, seg, widx, c)
+        G.grouped_gemm_i8(a, a_s, w4a8_kernel.expand_int8(packed, s4, z4), b_s, seg, widx, want)
+        assert torch.equal(c, want)
+
+
+def test_w4a8_range_check_matches_the_host_form():
+    """One scale group at a time is pushed over the end of int8, by its largest, its smallest or no nibble that it holds."""
+    from types import SimpleNamespace
+    from llm_kernels_b200.moe.all2all_moe import DeepseekV3MoE
+    g = torch.Generator().manual_seed(5)
+    for n, s, z, lo, hi, want in ((0, 9, 0, 0, 14, True), (9, 9, 0, 0, 15, False), (255, -9, 0, 0, 15, False), (131, 9, 15, 1, 15, True),
+                                  (131, 9, 15, 0, 15, False), (7, 1, -113, 0, 14, True), (7, 1, -113, 0, 15, False), (200, -128, 3, 3, 4, True), (200, -128, 3, 2, 3, False)):
+        q = torch.randint(0, 16, (1, 256, 384), generator=g)
+        q[0, n, 128:256] = torch.randint(lo, hi + 1, (128,), generator=g)
+        q[0, n, 130], q[0, n, 255] = lo, hi
+        s4 = torch.ones(1, 256, 3, dtype=torch.int8)
+        z4 = torch.full((1, 256, 3), 8, dtype=torch.int8)
+        s4[0, n, 1], z4[0, n, 1] = s, z
+        words = sum(q.view(1, 32, 8, 384)[:, :, i] << (4 * i) for i in range(8))
+        packed = torch.where(words >= 2 ** 31, words - 2 ** 32, words).to(torch.int32)
+        for dev in ("cpu", "cuda"):
+            fake = SimpleNamespace(w13_qweight=packed.to(dev), w13_s4=s4.to(dev), w13_z4=z4.to(dev), _buffers_cache={})
+            assert DeepseekV3MoE._raw_nibbles_ok(fake, "w13") == want, (n, s, z, lo, hi, dev)
