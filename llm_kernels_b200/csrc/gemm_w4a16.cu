@@ -9,18 +9,17 @@
 // the tokens on the M side.  The tokens are the N = 16..CHUNK columns, so few rows cost little tensor-core time.
 //
 // Measured on 8 experts of a Mixtral layer (gate/up N 28672 K 4096, then down N 4096 K 14336; us; tokens on the M side and
-// weights through shared memory -> here): 1-16 rows per expert 436 + 219 -> 205 + 108, 64 rows 440 + 221 -> 213 + 111,
-// 128 rows 451 + 225 -> 287 + 121, 256 rows 821 + 438 -> 524 + 228.  A 64-k block of 256 channels takes 910 cycles: 1000 for
-// the conversion by each of the two converter groups (they alternate), 150 for the issue of the MMAs.  The roles that are one
-// thread are entered through elect.sync: under `lane == 0` every tcgen05 instruction took about 90 cycles to issue (1340
-// cycles per block).
+// weights through shared memory -> here): 1-16 rows per expert 436 + 219 -> 186 + 98, 64 rows 440 + 221 -> 223 + 101,
+// 128 rows 451 + 225 -> 291 + 120, 256 rows 821 + 438 -> 514 + 222.  The roles that are one thread are entered through
+// elect.sync: under `lane == 0` every tcgen05 instruction took about 90 cycles to issue, 750 cycles for the MMAs of 64 k
+// instead of 150.  Even so the MMA thread's barriers counted: one hand-over per 128 k instead of two 205 + 108 -> 186 + 98.
 //
 // One persistent CTA per SM, 768 threads:
 //   warp 0       TMA producer of the packed words: two boxes of 128 channels x 128 B (256 k) and their (scale, zero)
 //                pairs as bulk copies, 4 slots of 34 KB
-//   warp 2       TMA producer of the token rows: box of 16/32/64/128 rows x 64 k, 64 KB ring
-//   warps 8-23   converters: warp w serves TMEM lanes 32 (w % 4).. of channel half (w / 4) % 2 and every other 64-k block
-//   warp 1       owns TMEM: 4 operand stages x 2 halves x 32 columns, 256 columns of accumulators; per 64-k block 2 x 4
+//   warp 2       TMA producer of the token rows: two boxes of 16/32/64/128 rows x 64 k, 64 KB ring
+//   warps 8-23   converters: warp w serves TMEM lanes 32 (w % 4).. of channel half (w / 4) % 2 and every other K block of 128
+//   warp 1       owns TMEM: 2 operand stages of 128 columns, 256 columns of accumulators; per K block 2 x 8
 //                tcgen05.mma.kind::f16 (M128, N = tokens, K16); the whole K loop accumulates in TMEM
 //   warps 4-7    tile epilogue (plain, or act(gate) * up); with CHUNK = 64 it overlaps the next tile
 //
@@ -37,12 +36,13 @@
 namespace b200moe {
 namespace w4a16 {
 
-constexpr int kWStages = 4, kOpStages = 4;
+constexpr int kWStages = 4, kOpStages = 2;
 constexpr uint32_t kWBytes = 2 * 128 * 128;            // two halves of 128 channels x 32 words (256 k)
 constexpr uint32_t kPairBytes = 128 * 4;               // (scale, zero) of one half and one 128-k group
 constexpr uint32_t kWSlot = kWBytes + 4 * kPairBytes;  // [group][half][128] pairs behind the words
-constexpr uint32_t kTRing = 65536;                     // token ring: 8 slots of 64 rows or 4 of 128 rows, 128 B each
-constexpr int kMaxTStages = 8;
+constexpr uint32_t kTRing = 65536;                     // token ring: 4 slots of 64 rows or 2 of 128 rows, two boxes of 64 k each
+constexpr int kMaxTStages = 4;
+constexpr uint32_t kOpCols = 128;                      // operand stage: [64-k block of the pair][half][32 columns]
 constexpr int kThreads = 768, kEpiWarp0 = 4, kEpiWarps = 4, kConvWarp0 = 8, kConvWarps = 16;
 constexpr uint32_t kAccCol = 256;                      // first accumulator column
 static_assert(kWSlot % 1024 == 0, "the 128-byte swizzle needs 1 KB aligned slots");
@@ -128,7 +128,7 @@ __device__ __forceinline__ Affine make_affine(uint32_t scale_zero) {
   // 128 + z and 128 + 8 z are bf16 numbers when z is a whole number of 0..15, and s / 8 is exact unless it underflows:
   // then the one subtraction gives q - z (8 (q - z)) exactly and the product rounds the same real number as
   // (q - z) * s.  Zero points or scales outside take the general form.
-  a.whole = z >= 0.f && z <= 15.f && z == truncf(z) && ((sb & 0x7F80u) >= (4u << 7) || (sb & 0x7FFFu) == 0u);
+  a.whole = z >= 0.f && z <= 15.f && z == (z + 12582912.f) - 12582912.f && ((sb & 0x7F80u) >= (4u << 7) || (sb & 0x7FFFu) == 0u);
   a.c = bf2_bits(__floats2bfloat162_rn(128.f + z, 128.f + 8.f * z));
   a.s = bf2_bits(__floats2bfloat162_rn(s, s * 0.125f));
   return a;
@@ -148,7 +148,7 @@ template <int CHUNK>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_w4a16_kernel(const __grid_constant__ w4::RowMaps tmap_a, const __grid_constant__ CUtensorMap tmap_p,
                   const __grid_constant__ Params p) {
-  constexpr int kTStages = static_cast<int>(kTRing / (CHUNK * 128));
+  constexpr int kTStages = static_cast<int>(kTRing / (CHUNK * 256));
   constexpr int kAccStages = 128 / CHUNK;              // CHUNK = 64: two, CHUNK = 128: one
   static_assert(kTStages <= kMaxTStages && kAccStages >= 1, "");
   extern __shared__ uint8_t smem_raw[];
@@ -157,8 +157,8 @@ gemm_w4a16_kernel(const __grid_constant__ w4::RowMaps tmap_a, const __grid_const
   Tail* sh = reinterpret_cast<Tail*>(smem_t + kTRing);
   volatile int* abort_flag = &sh->abort_flag;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int KS = p.K / 64;                             // 64-k blocks; even, since K is a multiple of 128
-  const int KW = (KS + 3) / 4;                         // 256-k slots of packed words, the last one maybe half
+  const int KG = p.K / 128;                            // K blocks: one scale group, two 64-k boxes of the swizzle
+  const int KW = (KG + 1) / 2;                         // 256-k slots of packed words, the last one maybe half
   const int num_ct = p.fused ? p.N / 256 : (p.N + 255) / 256;
 
   if (threadIdx.x == 0) {
@@ -219,7 +219,7 @@ gemm_w4a16_kernel(const __grid_constant__ w4::RowMaps tmap_a, const __grid_const
       for (int kw = 0; kw < KW; ++kw) {
         if (!ptx::mbar_wait(&sh->w_empty[stage], phase ^ 1u, abort_flag)) { ok = false; break; }
         uint8_t* sw = smem + size_t(stage) * kWSlot;
-        const bool two = kw * 4 + 2 < KS;              // the slot's second 128-k group exists
+        const bool two = kw * 2 + 1 < KG;              // the slot's second 128-k group exists
         ptx::mbar_arrive_expect_tx(&sh->w_full[stage], (kWBytes / 2 + kPairBytes * (two ? 2u : 1u)) * (second ? 2u : 1u));
         armed.arm(stage, phase);
         ptx::tma_load_2d(sw, &tmap_p, &sh->w_full[stage], kw * 32, row0);          // words past K: zero fill
@@ -243,11 +243,13 @@ gemm_w4a16_kernel(const __grid_constant__ w4::RowMaps tmap_a, const __grid_const
     for (int t = first; ok && t < total; t += step) {
       const Tile tl = decode<CHUNK>(sh, p, t, num_ct);
       const int sel = tl.tn <= 16 ? 0 : (tl.tn <= 32 ? 1 : (tl.tn <= 64 ? 2 : 3));
-      for (int ks = 0; ks < KS; ++ks) {
+      for (int kg = 0; kg < KG; ++kg) {
         if (!ptx::mbar_wait(&sh->t_empty[stage], phase ^ 1u, abort_flag)) { ok = false; break; }
-        ptx::mbar_arrive_expect_tx(&sh->t_full[stage], (16u << sel) * 128u);
+        ptx::mbar_arrive_expect_tx(&sh->t_full[stage], (16u << sel) * 256u);
         armed.arm(stage, phase);
-        ptx::tma_load_2d(smem_t + size_t(stage) * (CHUNK * 128), &tmap_a.m[sel], &sh->t_full[stage], ks * 128, tl.m0);
+        uint8_t* slot = smem_t + size_t(stage) * (CHUNK * 256);
+        ptx::tma_load_2d(slot, &tmap_a.m[sel], &sh->t_full[stage], kg * 256, tl.m0);
+        ptx::tma_load_2d(slot + CHUNK * 128, &tmap_a.m[sel], &sh->t_full[stage], kg * 256 + 128, tl.m0);
         if (++stage == kTStages) { stage = 0; phase ^= 1u; }
       }
     }
@@ -262,15 +264,17 @@ gemm_w4a16_kernel(const __grid_constant__ w4::RowMaps tmap_a, const __grid_const
       const uint32_t idesc = ptx::umma_idesc(1, 1, 1, 128, static_cast<uint32_t>(tl.tn));    // D f32, A and B bf16
       if (!ptx::mbar_wait(&sh->acc_empty[as], pacc ^ 1u, abort_flag)) break;     // the stage's previous tile has been read
       const uint32_t d = tmem_base + kAccCol + static_cast<uint32_t>(as) * (2 * CHUNK);
-      for (int ks = 0; ks < KS; ++ks) {
+      for (int kg = 0; kg < KG; ++kg) {
         if (!ptx::mbar_wait(&sh->t_full[st], pt, abort_flag) || !ptx::mbar_wait(&sh->op_full[so], po, abort_flag)) { ok = false; break; }
         ptx::tc_fence_after_sync();
-        const uint32_t a = tmem_base + static_cast<uint32_t>(so) * 64u;
-        const uint64_t tdesc = ptx::umma_desc_sw128(ptx::smem_u32(smem_t + size_t(st) * (CHUNK * 128)));
+        const uint32_t a = tmem_base + static_cast<uint32_t>(so) * kOpCols;
+        const uint64_t tdesc = ptx::umma_desc_sw128(ptx::smem_u32(smem_t + size_t(st) * (CHUNK * 256)));
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {      // halves alternate: an instruction does not wait for the one that feeds its accumulator
-          ptx::umma_f16_ts(d, a + 8u * k, tdesc + 2 * k, idesc, (ks > 0 || k > 0) ? 1u : 0u);
-          ptx::umma_f16_ts(d + CHUNK, a + 32u + 8u * k, tdesc + 2 * k, idesc, (ks > 0 || k > 0) ? 1u : 0u);
+        for (int k = 0; k < 8; ++k) {      // halves alternate: an instruction does not wait for the one that feeds its accumulator
+          const uint64_t td = tdesc + (k >> 2) * (CHUNK * 128 >> 4) + 2 * (k & 3);
+          const uint32_t ak = a + 64u * (k >> 2) + 8u * (k & 3), more = (kg > 0 || k > 0) ? 1u : 0u;
+          ptx::umma_f16_ts(d, ak, td, idesc, more);
+          ptx::umma_f16_ts(d + CHUNK, ak + 32u, td, idesc, more);
         }
         ptx::umma_commit(&sh->op_empty[so]);
         ptx::umma_commit(&sh->t_empty[st]);
@@ -282,51 +286,59 @@ gemm_w4a16_kernel(const __grid_constant__ w4::RowMaps tmap_a, const __grid_const
       if (++as == kAccStages) { as = 0; pacc ^= 1u; }
     }
   } else if (warp >= kConvWarp0) {
-    // ---- converters: thread = output channel, one 64-k block (eight packed words) at a time --------------------------
+    // ---- converters: thread = output channel, one K block (16 packed words) at a time; the two groups take turns ------
     const int cw = warp - kConvWarp0;
     const int q = cw & 3, half = (cw >> 2) & 1, par = cw >> 3;   // kConvWarp0 % 4 == 0: TMEM lane quarter = warp % 4
     const int row = q * 32 + lane;                                // channel within the half = TMEM lane
     const uint8_t* my_w = smem + half * (kWBytes / 2) + row * 128;
     const uint8_t* my_sz = smem + kWBytes + half * kPairBytes + row * 4;
-    const uint32_t my_t = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(half) * 32u;
-    int sw = 0, so = par;
+    // operand stage = group: the K blocks of all tiles in turn, stage 0 and stage 1 alternating
+    const uint32_t my_t = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(par) * kOpCols + static_cast<uint32_t>(half) * 32u;
+    int sw = 0, turn = 0;
     uint32_t pw = 0, po = 0;
     bool ok = true;
     for (int t = first; ok && t < total; t += step) {
       for (int kw = 0; ok && kw < KW; ++kw) {
         if (!warp_wait(&sh->w_full[sw], pw, abort_flag)) { ok = false; break; }
-#pragma unroll 1
-        for (int s = par; s < 4; s += 2) {                        // this warp's 64-k blocks of the slot
-          if (kw * 4 + s >= KS) break;
+        const int blocks = min(2, KG - kw * 2);
+        const int mine = (turn ^ par) & 1;                        // this group's K block of the slot
+        turn += blocks;
+        if (mine < blocks) {
           const uint8_t* src = my_w + size_t(sw) * kWSlot;
-          const uint4 wa = *reinterpret_cast<const uint4*>(src + (((2 * s) ^ (row & 7)) << 4));
-          const uint4 wb = *reinterpret_cast<const uint4*>(src + (((2 * s + 1) ^ (row & 7)) << 4));
-          const uint32_t sz = *reinterpret_cast<const uint32_t*>(my_sz + size_t(sw) * kWSlot + (s >> 1) * (2 * kPairBytes));
-          const uint32_t wd[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
+          const uint32_t sz = *reinterpret_cast<const uint32_t*>(my_sz + size_t(sw) * kWSlot + mine * (2 * kPairBytes));
           const Affine a = make_affine(sz);
-          uint32_t r[32];
-          if (__all_sync(0xffffffffu, a.whole)) {
+          const bool whole = __all_sync(0xffffffffu, a.whole);
+#pragma unroll 1
+          for (int s = 0; s < 2; ++s) {                           // 64 k each
+            const int ch = mine * 4 + s * 2;
+            const uint4 wa = *reinterpret_cast<const uint4*>(src + ((ch ^ (row & 7)) << 4));
+            const uint4 wb = *reinterpret_cast<const uint4*>(src + (((ch + 1) ^ (row & 7)) << 4));
+            const uint32_t wd[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
+            uint32_t r[32];
+            if (whole) {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) convert_word(wd[i], a, r + 4 * i);
-          } else {
+              for (int i = 0; i < 8; ++i) convert_word(wd[i], a, r + 4 * i);
+            } else {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              const uint4 v = dequant_word_bf16(wd[i], sz);
-              r[4 * i] = v.x; r[4 * i + 1] = v.y; r[4 * i + 2] = v.z; r[4 * i + 3] = v.w;
+              for (int i = 0; i < 8; ++i) {
+                const uint4 v = dequant_word_bf16(wd[i], sz);
+                r[4 * i] = v.x; r[4 * i + 1] = v.y; r[4 * i + 2] = v.z; r[4 * i + 3] = v.w;
+              }
             }
+            if (s == 0) {
+              if (!warp_wait(&sh->op_empty[par], po ^ 1u, abort_flag)) { ok = false; break; }
+              ptx::tc_fence_after_sync();
+            }
+            ptx::tmem_st32(my_t + static_cast<uint32_t>(s) * 64u, r);
           }
-          if (!warp_wait(&sh->op_empty[so], po ^ 1u, abort_flag)) { ok = false; break; }
-          ptx::tc_fence_after_sync();
-          ptx::tmem_st32(my_t + static_cast<uint32_t>(so) * 64u, r);
+          if (!ok) break;
           ptx::tmem_st_wait();
           ptx::tc_fence_before_sync();
           __syncwarp();
-          if (lane == 0) ptx::mbar_arrive(&sh->op_full[so]);
-          so += 2;
-          if (so >= kOpStages) { so = par; po ^= 1u; }
+          if (lane == 0) ptx::mbar_arrive(&sh->op_full[par]);
+          po ^= 1u;
         }
-        if (!ok) break;
-        if (lane == 0) ptx::mbar_arrive(&sh->w_empty[sw]);       // after the __syncwarp of the last block: every lane has read
+        if (lane == 0) ptx::mbar_arrive(&sh->w_empty[sw]);        // converged: every lane has read its words
         if (++sw == kWStages) { sw = 0; pw ^= 1u; }
       }
     }
@@ -385,8 +397,9 @@ gemm_w4a16_kernel(const __grid_constant__ w4::RowMaps tmap_a, const __grid_const
 }
 
 // Average rows per group above which a tile takes 128 tokens (one set of accumulators) instead of 64 (two sets, the epilogue
-// overlaps).  Gate/up above, us: 64 rows per group 213 with chunks of 64; 96 rows 262 with chunks of 128, where two chunks of
-// 64 would be 2 x 210.  Groups are ragged, so the line is below 64: from about 48 on average some need a second chunk of 64.
+// overlaps).  Gate/up above, us: 64 rows per group 213 with chunks of 64, 223 with chunks of 128; 96 rows 263 with chunks of
+// 128, where two chunks of 64 would be about 2 x 200.  Groups are ragged, so the line is below 64: from about 48 on average
+// some need a second chunk of 64.
 constexpr int kWideChunkRows = 48;
 
 template <int CHUNK>
