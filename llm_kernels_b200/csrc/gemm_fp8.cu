@@ -129,12 +129,15 @@ __device__ __forceinline__ Tile decode_tile(const SharedTail* sh, const GemmPara
   // inside a group: bands of p.band columns, every band down all m-tiles of the group; split-K launches keep whole rows,
   // from which the MMA issuer derives its split
   const int m_tiles = sh->pref[lo + 1] - sh->pref[lo];
-  const int rem = t - sh->pref[lo] * per;
-  const int band_cols = min(p.band, per);
-  const int band = rem / (m_tiles * band_cols);
-  const int in_band = rem - band * (m_tiles * band_cols);
-  const int cols = min(band_cols, per - band * band_cols);
-  const int m = in_band / cols, col = band * band_cols + in_band - m * cols;
+  int m = mt - sh->pref[lo], col = t - mt * per;
+  if (p.band < per) {
+    const int rem = t - sh->pref[lo] * per;
+    const int band = rem / (m_tiles * p.band);
+    const int in_band = rem - band * (m_tiles * p.band);
+    const int cols = min(p.band, per - band * p.band);
+    m = in_band / cols;
+    col = band * p.band + in_band - m * cols;
+  }
   Tile tl;
   tl.m0 = sh->seg[lo] + m * bmt + m_off;
   tl.m_end = sh->seg[lo + 1];
@@ -254,13 +257,19 @@ gemm_block_kernel(const __grid_constant__ RowMaps tmap_a,
   const int total_tiles = sh->pref[p.num_groups] * num_n_tiles * p.ksplits;
   const int KBs = (KB + p.ksplits - 1) / p.ksplits;   // K blocks per split
 
+  // The thread of a single-thread role.  elect.sync makes TMA and MMA instructions several times faster to issue than a
+  // lane == 0 branch; in pairs, whose leader issues for two SMs, that counts (w4a16 prefill of 8192 tokens 6319 -> 6077 us).
+  // The other launches wait for their promotion or their loads anyway, and lose with it (fp8 layer of 4096 tokens 3786 ->
+  // 3867 us).
+  auto one_thread = [&]() { if constexpr (PAIR) return ptx::elect_one(); else return lane == 0; };
+
   // Register hand-over: the producer/MMA warpgroup keeps 56 registers per thread, the two
   // promotion warpgroups grow to 224 (384 x 168 = 128 x 56 + 256 x 224).
   if (warp < kFirstEpiWarp) {
     ptx::setmaxnreg_dec<56>();
   if (warp == 0) {
     // ================================ TMA producer ================================
-    if (ptx::elect_one()) {
+    if (one_thread()) {
       int stage = 0; uint32_t phase = 0;
       uint32_t armed = 0, armed_parity = 0;
       bool ok = true;
@@ -325,7 +334,7 @@ gemm_block_kernel(const __grid_constant__ RowMaps tmap_a,
     }
   } else if (warp == 1) {
     // ================================ MMA issuer ==================================
-    if (leader && ptx::elect_one()) {
+    if (leader && one_thread()) {
       // D f32 (1) / s32 (2); operand formats: e4m3 = 0, signed int8 = 1, bf16 = 1
       constexpr uint32_t idesc = KIND == kFp8 ? ptx::umma_idesc(1, 0, 0, BMT, BN)
                                  : (KIND == kI8 ? ptx::umma_idesc(2, 1, 1, BMT, BN)
