@@ -20,7 +20,8 @@
 //     channel per 32-bit column: the converters transpose bytes in registers and store with the one tcgen05.st shape whose
 //     register layout fits, 0.7 instructions per weight and no shared-memory write or MMA read of the operand.
 //
-// What bounds it: see the figures.  64 experts, gate/up N 4096 K 7168 then down N 7168 K 2048, us (operand in shared memory,
+// What bounds it: issue slots (62 % at 16 rows per expert), first of the conversion, from about 32 rows on of the promotion.
+// 64 experts, gate/up N 4096 K 7168 then down N 7168 K 2048, us (operand in shared memory,
 // roles entered by lane == 0, four promotion warps with integer multiply-adds -> here): 1 row per expert 338 + 186 -> 218 +
 // 129, 16 rows 358 + 189 -> 221 + 131 (4.4 TB/s of packed weights), 48 rows 566 + 291 -> 355 + 210, 64 rows 690 + 377 ->
 // 416 + 244, 94 rows 1100 + 606 -> 706 + 384, 256 rows 2845 + 1491 -> 1643 + 897.
