@@ -128,3 +128,18 @@ def test_w4a8_range_check_matches_the_host_form():
         for dev in ("cpu", "cuda"):
             fake = SimpleNamespace(w13_qweight=packed.to(dev), w13_s4=s4.to(dev), w13_z4=z4.to(dev), _buffers_cache={})
             assert DeepseekV3MoE._raw_nibbles_ok(fake, "w13") == want, (n, s, z, lo, hi, dev)
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 128, 128), (24, 4096, 7168), (100, 1152, 640), (128, 512, 2048), (129, 512, 2048)])
+def test_w4a8_gemm_splits_against_64_bits(M, N, K):
+    """The K splits of few rows and the single launch of more: integer dot products are exact, so what is left is the f32
+    scaling and sum of K / 128 blocks, at most about sqrt(K / 128) roundings of 6e-8 in the 2-norm."""
+    from llm_kernels_b200.quantization import w4a8_kernel
+    dev = torch.device("cuda:0")
+    g = torch.Generator(device=dev).manual_seed(6)
+    packed, s, s4, z4 = w4a8_kernel.weight_quant(torch.randn(N, K, generator=g, device=dev) * 0.02)
+    a, a_s = w4a8_kernel.act_quant(torch.randn(M, K, generator=g, device=dev).to(torch.bfloat16))
+    c = w4a8_kernel.w4a8_gemm(a, a_s, packed, s, s4, z4, out_dtype=torch.float32)
+    w = w4a8_kernel.expand_int8(packed, s4, z4).double() * s.double().repeat_interleave(128, 0).repeat_interleave(128, 1)
+    want = (a.double() * a_s.double().repeat_interleave(128, 1)) @ w.t()
+    assert float((c - want).norm() / want.norm()) < 6e-8 * max(4.0, (K / 128) ** 0.5)
