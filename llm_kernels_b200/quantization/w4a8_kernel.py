@@ -80,15 +80,16 @@ def w4a8_gemm(a: torch.Tensor, a_s: torch.Tensor, b: torch.Tensor, b_s: torch.Te
     Nn = w8.shape[0]
     c = a.new_empty(*a.size()[:-1], Nn, dtype=out_dtype or torch.get_default_dtype())
     ks = _split_k(M, Nn, K)
-    if ks > 1 and M > 0 and _opts() is None:
+    a_s, b_s = a_s.reshape(M, -1).float(), b_s.float()
+    # The split launch takes its sizes and strides from M, N and K alone, so it serves operands that agree on them; any
+    # others go to the grouped launch, which checks them and reads the scales by their own stride.
+    if ks > 1 and _opts() is None and tuple(w8.shape) == (Nn, K) and a_s.shape[1] * 128 == K:
         N.require_cuda(a, a_s, b_s)
         assert a.dtype == torch.int8
-        a_s, b_s = a_s.reshape(M, -1).float(), b_s.float()
         part = _workspace(a.device, ks * M * Nn * 4)
         N.check(N.lib().b200moe_gemm_i8_block_splitk(N.ptr(a), N.ptr(a_s), N.ptr(w8), N.ptr(b_s), N.ptr(c),
                                                      N.dtype_code(c.dtype), M, Nn, K, ks, N.ptr(part), part.numel(),
                                                      N.stream()))
         return c
-    grouped_gemm_i8(a.view(M, K), a_s.reshape(M, -1).float(), w8.unsqueeze(0), b_s.float().unsqueeze(0), None, None,
-                    c.view(M, Nn))
+    grouped_gemm_i8(a.view(M, K), a_s, w8.unsqueeze(0), b_s.unsqueeze(0), None, None, c.view(M, Nn))
     return c

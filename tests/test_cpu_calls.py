@@ -1,0 +1,56 @@
+"""What the Python layer hands to the library, seen on the host: the launches are replaced by a recorder (or, where only the
+library's argument checks matter, reach the library itself, which checks before it launches)."""
+import pytest
+import torch
+
+
+@pytest.fixture
+def host(monkeypatch):
+    """CPU tensors pass for the current device's."""
+    from llm_kernels_b200 import _native as N, build
+    build.build()
+    monkeypatch.setattr(N, "require_cuda", lambda *tensors: None)
+    monkeypatch.setattr(N, "stream", lambda: 0)
+    return N
+
+
+class Recorder:
+    """Stands in for the loaded library: every entry point succeeds and is noted; `on` maps names to replacements."""
+
+    def __init__(self, **on):
+        self.calls, self.on = [], on
+
+    def __getattr__(self, name):
+        def call(*args):
+            self.calls.append((name, args))
+            return self.on[name](*args) if name in self.on else 0
+        return call
+
+    def names(self):
+        return [n for n, _ in self.calls]
+
+
+def _w4a8_operands(M, K, kw, scale_cols):
+    """int8 rows of K, a weight of 256 channels x kw, `scale_cols` activation scales per row."""
+    return (torch.zeros(M, K, dtype=torch.int8), torch.ones(M, scale_cols), torch.zeros(32, kw, dtype=torch.int32),
+            torch.ones(2, kw // 128), torch.ones(256, kw // 128, dtype=torch.int8), torch.ones(256, kw // 128, dtype=torch.int8))
+
+
+@pytest.mark.parametrize("M", [24, 200])
+@pytest.mark.parametrize("K,kw,scale_cols", [(1024, 512, 8), (512, 1024, 4), (1024, 1024, 4)])
+def test_w4a8_gemm_refuses_operands_that_disagree(host, monkeypatch, M, K, kw, scale_cols):
+    """A weight of another K, or too few activation scales, is refused for few rows as for many."""
+    from llm_kernels_b200.quantization import w4a8_kernel
+    monkeypatch.setattr(w4a8_kernel, "expand_int8", lambda b, s4, z4: torch.zeros(8 * b.shape[0], b.shape[1], dtype=torch.int8))
+    with pytest.raises(AssertionError):
+        w4a8_kernel.w4a8_gemm(*_w4a8_operands(M, K, kw, scale_cols))
+
+
+@pytest.mark.parametrize("M", [24, 200])
+def test_w4a8_gemm_reads_wider_scales_by_their_own_stride(host, monkeypatch, M):
+    from llm_kernels_b200.quantization import w4a8_kernel
+    lib = Recorder()
+    monkeypatch.setattr(host, "_lib", lib)
+    w4a8_kernel.w4a8_gemm(*_w4a8_operands(M, 1024, 1024, 11))
+    name, args = lib.calls[-1]
+    assert name == "b200moe_grouped_gemm_i8" and args[3] == 11
