@@ -175,6 +175,11 @@ class MoEGate(nn.Module):
         return t
 
 
+def _is_plain(t, dtype, shape):
+    """Whether t is a contiguous tensor of this type and shape."""
+    return t is not None and t.dtype == dtype and t.shape == shape and t.is_contiguous()
+
+
 class DeepseekV3MoE(nn.Module):
     """A mixed expert module (reference :120-286) over quantized fused expert weights.
 
@@ -279,6 +284,9 @@ class DeepseekV3MoE(nn.Module):
             reg("shared_w13", z(1, 2 * Is, H, dtype=torch.bfloat16))     # [gate_proj ; up_proj]
             reg("shared_w2", z(1, H, Is, dtype=torch.bfloat16))          # down_proj
             self._shared_stream = None
+        # types and shapes of the tensors above, as the one-call pass reads them, and the sizes that they were made from
+        self._layout = {n: (t.dtype, t.shape) for n, t in self._buffers.items()}
+        self._sizes = (E, H, I)
         # int4 methods: up to this many rows per expert group on average the dequantization runs inside the GEMMs
         # (every tile converts its weights once); above it the weights are expanded once per forward instead
         # Whole w4a8 layer (256 experts, hidden 7168), us expanded -> inside the GEMMs: 47 rows 7785 -> 2509, 94 rows 8019 -> 4755,
@@ -398,8 +406,13 @@ class DeepseekV3MoE(nn.Module):
         a weight, the router or a setting changed since the last pass: `key` is everything the structure was made from."""
         gate, bufs, cfg = self.gate, self._buffers, self.config
         w, bias = gate.weight, gate.e_score_correction_bias
-        tensors = [w, bias]
-        tensors += [t for n, t in bufs.items() if t is not None]
+        E, H, I = self._sizes
+        # tensors of another type, shape or stride than the layer's own: the separate calls check them one by one
+        if ((cfg.n_routed_experts, cfg.hidden_size, cfg.moe_intermediate_size) != self._sizes
+                or not _is_plain(w, torch.float32, (E, H)) or not _is_plain(bias, torch.float32, (E,))
+                or not all(_is_plain(bufs.get(n), *want) for n, want in self._layout.items())):
+            return None
+        tensors = [w, bias, *(bufs[n] for n in self._layout)]
         key = [v for t in tensors for v in (t.data_ptr(), t._version)]
         key += [self.method, self._gelu, gate.scoring_func, gate.topk_method, gate.top_k, gate.n_group, gate.topk_group,
                 gate.norm_topk_prob, gate.routed_scaling_factor]
@@ -407,15 +420,14 @@ class DeepseekV3MoE(nn.Module):
             return self._native[1]
         self._native = None
         if (gate.scoring_func not in ("sigmoid", "softmax") or gate.topk_method != "noaux_tc" or type(gate) is not MoEGate
-                or w.dtype != torch.float32 or bias.dtype != torch.float32 or gate.top_k != cfg.num_experts_per_tok):
+                or gate.top_k != cfg.num_experts_per_tok):
             return None
         N.require_cuda(*tensors)
-        assert all(t.is_contiguous() for t in tensors)
         w3 = gate._split_weight(w)
-        d = N.Layer(struct_bytes=C.sizeof(N.Layer), act=int(self._gelu), experts=cfg.n_routed_experts, top_k=gate.top_k,
+        d = N.Layer(struct_bytes=C.sizeof(N.Layer), act=int(self._gelu), experts=E, top_k=gate.top_k,
                     n_group=gate.n_group, topk_group=gate.topk_group, scoring=0 if gate.scoring_func == "sigmoid" else 1,
                     norm_topk_prob=1 if gate.norm_topk_prob else 0, scaling=float(gate.routed_scaling_factor),
-                    router_rows=w3.shape[0], hidden=cfg.hidden_size, inter=cfg.moe_intermediate_size,
+                    router_rows=w3.shape[0], hidden=H, inter=I,
                     router_w3=N.ptr(w3), router_bias=N.ptr(bias), status=N.ptr(self._status))
         for n in ("w13", "w2"):
             if self.method == "fp8_block":

@@ -54,3 +54,46 @@ def test_w4a8_gemm_reads_wider_scales_by_their_own_stride(host, monkeypatch, M):
     w4a8_kernel.w4a8_gemm(*_w4a8_operands(M, 1024, 1024, 11))
     name, args = lib.calls[-1]
     assert name == "b200moe_grouped_gemm_i8" and args[3] == 11
+
+
+@pytest.fixture
+def layer_host(host, monkeypatch):
+    """make(method) -> (layer on the host, bf16 tokens, recorder of its launches)."""
+    from llm_kernels_b200.moe import group_gemm_kernel as G
+    from llm_kernels_b200.moe.all2all_moe import DeepseekV3MoE
+    from llm_kernels_b200.workloads import LayerShape, make_config
+    monkeypatch.setattr(G, "_workspace", lambda device, nbytes: torch.empty(1024, dtype=torch.uint8))
+
+    def make(method="fp8_block", cls=DeepseekV3MoE, **on):
+        lib = Recorder(b200moe_layer_workspace_bytes=lambda d, T: 4096, b200moe_router_ksplits=lambda T, H, E: 1, **on)
+        monkeypatch.setattr(host, "_lib", lib)
+        shape = LayerShape("host", 4, 256, 128, 8, 2, 1, 1, "sigmoid", 1.0, 0, method=method)
+        layer = cls(make_config(shape), device="cpu").eval()
+        return layer, torch.zeros(1, 4, 256, dtype=torch.bfloat16), lib
+    return make
+
+
+@pytest.mark.parametrize("method", ["fp8_block", "w4a16", "w4a8"])
+def test_layer_pass_is_one_call(layer_host, method):
+    layer, x, lib = layer_host(method)
+    assert layer(x).shape == x.shape and lib.names()[-1] == "b200moe_layer_forward"
+    assert not any(n.startswith("b200moe_grouped") for n in lib.names())
+
+
+@pytest.mark.parametrize("method,name,change", [
+    ("fp8_block", "w13_weight_scale", lambda t: t.to(torch.bfloat16)),
+    ("fp8_block", "w2_weight_scale", lambda t: t.double()),
+    ("fp8_block", "w13_weight", lambda t: torch.cat([t.view(torch.uint8)] * 2, dim=2).view(t.dtype)),
+    ("w4a16", "w2_scale", lambda t: t.float()),
+    ("w4a16", "w13_qweight", lambda t: t.to(torch.int64)),
+    ("w4a8", "w2_weight_scale", lambda t: t.half()),
+    ("w4a8", "w13_s4", lambda t: torch.cat([t, t], dim=2))])
+def test_layer_refuses_weights_of_another_type_or_shape(layer_host, method, name, change):
+    """The one-call pass reads raw pointers: what the separate launches refuse must not reach it."""
+    layer, x, lib = layer_host(method)
+    layer(x)
+    setattr(layer, name, change(getattr(layer, name)))
+    lib.calls.clear()
+    with pytest.raises((AssertionError, RuntimeError)):
+        layer(x)
+    assert "b200moe_layer_forward" not in lib.names()
