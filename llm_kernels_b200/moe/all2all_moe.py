@@ -401,9 +401,10 @@ class DeepseekV3MoE(nn.Module):
             self._shared_finish(fork, y)
         return y.view(*orig_shape)
 
-    def _describe(self):
-        """The layer as the C structure of b200moe_layer_forward, or None where that call does not apply.  Rebuilt when
-        a weight, the router or a setting changed since the last pass: `key` is everything the structure was made from."""
+    def _describe(self, x):
+        """The layer as the C structure of b200moe_layer_forward, or None where that call does not apply to x.  Rebuilt
+        when a weight, the router or a setting changed since the last pass: `key` is everything the structure was made
+        from.  What a pass needs of its tensors is looked at in every pass."""
         gate, bufs, cfg = self.gate, self._buffers, self.config
         w, bias = gate.weight, gate.e_score_correction_bias
         E, H, I = self._sizes
@@ -413,6 +414,7 @@ class DeepseekV3MoE(nn.Module):
                 or not all(_is_plain(bufs.get(n), *want) for n, want in self._layout.items())):
             return None
         tensors = [w, bias, *(bufs[n] for n in self._layout)]
+        N.require_cuda(x, *tensors)
         key = [v for t in tensors for v in (t.data_ptr(), t._version)]
         key += [self.method, self._gelu, gate.scoring_func, gate.topk_method, gate.top_k, gate.n_group, gate.topk_group,
                 gate.norm_topk_prob, gate.routed_scaling_factor]
@@ -422,7 +424,6 @@ class DeepseekV3MoE(nn.Module):
         if (gate.scoring_func not in ("sigmoid", "softmax") or gate.topk_method != "noaux_tc" or type(gate) is not MoEGate
                 or gate.top_k != cfg.num_experts_per_tok):
             return None
-        N.require_cuda(*tensors)
         w3 = gate._split_weight(w)
         d = N.Layer(struct_bytes=C.sizeof(N.Layer), act=int(self._gelu), experts=E, top_k=gate.top_k,
                     n_group=gate.n_group, topk_group=gate.topk_group, scoring=0 if gate.scoring_func == "sigmoid" else 1,
@@ -465,8 +466,7 @@ class DeepseekV3MoE(nn.Module):
                 T * self.num_experts_per_tok > self.w4_fused_rows_per_group * self.experts_per_rank):
             return None
         assert not self.gate.training
-        N.require_cuda(x)
-        if self._describe() is None:
+        if self._describe(x) is None:
             return None
         lib, desc = N.lib(), self._native[2]
         need = lib.b200moe_layer_workspace_bytes(desc, T)

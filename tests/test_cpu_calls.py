@@ -97,3 +97,19 @@ def test_layer_refuses_weights_of_another_type_or_shape(layer_host, method, name
     with pytest.raises((AssertionError, RuntimeError)):
         layer(x)
     assert "b200moe_layer_forward" not in lib.names()
+
+
+def test_layer_refuses_weights_of_another_device_in_every_pass(layer_host, host, monkeypatch):
+    """x on the current device is not enough, also once a pass has gone through."""
+    layer, x, lib = layer_host()
+    current = [x, *layer.state_dict(keep_vars=True).values()]
+
+    def require_cuda(*tensors):
+        if not all(t is None or any(t.data_ptr() == c.data_ptr() for c in current) for t in tensors):
+            raise RuntimeError("not on the current device")
+    monkeypatch.setattr(host, "require_cuda", require_cuda)
+    layer(x)
+    x = torch.ones_like(x)
+    current = [x]                                    # the caller has moved on to another device
+    with pytest.raises(RuntimeError, match="current device"):
+        layer(x)
