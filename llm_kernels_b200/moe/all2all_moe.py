@@ -384,7 +384,7 @@ class DeepseekV3MoE(nn.Module):
     # ---- forward ---------------------------------------------------------------------
     @torch.no_grad()
     def forward(self, hidden_states):
-        if self.ep_size == 1 and self.stage_events is None:
+        if self.ep_size == 1 and self.stage_events is None and G._opts() is None:     # the one call takes no GEMM options
             y = self._forward_native(hidden_states)
             if y is not None:
                 return y

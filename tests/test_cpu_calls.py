@@ -113,3 +113,13 @@ def test_layer_refuses_weights_of_another_device_in_every_pass(layer_host, host,
     current = [x]                                    # the caller has moved on to another device
     with pytest.raises(RuntimeError, match="current device"):
         layer(x)
+
+
+def test_layer_passes_gemm_options_on(layer_host):
+    """gemm_options around a layer reaches its grouped GEMMs."""
+    from llm_kernels_b200.moe import group_gemm_kernel as G
+    layer, x, lib = layer_host()
+    with G.gemm_options(max_ctas=7):
+        layer(x)
+    gemms = [args for n, args in lib.calls if n == "b200moe_grouped_gemm_fp8"]
+    assert len(gemms) == 2 and all(args[-2]._obj.max_ctas == 7 for args in gemms)
