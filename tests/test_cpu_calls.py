@@ -123,3 +123,46 @@ def test_layer_passes_gemm_options_on(layer_host):
         layer(x)
     gemms = [args for n, args in lib.calls if n == "b200moe_grouped_gemm_fp8"]
     assert len(gemms) == 2 and all(args[-2]._obj.max_ctas == 7 for args in gemms)
+
+
+def _hook(seen):
+    return lambda *a: seen.append(1)
+
+
+@pytest.mark.parametrize("how", ["forward hook", "pre-forward hook", "global hook", "instance forward", "gate class", "infer override", "infer on the instance"])
+def test_layer_runs_what_replaces_its_gate_or_pipeline(layer_host, how):
+    from llm_kernels_b200.moe.all2all_moe import DeepseekV3MoE, MoEGate
+    seen = []
+
+    class Other(DeepseekV3MoE):
+        def triton_group_gemm_moe_infer(self, x, idx, w):
+            seen.append(1)
+            return super().triton_group_gemm_moe_infer(x, idx, w)
+
+    class OtherGate(MoEGate):
+        def forward(self, x):
+            seen.append(1)
+            return super().forward(x)
+
+    layer, x, lib = layer_host(cls=Other if how == "infer override" else DeepseekV3MoE)
+    if how != "infer override":
+        layer(x)                                     # a pass before the change must not decide for the ones after it
+    handle, gate_forward, infer = None, layer.gate.forward, layer.triton_group_gemm_moe_infer
+    if how == "forward hook":
+        layer.gate.register_forward_hook(_hook(seen))
+    elif how == "pre-forward hook":
+        layer.gate.register_forward_pre_hook(_hook(seen))
+    elif how == "global hook":
+        handle = torch.nn.modules.module.register_module_forward_hook(lambda m, i, o: seen.append(1) if m is layer.gate else None)
+    elif how == "instance forward":
+        layer.gate.forward = lambda h: (seen.append(1), gate_forward(h))[1]
+    elif how == "gate class":
+        layer.gate.__class__ = OtherGate
+    elif how == "infer on the instance":
+        layer.triton_group_gemm_moe_infer = lambda *a: (seen.append(1), infer(*a))[1]
+    try:
+        layer(x)
+    finally:
+        if handle is not None:
+            handle.remove()
+    assert seen == [1]
