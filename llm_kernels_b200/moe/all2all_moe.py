@@ -417,6 +417,8 @@ class DeepseekV3MoE(nn.Module):
         when a weight, the router or a setting changed since the last pass: `key` is everything the structure was made
         from.  What a pass needs of its tensors is looked at in every pass."""
         gate, bufs, cfg = self.gate, self._buffers, self.config
+        if gate.scoring_func not in ("sigmoid", "softmax") or gate.topk_method != "noaux_tc":      # the gate says why
+            return None
         w, bias = gate.weight, gate.e_score_correction_bias
         E, H, I = self._sizes
         # tensors of another type, shape or stride than the layer's own: the separate calls check them one by one
@@ -432,8 +434,7 @@ class DeepseekV3MoE(nn.Module):
         if self._native is not None and self._native[0] == key:
             return self._native[1]
         self._native = None
-        if (gate.scoring_func not in ("sigmoid", "softmax") or gate.topk_method != "noaux_tc"
-                or gate.top_k != cfg.num_experts_per_tok):
+        if gate.top_k != cfg.num_experts_per_tok:
             return None
         w3 = gate._split_weight(w)
         d = N.Layer(struct_bytes=C.sizeof(N.Layer), act=int(self._gelu), experts=E, top_k=gate.top_k,

@@ -64,11 +64,14 @@ def layer_host(host, monkeypatch):
     from llm_kernels_b200.workloads import LayerShape, make_config
     monkeypatch.setattr(G, "_workspace", lambda device, nbytes: torch.empty(1024, dtype=torch.uint8))
 
-    def make(method="fp8_block", cls=DeepseekV3MoE, **on):
+    def make(method="fp8_block", cls=DeepseekV3MoE, config={}, **on):
         lib = Recorder(b200moe_layer_workspace_bytes=lambda d, T: 4096, b200moe_router_ksplits=lambda T, H, E: 1, **on)
         monkeypatch.setattr(host, "_lib", lib)
         shape = LayerShape("host", 4, 256, 128, 8, 2, 1, 1, "sigmoid", 1.0, 0, method=method)
-        layer = cls(make_config(shape), device="cpu").eval()
+        cfg = make_config(shape)
+        for name, value in config.items():
+            setattr(cfg, name, value)
+        layer = cls(cfg, device="cpu").eval()
         return layer, torch.zeros(1, 4, 256, dtype=torch.bfloat16), lib
     return make
 
@@ -166,3 +169,11 @@ def test_layer_runs_what_replaces_its_gate_or_pipeline(layer_host, how):
         if handle is not None:
             handle.remove()
     assert seen == [1]
+
+
+@pytest.mark.parametrize("name,value", [("topk_method", "greedy"), ("topk_method", "group_limited_greedy"), ("scoring_func", "relu")])
+def test_layer_names_an_unsupported_router(layer_host, name, value):
+    """Such a gate has no correction bias for the layer to read."""
+    layer, x, lib = layer_host(config={name: value})
+    with pytest.raises(NotImplementedError, match=value if name == "topk_method" else "scoring"):
+        layer(x)
