@@ -413,9 +413,9 @@ class DeepseekV3MoE(nn.Module):
                          or nn.modules.module._global_forward_pre_hooks))
 
     def _describe(self, x):
-        """The layer as the C structure of b200moe_layer_forward, or None where that call does not apply to x.  Rebuilt
-        when a weight, the router or a setting changed since the last pass: `key` is everything the structure was made
-        from.  What a pass needs of its tensors is looked at in every pass."""
+        """The layer as the C structure of b200moe_layer_forward, or None where that call does not apply to x.  `key` is
+        everything the structure was made from, pointers and settings; it is rebuilt when one of them differs from the last
+        pass's.  What a pass needs of its tensors is looked at in every pass."""
         gate, bufs, cfg = self.gate, self._buffers, self.config
         if gate.scoring_func not in ("sigmoid", "softmax") or gate.topk_method != "noaux_tc":      # the gate says why
             return None
@@ -428,31 +428,31 @@ class DeepseekV3MoE(nn.Module):
             return None
         tensors = [w, bias, *(bufs[n] for n in self._layout)]
         N.require_cuda(x, *tensors)
-        key = [v for t in tensors for v in (t.data_ptr(), t._version)]
-        key += [self.method, self._gelu, gate.scoring_func, gate.topk_method, gate.top_k, gate.n_group, gate.topk_group,
-                gate.norm_topk_prob, gate.routed_scaling_factor]
-        if self._native is not None and self._native[0] == key:
-            return self._native[1]
-        self._native = None
         if gate.top_k != cfg.num_experts_per_tok:
             return None
-        w3 = gate._split_weight(w)
-        d = N.Layer(struct_bytes=C.sizeof(N.Layer), act=int(self._gelu), experts=E, top_k=gate.top_k,
+        w3, pairs = gate._split_weight(w), {"w13": None, "w2": None}
+        for n in pairs:
+            if self.method == "w4a16":
+                pairs[n] = self._pairs(n, "_scale", "_zero")
+            elif self.method == "w4a8":
+                if not self._raw_nibbles_ok(n):
+                    return None
+                pairs[n] = self._pairs(n)
+        key = [t.data_ptr() for t in tensors] + [w3.data_ptr()] + [N.ptr(t) for t in pairs.values()]
+        key += [self.method, self._gelu, gate.scoring_func, gate.top_k, gate.n_group, gate.topk_group, gate.norm_topk_prob,
+                gate.routed_scaling_factor]
+        if self._native is not None and self._native[0] == key:
+            return self._native[1]
+        d = N.Layer(struct_bytes=C.sizeof(N.Layer), method=("fp8_block", "w4a16", "w4a8").index(self.method),
+                    act=int(self._gelu), experts=E, top_k=gate.top_k,
                     n_group=gate.n_group, topk_group=gate.topk_group, scoring=0 if gate.scoring_func == "sigmoid" else 1,
                     norm_topk_prob=1 if gate.norm_topk_prob else 0, scaling=float(gate.routed_scaling_factor),
                     router_rows=w3.shape[0], hidden=H, inter=I,
                     router_w3=N.ptr(w3), router_bias=N.ptr(bias), status=N.ptr(self._status))
-        for n in ("w13", "w2"):
-            if self.method == "fp8_block":
-                d.method, parts = 0, (bufs[n + "_weight"], bufs[n + "_weight_scale"], None)
-            elif self.method == "w4a16":
-                d.method, parts = 1, (bufs[n + "_qweight"], None, self._pairs(n, "_scale", "_zero"))
-            else:
-                if not self._raw_nibbles_ok(n):
-                    return None
-                d.method, parts = 2, (bufs[n + "_qweight"], bufs[n + "_weight_scale"], self._pairs(n))
-            for suffix, t in zip(("", "_scale", "_pairs"), parts):
-                setattr(d, n + suffix, N.ptr(t))
+        for n in pairs:
+            setattr(d, n, N.ptr(bufs[n + ("_weight" if self.method == "fp8_block" else "_qweight")]))
+            setattr(d, n + "_scale", N.ptr(bufs.get(n + "_weight_scale")))
+            setattr(d, n + "_pairs", N.ptr(pairs[n]))
         keep = [w3]
         if self.n_shared:
             if self._shared_stream is None:

@@ -177,3 +177,39 @@ def test_layer_names_an_unsupported_router(layer_host, name, value):
     layer, x, lib = layer_host(config={name: value})
     with pytest.raises(NotImplementedError, match=value if name == "topk_method" else "scoring"):
         layer(x)
+
+
+def test_layer_takes_weights_made_under_inference_mode(layer_host):
+    """Inference tensors have no version to compare."""
+    layer, x, lib = layer_host()
+    with torch.inference_mode():
+        for name in ("w13_weight", "w13_weight_scale", "w2_weight", "w2_weight_scale"):
+            setattr(layer, name, getattr(layer, name).clone())
+    layer(x)
+    layer(x)
+    assert lib.names().count("b200moe_layer_forward") == 2
+
+
+def test_layer_structure_follows_weights_and_settings(layer_host):
+    """What the library reads in a pass is what the layer holds at that moment."""
+    from ctypes import POINTER, cast
+    from llm_kernels_b200 import _native as N
+    seen = []
+    layer, x, lib = layer_host("w4a16", b200moe_layer_forward=lambda d, *a: seen.append(N.Layer.from_buffer_copy(cast(d, POINTER(N.Layer))[0])) or 0)
+    layer(x)
+    layer(x)
+    assert bytes(seen[0]) == bytes(seen[1])
+    layer.w2_zero += 1                                     # in place: another copy of the pairs
+    old = layer.w13_qweight
+    layer.w13_qweight = old.clone()
+    layer.gate.routed_scaling_factor = 3.5
+    layer.gate.weight.data.add_(1.0)
+    with torch.no_grad():
+        layer.gate.weight.add_(1.0)
+    layer(x)
+    d = seen[2]
+    assert d.w13 == layer.w13_qweight.data_ptr() != old.data_ptr() and d.scaling == 3.5
+    assert d.w2 == layer.w2_qweight.data_ptr() and d.router_bias == layer.gate.e_score_correction_bias.data_ptr()
+    assert torch.equal(layer._pairs("w2", "_scale", "_zero")[..., 1], layer.w2_zero.transpose(1, 2))
+    assert d.w2_pairs == layer._pairs("w2", "_scale", "_zero").data_ptr() and d.router_w3 == layer.gate._w3.data_ptr()
+    assert torch.equal(layer.gate._w3[:8].float().view(8, 3, 256).sum(1), layer.gate.weight)
