@@ -296,9 +296,8 @@ class DeepseekV3MoE(nn.Module):
         self._buffers_cache = {}
         self._status = torch.zeros(1, dtype=torch.int32, device=dev)
         self._last_recv_rows = None
-        self._last, self._last_tokens = None, 0
+        self._last, self._last_pass = None, None
         self._native = None               # (key, structure, its address, what it points to) of _describe
-        self._workspace = None
         # Optional per-stage timing: set to a list and every forward appends
         # (stage name, CUDA event recorded when the stage's launches were queued).
         self.stage_events = None
@@ -389,6 +388,7 @@ class DeepseekV3MoE(nn.Module):
             y = self._forward_native(hidden_states)
             if y is not None:
                 return y
+        self._last_pass = None
         orig_shape = hidden_states.shape
         self._mark("start")
         topk_idx, topk_weight = self.gate(hidden_states)
@@ -481,23 +481,25 @@ class DeepseekV3MoE(nn.Module):
         if self._describe(x) is None:
             return None
         lib, desc = N.lib(), self._native[2]
-        need = lib.b200moe_layer_workspace_bytes(desc, T)
-        ws = self._workspace
-        if ws is None or ws.numel() < need:
-            ws = self._workspace = torch.empty(need, dtype=torch.uint8, device=self._dev)
+        # Every pass has a workspace of its own: passes on other streams or threads and captured graphs may run beside it.
+        # The last one is only kept for time_expert_gemms; it is let go first, so that this pass can have the same memory.
+        self._last = self._last_pass = None
+        ws = torch.empty(lib.b200moe_layer_workspace_bytes(desc, T), dtype=torch.uint8, device=self._dev)
         y = torch.empty_like(x)
         N.check(lib.b200moe_layer_forward(desc, x.data_ptr(), y.data_ptr(), T, ws.data_ptr(), ws.numel(), N.stream()))
-        self._last_recv_rows, self._last = T * self.num_experts_per_tok, None
-        self._last_tokens = T
+        self._last_recv_rows = T * self.num_experts_per_tok
+        if self.method == "fp8_block":
+            self._last_pass = (self._native, ws, T)
         return y
 
     def _last_rows(self):
         """(permuted rows, row count, group table, weight indices) of the last forward."""
-        if self._last is None and self._last_tokens:
+        if self._last is None and self._last_pass is not None:
+            native, ws, T = self._last_pass
             send, seg = C.c_int64(), C.c_int64()
-            H, S, E = self.config.hidden_size, self._last_recv_rows, self.config.n_routed_experts
-            N.check(N.lib().b200moe_layer_workspace_layout(self._native[2], self._last_tokens, C.byref(send), C.byref(seg)))
-            ws, rec = self._workspace, self._record_bytes(H)
+            E, H, _ = self._sizes
+            S, rec = T * native[1].top_k, self._record_bytes(H)
+            N.check(N.lib().b200moe_layer_workspace_layout(native[2], T, C.byref(send), C.byref(seg)))
             self._last = (ws[send.value:send.value + S * rec].view(S, rec), S,
                           ws[seg.value:seg.value + 8 * (E + 1)].view(torch.int64), None)
         return self._last
@@ -529,7 +531,6 @@ class DeepseekV3MoE(nn.Module):
             graph.replay()
             return static_out
         run.graph, run.static_input, run.static_output = graph, static_in, static_out
-        run.workspace = self._workspace     # the graph's kernels keep using it, whatever later passes allocate
         return run
 
     # the reference's unfused entry point routes to the same pipeline

@@ -213,3 +213,42 @@ def test_layer_structure_follows_weights_and_settings(layer_host):
     assert torch.equal(layer._pairs("w2", "_scale", "_zero")[..., 1], layer.w2_zero.transpose(1, 2))
     assert d.w2_pairs == layer._pairs("w2", "_scale", "_zero").data_ptr() and d.router_w3 == layer.gate._w3.data_ptr()
     assert torch.equal(layer.gate._w3[:8].float().view(8, 3, 256).sum(1), layer.gate.weight)
+
+
+def _twice(layer, x, lib, entry, note):
+    """Runs a second pass of the layer in the middle of the first one's call of `entry`; returns what `note` made of the
+    arguments of both, the outer one first."""
+    seen = []
+
+    def outer(*args):
+        seen.append(note(*args))
+        if len(seen) == 1:
+            layer(x)
+        return 0
+    lib.on[entry] = outer
+    layer(x)
+    return seen
+
+
+def test_layer_passes_that_overlap_have_workspaces_of_their_own(layer_host):
+    """Another stream or thread, or a captured graph, can be in the middle of a pass."""
+    layer, x, lib = layer_host()
+    a, b = _twice(layer, x, lib, "b200moe_layer_forward", lambda d, x, y, T, ws, nbytes, stream: range(ws, ws + nbytes))
+    assert a.stop <= b.start or b.stop <= a.start
+
+
+def test_layer_keeps_the_last_rows_for_the_gemm_timing(layer_host):
+    """_last_rows describes the last pass, whichever path it took."""
+    layer, x, lib = layer_host()
+
+    def layout(d, T, send, seg):
+        send._obj.value, seg._obj.value = 0, 3584
+        return 0
+    lib.on["b200moe_layer_workspace_layout"] = layout
+    layer(x)
+    buf, rows, seg, widx = layer._last_rows()
+    assert rows == 8 and buf.shape == (8, 272) and seg.shape == (9,) and widx is None
+    layer.stage_events = []
+    layer._mark = lambda name: None
+    layer(x)
+    assert layer._last_rows()[0] is layer._last[0] and layer._last_rows()[0].data_ptr() != buf.data_ptr()
