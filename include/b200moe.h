@@ -466,7 +466,8 @@ typedef struct b200moe_layer {
   const void *w2, *w2_scale, *w2_pairs;
   int64_t shared_inter;              /* width of the shared experts, 0 = none */
   const void *shared_w13, *shared_w2;        /* bf16 [2*shared_inter, hidden], [hidden, shared_inter] */
-  void *side_stream, *fork_event, *join_event;   /* cudaStream_t / cudaEvent_t of the caller (shared experts only) */
+  void* side_stream;                 /* cudaStream_t on which the shared experts' gate/up runs beside the routed path */
+  void *fork_event, *join_event;     /* not read: every pass orders the two streams with events of its own */
   int32_t* status;                   /* device status word of the GEMMs, may be NULL */
 } b200moe_layer;
 /* Bytes of workspace a pass of T tokens needs (256-byte aligned); -1 for a bad descriptor. */

@@ -69,6 +69,43 @@ extern "C" int b200moe_layer_workspace_layout(const b200moe_layer* L, int64_t T,
   return B200MOE_OK;
 }
 
+// A side stream's part in one pass, with events of its own, since other passes may be using the same side stream.
+class SideWork {
+ public:
+  explicit SideWork(cudaStream_t main) : main_(main) {}
+  ~SideWork() {
+    if (fork_) cudaEventDestroy(fork_);      // released by the runtime once the work recorded in them is through
+    if (done_) cudaEventDestroy(done_);
+  }
+  int fork(cudaStream_t side) {
+    side_ = side;
+    if (int rc = check(cudaEventCreateWithFlags(&fork_, cudaEventDisableTiming))) return rc;
+    if (int rc = check(cudaEventCreateWithFlags(&done_, cudaEventDisableTiming))) return rc;
+    if (int rc = check(cudaEventRecord(fork_, main_))) return rc;
+    if (int rc = check(cudaStreamWaitEvent(side_, fork_, 0))) return rc;
+    forked_ = true;
+    return B200MOE_OK;
+  }
+  int done() {                               // what the side stream holds now is what the pass waits for
+    recorded_ = true;
+    return check(cudaEventRecord(done_, side_));
+  }
+  int join() {
+    if (!forked_) return B200MOE_OK;
+    forked_ = false;
+    if (!recorded_) if (int rc = done()) return rc;
+    return check(cudaStreamWaitEvent(main_, done_, 0));
+  }
+
+ private:
+  static int check(cudaError_t e) {
+    return e == cudaSuccess ? B200MOE_OK : fail(B200MOE_LAUNCH_FAILED, "layer_forward: side stream: %s", cudaGetErrorString(e));
+  }
+  cudaStream_t main_, side_ = nullptr;
+  cudaEvent_t fork_ = nullptr, done_ = nullptr;
+  bool forked_ = false, recorded_ = false;
+};
+
 #define STEP(call) do { if (int rc_ = (call)) return rc_; } while (0)
 
 extern "C" int b200moe_layer_forward(const b200moe_layer* Lp, const void* x, void* y, int64_t T, void* workspace,
@@ -93,20 +130,17 @@ extern "C" int b200moe_layer_forward(const b200moe_layer* Lp, const void* x, voi
   void* h = ws + p.h;
   auto* h_s = reinterpret_cast<float*>(ws + p.h_s);
   void* down = ws + p.down;
-  cudaStream_t st = as_stream(stream);
+  SideWork side(as_stream(stream));
 
   STEP(b200moe_router_logits_bf16x3(x, L.router_w3, part, T, H, L.router_rows, p.ksplits, stream));
   STEP(b200moe_router_select(part, p.ksplits, L.router_rows, L.router_bias, T, L.experts, L.top_k, L.n_group, L.topk_group,
                              L.scoring, L.norm_topk_prob, L.scaling, idx, wts, stream));
   if (L.shared_inter) {
     // gate/up of the shared experts needs only x: on the side stream it fills the SMs the routed path leaves idle
-    cudaStream_t side = as_stream(L.side_stream);
-    cudaEvent_t fork = static_cast<cudaEvent_t>(L.fork_event), join = static_cast<cudaEvent_t>(L.join_event);
-    cudaEventRecord(fork, st);
-    cudaStreamWaitEvent(side, fork, 0);
+    STEP(side.fork(as_stream(L.side_stream)));
     STEP(b200moe_grouped_gemm_bf16(x, 2 * H, L.shared_w13, ws + p.shared_h, B200MOE_BF16, 2 * L.shared_inter, T,
                                    2 * L.shared_inter, H, 1, 1, nullptr, nullptr, L.act ? 5 : 2, L.status, nullptr, L.side_stream));
-    cudaEventRecord(join, side);
+    STEP(side.done());
   }
   STEP(b200moe_route_metadata(idx, p.S, L.experts, reinterpret_cast<int64_t*>(ws + p.ids), dst, seg, ws + p.scratch,
                               static_cast<size_t>(p.scratch_bytes), stream));
@@ -137,7 +171,7 @@ extern "C" int b200moe_layer_forward(const b200moe_layer* Lp, const void* x, voi
   }
   STEP(b200moe_post_reorder(down, B200MOE_BF16, y, dst, idx, wts, 0, E - 1, T, L.top_k, H, stream));
   if (L.shared_inter) {
-    cudaStreamWaitEvent(st, static_cast<cudaEvent_t>(L.join_event), 0);
+    STEP(side.join());
     STEP(b200moe_grouped_gemm_bf16(ws + p.shared_h, 2 * L.shared_inter, L.shared_w2, y, B200MOE_BF16, 2 * H, T, H, L.shared_inter,
                                    1, 1, nullptr, nullptr, 3, L.status, nullptr, stream));
   }

@@ -457,13 +457,9 @@ class DeepseekV3MoE(nn.Module):
         if self.n_shared:
             if self._shared_stream is None:
                 self._shared_stream = torch.cuda.Stream(device=self._dev)
-            ev = [torch.cuda.Event(), torch.cuda.Event()]
-            for e in ev:
-                e.record()                      # creates the handle
             d.shared_inter = bufs["shared_w2"].shape[2]
             d.shared_w13, d.shared_w2 = N.ptr(bufs["shared_w13"]), N.ptr(bufs["shared_w2"])
-            d.side_stream, d.fork_event, d.join_event = self._shared_stream.cuda_stream, ev[0].cuda_event, ev[1].cuda_event
-            keep += ev
+            d.side_stream = self._shared_stream.cuda_stream
         self._native = (key, d, C.addressof(d), keep)
         return d
 

@@ -252,3 +252,18 @@ def test_layer_keeps_the_last_rows_for_the_gemm_timing(layer_host):
     layer._mark = lambda name: None
     layer(x)
     assert layer._last_rows()[0] is layer._last[0] and layer._last_rows()[0].data_ptr() != buf.data_ptr()
+
+
+def test_layer_passes_that_overlap_share_no_events(layer_host, monkeypatch):
+    """With shared experts a pass orders two streams; an event recorded again by another pass would order the wrong work.
+    The library makes them, so none is handed over."""
+    from ctypes import POINTER, cast
+    from types import SimpleNamespace
+    from llm_kernels_b200 import _native as N
+    handles = iter(range(1, 100))
+    monkeypatch.setattr(torch.cuda, "Stream", lambda device=None: SimpleNamespace(cuda_stream=next(handles)))
+    monkeypatch.setattr(torch.cuda, "Event", lambda: SimpleNamespace(cuda_event=next(handles), record=lambda: None))
+    layer, x, lib = layer_host(config={"n_shared_experts": 1})
+    a, b = _twice(layer, x, lib, "b200moe_layer_forward", lambda d, *rest: N.Layer.from_buffer_copy(cast(d, POINTER(N.Layer))[0]))
+    assert a.side_stream == b.side_stream == 1 and a.shared_inter == 128
+    assert not {a.fork_event, a.join_event} & {b.fork_event, b.join_event} - {None}
