@@ -69,11 +69,13 @@ extern "C" int b200moe_layer_workspace_layout(const b200moe_layer* L, int64_t T,
   return B200MOE_OK;
 }
 
-// A side stream's part in one pass, with events of its own, since other passes may be using the same side stream.
+// A side stream's part in one pass: forked from the pass's stream and joined to it on every way out, with events of its own,
+// since other passes may be using the same side stream.
 class SideWork {
  public:
   explicit SideWork(cudaStream_t main) : main_(main) {}
   ~SideWork() {
+    join();
     if (fork_) cudaEventDestroy(fork_);      // released by the runtime once the work recorded in them is through
     if (done_) cudaEventDestroy(done_);
   }
