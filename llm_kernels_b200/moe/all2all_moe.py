@@ -297,7 +297,7 @@ class DeepseekV3MoE(nn.Module):
         self._status = torch.zeros(1, dtype=torch.int32, device=dev)
         self._last_recv_rows = None
         self._last, self._last_pass = None, None
-        self._native = None               # (key, structure, its address, what it points to) of _describe
+        self._native = None               # what _describe returned last
         # Optional per-stage timing: set to a list and every forward appends
         # (stage name, CUDA event recorded when the stage's launches were queued).
         self.stage_events = None
@@ -413,9 +413,9 @@ class DeepseekV3MoE(nn.Module):
                          or nn.modules.module._global_forward_pre_hooks))
 
     def _describe(self, x):
-        """The layer as the C structure of b200moe_layer_forward, or None where that call does not apply to x.  `key` is
-        everything the structure was made from, pointers and settings; it is rebuilt when one of them differs from the last
-        pass's.  What a pass needs of its tensors is looked at in every pass."""
+        """(key, the layer as the C structure of b200moe_layer_forward, its address, what it points to), or None where that
+        call does not apply to x.  `key` is everything the structure was made from, pointers and settings; it is rebuilt
+        when one of them differs from the last pass's.  What a pass needs of its tensors is looked at in every pass."""
         gate, bufs, cfg = self.gate, self._buffers, self.config
         if gate.scoring_func not in ("sigmoid", "softmax") or gate.topk_method != "noaux_tc":      # the gate says why
             return None
@@ -441,8 +441,9 @@ class DeepseekV3MoE(nn.Module):
         key = [t.data_ptr() for t in tensors] + [w3.data_ptr()] + [N.ptr(t) for t in pairs.values()]
         key += [self.method, self._gelu, gate.scoring_func, gate.top_k, gate.n_group, gate.topk_group, gate.norm_topk_prob,
                 gate.routed_scaling_factor]
-        if self._native is not None and self._native[0] == key:
-            return self._native[1]
+        native = self._native
+        if native is not None and native[0] == key:
+            return native
         d = N.Layer(struct_bytes=C.sizeof(N.Layer), method=("fp8_block", "w4a16", "w4a8").index(self.method),
                     act=int(self._gelu), experts=E, top_k=gate.top_k,
                     n_group=gate.n_group, topk_group=gate.topk_group, scoring=0 if gate.scoring_func == "sigmoid" else 1,
@@ -453,15 +454,14 @@ class DeepseekV3MoE(nn.Module):
             setattr(d, n, N.ptr(bufs[n + ("_weight" if self.method == "fp8_block" else "_qweight")]))
             setattr(d, n + "_scale", N.ptr(bufs.get(n + "_weight_scale")))
             setattr(d, n + "_pairs", N.ptr(pairs[n]))
-        keep = [w3]
         if self.n_shared:
             if self._shared_stream is None:
                 self._shared_stream = torch.cuda.Stream(device=self._dev)
             d.shared_inter = bufs["shared_w2"].shape[2]
             d.shared_w13, d.shared_w2 = N.ptr(bufs["shared_w13"]), N.ptr(bufs["shared_w2"])
             d.side_stream = self._shared_stream.cuda_stream
-        self._native = (key, d, C.addressof(d), keep)
-        return d
+        self._native = native = (key, d, C.addressof(d), (w3, pairs))
+        return native
 
     def _forward_native(self, hidden_states):
         """One pass of a single-rank layer as one host call (b200moe_layer_forward); None where the layer's state needs
@@ -474,9 +474,10 @@ class DeepseekV3MoE(nn.Module):
                 T * self.num_experts_per_tok > self.w4_fused_rows_per_group * self.experts_per_rank):
             return None
         assert not self.gate.training
-        if self._describe(x) is None:
+        native = self._describe(x)          # held to the end of the pass: another thread's pass may build a new one
+        if native is None:
             return None
-        lib, desc = N.lib(), self._native[2]
+        lib, desc = N.lib(), native[2]
         # Every pass has a workspace of its own: passes on other streams or threads and captured graphs may run beside it.
         # The last one is only kept for time_expert_gemms; it is let go first, so that this pass can have the same memory.
         self._last = self._last_pass = None
@@ -485,7 +486,7 @@ class DeepseekV3MoE(nn.Module):
         N.check(lib.b200moe_layer_forward(desc, x.data_ptr(), y.data_ptr(), T, ws.data_ptr(), ws.numel(), N.stream()))
         self._last_recv_rows = T * self.num_experts_per_tok
         if self.method == "fp8_block":
-            self._last_pass = (self._native, ws, T)
+            self._last_pass = (native, ws, T)
         return y
 
     def _last_rows(self):

@@ -267,3 +267,28 @@ def test_layer_passes_that_overlap_share_no_events(layer_host, monkeypatch):
     a, b = _twice(layer, x, lib, "b200moe_layer_forward", lambda d, *rest: N.Layer.from_buffer_copy(cast(d, POINTER(N.Layer))[0]))
     assert a.side_stream == b.side_stream == 1 and a.shared_inter == 128
     assert not {a.fork_event, a.join_event} & {b.fork_event, b.join_event} - {None}
+
+
+def test_layer_pass_keeps_what_its_structure_points_to(layer_host):
+    """A pass after a change of the weights, in another thread, must not free what a pass in flight reads: the structure
+    itself, the split router weight, the pairs."""
+    import gc
+    import weakref
+    layer, x, lib = layer_host("w4a16")
+    layer(x)
+    held = [weakref.ref(layer._native[1]), *(weakref.ref(t) for t in (layer.gate._w3, layer._pairs("w2", "_scale", "_zero")))]
+    alive = []
+
+    def note(*args):
+        if alive:
+            gc.collect()
+            alive.append([r() is not None for r in held])
+        else:
+            alive.append(None)
+            layer.w2_zero += 1
+            with torch.no_grad():
+                layer.gate.weight.add_(1.0)
+    _twice(layer, x, lib, "b200moe_layer_forward", note)
+    assert alive[1] == [True] * 3
+    gc.collect()
+    assert [r() is not None for r in held] == [False] * 3
