@@ -193,6 +193,7 @@ class DeepseekV3MoE(nn.Module):
     """
 
     METHODS = ("fp8_block", "w4a16", "w4a8")
+    _native = _last_pass = _layout = None        # of a layer that an earlier version has saved as a whole: no one-call passes
 
     def __init__(self, config, device=None):
         super().__init__()
@@ -301,6 +302,10 @@ class DeepseekV3MoE(nn.Module):
         # Optional per-stage timing: set to a list and every forward appends
         # (stage name, CUDA event recorded when the stage's launches were queued).
         self.stage_events = None
+
+    def __getstate__(self):
+        """Copies and pickles leave out what belongs to the passes of this object: raw pointers."""
+        return dict(self.__dict__, _native=None, _last_pass=None)
 
     def _mark(self, name):
         if self.stage_events is not None:
@@ -417,8 +422,8 @@ class DeepseekV3MoE(nn.Module):
         call does not apply to x.  `key` is everything the structure was made from, pointers and settings; it is rebuilt
         when one of them differs from the last pass's.  What a pass needs of its tensors is looked at in every pass."""
         gate, bufs, cfg = self.gate, self._buffers, self.config
-        if gate.scoring_func not in ("sigmoid", "softmax") or gate.topk_method != "noaux_tc":      # the gate says why
-            return None
+        if self._layout is None or gate.scoring_func not in ("sigmoid", "softmax") or gate.topk_method != "noaux_tc":
+            return None                                                                    # the gate says what it lacks
         w, bias = gate.weight, gate.e_score_correction_bias
         E, H, I = self._sizes
         # tensors of another type, shape or stride than the layer's own: the separate calls check them one by one

@@ -292,3 +292,26 @@ def test_layer_pass_keeps_what_its_structure_points_to(layer_host):
     assert alive[1] == [True] * 3
     gc.collect()
     assert [r() is not None for r in held] == [False] * 3
+
+
+@pytest.mark.parametrize("method", ["fp8_block", "w4a8"])
+def test_layer_can_be_copied_after_a_pass(layer_host, method):
+    import copy
+    import io
+    layer, x, lib = layer_host(method)
+    layer(x)
+    file = io.BytesIO()
+    torch.save(layer, file)
+    file.seek(0)
+    for twin in (copy.deepcopy(layer), torch.load(file, weights_only=False)):
+        assert twin._native is None and twin._last_pass is None
+        twin(x)
+        assert twin._native[1].w13 == next(iter(twin.buffers())).data_ptr() != layer._native[1].w13
+
+
+def test_layer_saved_by_an_earlier_version_runs(layer_host):
+    layer, x, lib = layer_host()
+    for name in ("_native", "_last_pass", "_layout", "_sizes"):
+        del layer.__dict__[name]
+    layer(x)
+    assert lib.names().count("b200moe_grouped_gemm_fp8") == 2
