@@ -388,11 +388,9 @@ class DeepseekV3MoE(nn.Module):
     # ---- forward ---------------------------------------------------------------------
     @torch.no_grad()
     def forward(self, hidden_states):
-        # the one call takes no GEMM options and marks no stages
-        if self.ep_size == 1 and self.stage_events is None and G._opts() is None and self._runs_as_written():
-            y = self._forward_native(hidden_states)
-            if y is not None:
-                return y
+        y = self._forward_native(hidden_states)
+        if y is not None:
+            return y
         self._last_pass = None
         orig_shape = hidden_states.shape
         self._mark("start")
@@ -468,20 +466,27 @@ class DeepseekV3MoE(nn.Module):
         self._native = native = (key, d, C.addressof(d), (w3, pairs))
         return native
 
-    def _forward_native(self, hidden_states):
-        """One pass of a single-rank layer as one host call (b200moe_layer_forward); None where the layer's state needs
-        the separate calls (stages that expand the int4 weights first)."""
+    def _native_for(self, x):
+        """What _describe gives, where a pass over the contiguous tensor x is one call; else None: the one call takes no
+        GEMM options, marks no stages and expands no int4 weights first."""
+        if self.ep_size != 1 or self.stage_events is not None or G._opts() is not None or not self._runs_as_written():
+            return None
         H = self.config.hidden_size
-        x = hidden_states if hidden_states.is_contiguous() else hidden_states.contiguous()
         T = x.numel() // H
         if x.dtype != torch.bfloat16 or T == 0 or x.shape[-1] != H or (
                 self.method != "fp8_block" and
                 T * self.num_experts_per_tok > self.w4_fused_rows_per_group * self.experts_per_rank):
             return None
         assert not self.gate.training
-        native = self._describe(x)          # held to the end of the pass: another thread's pass may build a new one
+        return self._describe(x)
+
+    def _forward_native(self, hidden_states):
+        """One pass of a single-rank layer as one host call (b200moe_layer_forward); None where it takes separate ones."""
+        x = hidden_states if hidden_states.is_contiguous() else hidden_states.contiguous()
+        native = self._native_for(x)        # held to the end of the pass: another thread's pass may build a new one
         if native is None:
             return None
+        T = x.numel() // self.config.hidden_size
         lib, desc = N.lib(), native[2]
         # Every pass has a workspace of its own: passes on other streams or threads and captured graphs may run beside it.
         # The last one is only kept for time_expert_gemms; it is let go first, so that this pass can have the same memory.
@@ -511,7 +516,8 @@ class DeepseekV3MoE(nn.Module):
         returns `run(x) -> y` (single-rank layers).  The layer's launch sequence is fixed and reads nothing
         back to the host.  For small batches, where the step is a dozen launches of a few microseconds
         each, replaying the graph removes the per-launch host cost.  `y` is a static buffer that the next
-        `run` overwrites; a device-side timeout still shows up in `check_status()`.  Restricted to
+        `run` overwrites; a device-side timeout still shows up in `check_status()`.  Weights may be loaded in place between
+        runs: where the graph holds operands made from them, `run` captures the pass again.  Restricted to
         ep_size == 1: an expert-parallel step interleaves NCCL collectives with kernels that store into
         peer-mapped buffers, and capturing that sequence is not supported here."""
         assert self.ep_size == 1, "make_graphed supports ep_size == 1"
@@ -524,16 +530,38 @@ class DeepseekV3MoE(nn.Module):
                 self(static_in)
         cur.wait_stream(side)
         torch.cuda.synchronize(self._dev)
-        graph = torch.cuda.CUDAGraph()
-        with torch.cuda.graph(graph):
-            static_out = self(static_in)
+
+        def capture():
+            run.state = self._baked_in(static_in)
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph):
+                run.latest = self(static_in)
+            run.graph = graph
+            # read by address in every replay, whatever later passes put in their place
+            run.operands = (self._native, getattr(self.gate, "_w3", None), getattr(self.gate, "_partials", None),
+                            list(self._buffers_cache.values()))
 
         def run(x: torch.Tensor) -> torch.Tensor:
             static_in.copy_(x, non_blocking=True)
-            graph.replay()
-            return static_out
-        run.graph, run.static_input, run.static_output = graph, static_in, static_out
+            if self._baked_in(static_in) != run.state:
+                torch.cuda.synchronize(self._dev)            # replays of the old graph are through
+                capture()
+            run.graph.replay()
+            if run.latest is not run.static_output:
+                run.static_output.copy_(run.latest)
+            return run.static_output
+        capture()
+        run.static_input, run.static_output = static_in, run.latest
         return run
+
+    @torch.no_grad()
+    def _baked_in(self, x):
+        """What a captured pass over x has taken for granted: the addresses and settings of a one-call pass (the router's
+        split weight and the int4 pairs are new tensors once their sources have changed), or every tensor's state."""
+        native = self._native_for(x)
+        if native is not None:
+            return native[0]
+        return [(t.data_ptr(), 0 if t.is_inference() else t._version) for t in (*self.parameters(), *self.buffers())]
 
     # the reference's unfused entry point routes to the same pipeline
     def moe_infer(self, x, topk_ids, topk_weight):

@@ -42,3 +42,56 @@ def test_refused_pass_leaves_the_side_stream_joined():
     layer.w13_weight = w
     assert torch.isfinite(layer(x)).all()
     layer.check_status()
+
+
+@pytest.mark.parametrize("method", ["fp8_block", "w4a16", "w4a8"])
+@pytest.mark.parametrize("what", ["router", "expert"])
+def test_graph_follows_weights_loaded_in_place(method, what):
+    """The split router weight and the int4 pairs are made from the weights: a replay must not go on with the old ones, nor
+    read memory that an eager pass after the change has freed."""
+    layer, x = _layer(method)
+    other, _ = _layer(method, seed=4)
+    run = layer.make_graphed(x)
+    out = run.static_output
+    before = run(x).clone()
+    if what == "router":
+        with torch.no_grad():
+            layer.gate.weight.copy_(other.gate.weight)
+    else:
+        for name, t in layer.named_buffers():
+            t.copy_(dict(other.named_buffers())[name])
+    got = run(x)
+    assert got is out
+    got = got.clone()
+    want = layer(x).clone()
+    assert torch.equal(got, want) and not torch.equal(got, before)
+    junk = [torch.full((1 << 20,), float("nan"), device=x.device) for _ in range(8)]      # freed memory would be taken by these
+    assert torch.equal(run(x), want) and len(junk) == 8
+    layer.check_status()
+
+
+@pytest.mark.parametrize("shared", [0, 1])
+def test_passes_of_two_threads_and_streams(shared):
+    """Two threads, each on a stream of its own, run one layer on different tokens; a graph of it is replayed beside them."""
+    import threading
+    layer, x = _layer(shared=shared, tokens=96)
+    xs = [x, x.flip(1).contiguous(), x.roll(5, 1).contiguous()]
+    want = [layer(t).clone() for t in xs]
+    run = layer.make_graphed(xs[2])
+    torch.cuda.synchronize()
+    wrong = []
+
+    def work(i):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(50):
+                y = run(xs[2]) if i == 2 else layer(xs[i])
+                torch.cuda.current_stream().synchronize()
+                if not torch.equal(y, want[i]):
+                    wrong.append(i)
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(3)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
+    layer.check_status()
