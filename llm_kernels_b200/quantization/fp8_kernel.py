@@ -52,18 +52,6 @@ def weight_dequant(x: torch.Tensor, s: torch.Tensor, block_size: int = 128) -> t
     return y
 
 
-_workspaces = {}
-
-
-def _workspace(device, nbytes: int) -> torch.Tensor:
-    """One scratch buffer per device and stream."""
-    key = (device, N.stream())
-    ws = _workspaces.get(key)
-    if ws is None or ws.numel() < nbytes:
-        ws = _workspaces[key] = torch.empty(nbytes, dtype=torch.uint8, device=device)
-    return ws
-
-
 def _split_k(M: int, Nn: int, K: int) -> int:
     """K splits for a small-M product: enough tiles to occupy the 148 SMs, every split non-empty."""
     if M > 128:
@@ -74,6 +62,12 @@ def _split_k(M: int, Nn: int, K: int) -> int:
     while ks > 1 and -(-kb // ks) * (ks - 1) >= kb:
         ks -= 1
     return ks
+
+
+def _partials(a: torch.Tensor, n: int) -> torch.Tensor:
+    """Scratch of one call's K splits.  Nothing is kept between calls: the caching allocator orders its memory by stream and
+    gives a captured call memory of its graph, and calls of two threads on one stream must not meet in one buffer."""
+    return torch.empty(n, dtype=torch.float32, device=a.device)
 
 
 def fp8_gemm(a: torch.Tensor, a_s: torch.Tensor, b: torch.Tensor, b_s: torch.Tensor,
@@ -93,10 +87,10 @@ def fp8_gemm(a: torch.Tensor, a_s: torch.Tensor, b: torch.Tensor, b_s: torch.Ten
     c = a.new_empty(*a.size()[:-1], Nn, dtype=out_dtype or torch.get_default_dtype())
     ks = _split_k(M, Nn, K) if ksplits is None else int(ksplits)
     if ks > 1 and M > 0:
-        part = _workspace(a.device, ks * M * Nn * 4)
+        part = _partials(a, ks * M * Nn)
         N.check(N.lib().b200moe_gemm_fp8_block_splitk(N.ptr(a), N.ptr(a_s), N.ptr(b), N.ptr(b_s), N.ptr(c),
                                                       N.dtype_code(c.dtype), M, Nn, K, ks, N.ptr(part),
-                                                      part.numel(), N.stream()))
+                                                      part.numel() * 4, N.stream()))
         return c
     N.check(N.lib().b200moe_gemm_fp8_block(N.ptr(a), N.ptr(a_s), N.ptr(b), N.ptr(b_s), N.ptr(c),
                                            N.dtype_code(c.dtype), M, Nn, K, N.stream()))

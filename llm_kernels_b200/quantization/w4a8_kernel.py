@@ -69,7 +69,7 @@ def w4a8_gemm(a: torch.Tensor, a_s: torch.Tensor, b: torch.Tensor, b_s: torch.Te
     """c[..., N] = a[..., K] (int8) . dequant(b)^T with per-K-block scales (reference :406-448).  Few rows (M <= 128) split
     the K loop over all SMs as fp8_gemm does: one m-tile alone kept N / 256 of them busy (M = 24, N = 4096, K = 7168)."""
     from ..moe.group_gemm_kernel import _opts, grouped_gemm_i8
-    from .fp8_kernel import _split_k, _workspace
+    from .fp8_kernel import _partials, _split_k
     assert a.is_contiguous() and b.is_contiguous(), 'Input tensors must be contiguous'
     assert a_s.is_contiguous() and b_s.is_contiguous(), 'Scaling factor tensors must be contiguous'
     assert b_s4.is_contiguous() and b_z4.is_contiguous(), 'Scaling factor and zero point tensors must be contiguous'
@@ -86,10 +86,10 @@ def w4a8_gemm(a: torch.Tensor, a_s: torch.Tensor, b: torch.Tensor, b_s: torch.Te
     if ks > 1 and _opts() is None and tuple(w8.shape) == (Nn, K) and a_s.shape[1] * 128 == K:
         N.require_cuda(a, a_s, b_s)
         assert a.dtype == torch.int8
-        part = _workspace(a.device, ks * M * Nn * 4)
+        part = _partials(a, ks * M * Nn)
         N.check(N.lib().b200moe_gemm_i8_block_splitk(N.ptr(a), N.ptr(a_s), N.ptr(w8), N.ptr(b_s), N.ptr(c),
-                                                     N.dtype_code(c.dtype), M, Nn, K, ks, N.ptr(part), part.numel(),
-                                                     N.stream()))
+                                                     N.dtype_code(c.dtype), M, Nn, K, ks, N.ptr(part),
+                                                     part.numel() * 4, N.stream()))
         return c
     grouped_gemm_i8(a.view(M, K), a_s, w8.unsqueeze(0), b_s.unsqueeze(0), None, None, c.view(M, Nn))
     return c

@@ -315,3 +315,26 @@ def test_layer_saved_by_an_earlier_version_runs(layer_host):
         del layer.__dict__[name]
     layer(x)
     assert lib.names().count("b200moe_grouped_gemm_fp8") == 2
+
+
+@pytest.mark.parametrize("kind", ["fp8", "w4a8"])
+def test_split_gemms_that_overlap_have_partials_of_their_own(host, monkeypatch, kind):
+    """The product and the sum of its splits are two launches: another thread's call can come between them."""
+    from llm_kernels_b200.quantization import fp8_kernel, w4a8_kernel
+    f8 = torch.float8_e4m3fn
+    seen = []
+
+    def call():
+        if kind == "w4a8":
+            return w4a8_kernel.w4a8_gemm(*_w4a8_operands(24, 1024, 1024, 8))
+        return fp8_kernel.fp8_gemm(torch.zeros(24, 1024, dtype=f8), torch.ones(24, 8), torch.zeros(256, 1024, dtype=f8), torch.ones(2, 8))
+
+    def outer(*args):
+        seen.append(range(args[10], args[10] + args[11]))
+        if len(seen) == 1:
+            call()
+        return 0
+    monkeypatch.setattr(host, "_lib", Recorder(b200moe_gemm_i8_block_splitk=outer, b200moe_gemm_fp8_block_splitk=outer))
+    call()
+    a, b = seen
+    assert len(a) == 8 * 24 * 256 * 4 and (a.stop <= b.start or b.stop <= a.start)
