@@ -95,3 +95,19 @@ def test_passes_of_two_threads_and_streams(shared):
         t.join()
     assert not wrong
     layer.check_status()
+
+
+@pytest.mark.parametrize("tokens", [40, 400])
+def test_w4a8_first_pass_can_be_captured(tokens):
+    """10 and 100 rows per expert: whether the weights fit the fused GEMMs is not known yet and cannot be asked during a
+    capture, so the graph expands them; the bits are the same."""
+    layer, x = _layer("w4a8", tokens=tokens)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = layer(x)
+    graph.replay()
+    torch.cuda.synchronize()
+    got = y.clone()
+    assert torch.equal(got, layer(x)) and layer._native is not None
+    layer.check_status()
