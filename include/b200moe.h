@@ -96,7 +96,10 @@ B200MOE_API int b200moe_gemm_fp8_block_splitk(const void* a, const float* a_s, c
                                   void* c, int c_dtype, int64_t M, int64_t N, int64_t K, int ksplits,
                                   float* partials, int64_t partials_bytes, void* stream);
 
-/* The same for int8 operands (the w4a8 product once its weights are int8, quantization/w4a8_kernel.py:406-448). */
+/* Both for int8 operands (the w4a8 product once its weights are int8, quantization/w4a8_kernel.py:406-448). */
+B200MOE_API int b200moe_gemm_i8_block(const void* a, const float* a_s, const void* b, const float* b_s,
+                          void* c, int c_dtype, int64_t M, int64_t N, int64_t K,
+                          void* stream);
 B200MOE_API int b200moe_gemm_i8_block_splitk(const void* a, const float* a_s, const void* b, const float* b_s,
                                  void* c, int c_dtype, int64_t M, int64_t N, int64_t K, int ksplits,
                                  float* partials, int64_t partials_bytes, void* stream);

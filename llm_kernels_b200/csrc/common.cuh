@@ -25,6 +25,10 @@ int check_launch(const char* what);
 // Opts a kernel in to `bytes` of dynamic shared memory on the current device, once per kernel and device.
 int set_dynamic_smem(const void* kernel, size_t bytes);
 
+// b200moe_grouped_gemm_bf16 (gemm_fp8.cu) on one group of all M rows, which needs no group table; a [M, K] contiguous.
+int dense_gemm_bf16(const void* a, const void* b, void* c, int64_t c_row_stride_bytes, int64_t M, int64_t N, int64_t K,
+                    int epilogue, int32_t* status_word, void* stream);
+
 #define B200MOE_REQUIRE(cond, status, ...)                 \
   do {                                                     \
     if (!(cond)) return ::b200moe::fail((status), __VA_ARGS__); \

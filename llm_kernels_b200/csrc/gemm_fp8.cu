@@ -674,23 +674,33 @@ static int launch_gemm(const void* a, int64_t a_stride, const void* b, GemmParam
 
 using namespace b200moe;
 
-extern "C" int b200moe_gemm_fp8_block(const void* a, const float* a_s, const void* b,
-                                      const float* b_s, void* c, int c_dtype, int64_t M,
-                                      int64_t N, int64_t K, void* stream) {
-  B200MOE_REQUIRE(a && a_s && b && b_s && c, B200MOE_BAD_ARG, "gemm_fp8_block: null pointer");
+template <int KIND>
+static int gemm_dense(const char* who, const void* a, const float* a_s, const void* b, const float* b_s, void* c, int c_dtype,
+                      int64_t M, int64_t N, int64_t K, void* stream) {
+  B200MOE_REQUIRE(a && a_s && b && b_s && c, B200MOE_BAD_ARG, "%s: null pointer", who);
   B200MOE_REQUIRE(M >= 0 && M < (int64_t(1) << 31) && N > 0 && K > 0 && K % 128 == 0 && N % 128 == 0 && N * K < (int64_t(1) << 40),
-                  B200MOE_BAD_SHAPE, "gemm_fp8_block: M=%lld N=%lld K=%lld (N and K must be multiples of 128)",
-                  (long long)M, (long long)N, (long long)K);
+                  B200MOE_BAD_SHAPE, "%s: M=%lld N=%lld K=%lld (N and K must be multiples of 128)",
+                  who, (long long)M, (long long)N, (long long)K);
   B200MOE_REQUIRE(c_dtype == B200MOE_F32 || c_dtype == B200MOE_F16 || c_dtype == B200MOE_BF16, B200MOE_BAD_DTYPE,
-                  "gemm_fp8_block: c dtype %d", c_dtype);
+                  "%s: c dtype %d", who, c_dtype);
   B200MOE_REQUIRE(aligned(a, 16) && aligned(b, 16) && aligned(c, 16), B200MOE_BAD_ALIGN,
-                  "gemm_fp8_block: Input tensors must be 16-byte aligned");
+                  "%s: Input tensors must be 16-byte aligned", who);
   if (M == 0) return B200MOE_OK;
   const int esz = c_dtype == B200MOE_F32 ? 4 : 2;
   GemmParams p{a_s, K / 128, b_s, c, N * esz, nullptr, 0, nullptr, nullptr, M,
                static_cast<int>(N), static_cast<int>(K), 1, 1, c_dtype, 0, nullptr, 1, 0, 0, nullptr, nullptr, 0, 0};
   const int64_t tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
-  return launch_gemm<kFp8>(a, K, b, p, tiles, as_stream(stream));
+  return launch_gemm<KIND>(a, K, b, p, tiles, as_stream(stream));
+}
+
+extern "C" int b200moe_gemm_fp8_block(const void* a, const float* a_s, const void* b, const float* b_s, void* c, int c_dtype,
+                                      int64_t M, int64_t N, int64_t K, void* stream) {
+  return gemm_dense<kFp8>("gemm_fp8_block", a, a_s, b, b_s, c, c_dtype, M, N, K, stream);
+}
+
+extern "C" int b200moe_gemm_i8_block(const void* a, const float* a_s, const void* b, const float* b_s, void* c, int c_dtype,
+                                     int64_t M, int64_t N, int64_t K, void* stream) {
+  return gemm_dense<kI8>("gemm_i8_block", a, a_s, b, b_s, c, c_dtype, M, N, K, stream);
 }
 
 namespace b200moe {
@@ -811,10 +821,9 @@ extern "C" int b200moe_grouped_gemm_fp8(const void* a, int64_t a_row_stride_byte
 
 // ---- int8 x int8 (w4a8 after the int4 -> int8 step) and bf16 x bf16 (w4a16 after dequantization) ----
 static int check_grouped_common(const char* who, const void* a, const void* b, const void* c,
-                                const int64_t* seg, int64_t a_stride, int64_t kbytes, int64_t M_total,
+                                int64_t a_stride, int64_t kbytes, int64_t M_total,
                                 int64_t N, int num_groups, int num_weights) {
-  // one group over all rows needs no table
-  B200MOE_REQUIRE(a && b && c && (seg || num_groups == 1), B200MOE_BAD_ARG, "%s: null pointer", who);
+  B200MOE_REQUIRE(a && b && c, B200MOE_BAD_ARG, "%s: null pointer", who);
   B200MOE_REQUIRE(M_total >= 0 && M_total < (int64_t(1) << 31) && N > 0 && N % 128 == 0 && kbytes > 0 && kbytes % 128 == 0,
                   B200MOE_BAD_SHAPE, "%s: M=%lld N=%lld (N must be a multiple of 128, K of 128 bytes)", who,
                   (long long)M_total, (long long)N);
@@ -832,7 +841,8 @@ extern "C" int b200moe_grouped_gemm_i8(const void* a, int64_t a_row_stride_bytes
                                        int64_t K, int num_groups, int num_weights,
                                        const int64_t* seg_indptr, const int64_t* weight_indices,
                                        int32_t* status_word, const b200moe_gemm_opts* opts, void* stream) {
-  if (int rc = check_grouped_common("grouped_gemm_i8", a, b, c, seg_indptr, a_row_stride_bytes, K, M_total, N,
+  B200MOE_REQUIRE(seg_indptr, B200MOE_BAD_ARG, "grouped_gemm_i8: null pointer");
+  if (int rc = check_grouped_common("grouped_gemm_i8", a, b, c, a_row_stride_bytes, K, M_total, N,
                                     num_groups, num_weights)) return rc;
   B200MOE_REQUIRE(a_s && b_s && a_s_row_stride >= K / 128, B200MOE_BAD_ARG, "grouped_gemm_i8: scales");
   B200MOE_REQUIRE(c_dtype == B200MOE_F32 || c_dtype == B200MOE_F16 || c_dtype == B200MOE_BF16, B200MOE_BAD_DTYPE,
@@ -850,7 +860,7 @@ static int grouped_gemm_16bit(bool f16, const void* a, int64_t a_row_stride_byte
                               int64_t K, int num_groups, int num_weights,
                               const int64_t* seg_indptr, const int64_t* weight_indices,
                               int epilogue, int32_t* status_word, const b200moe_gemm_opts* opts, void* stream) {
-  if (int rc = check_grouped_common("grouped_gemm_bf16", a, b, c, seg_indptr, a_row_stride_bytes, 2 * K, M_total, N,
+  if (int rc = check_grouped_common("grouped_gemm_bf16", a, b, c, a_row_stride_bytes, 2 * K, M_total, N,
                                     num_groups, num_weights)) return rc;
   B200MOE_REQUIRE(epilogue == 0 || epilogue == 3 || ((epilogue == 2 || epilogue == 5) && !f16), B200MOE_BAD_ARG,
                   "grouped_gemm_bf16: epilogue %d (0 plain, 2 SiLU*up / 5 GELU*up with bf16 operands, 3 plain added to c)", epilogue);
@@ -880,6 +890,7 @@ extern "C" int b200moe_grouped_gemm_bf16(const void* a, int64_t a_row_stride_byt
                                          const int64_t* seg_indptr, const int64_t* weight_indices,
                                          int epilogue, int32_t* status_word, const b200moe_gemm_opts* opts,
                                          void* stream) {
+  B200MOE_REQUIRE(seg_indptr, B200MOE_BAD_ARG, "grouped_gemm_bf16: null pointer");
   return grouped_gemm_16bit(false, a, a_row_stride_bytes, b, c, c_dtype, c_row_stride_bytes, M_total, N, K,
                             num_groups, num_weights, seg_indptr, weight_indices, epilogue, status_word, opts, stream);
 }
@@ -889,8 +900,15 @@ extern "C" int b200moe_grouped_gemm_f16(const void* a, int64_t a_row_stride_byte
                                         int64_t K, int num_groups, int num_weights,
                                         const int64_t* seg_indptr, const int64_t* weight_indices,
                                         int32_t* status_word, const b200moe_gemm_opts* opts, void* stream) {
+  B200MOE_REQUIRE(seg_indptr, B200MOE_BAD_ARG, "grouped_gemm_f16: null pointer");
   return grouped_gemm_16bit(true, a, a_row_stride_bytes, b, c, c_dtype, c_row_stride_bytes, M_total, N, K,
                             num_groups, num_weights, seg_indptr, weight_indices, 0, status_word, opts, stream);
+}
+
+int b200moe::dense_gemm_bf16(const void* a, const void* b, void* c, int64_t c_row_stride_bytes, int64_t M, int64_t N, int64_t K,
+                             int epilogue, int32_t* status_word, void* stream) {
+  return grouped_gemm_16bit(false, a, 2 * K, b, c, B200MOE_BF16, c_row_stride_bytes, M, N, K, 1, 1, nullptr, nullptr, epilogue,
+                            status_word, nullptr, stream);
 }
 
 // ---- router logits on the tensor cores ------------------------------------------------------

@@ -140,8 +140,8 @@ extern "C" int b200moe_layer_forward(const b200moe_layer* Lp, const void* x, voi
   if (L.shared_inter) {
     // gate/up of the shared experts needs only x: on the side stream it fills the SMs the routed path leaves idle
     STEP(side.fork(as_stream(L.side_stream)));
-    STEP(b200moe_grouped_gemm_bf16(x, 2 * H, L.shared_w13, ws + p.shared_h, B200MOE_BF16, 2 * L.shared_inter, T,
-                                   2 * L.shared_inter, H, 1, 1, nullptr, nullptr, L.act ? 5 : 2, L.status, nullptr, L.side_stream));
+    STEP(dense_gemm_bf16(x, L.shared_w13, ws + p.shared_h, 2 * L.shared_inter, T, 2 * L.shared_inter, H, L.act ? 5 : 2, L.status,
+                         L.side_stream));
     STEP(side.done());
   }
   STEP(b200moe_route_metadata(idx, p.S, L.experts, reinterpret_cast<int64_t*>(ws + p.ids), dst, seg, ws + p.scratch,
@@ -174,8 +174,7 @@ extern "C" int b200moe_layer_forward(const b200moe_layer* Lp, const void* x, voi
   STEP(b200moe_post_reorder(down, B200MOE_BF16, y, dst, idx, wts, 0, E - 1, T, L.top_k, H, stream));
   if (L.shared_inter) {
     STEP(side.join());
-    STEP(b200moe_grouped_gemm_bf16(ws + p.shared_h, 2 * L.shared_inter, L.shared_w2, y, B200MOE_BF16, 2 * H, T, H, L.shared_inter,
-                                   1, 1, nullptr, nullptr, 3, L.status, nullptr, stream));
+    STEP(dense_gemm_bf16(ws + p.shared_h, L.shared_w2, y, 2 * H, T, H, L.shared_inter, 3, L.status, stream));
   }
   return B200MOE_OK;
 }

@@ -234,7 +234,7 @@ def permute_quant_fp8_push(x, src2dst, topk_ids, seg_indptr, dst_base, rec_bytes
 
 def grouped_gemm_i8(a, a_s, b, b_s, seg_indptr, weight_indices, c, status_word=None):
     """tcgen05 grouped int8 GEMM with blockwise f32 scales (the w4a8 path once the weights are
-    int8; seg_indptr None: one group of all rows).  a int8 [M,K], a_s f32 [M,K/128], b int8 [W,N,K], b_s f32 [W,N/128,K/128]."""
+    int8).  a int8 [M,K], a_s f32 [M,K/128], b int8 [W,N,K], b_s f32 [W,N/128,K/128]."""
     N.require_cuda(a, a_s, b, b_s, c)
     assert a.dtype == torch.int8 and b.dtype == torch.int8 and a_s.dtype == torch.float32 and b_s.dtype == torch.float32
     assert b.is_contiguous() and b_s.is_contiguous() and a.stride(1) == 1 and a_s.stride(1) == 1
@@ -243,8 +243,8 @@ def grouped_gemm_i8(a, a_s, b, b_s, seg_indptr, weight_indices, c, status_word=N
     assert Kb == K
     N.check(N.lib().b200moe_grouped_gemm_i8(
         N.ptr(a), a.stride(0), N.ptr(a_s), a_s.stride(0), N.ptr(b), N.ptr(b_s), N.ptr(c), N.dtype_code(c.dtype),
-        c.stride(0) * c.element_size(), M, Nn, K, 1 if seg_indptr is None else seg_indptr.numel() - 1, W,
-        N.ptr(seg_indptr), N.ptr(weight_indices), N.ptr(status_word), _opts(), N.stream()))
+        c.stride(0) * c.element_size(), M, Nn, K, seg_indptr.numel() - 1, W, N.ptr(seg_indptr),
+        N.ptr(weight_indices), N.ptr(status_word), _opts(), N.stream()))
     return c
 
 

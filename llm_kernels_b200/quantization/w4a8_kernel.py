@@ -81,15 +81,18 @@ def w4a8_gemm(a: torch.Tensor, a_s: torch.Tensor, b: torch.Tensor, b_s: torch.Te
     c = a.new_empty(*a.size()[:-1], Nn, dtype=out_dtype or torch.get_default_dtype())
     ks = _split_k(M, Nn, K)
     a_s, b_s = a_s.reshape(M, -1).float(), b_s.float()
-    # The split launch takes its sizes and strides from M, N and K alone, so it serves operands that agree on them; any
+    # The dense launches take their sizes and strides from M, N and K alone, so they serve operands that agree on them; any
     # others go to the grouped launch, which checks them and reads the scales by their own stride.
-    if ks > 1 and _opts() is None and tuple(w8.shape) == (Nn, K) and a_s.shape[1] * 128 == K:
+    if _opts() is None and tuple(w8.shape) == (Nn, K) and a_s.shape[1] * 128 == K:
         N.require_cuda(a, a_s, b_s)
         assert a.dtype == torch.int8
-        part = _partials(a, ks * M * Nn)
-        N.check(N.lib().b200moe_gemm_i8_block_splitk(N.ptr(a), N.ptr(a_s), N.ptr(w8), N.ptr(b_s), N.ptr(c),
-                                                     N.dtype_code(c.dtype), M, Nn, K, ks, N.ptr(part),
-                                                     part.numel() * 4, N.stream()))
+        args = (N.ptr(a), N.ptr(a_s), N.ptr(w8), N.ptr(b_s), N.ptr(c), N.dtype_code(c.dtype), M, Nn, K)
+        if ks > 1:
+            part = _partials(a, ks * M * Nn)
+            N.check(N.lib().b200moe_gemm_i8_block_splitk(*args, ks, N.ptr(part), part.numel() * 4, N.stream()))
+        else:
+            N.check(N.lib().b200moe_gemm_i8_block(*args, N.stream()))
         return c
-    grouped_gemm_i8(a.view(M, K), a_s, w8.unsqueeze(0), b_s.unsqueeze(0), None, None, c.view(M, Nn))
+    seg = torch.tensor([0, M], dtype=torch.int64, device=a.device)
+    grouped_gemm_i8(a.view(M, K), a_s, w8.unsqueeze(0), b_s.unsqueeze(0), seg, None, c.view(M, Nn))
     return c

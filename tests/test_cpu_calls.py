@@ -338,3 +338,12 @@ def test_split_gemms_that_overlap_have_partials_of_their_own(host, monkeypatch, 
     call()
     a, b = seen
     assert len(a) == 8 * 24 * 256 * 4 and (a.stop <= b.start or b.stop <= a.start)
+
+
+def test_grouped_gemms_refuse_a_missing_group_table(host):
+    """Also for one group, and before anything else decides that there is nothing to do (no rows)."""
+    lib, bf = host.lib(), host.BF16
+    assert lib.b200moe_grouped_gemm_i8(16, 128, 16, 1, 16, 16, 16, bf, 256, 0, 128, 128, 1, 1, None, None, None, None, None) == 4
+    for fn, tail in ((lib.b200moe_grouped_gemm_bf16, (0, None, None, None)), (lib.b200moe_grouped_gemm_f16, (None, None, None))):
+        assert fn(16, 256, 16, 16, bf, 256, 0, 128, 128, 1, 1, None, None, *tail) == 4
+        assert fn(16, 256, 16, 16, bf, 256, 0, 128, 128, 1, 1, 16, None, *tail) == 0
