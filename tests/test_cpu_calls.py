@@ -347,3 +347,17 @@ def test_grouped_gemms_refuse_a_missing_group_table(host):
     for fn, tail in ((lib.b200moe_grouped_gemm_bf16, (0, None, None, None)), (lib.b200moe_grouped_gemm_f16, (None, None, None))):
         assert fn(16, 256, 16, 16, bf, 256, 0, 128, 128, 1, 1, None, None, *tail) == 4
         assert fn(16, 256, 16, 16, bf, 256, 0, 128, 128, 1, 1, 16, None, *tail) == 0
+
+
+def test_package_imports_on_a_torch_without_cuda():
+    """The host-only parts (configurations, bit packing on the CPU, plans) need no CUDA in torch."""
+    import os
+    import subprocess
+    import sys
+    code = ("import torch\n"
+            "for name in [n for n in dir(torch._C) if n.startswith('_cuda_get')]:\n"
+            "    delattr(torch._C, name)\n"
+            "import llm_kernels_b200._native, llm_kernels_b200.moe.all2all_moe, llm_kernels_b200.workloads\n")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    done = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True)
+    assert done.returncode == 0, done.stderr
