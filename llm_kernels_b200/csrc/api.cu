@@ -1,6 +1,5 @@
 // Status strings and the per-thread last-error message of the C ABI.
 #include <mutex>
-#include <vector>
 
 #include "common.cuh"
 
@@ -26,15 +25,16 @@ int check_launch(const char* what) {
 int set_dynamic_smem(const void* kernel, size_t bytes) {
   struct Entry { const void* kernel; int dev; size_t bytes; };
   static std::mutex mu;
-  static std::vector<Entry> done;
+  static Entry done[128];          // no allocation, which could throw through a C entry; beyond it the call is only repeated
+  static int count = 0;
   int dev = -1;
   cudaGetDevice(&dev);
   std::lock_guard<std::mutex> lock(mu);
-  for (const Entry& e : done)
-    if (e.kernel == kernel && e.dev == dev && e.bytes >= bytes) return B200MOE_OK;
+  for (int i = 0; i < count; ++i)
+    if (done[i].kernel == kernel && done[i].dev == dev && done[i].bytes >= bytes) return B200MOE_OK;
   const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
   if (e != cudaSuccess) return fail(B200MOE_LAUNCH_FAILED, "%zu bytes of shared memory: %s", bytes, cudaGetErrorString(e));
-  done.push_back({kernel, dev, bytes});
+  if (count < 128) done[count++] = {kernel, dev, bytes};
   return B200MOE_OK;
 }
 
