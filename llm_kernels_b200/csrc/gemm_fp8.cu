@@ -60,7 +60,7 @@ constexpr uint32_t kTmemCols = 512;
 // before, all n-tiles of an m-tile first: bands gain nothing there (fp8 layer of 4096 tokens, 29 MB per expert: 1 % slower).
 constexpr int kBand = 8;
 constexpr int64_t kBandMinBytes = 48 << 20;
-constexpr int kPairRowsPerGroup = 768;   // see launch_gemm
+constexpr int kPairRowsPerGroup = 768;   // see pairs_pay
 
 struct SharedTail {
   uint64_t full[kMaxStages];
@@ -636,6 +636,22 @@ static int launch_gemm_as(const RowMaps& ma, const CUtensorMap& mb, const GemmPa
   return check_launch("gemm_block_kernel");
 }
 
+// Whether a launch of 16-bit operands without options runs in CTA pairs: a pair moves a third less from L2 to its SMs, which
+// at the power cap is time.  The block-scaled kinds are bound by their promotion and gain nothing.  us, single -> pair:
+//   rows per group (8 groups, gate/up N 28672 K 4096, then down N 4096 K 14336): 300 656-685 -> 724 and 365 -> 431 (256-row
+//     tiles pad more), 1024 1711-1828 -> 1577 and 770-838 -> 718, 2048 3440-3626 -> 2764 and 1698-1757 -> 1597; one group of
+//     768 rows, N 4096 K 7168: 75 -> 66
+//   K (one group of 768 to 4096 rows; a short K loop does not make up for the pair's longer tile epilogue): from 2048 on
+//     every epilogue gains or is even (N 4096: plain 77 -> 67, gate/up 85 -> 77), below it fused and adding ones lose 1 to 2 us
+//     (K 1024: gate/up 41 -> 42 and 65 -> 67, adding 53 -> 54), at 512 all do
+//   tiles of a plain epilogue at K 1024: 48 and 96 of them 27.8 -> 28.0 and 28.3 -> 28.9, 192 and more 38 -> 35 and 52 -> 46
+static bool pairs_pay(const GemmParams& p, int sms) {
+  if (p.M_total < kPairRowsPerGroup * static_cast<int64_t>(p.num_groups)) return false;
+  const int K = p.K / 2;
+  const int64_t tiles = ((p.M_total + BM - 1) / BM) * ((p.N + BN - 1) / BN);
+  return K >= 2048 || (K >= 1024 && !p.swiglu && !p.accumulate && tiles > sms);
+}
+
 // opts (may be null): per-call launch options of the grouped GEMMs (b200moe_gemm_opts).
 template <int KIND>
 static int launch_gemm(const void* a, int64_t a_stride, const void* b, GemmParams p, int64_t tiles_hint,
@@ -659,12 +675,8 @@ static int launch_gemm(const void* a, int64_t a_stride, const void* b, GemmParam
   if (max_ctas > 0 && max_ctas < grid) grid = max_ctas;
   if (tiles_hint > 0 && tiles_hint < grid) grid = static_cast<int>(tiles_hint);
   // N must cover both halves of a pair's tile; split-K launches stay single.
-  // Without options, 16-bit operands with many rows per group run in pairs: a pair moves a third less from L2 to its SMs,
-  // which at the power cap is time.  Rows per group, us single -> pair (8 groups, gate/up N 28672 K 4096, then down N 4096
-  // K 14336): 300 656-685 -> 724 and 365 -> 431 (256-row tiles pad more), 1024 1711-1828 -> 1577 and 770-838 -> 718,
-  // 2048 3440-3626 -> 2764 and 1698-1757 -> 1597.  The block-scaled kinds are bound by their promotion: no gain.
   constexpr bool k16bit = KIND == kBf16 || KIND == kF16;
-  bool pair = pair_mode == 1 || (k16bit && !opts && p.M_total >= kPairRowsPerGroup * static_cast<int64_t>(p.num_groups));
+  bool pair = pair_mode == 1 || (k16bit && !opts && pairs_pay(p, sms));
   if (p.ksplits > 1 || grid < 2 || (!p.swiglu && p.N % BN != 0)) pair = false;
   if (pair) return launch_gemm_as<KIND, true>(ma, mb, p, grid & ~1, st);
   return launch_gemm_as<KIND, false>(ma, mb, p, grid, st);
