@@ -25,6 +25,51 @@ def _layer(method="fp8_block", act="silu", shared=0, tokens=37, hidden=512, inte
     return layer, WL.tokens(shape).to(dev).view(1, tokens, hidden)
 
 
+def _separate(layer, x):
+    """The same pass as one launch after the other."""
+    layer.stage_events = []
+    y = layer(x).clone()
+    assert any(name == "post_reorder" for name, _ in layer.stage_events)
+    layer.stage_events = None
+    return y
+
+
+@pytest.mark.parametrize("method", ["fp8_block", "w4a16", "w4a8"])
+@pytest.mark.parametrize("act,shared", [("silu", 0), ("gelu", 0), ("silu", 2), ("gelu", 1)])
+@pytest.mark.parametrize("tokens", [1, 37, 130, 768])
+def test_one_call_pass_is_bit_identical_to_separate_launches(method, act, shared, tokens):
+    """One row in all, few and many rows per expert, shared experts in single CTAs and in pairs (768 rows, hidden 2048)."""
+    layer, x = _layer(method, act, shared, tokens, hidden=2048 if tokens == 768 else 512)
+    y = layer(x).clone()
+    assert layer._native is not None
+    layer._native = None
+    assert torch.equal(y, _separate(layer, x)) and layer._native is None
+    layer.check_status()
+
+
+def test_one_call_pass_after_changes():
+    """Weights loaded in place, a replaced router weight and a changed setting: the next pass has them."""
+    layer, x = _layer("w4a8")
+    other, _ = _layer("w4a8", seed=8)
+    seen = [layer(x).clone()]
+    for name, t in layer.named_buffers():
+        t.copy_(dict(other.named_buffers())[name])
+    seen.append(layer(x).clone())
+    layer.gate.weight = torch.nn.Parameter(other.gate.weight.detach().clone())
+    seen.append(layer(x).clone())
+    assert torch.equal(seen[-1], other(x))
+    layer.gate.routed_scaling_factor = 2.0
+    seen.append(layer(x).clone())
+    assert torch.equal(seen[-1], _separate(layer, x))
+    assert not any(torch.equal(a, b) for a, b in zip(seen, seen[1:]))
+    layer.w13_s4[0, 0, 0], layer.w13_z4[0, 0, 0] = 127, 0         # (q - 0) * 127 leaves int8: only expansion is right
+    layer.w13_qweight[0, 0, 0] |= 0xF
+    y = layer(x).clone()
+    layer.w4_fused_rows_per_group = 0
+    assert torch.equal(y, layer(x)) and not layer._raw_nibbles_ok("w13")
+    layer.check_status()
+
+
 def test_refused_pass_leaves_the_side_stream_joined():
     """A launch is refused by the host checks after the shared experts' gate/up has been forked off: a capture around it
     can only end if the side stream has been joined again."""

@@ -1,20 +1,36 @@
 """The GEMMs for few rows per group (csrc/gemm_fp8_rows.cu, csrc/gemm_w4a16.cu) against the 128-token tiles of
 csrc/gemm_fp8.cu, which the other test files compare with the oracle."""
+import os
+import re
+
 import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
 
-# rows per group: none, one, around the 16-token steps, a full 64-token chunk and its neighbours
-ROWS = [0, 1, 15, 16, 17, 0, 33, 48, 49, 63, 64, 65, 3]
+# rows per group: none, one, around the 16-token steps, a full 64-token chunk and its neighbours; two chunks and a rest
+ROWS = [0, 1, 15, 16, 17, 0, 33, 48, 49, 63, 64, 65, 3, 0, 1, 0, 130, 1, 0, 2, 32, 31, 0, 0, 1, 0]
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "llm_kernels_b200", "csrc")
+
+
+def _limit():
+    """Rows per group on average up to which fp8 products take the kernel under test."""
+    return int(re.search(r"kMaxRowsPerGroup = (\d+);", open(os.path.join(CSRC, "gemm_rows.cuh")).read()).group(1))
+
+
+def _bits(t):
+    return t.view({2: torch.int16, 4: torch.int32}[t.element_size()])
 
 
 def _operands(rows, N, K, seed):
+    """Every eleventh row is zero, whose e4m3 codes are NaN with a scale of zero."""
     from llm_kernels_b200.quantization import fp8_kernel
     dev = torch.device("cuda:0")
     g = torch.Generator(device=dev).manual_seed(seed)
     W, M = len(rows), sum(rows)
-    a, a_s = fp8_kernel.act_quant(torch.randn(M, K, generator=g, device=dev).to(torch.bfloat16))
+    x = torch.randn(M, K, generator=g, device=dev).to(torch.bfloat16)
+    x[5::11] = 0
+    a, a_s = fp8_kernel.act_quant(x)
     b, b_s = fp8_kernel.weight_quant(torch.randn(W * N, K, generator=g, device=dev) * 0.02)
     seg = torch.tensor([0] + torch.tensor(rows).cumsum(0).tolist(), dtype=torch.int64, device=dev)
     widx = torch.randperm(W, generator=g, device=dev)
@@ -26,26 +42,46 @@ def _operands(rows, N, K, seed):
 def test_rows_kernel_plain_is_bit_identical(N, K, dtype):
     """Same promotion (one FMA per value and K block, in K order), so the same bits."""
     from llm_kernels_b200.moe import group_gemm_kernel as G
+    assert sum(ROWS) <= _limit() * len(ROWS)                     # else both calls run the same kernel
     a, a_s, b, b_s, seg, widx = _operands(ROWS, N, K, 1)
     c = torch.empty(a.shape[0], N, dtype=dtype, device=a.device)
     want = torch.empty_like(c)
     G.grouped_gemm_fp8(a, a_s, b, b_s, seg, widx, c)
     with G.gemm_options():
         G.grouped_gemm_fp8(a, a_s, b, b_s, seg, widx, want)
-    assert torch.equal(c, want)
+    assert torch.equal(_bits(c), _bits(want))
+
+
+@pytest.mark.parametrize("groups", [1, 3])
+@pytest.mark.parametrize("more", [0, 1])
+def test_rows_kernel_at_its_limit(groups, more):
+    """The last number of rows that takes the kernel and the first that does not, against 64-bit sums: e4m3 products are exact,
+    so what is left are the roundings of K / 128 scaled block sums and of the f32 sum inside the tensor core."""
+    from llm_kernels_b200.moe import group_gemm_kernel as G
+    rows = [_limit()] * groups
+    rows[-1] += more
+    a, a_s, b, b_s, seg, widx = _operands(rows, 384, 640, 5)
+    a = torch.where(a_s.repeat_interleave(128, -1) > 0, a.float(), 0.0).to(a.dtype)
+    c = G.grouped_gemm_fp8(a, a_s, b, b_s, seg, widx, torch.empty(a.shape[0], 384, device=a.device))
+    wide = lambda t, s: t.double() * s.double().repeat_interleave(128, -1)
+    for i in range(groups):
+        w = int(widx[i])
+        want = wide(a[seg[i]:seg[i + 1]], a_s[seg[i]:seg[i + 1]]) @ wide(b[w], b_s[w].repeat_interleave(128, 0)).t()
+        assert float((c[seg[i]:seg[i + 1]] - want).norm() / want.norm()) < 1e-4
 
 
 @pytest.mark.parametrize("epilogue", [1, 4])
 @pytest.mark.parametrize("N,K", [(256, 128), (768, 640)])
 def test_rows_kernel_fused_is_bit_identical(N, K, epilogue):
     from llm_kernels_b200.moe import group_gemm_kernel as G
+    assert sum(ROWS) <= _limit() * len(ROWS)
     a, a_s, b, b_s, seg, widx = _operands(ROWS, N, K, 2)
     M = a.shape[0]
     out = [(torch.empty(M, N // 2, dtype=torch.uint8, device=a.device), torch.empty(M, N // 256, device=a.device)) for _ in range(2)]
     G.grouped_gemm_fp8(a, a_s, b, b_s, seg, widx, *out[0], epilogue=epilogue)
     with G.gemm_options():
         G.grouped_gemm_fp8(a, a_s, b, b_s, seg, widx, *out[1], epilogue=epilogue)
-    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(_bits(out[0][1]), _bits(out[1][1]))
 
 
 @pytest.mark.parametrize("whole_zeros", [True, False])
