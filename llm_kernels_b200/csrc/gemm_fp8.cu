@@ -640,16 +640,16 @@ static int launch_gemm_as(const RowMaps& ma, const CUtensorMap& mb, const GemmPa
 // at the power cap is time.  The block-scaled kinds are bound by their promotion and gain nothing.  us, single -> pair:
 //   rows per group (8 groups, gate/up N 28672 K 4096, then down N 4096 K 14336): 300 656-685 -> 724 and 365 -> 431 (256-row
 //     tiles pad more), 1024 1711-1828 -> 1577 and 770-838 -> 718, 2048 3440-3626 -> 2764 and 1698-1757 -> 1597; one group of
-//     768 rows, N 4096 K 7168: 75 -> 66
-//   K (one group of 768 to 4096 rows; a short K loop does not make up for the pair's longer tile epilogue): from 2048 on
-//     every epilogue gains or is even (N 4096: plain 77 -> 67, gate/up 85 -> 77), below it fused and adding ones lose 1 to 2 us
-//     (K 1024: gate/up 41 -> 42 and 65 -> 67, adding 53 -> 54), at 512 all do
-//   tiles of a plain epilogue at K 1024: 48 and 96 of them 27.8 -> 28.0 and 28.3 -> 28.9, 192 and more 38 -> 35 and 52 -> 46
+//     768 rows, N 4096 K 7168: 63 -> 53
+//   K (one group of 768 to 4096 rows, N 1024 to 8192; the code evicted before each launch, as in a layer): from 1536 on every
+//     epilogue gains or is even (N 4096, 4096 rows: plain 57 -> 47, gate/up 63 -> 63; K 2048: 70 -> 59, 76 -> 68); at 1024
+//     gate/up and adding epilogues lose up to 2 us (57 -> 59, 78 -> 80); at 512 and 256 plain ones too (16 -> 18)
+//   tiles of a plain product at K 1024: 48 and 96 of them 18 -> 20 and 20 -> 20, 192 and more 29 -> 27 and 43 -> 38
 static bool pairs_pay(const GemmParams& p, int sms) {
   if (p.M_total < kPairRowsPerGroup * static_cast<int64_t>(p.num_groups)) return false;
   const int K = p.K / 2;
   const int64_t tiles = ((p.M_total + BM - 1) / BM) * ((p.N + BN - 1) / BN);
-  return K >= 2048 || (K >= 1024 && !p.swiglu && !p.accumulate && tiles > sms);
+  return K >= 1536 || (K >= 1024 && !p.swiglu && !p.accumulate && tiles > sms);
 }
 
 // opts (may be null): per-call launch options of the grouped GEMMs (b200moe_gemm_opts).
