@@ -64,12 +64,6 @@ def _split_k(M: int, Nn: int, K: int) -> int:
     return ks
 
 
-def _partials(a: torch.Tensor, n: int) -> torch.Tensor:
-    """Scratch of one call's K splits.  Nothing is kept between calls: the caching allocator orders its memory by stream and
-    gives a captured call memory of its graph, and calls of two threads on one stream must not meet in one buffer."""
-    return torch.empty(n, dtype=torch.float32, device=a.device)
-
-
 def fp8_gemm(a: torch.Tensor, a_s: torch.Tensor, b: torch.Tensor, b_s: torch.Tensor,
              out_dtype: torch.dtype = None, ksplits: int = None) -> torch.Tensor:
     """c[..., N] = a[..., K] . b[N, K]^T with 1x128 / 128x128 f32 block scales, in the
@@ -87,7 +81,9 @@ def fp8_gemm(a: torch.Tensor, a_s: torch.Tensor, b: torch.Tensor, b_s: torch.Ten
     c = a.new_empty(*a.size()[:-1], Nn, dtype=out_dtype or torch.get_default_dtype())
     ks = _split_k(M, Nn, K) if ksplits is None else int(ksplits)
     if ks > 1 and M > 0:
-        part = _partials(a, ks * M * Nn)
+        # The splits' scratch belongs to the call: the caching allocator orders its memory by stream and gives a captured call
+        # memory of its graph, and calls of two threads on one stream must not meet in one buffer.
+        part = a_s.new_empty(ks * M * Nn)
         N.check(N.lib().b200moe_gemm_fp8_block_splitk(N.ptr(a), N.ptr(a_s), N.ptr(b), N.ptr(b_s), N.ptr(c),
                                                       N.dtype_code(c.dtype), M, Nn, K, ks, N.ptr(part),
                                                       part.numel() * 4, N.stream()))

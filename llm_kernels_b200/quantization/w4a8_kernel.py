@@ -10,7 +10,9 @@ from typing import Tuple
 import torch
 
 from .. import _native as N
+from ..moe.group_gemm_kernel import _opts, grouped_gemm_i8
 from . import int8_kernel
+from .fp8_kernel import _split_k
 
 PACKING_BITS = 32
 W_BITS = 4
@@ -68,8 +70,6 @@ def w4a8_gemm(a: torch.Tensor, a_s: torch.Tensor, b: torch.Tensor, b_s: torch.Te
               pack_direction: str = "row", out_dtype: torch.dtype = None) -> torch.Tensor:
     """c[..., N] = a[..., K] (int8) . dequant(b)^T with per-K-block scales (reference :406-448).  Few rows (M <= 128) split
     the K loop over all SMs as fp8_gemm does: one m-tile alone kept N / 256 of them busy (M = 24, N = 4096, K = 7168)."""
-    from ..moe.group_gemm_kernel import _opts, grouped_gemm_i8
-    from .fp8_kernel import _partials, _split_k
     assert a.is_contiguous() and b.is_contiguous(), 'Input tensors must be contiguous'
     assert a_s.is_contiguous() and b_s.is_contiguous(), 'Scaling factor tensors must be contiguous'
     assert b_s4.is_contiguous() and b_z4.is_contiguous(), 'Scaling factor and zero point tensors must be contiguous'
@@ -88,7 +88,7 @@ def w4a8_gemm(a: torch.Tensor, a_s: torch.Tensor, b: torch.Tensor, b_s: torch.Te
         assert a.dtype == torch.int8
         args = (N.ptr(a), N.ptr(a_s), N.ptr(w8), N.ptr(b_s), N.ptr(c), N.dtype_code(c.dtype), M, Nn, K)
         if ks > 1:
-            part = _partials(a, ks * M * Nn)
+            part = a_s.new_empty(ks * M * Nn)          # the call's own, as in fp8_gemm
             N.check(N.lib().b200moe_gemm_i8_block_splitk(*args, ks, N.ptr(part), part.numel() * 4, N.stream()))
         else:
             N.check(N.lib().b200moe_gemm_i8_block(*args, N.stream()))
