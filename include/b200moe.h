@@ -153,6 +153,9 @@ B200MOE_API int b200moe_router_topk(const void* x, int x_dtype, const float* w, 
                         int scoring, int norm_topk_prob, float routed_scaling_factor,
                         int64_t* topk_idx, float* topk_weight, void* stream);
 
+/* K splits with which b200moe_router_logits_bf16x3 should run for T tokens and E padded expert rows. */
+B200MOE_API int b200moe_router_ksplits(int64_t T, int64_t H, int E);
+
 /* Tensor-core form of the same router for large expert counts, in two launches.
  * b200moe_router_logits_bf16x3: logits x . W^T with f32-equivalent precision out of bf16
  * MMAs: w3 bf16 [E, 3H] holds, per expert row, the three bf16 parts hi | mid | lo of the f32
@@ -163,8 +166,6 @@ B200MOE_API int b200moe_router_topk(const void* x, int x_dtype, const float* w, 
  * b200moe_router_select: adds the partials in index order and applies the scoring,
  * group-limited selection and weight normalisation exactly as b200moe_router_topk, over
  * the first E columns of rows that are partials_row_stride floats apart (the padded count). */
-/* K splits with which b200moe_router_logits_bf16x3 should run for T tokens and E padded expert rows. */
-B200MOE_API int b200moe_router_ksplits(int64_t T, int64_t H, int E);
 B200MOE_API int b200moe_router_logits_bf16x3(const void* x_bf16, const void* w3_bf16, float* partials,
                                  int64_t T, int64_t H, int E, int ksplits, void* stream);
 B200MOE_API int b200moe_router_select(const float* partials, int nsplit, int64_t partials_row_stride,
@@ -396,11 +397,12 @@ B200MOE_API int b200moe_grouped_gemm_w4a8(const void* a, int64_t a_row_stride_by
 /* Grouped w4a16 GEMM (asymmetric group-128 int4 weights, bf16 activations) with the dequantization inside the kernel:
  * the counterpart, for few rows per group, of the reference's w4a16 kernel that dequantizes in registers
  * (fast_dequant/simple_marlin/marlin_w4a16_gemm.cu:44-64, 86-280), here with a zero-point and bf16.  Packed words travel
- * from HBM as they are; converter warps turn each word into eight bf16 values (q - zero) * scale (0x4300 | q is the bf16
- * number 128 + q; two exact subtractions, one rounded product) and write the operand tile the tensor core reads; the
- * K loop accumulates in TMEM.  Bit-identical to b200moe_w4a16_expand_bf16 followed by b200moe_grouped_gemm_bf16.
+ * from HBM as they are; converter warps turn each word into eight bf16 values (q - zero) * scale (exact difference, one
+ * rounded product) and store them as the tensor core's operand in tensor memory; the K loop accumulates there too.
+ * Bit-identical to b200moe_w4a16_expand_bf16 followed by b200moe_grouped_gemm_bf16.
  *   a bf16 [M_total, K]; b_packed int32 [num_weights, N, K/8] (pack_weights_over_cols, quantization/bitpack.py:38-67);
- *   scale_zero_t bf16 [num_weights, K/128, N, 2]: (scale, zero) pairs with one K group's pairs contiguous.
+ *   scale_zero_t bf16 [num_weights, K/128, N, 2]: (scale, zero) pairs with one K group's pairs contiguous, 16-byte
+ *   aligned (bulk copies read it: a base of lesser alignment is refused, it would fault).
  *   epilogue 0: c [M_total, N] f32/f16/bf16; 2 / 5: SiLU(gate)*up / GELU(gate)*up, c bf16 [M_total, N/2].
  *   K % 128 == 0, N % 128 == 0 (fused epilogues: N % 256 == 0). */
 B200MOE_API int b200moe_grouped_gemm_w4a16(const void* a, int64_t a_row_stride_bytes, const void* b_packed,
@@ -452,11 +454,14 @@ B200MOE_API int b200moe_marlin_pack(const int32_t* q, void* packed_i32, const vo
 /* ======================= one pass of a single-rank layer ================== */
 /* DeepseekV3MoE.forward (moe/all2all_moe.py:167-184) at ep_size 1 as one host call: router, permutation
  * metadata, permute (+ quantize), the two grouped GEMMs, weighted un-permute and, when shared_inter != 0, the
- * shared experts (:161-165, 182-183).  Same kernels, same order and same results as the separate calls. */
+ * shared experts (:161-165, 182-183).  Same kernels, same order and same results as the separate calls.  A step that is
+ * refused ends the pass with its status: what was launched before it runs on, and the side stream is joined either way.
+ * The descriptor is only read; passes may overlap if each has a workspace of its own. */
 enum { B200MOE_LAYER_FP8 = 0, B200MOE_LAYER_W4A16 = 1, B200MOE_LAYER_W4A8 = 2 };
 typedef struct b200moe_layer {
   int32_t struct_bytes;              /* sizeof(b200moe_layer) */
-  int32_t method;                    /* B200MOE_LAYER_*: which grouped GEMM pair, hence which weight layout */
+  int32_t method;                    /* B200MOE_LAYER_*: which grouped GEMM pair, hence which weight layout; W4A8 only for
+                                        weights that b200moe_w4a8_range_check passes */
   int32_t act;                       /* 0 = SiLU, 1 = tanh-GELU */
   int32_t experts, top_k, n_group, topk_group, scoring, norm_topk_prob;
   float scaling;

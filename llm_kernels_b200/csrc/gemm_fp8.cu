@@ -58,6 +58,9 @@ constexpr uint32_t kTmemCols = 512;
 // 2304 tokens): near the square that touches the fewest bytes, and small enough that the weights of a band (17 MB for a
 // K of 8 KB) stay in L2 while the band walks down the group.  Weights that L2 holds next to the tokens are walked as
 // before, all n-tiles of an m-tile first: bands gain nothing there (fp8 layer of 4096 tokens, 29 MB per expert: 1 % slower).
+// Around and above the line, us without -> with bands (single CTAs): 8 groups of 2048 rows, bf16, 49 MB (N 7168 K 3584)
+// 697 -> 643, 56 MB 812 -> 743, 112 MB 1719 -> 1462; fp8 51 MB 944 -> 951, 59 MB (N 4096 K 14336) 1000 -> 988, 117 MB
+// (N 28672 K 4096) 3017 -> 2565; 300 rows per group, fp8: 235 -> 228, 263 -> 227, 583 -> 529.
 constexpr int kBand = 8;
 constexpr int64_t kBandMinBytes = 48 << 20;
 constexpr int kPairRowsPerGroup = 768;   // see pairs_pay
@@ -258,7 +261,8 @@ gemm_block_kernel(const __grid_constant__ RowMaps tmap_a,
   const int KBs = (KB + p.ksplits - 1) / p.ksplits;   // K blocks per split
 
   // The thread of a single-thread role.  elect.sync makes TMA and MMA instructions several times faster to issue than a
-  // lane == 0 branch; in pairs, whose leader issues for two SMs, that counts (w4a16 prefill of 8192 tokens 6319 -> 6077 us).
+  // lane == 0 branch; in pairs, whose leader issues for two SMs, that counts (w4a16 prefill of 8192 tokens 6.42 -> 5.88 ms,
+  // three runs of both in turn).
   // The other launches wait for their promotion or their loads anyway, and lose with it (fp8 layer of 4096 tokens 3786 ->
   // 3867 us).
   auto one_thread = [&]() { if constexpr (PAIR) return ptx::elect_one(); else return lane == 0; };

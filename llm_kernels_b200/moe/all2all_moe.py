@@ -289,9 +289,11 @@ class DeepseekV3MoE(nn.Module):
         self._layout = {n: (t.dtype, t.shape) for n, t in self._buffers.items()}
         self._sizes = (E, H, I)
         # int4 methods: up to this many rows per expert group on average the dequantization runs inside the GEMMs
-        # (every tile converts its weights once); above it the weights are expanded once per forward instead
-        # Whole w4a8 layer (256 experts, hidden 7168), us expanded -> inside the GEMMs: 47 rows 7785 -> 2509, 94 rows 8019 -> 4755,
-        # 128 rows 8901 -> 6215, 192 rows 10528 -> 8967, 256 rows 11871 -> 11467.
+        # (every tile converts its weights once); above it the weights are expanded once per forward instead.
+        # Whole layer, us expanded -> inside the GEMMs.  w4a8 (256 experts, hidden 7168): 96 rows 7963 -> 4781, 192 rows
+        # 10175 -> 8723, 224 rows 10348 -> 10064, 256 rows 11474 -> 11735: the crossing is between 224 and 256.
+        # w4a16 (8 experts of 4096 x 14336): 128 rows 1547 -> 653, 256 rows 1834 -> 1015, 512 rows 2363 -> 1730, 768 rows
+        # 2832 -> 2595, 1024 rows 3165 -> 3258: its line of 256 is that of an earlier kernel, the crossing is near 1000.
         self.w4_fused_rows_per_group = int(getattr(config, "w4_fused_rows_per_group",
                                                    256 if self.method == "w4a16" else 192))
         self._buffers_cache = {}
