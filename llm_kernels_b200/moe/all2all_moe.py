@@ -432,7 +432,7 @@ class DeepseekV3MoE(nn.Module):
                 or not all(_is_plain(bufs.get(n), *want) for n, want in self._layout.items())):
             return None
         tensors = [w, bias, *(bufs[n] for n in self._layout)]
-        N.require_cuda(x, *tensors)
+        N.require_cuda(x, self._status, *tensors)        # the status word and the scratch stay where the layer was made
         if gate.top_k != cfg.num_experts_per_tok:
             return None
         w3, pairs = gate._split_weight(w), {"w13": None, "w2": None}

@@ -105,7 +105,7 @@ def test_layer_refuses_weights_of_another_type_or_shape(layer_host, method, name
 def test_layer_refuses_weights_of_another_device_in_every_pass(layer_host, host, monkeypatch):
     """x on the current device is not enough, also once a pass has gone through."""
     layer, x, lib = layer_host()
-    current = [x, *layer.state_dict(keep_vars=True).values()]
+    current = [x, layer._status, *layer.state_dict(keep_vars=True).values()]
 
     def require_cuda(*tensors):
         if not all(t is None or any(t.data_ptr() == c.data_ptr() for c in current) for t in tensors):
@@ -361,3 +361,16 @@ def test_package_imports_on_a_torch_without_cuda():
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     done = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True)
     assert done.returncode == 0, done.stderr
+
+
+def test_layer_moved_to_another_device_is_refused(layer_host, host, monkeypatch):
+    """Module.to moves weights and buffers; the layer's scratch and status word stay on the device that it was made for."""
+    layer, x, lib = layer_host()
+    elsewhere = layer._status
+
+    def require_cuda(*tensors):
+        if any(t is elsewhere for t in tensors):
+            raise RuntimeError("not on the current device")
+    monkeypatch.setattr(host, "require_cuda", require_cuda)
+    with pytest.raises(RuntimeError, match="current device"):
+        layer(x)
