@@ -146,7 +146,8 @@ __device__ __forceinline__ void promote2(float& acc0, float& acc1, uint32_t d0, 
   ptx::unpack_f32x2(r, acc0, acc1);
 }
 
-// One token of the fused epilogue: 128 gate and 128 up values of the stage -> int8 row and its scale.
+// One token of the fused epilogue: 128 gate and 128 up values of the stage -> int8 row and its scale.  128 values that are all
+// NaN (a token with an infinite value) have a NaN scale, as the reference's maximum gives; act_quant gives them a scale of 0.
 __device__ __forceinline__ void emit_row(const Tail8* sh, const Params8& p, const Tile8& tl, int m) {
   const int lane = threadIdx.x & 31;
   const uint2 gv = *reinterpret_cast<const uint2*>(&sh->stage[m][lane * 4]);
