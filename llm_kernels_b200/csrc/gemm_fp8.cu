@@ -392,6 +392,7 @@ gemm_block_kernel(const __grid_constant__ RowMaps tmap_a,
     int as = 0; uint32_t aphase = 0;
     int it = 0;
     bool ok = true;
+    const bool one_tile = total_tiles <= nworkers;
     // Per-tile scale pointers and the first K block's scales; fetched one tile ahead so that the
     // global-load latency hides behind the previous tile's epilogue.
     struct ScaleCursor { const float* as_ptr; const float* bs0_ptr; const float* bs1_ptr; float sa, b0, b1; };
@@ -483,7 +484,60 @@ gemm_block_kernel(const __grid_constant__ RowMaps tmap_a,
         for (int half = 0; half < 2; ++half) {
           const int col0 = tl.nt * BN + half * 128 + hsel * 64;
           if (col0 >= p.N) continue;                       // warp-uniform
-          if (p.c_dtype == B200MOE_F32) {
+          // A thread owns contiguous bytes of ITS row, so a direct store touches 32 cache lines per instruction.  Transpose
+          // 128 bytes per row through shared memory (16 rows at a time, 16-byte chunks XOR-swizzled by the row) so that 8
+          // lanes write one full 128-byte piece of a row (the router's f32 partial sums of 4096 tokens, direct -> this way: 88 -> 69
+          // us).  f32 rows of a launch with one tile per CTA (split K) are stored directly all the same: there this code is
+          // fetched for one use, which costs more (router of one token 13.7 us direct, 18.8 us this way).
+          uint8_t* stg = sh->out_stage[e];
+          auto store_piece = [&](const uint4 (&v)[8], int64_t col_bytes) {
+#pragma unroll
+            for (int part = 0; part < 2; ++part) {
+              if (tl.m0 + q * 32 + part * 16 >= tl.m_end) break;             // warp-uniform
+              if ((lane >> 4) == part) {
+                const int r = lane & 15;
+#pragma unroll
+                for (int c = 0; c < 8; ++c)
+                  *reinterpret_cast<uint4*>(stg + r * 128 + ((c ^ (r & 7)) << 4)) = v[c];
+              }
+              __syncwarp();
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const int r = (lane >> 3) + 4 * i;               // row inside this 16-row part
+                const int cc = lane & 7;
+                uint4 val = *reinterpret_cast<const uint4*>(stg + r * 128 + ((cc ^ (r & 7)) << 4));
+                const int orow_in = tl.m0 + q * 32 + part * 16 + r;
+                if (orow_in < tl.m_end) {
+                  const int64_t orow = p.c_row_map ? p.c_row_map[orow_in] : orow_in;
+                  uint8_t* dst = p.c_row_addr ? reinterpret_cast<uint8_t*>(p.c_row_addr[orow_in])
+                                              : static_cast<uint8_t*>(p.c) + tl.ks * p.split_stride + orow * p.c_stride;
+                  uint4* out = reinterpret_cast<uint4*>(dst + col_bytes + cc * 16);
+                  if (p.accumulate) {
+                    const uint4 old = *out;
+                    const uint32_t* o = &old.x;
+                    uint32_t* n = &val.x;
+#pragma unroll
+                    for (int i2 = 0; i2 < 4; ++i2) {
+                      if (p.c_dtype == B200MOE_BF16) {
+                        const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&o[i2]));
+                        const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&n[i2]));
+                        const __nv_bfloat162 t2 = __floats2bfloat162_rn(a.x + b.x, a.y + b.y);
+                        n[i2] = *reinterpret_cast<const uint32_t*>(&t2);
+                      } else {
+                        const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&o[i2]));
+                        const float2 b = __half22float2(*reinterpret_cast<const __half2*>(&n[i2]));
+                        const __half2 t2 = __floats2half2_rn(a.x + b.x, a.y + b.y);
+                        n[i2] = *reinterpret_cast<const uint32_t*>(&t2);
+                      }
+                    }
+                  }
+                  *out = val;
+                }
+              }
+              __syncwarp();
+            }
+          };
+          if (p.c_dtype == B200MOE_F32 && one_tile) {
             if (row_ok) {
               const int64_t orow = p.c_row_map ? p.c_row_map[row] : row;
               uint8_t* dst = p.c_row_addr ? reinterpret_cast<uint8_t*>(p.c_row_addr[row])
@@ -492,10 +546,19 @@ gemm_block_kernel(const __grid_constant__ RowMaps tmap_a,
             }
             continue;
           }
-          // 16-bit outputs: a thread owns 128 contiguous bytes of ITS row, so a direct store touches
-          // 32 cache lines per instruction.  Transpose through shared memory (16 rows at a time,
-          // 16-byte chunks XOR-swizzled by the row) so that 8 lanes write one full 128-byte row.
           uint4 v[8];
+          if (p.c_dtype == B200MOE_F32) {
+#pragma unroll
+            for (int piece = 0; piece < 2; ++piece) {
+#pragma unroll
+              for (int c = 0; c < 8; ++c) {
+                const float* f = acc + half * 64 + piece * 32 + c * 4;
+                v[c] = make_uint4(__float_as_uint(f[0]), __float_as_uint(f[1]), __float_as_uint(f[2]), __float_as_uint(f[3]));
+              }
+              store_piece(v, static_cast<int64_t>(col0 + piece * 32) * 4);
+            }
+            continue;
+          }
 #pragma unroll
           for (int c = 0; c < 8; ++c) {
             uint32_t w[4];
@@ -507,51 +570,7 @@ gemm_block_kernel(const __grid_constant__ RowMaps tmap_a,
             }
             v[c] = make_uint4(w[0], w[1], w[2], w[3]);
           }
-          uint8_t* stg = sh->out_stage[e];
-#pragma unroll
-          for (int part = 0; part < 2; ++part) {
-            if ((lane >> 4) == part) {
-              const int r = lane & 15;
-#pragma unroll
-              for (int c = 0; c < 8; ++c)
-                *reinterpret_cast<uint4*>(stg + r * 128 + ((c ^ (r & 7)) << 4)) = v[c];
-            }
-            __syncwarp();
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const int r = (lane >> 3) + 4 * i;               // row inside this 16-row part
-              const int cc = lane & 7;
-              uint4 val = *reinterpret_cast<const uint4*>(stg + r * 128 + ((cc ^ (r & 7)) << 4));
-              const int orow_in = tl.m0 + q * 32 + part * 16 + r;
-              if (orow_in < tl.m_end) {
-                const int64_t orow = p.c_row_map ? p.c_row_map[orow_in] : orow_in;
-                uint8_t* dst = p.c_row_addr ? reinterpret_cast<uint8_t*>(p.c_row_addr[orow_in])
-                                            : static_cast<uint8_t*>(p.c) + tl.ks * p.split_stride + orow * p.c_stride;
-                uint4* out = reinterpret_cast<uint4*>(dst + static_cast<int64_t>(col0) * 2 + cc * 16);
-                if (p.accumulate) {
-                  const uint4 old = *out;
-                  const uint32_t* o = &old.x;
-                  uint32_t* n = &val.x;
-#pragma unroll
-                  for (int i2 = 0; i2 < 4; ++i2) {
-                    if (p.c_dtype == B200MOE_BF16) {
-                      const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&o[i2]));
-                      const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&n[i2]));
-                      const __nv_bfloat162 t2 = __floats2bfloat162_rn(a.x + b.x, a.y + b.y);
-                      n[i2] = *reinterpret_cast<const uint32_t*>(&t2);
-                    } else {
-                      const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&o[i2]));
-                      const float2 b = __half22float2(*reinterpret_cast<const __half2*>(&n[i2]));
-                      const __half2 t2 = __floats2half2_rn(a.x + b.x, a.y + b.y);
-                      n[i2] = *reinterpret_cast<const uint32_t*>(&t2);
-                    }
-                  }
-                }
-                *out = val;
-              }
-            }
-            __syncwarp();
-          }
+          store_piece(v, static_cast<int64_t>(col0) * 2);
         }
       } else if (p.swiglu == 2) {
         // SwiGLU with the reference's roundings, written as bf16 (no re-quantization)

