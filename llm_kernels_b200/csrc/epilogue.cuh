@@ -40,11 +40,13 @@ __device__ __forceinline__ float bf16r(float v) { return __bfloat162float(__floa
 
 // Activation of the fused "act(gate) * up" epilogues, evaluated in f32 on the bf16-rounded gate value:
 // act 0 = SiLU (moe/group_gemm_kernel.py:158-162), act 1 = tanh-GELU with tanh(x) = 2 sigmoid(2x) - 1 (:176-224).
-__device__ __forceinline__ float gate_act(float g, int act) {
-  if (act == 0) return g * __fdividef(1.0f, 1.0f + __expf(-g));
+template <int ACT>
+__device__ __forceinline__ float gate_act(float g) {
+  if (ACT == 0) return g * __fdividef(1.0f, 1.0f + __expf(-g));
   const float inner = 0.7978845608028654f * (g + 0.044715f * g * g * g);
   const float th = 2.f * __fdividef(1.0f, 1.0f + __expf(-2.f * inner)) - 1.f;
   return 0.5f * g * (1.f + th);
 }
+__device__ __forceinline__ float gate_act(float g, int act) { return act == 0 ? gate_act<0>(g) : gate_act<1>(g); }
 
 }  // namespace b200moe

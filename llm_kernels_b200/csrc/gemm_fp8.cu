@@ -185,6 +185,19 @@ __device__ __forceinline__ void promote32(float* acc, const uint32_t (&r)[32], f
   }
 }
 
+// acc[j] <- act(acc[j]) * acc[64 + j] for a thread's 64 columns, with the roundings of the unfused chain (GEMM output, activation
+// and product each to bf16).  One loop per activation: with the choice inside, the unrolled loop's instructions for the other
+// activation lay between those in use, and a small problem waited for their fetch.
+__device__ __forceinline__ void gate_up(float (&acc)[128], int act) {
+  if (act == 0) {
+#pragma unroll
+    for (int j = 0; j < 64; ++j) acc[j] = bf16r(bf16r(gate_act<0>(bf16r(acc[j]))) * bf16r(acc[64 + j]));
+  } else {
+#pragma unroll
+    for (int j = 0; j < 64; ++j) acc[j] = bf16r(bf16r(gate_act<1>(bf16r(acc[j]))) * bf16r(acc[64 + j]));
+  }
+}
+
 // PAIR: the kernel is launched in clusters of two CTAs that share one 256 x 256 tile
 // (tcgen05 cta_group::2).  CTA r of the pair loads rows [128 r, 128 r + 128) of the activation tile
 // and the r-th 128-row box of the weight tile, so each SM moves 32 KB per K block through the
@@ -484,60 +497,45 @@ gemm_block_kernel(const __grid_constant__ RowMaps tmap_a,
         for (int half = 0; half < 2; ++half) {
           const int col0 = tl.nt * BN + half * 128 + hsel * 64;
           if (col0 >= p.N) continue;                       // warp-uniform
-          // A thread owns contiguous bytes of ITS row, so a direct store touches 32 cache lines per instruction.  Transpose
-          // 128 bytes per row through shared memory (16 rows at a time, 16-byte chunks XOR-swizzled by the row) so that 8
-          // lanes write one full 128-byte piece of a row (the router's f32 partial sums of 4096 tokens, direct -> this way: 88 -> 69
-          // us).  f32 rows of a launch with one tile per CTA (split K) are stored directly all the same: there this code is
-          // fetched for one use, which costs more (router of one token 13.7 us direct, 18.8 us this way).
-          uint8_t* stg = sh->out_stage[e];
-          auto store_piece = [&](const uint4 (&v)[8], int64_t col_bytes) {
+          if constexpr (!kPromote) {
+            // f32 rows of a launch with several tiles per CTA (the router's partial sums) go through shared memory as the
+            // 16-bit rows below, 32 columns at a time: 4096 tokens 88 -> 58 us.  With one tile per CTA this code is fetched
+            // for one use, which costs more than the direct stores (one token 13.7 us direct, 18.8 us this way); in the
+            // block-scaled kinds its registers slow every tile down (4096 x 7168 x 7168: 248 -> 259 us).
+            if (p.c_dtype == B200MOE_F32 && !one_tile) {
+              uint8_t* stg = sh->out_stage[e];
 #pragma unroll
-            for (int part = 0; part < 2; ++part) {
-              if (tl.m0 + q * 32 + part * 16 >= tl.m_end) break;             // warp-uniform
-              if ((lane >> 4) == part) {
-                const int r = lane & 15;
+              for (int piece = 0; piece < 2; ++piece) {
 #pragma unroll
-                for (int c = 0; c < 8; ++c)
-                  *reinterpret_cast<uint4*>(stg + r * 128 + ((c ^ (r & 7)) << 4)) = v[c];
-              }
-              __syncwarp();
+                for (int part = 0; part < 2; ++part) {
+                  if ((lane >> 4) == part) {
+                    const int r = lane & 15;
 #pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                const int r = (lane >> 3) + 4 * i;               // row inside this 16-row part
-                const int cc = lane & 7;
-                uint4 val = *reinterpret_cast<const uint4*>(stg + r * 128 + ((cc ^ (r & 7)) << 4));
-                const int orow_in = tl.m0 + q * 32 + part * 16 + r;
-                if (orow_in < tl.m_end) {
-                  const int64_t orow = p.c_row_map ? p.c_row_map[orow_in] : orow_in;
-                  uint8_t* dst = p.c_row_addr ? reinterpret_cast<uint8_t*>(p.c_row_addr[orow_in])
-                                              : static_cast<uint8_t*>(p.c) + tl.ks * p.split_stride + orow * p.c_stride;
-                  uint4* out = reinterpret_cast<uint4*>(dst + col_bytes + cc * 16);
-                  if (p.accumulate) {
-                    const uint4 old = *out;
-                    const uint32_t* o = &old.x;
-                    uint32_t* n = &val.x;
-#pragma unroll
-                    for (int i2 = 0; i2 < 4; ++i2) {
-                      if (p.c_dtype == B200MOE_BF16) {
-                        const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&o[i2]));
-                        const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&n[i2]));
-                        const __nv_bfloat162 t2 = __floats2bfloat162_rn(a.x + b.x, a.y + b.y);
-                        n[i2] = *reinterpret_cast<const uint32_t*>(&t2);
-                      } else {
-                        const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&o[i2]));
-                        const float2 b = __half22float2(*reinterpret_cast<const __half2*>(&n[i2]));
-                        const __half2 t2 = __floats2half2_rn(a.x + b.x, a.y + b.y);
-                        n[i2] = *reinterpret_cast<const uint32_t*>(&t2);
-                      }
+                    for (int c = 0; c < 8; ++c) {
+                      const float* f = acc + half * 64 + piece * 32 + c * 4;
+                      *reinterpret_cast<float4*>(stg + r * 128 + ((c ^ (r & 7)) << 4)) = make_float4(f[0], f[1], f[2], f[3]);
                     }
                   }
-                  *out = val;
+                  __syncwarp();
+#pragma unroll
+                  for (int i = 0; i < 4; ++i) {
+                    const int r = (lane >> 3) + 4 * i, cc = lane & 7;
+                    const int orow_in = tl.m0 + q * 32 + part * 16 + r;
+                    if (orow_in < tl.m_end) {
+                      const int64_t orow = p.c_row_map ? p.c_row_map[orow_in] : orow_in;
+                      uint8_t* dst = p.c_row_addr ? reinterpret_cast<uint8_t*>(p.c_row_addr[orow_in])
+                                                  : static_cast<uint8_t*>(p.c) + tl.ks * p.split_stride + orow * p.c_stride;
+                      *reinterpret_cast<float4*>(dst + static_cast<int64_t>(col0 + piece * 32) * 4 + cc * 16) =
+                          *reinterpret_cast<const float4*>(stg + r * 128 + ((cc ^ (r & 7)) << 4));
+                    }
+                  }
+                  __syncwarp();
                 }
               }
-              __syncwarp();
+              continue;
             }
-          };
-          if (p.c_dtype == B200MOE_F32 && one_tile) {
+          }
+          if (p.c_dtype == B200MOE_F32) {
             if (row_ok) {
               const int64_t orow = p.c_row_map ? p.c_row_map[row] : row;
               uint8_t* dst = p.c_row_addr ? reinterpret_cast<uint8_t*>(p.c_row_addr[row])
@@ -546,19 +544,10 @@ gemm_block_kernel(const __grid_constant__ RowMaps tmap_a,
             }
             continue;
           }
+          // 16-bit outputs: a thread owns 128 contiguous bytes of ITS row, so a direct store touches
+          // 32 cache lines per instruction.  Transpose through shared memory (16 rows at a time,
+          // 16-byte chunks XOR-swizzled by the row) so that 8 lanes write one full 128-byte row.
           uint4 v[8];
-          if (p.c_dtype == B200MOE_F32) {
-#pragma unroll
-            for (int piece = 0; piece < 2; ++piece) {
-#pragma unroll
-              for (int c = 0; c < 8; ++c) {
-                const float* f = acc + half * 64 + piece * 32 + c * 4;
-                v[c] = make_uint4(__float_as_uint(f[0]), __float_as_uint(f[1]), __float_as_uint(f[2]), __float_as_uint(f[3]));
-              }
-              store_piece(v, static_cast<int64_t>(col0 + piece * 32) * 4);
-            }
-            continue;
-          }
 #pragma unroll
           for (int c = 0; c < 8; ++c) {
             uint32_t w[4];
@@ -570,17 +559,55 @@ gemm_block_kernel(const __grid_constant__ RowMaps tmap_a,
             }
             v[c] = make_uint4(w[0], w[1], w[2], w[3]);
           }
-          store_piece(v, static_cast<int64_t>(col0) * 2);
+          uint8_t* stg = sh->out_stage[e];
+#pragma unroll
+          for (int part = 0; part < 2; ++part) {
+            if ((lane >> 4) == part) {
+              const int r = lane & 15;
+#pragma unroll
+              for (int c = 0; c < 8; ++c)
+                *reinterpret_cast<uint4*>(stg + r * 128 + ((c ^ (r & 7)) << 4)) = v[c];
+            }
+            __syncwarp();
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const int r = (lane >> 3) + 4 * i;               // row inside this 16-row part
+              const int cc = lane & 7;
+              uint4 val = *reinterpret_cast<const uint4*>(stg + r * 128 + ((cc ^ (r & 7)) << 4));
+              const int orow_in = tl.m0 + q * 32 + part * 16 + r;
+              if (orow_in < tl.m_end) {
+                const int64_t orow = p.c_row_map ? p.c_row_map[orow_in] : orow_in;
+                uint8_t* dst = p.c_row_addr ? reinterpret_cast<uint8_t*>(p.c_row_addr[orow_in])
+                                            : static_cast<uint8_t*>(p.c) + tl.ks * p.split_stride + orow * p.c_stride;
+                uint4* out = reinterpret_cast<uint4*>(dst + static_cast<int64_t>(col0) * 2 + cc * 16);
+                if (p.accumulate) {
+                  const uint4 old = *out;
+                  const uint32_t* o = &old.x;
+                  uint32_t* n = &val.x;
+#pragma unroll
+                  for (int i2 = 0; i2 < 4; ++i2) {
+                    if (p.c_dtype == B200MOE_BF16) {
+                      const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&o[i2]));
+                      const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&n[i2]));
+                      const __nv_bfloat162 t2 = __floats2bfloat162_rn(a.x + b.x, a.y + b.y);
+                      n[i2] = *reinterpret_cast<const uint32_t*>(&t2);
+                    } else {
+                      const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&o[i2]));
+                      const float2 b = __half22float2(*reinterpret_cast<const __half2*>(&n[i2]));
+                      const __half2 t2 = __floats2half2_rn(a.x + b.x, a.y + b.y);
+                      n[i2] = *reinterpret_cast<const uint32_t*>(&t2);
+                    }
+                  }
+                }
+                *out = val;
+              }
+            }
+            __syncwarp();
+          }
         }
       } else if (p.swiglu == 2) {
         // SwiGLU with the reference's roundings, written as bf16 (no re-quantization)
-#pragma unroll
-        for (int j = 0; j < 64; ++j) {
-          const float g = bf16r(acc[j]);
-          const float u = bf16r(acc[64 + j]);
-          const float a = bf16r(gate_act(g, p.act));
-          acc[j] = a * u;
-        }
+        gate_up(acc, p.act);
         if (row_ok) {
           uint8_t* dst = static_cast<uint8_t*>(p.c) + static_cast<int64_t>(row) * p.c_stride;
           store_row64(reinterpret_cast<__nv_bfloat16*>(dst) + tl.nt * 128 + hsel * 64, acc);
@@ -588,16 +615,10 @@ gemm_block_kernel(const __grid_constant__ RowMaps tmap_a,
       } else {
         // SwiGLU with the reference's roundings (gate/up GEMM output, silu and the
         // product each rounded to bf16), then 1x128 e4m3 quantization of the row block.
+        gate_up(acc, p.act);
         float amax = 0.f;
 #pragma unroll
-        for (int j = 0; j < 64; ++j) {
-          const float g = bf16r(acc[j]);
-          const float u = bf16r(acc[64 + j]);
-          const float a = bf16r(gate_act(g, p.act));
-          const float h = bf16r(a * u);
-          acc[j] = h;
-          amax = fmaxf(amax, fabsf(h));
-        }
+        for (int j = 0; j < 64; ++j) amax = fmaxf(amax, fabsf(acc[j]));
         const int buf = it & 1;
         sh->amax[buf][hsel][r_in_tile] = amax;
         __syncwarp();
