@@ -29,6 +29,12 @@ int set_dynamic_smem(const void* kernel, size_t bytes);
 int dense_gemm_bf16(const void* a, const void* b, void* c, int64_t c_row_stride_bytes, int64_t M, int64_t N, int64_t K,
                     int epilogue, int32_t* status_word, void* stream);
 
+// Router logits of few tokens on the CUDA cores (router.cu), from the operands of b200moe_router_logits_bf16x3 (gemm_fp8.cu).
+// us, tensor cores with 16 splits -> here: hidden size 7168, 256 experts 18.6 -> 14.7 for one token, 18.8 -> 22.5 for four; 4096
+// and 128 rows 14.4 -> 10.3 and 14.4 -> 16.4.
+constexpr int64_t kRouterFewTokens = 2;
+int router_logits_few(const void* x_bf16, const void* w3_bf16, float* logits, int64_t T, int64_t H, int E, cudaStream_t st);
+
 #define B200MOE_REQUIRE(cond, status, ...)                 \
   do {                                                     \
     if (!(cond)) return ::b200moe::fail((status), __VA_ARGS__); \

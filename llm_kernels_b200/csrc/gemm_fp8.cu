@@ -978,7 +978,11 @@ int b200moe::dense_gemm_bf16(const void* a, const void* b, void* c, int64_t c_ro
 // (about 16 K blocks of 64): the f32 accumulator of the MMA truncates, and the error of a long chain reaches the
 // routing weights (measured 5e-5 relative for 4096-term dot products in two splits, below 1e-5 with short chains);
 // the partial sums are added with IEEE roundings by the selection kernel.
+//
+// A handful of tokens is a matrix-vector product: b200moe::router_logits_few (router.cu) reads the three parts once on all SMs
+// and leaves one sum.
 extern "C" int b200moe_router_ksplits(int64_t T, int64_t H, int E) {
+  if (T <= kRouterFewTokens) return 1;
   const int64_t tiles = std::max<int64_t>(1, ((T + BM - 1) / BM) * ((E + BN - 1) / BN));
   const int64_t kb = std::max<int64_t>(1, 3 * H / 64);
   int64_t ks = std::max<int64_t>(1, std::min<int64_t>(16, std::max<int64_t>(148 / tiles, (kb + 15) / 16)));
@@ -997,6 +1001,7 @@ extern "C" int b200moe_router_logits_bf16x3(const void* x_bf16, const void* w3_b
   B200MOE_REQUIRE(aligned(x_bf16, 16) && aligned(w3_bf16, 16) && aligned(partials, 16), B200MOE_BAD_ALIGN,
                   "router_logits_bf16x3: alignment");
   if (T == 0) return B200MOE_OK;
+  if (T <= kRouterFewTokens && ksplits == 1) return router_logits_few(x_bf16, w3_bf16, partials, T, H, E, as_stream(stream));
   GemmParams p{nullptr, 0, nullptr, partials, static_cast<int64_t>(E) * 4, nullptr, 0, nullptr, nullptr, T, E,
                static_cast<int>(3 * H * 2), 1, 1, B200MOE_F32, 0, nullptr, ksplits, T * static_cast<int64_t>(E) * 4,
                static_cast<int>(H * 2), nullptr, nullptr, 0, 0};

@@ -31,33 +31,38 @@ __device__ __forceinline__ uint32_t order_key(float v) {
   return (u & 0x80000000u) ? ~u : u | 0x80000000u;
 }
 
-// Phase B for one token by one warp.  v[j] is the f32 logit of expert lane + 32 j (J registers cover E experts), `sfc` E floats
-// of shared memory private to the warp (used by the group selection only).
+// Scores of one token's experts from their logits, in place in shared memory, by the calling warp (softmax; sigmoid scores need
+// no other expert and are formed where the logits are).
+__device__ __forceinline__ void softmax_scores(float* logit, int E) {
+  const int lane = threadIdx.x & 31;
+  float m = -INFINITY;
+#pragma unroll 1
+  for (int e = lane; e < E; e += 32) m = fmaxf(m, logit[e]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+  float sum = 0.f;
+#pragma unroll 1
+  for (int e = lane; e < E; e += 32) { const float ex = expf(logit[e] - m); logit[e] = ex; sum += ex; }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+#pragma unroll 1
+  for (int e = lane; e < E; e += 32) logit[e] = __fdiv_rn(logit[e], sum);
+}
+__device__ __forceinline__ float sigmoid_score(float logit) { return __fdiv_rn(1.f, 1.f + expf(-logit)); }
+
+// Phase B for one token by one warp.  `score` holds the E scores, `sfc` is E floats of scratch (used by the group selection
+// only), both in shared memory and private to the warp; J registers per lane cover E experts.
 //
-// What bounds it: the latency of eight dependent picks for a token.  Scores stay in registers and a pick is two redux.sync on
-// integer images of the scores; with scores in shared memory, a pick was eight loads and ten shuffles and the scan of the
-// groups met itself in one bank (256 experts, top-8 of 4 of 8 groups: one token 15.2 -> 9.4 us, 4096 tokens 37 -> 30 us).
+// What bounds it: the latency of eight dependent picks for a token, and for few tokens the fetch of this code.  The candidates
+// stay in registers and a pick is two redux.sync on integer images of the scores; with the candidates in shared memory, a pick
+// was eight loads and ten shuffles and the scan of the groups met itself in one bank.
 template <int J>
-__device__ void select_token(const RouterParams& p, int64_t t, float (&v)[J], float* sfc) {
+__device__ void select_token(const RouterParams& p, int64_t t, const float* score, float* sfc) {
   const int lane = threadIdx.x & 31;
   const int E = p.E;
-  if (p.scoring == 1) {
-    float m = -INFINITY;
+  float v[J];
 #pragma unroll
-    for (int j = 0; j < J; ++j) if (lane + 32 * j < E) m = fmaxf(m, v[j]);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    float sum = 0.f;
-#pragma unroll
-    for (int j = 0; j < J; ++j) if (lane + 32 * j < E) { v[j] = expf(v[j] - m); sum += v[j]; }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-#pragma unroll
-    for (int j = 0; j < J; ++j) v[j] = __fdiv_rn(v[j], sum);
-  } else {
-#pragma unroll
-    for (int j = 0; j < J; ++j) v[j] = __fdiv_rn(1.f, 1.f + expf(-v[j]));
-  }
+  for (int j = 0; j < J; ++j) v[j] = lane + 32 * j < E ? score[lane + 32 * j] : 0.f;
   float s[J];                                            // selection scores
 #pragma unroll
   for (int j = 0; j < J; ++j) {
@@ -136,13 +141,16 @@ __device__ void select_token(const RouterParams& p, int64_t t, float (&v)[J], fl
   }
 }
 
-// The logits of one token in shared memory -> select_token's registers.
+// The same from logits in shared memory.
 template <int J>
-__device__ __forceinline__ void select_from_shared(const RouterParams& p, int64_t t, const float* logit, float* sfc) {
-  float v[J];
-#pragma unroll
-  for (int j = 0; j < J; ++j) { const int e = (threadIdx.x & 31) + 32 * j; v[j] = e < p.E ? logit[e] : 0.f; }
-  select_token<J>(p, t, v, sfc);
+__device__ __forceinline__ void select_from_logits(const RouterParams& p, int64_t t, float* logit, float* sfc) {
+  if (p.scoring == 1) softmax_scores(logit, p.E);
+  else {
+#pragma unroll 1
+    for (int e = threadIdx.x & 31; e < p.E; e += 32) logit[e] = sigmoid_score(logit[e]);
+  }
+  __syncwarp();
+  select_token<J>(p, t, logit, sfc);
 }
 
 // ---- E <= 32: warp per token ------------------------------------------------------
@@ -181,7 +189,7 @@ __global__ void __launch_bounds__(256) router_small_kernel(const T* __restrict__
     }
   }
   __syncwarp();
-  select_from_shared<1>(p, t, s_logit[warp], s_sfc[warp]);
+  select_from_logits<1>(p, t, s_logit[warp], s_sfc[warp]);
 }
 
 // ---- E <= 256: 32 tokens x E tile, K chunks of 32 through shared memory -----------
@@ -251,38 +259,99 @@ __global__ void __launch_bounds__(256) router_tiled_kernel(const T* __restrict__
   __syncthreads();
   for (int a = 0; a < 4; ++a) {
     const int64_t t = t0 + ty * 4 + a;
-    if (t < p.T) select_from_shared<kMaxE / 32>(p, t, lg + (ty * 4 + a) * kMaxE, sf + ty * kMaxE);
+    if (t < p.T) select_from_logits<kMaxE / 32>(p, t, lg + (ty * 4 + a) * kMaxE, sf + ty * kMaxE);
     __syncwarp();
   }
 }
 
+// ---- logits of few tokens ------------------------------------------------------------------
+// logits[t, e] = x[t] . w[e] in f32, w given as its three bf16 parts side by side (hi + mid + lo = w exactly).  Bound by the
+// 6 E H bytes of the parts.  A block takes two experts and up to two tokens, four warps an expert, each a quarter of the columns;
+// their sums are added in order.
+constexpr int kFewTokens = 2;
+__global__ void __launch_bounds__(256) router_few_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w3,
+                                                         float* __restrict__ logits, int64_t T, int64_t H, int E) {
+  __shared__ float part[8][kFewTokens];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int e = static_cast<int>(blockIdx.x) * 2 + (warp >> 2);       // E is a multiple of 128
+  const int64_t t0 = static_cast<int64_t>(blockIdx.y) * kFewTokens;
+  const int tokens = static_cast<int>(min(T - t0, static_cast<int64_t>(kFewTokens)));
+  const __nv_bfloat16* w = w3 + static_cast<int64_t>(e) * 3 * H;
+  float acc[kFewTokens];
+#pragma unroll
+  for (int k = 0; k < kFewTokens; ++k) acc[k] = 0.f;
+#pragma unroll 2
+  for (int64_t h = ((warp & 3) * 32 + lane) * 8; h < H; h += 1024) {  // H is a multiple of 64
+    float hi[8], mid[8], lo[8];
+    load8(w + h, hi);
+    load8(w + H + h, mid);
+    load8(w + 2 * H + h, lo);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) hi[i] = (hi[i] + mid[i]) + lo[i];
+#pragma unroll
+    for (int k = 0; k < kFewTokens; ++k) {
+      if (k >= tokens) break;
+      float v[8];
+      load8(x + (t0 + k) * H + h, v);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[k] = fmaf(v[i], hi[i], acc[k]);
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < kFewTokens; ++k) {
+    if (k >= tokens) break;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
+    if (lane == 0) part[warp][k] = acc[k];
+  }
+  __syncthreads();
+  if (threadIdx.x < 2 * kFewTokens) {
+    const int k = threadIdx.x & (kFewTokens - 1), g = threadIdx.x / kFewTokens;
+    if (k < tokens)
+      logits[(t0 + k) * E + static_cast<int64_t>(blockIdx.x) * 2 + g] =
+          ((part[g * 4][k] + part[g * 4 + 1][k]) + part[g * 4 + 2][k]) + part[g * 4 + 3][k];
+  }
+}
+
+int router_logits_few(const void* x_bf16, const void* w3_bf16, float* logits, int64_t T, int64_t H, int E, cudaStream_t st) {
+  const dim3 grid(static_cast<unsigned>(E / 2), static_cast<unsigned>((T + kFewTokens - 1) / kFewTokens));
+  router_few_kernel<<<grid, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(x_bf16), static_cast<const __nv_bfloat16*>(w3_bf16), logits, T, H, E);
+  return check_launch("router_logits");
+}
+
 // ---- selection from precomputed logits (tensor-core path) ----------------------------------
-// One warp per token.  The partial sums are added in index order; the loads of 16 splits are in flight at a time.
+// Eight tokens per block.  All threads add the partial sums, an expert each (in index order, eight loads in flight), then a warp
+// selects for one token.  A thread per expert keeps the code short: with a warp per token all the way, eight experts per lane
+// unrolled, a single token waited longer for instructions than for data (decode of one token, with the logits above: 117 -> 108 us).
+constexpr int kSelectTokens = 8;
 template <int J>
 __global__ void __launch_bounds__(256) router_select_kernel(const float* __restrict__ partials,
                                                             int nsplit, int64_t row_stride, RouterParams p) {
-  extern __shared__ __align__(16) float smem[];   // [8 warps][E]
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t t = static_cast<int64_t>(blockIdx.x) * 8 + warp;
-  if (t >= p.T) return;
-  float v[J];
-#pragma unroll
-  for (int j = 0; j < J; ++j) v[j] = 0.f;
-  const float* src = partials + t * row_stride + lane;
+  extern __shared__ __align__(16) float smem[];   // [8 tokens][2][E]
+  const int warp = threadIdx.x >> 5;
+  const int64_t t0 = static_cast<int64_t>(blockIdx.x) * kSelectTokens;
+  const int tokens = static_cast<int>(min(p.T - t0, static_cast<int64_t>(kSelectTokens)));
   const int64_t step = p.T * row_stride;
-  constexpr int kAhead = J <= 8 ? 16 : 2;
-  for (int s0 = 0; s0 < nsplit; s0 += kAhead) {
-    float x[kAhead][J];
+#pragma unroll 1
+  for (int i = threadIdx.x; i < tokens * p.E; i += 256) {
+    const int k = i / p.E, e = i - k * p.E;
+    const float* src = partials + (t0 + k) * row_stride + e;
+    float v = 0.f;
+#pragma unroll 1
+    for (int s0 = 0; s0 < nsplit; s0 += 8) {
+      float x[8];
 #pragma unroll
-    for (int s = 0; s < kAhead; ++s)
+      for (int s = 0; s < 8; ++s) x[s] = s0 + s < nsplit ? src[(s0 + s) * step] : 0.f;
 #pragma unroll
-      for (int j = 0; j < J; ++j) x[s][j] = s0 + s < nsplit && lane + 32 * j < p.E ? src[(s0 + s) * step + 32 * j] : 0.f;
-#pragma unroll
-    for (int s = 0; s < kAhead; ++s)
-#pragma unroll
-      for (int j = 0; j < J; ++j) v[j] += x[s][j];       // past the last split: + 0, which changes nothing
+      for (int s = 0; s < 8; ++s) v += x[s];             // past the last split: + 0, which changes nothing
+    }
+    smem[k * 2 * p.E + e] = p.scoring == 1 ? v : sigmoid_score(v);
   }
-  select_token<J>(p, t, v, smem + warp * p.E);
+  __syncthreads();
+  if (warp >= tokens) return;
+  float* score = smem + warp * 2 * p.E;
+  if (p.scoring == 1) { softmax_scores(score, p.E); __syncwarp(); }
+  select_token<J>(p, t0 + warp, score, score + p.E);
 }
 
 constexpr size_t kTiledSmem = sizeof(float) * (kTM * kLd + kMaxE * kLd + kTM * kMaxE + 8 * kMaxE);
@@ -352,7 +421,9 @@ extern "C" int b200moe_router_select(const float* partials, int nsplit, int64_t 
   RouterParams p{nullptr, bias, T, 0, E, top_k, n_group, topk_group, scoring, norm_topk_prob,
                  routed_scaling_factor, topk_idx, topk_weight};
   const unsigned grid = static_cast<unsigned>((T + 7) / 8);
-  const size_t smem = sizeof(float) * 8 * E;                 // at most 32 KB
+  const size_t smem = sizeof(float) * kSelectTokens * 2 * E;
+  if (E > 256)
+    if (int rc = set_dynamic_smem(reinterpret_cast<const void*>(router_select_kernel<32>), sizeof(float) * kSelectTokens * 2 * 1024)) return rc;
   auto launch = [&](auto kernel) { kernel<<<grid, 256, smem, as_stream(stream)>>>(partials, nsplit, partials_row_stride, p); };
   if (E <= 32) launch(router_select_kernel<1>);
   else if (E <= 256) launch(router_select_kernel<8>);

@@ -1,0 +1,143 @@
+"""The launches around the GEMMs at the sizes where their routes and tiles change (csrc/router.cu, route.cu, permute.cu, quant.cu)."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _bits(t):
+    return t.contiguous().view({1: torch.uint8, 2: torch.int16, 4: torch.int32, 8: torch.int64}[t.element_size()])
+
+
+# one launch up to 65536 slots, chunks of 1024; three launches beyond.  Some ids lie outside [0, E).
+@pytest.mark.parametrize("n", [1, 31, 33, 1023, 1024, 1025, 5000, 65535, 65536, 65537])
+@pytest.mark.parametrize("E", [1, 7, 256, 1024])
+def test_sort_is_stable_at_its_chunk_edges(n, E):
+    from llm_kernels_b200.moe import group_gemm_kernel as G
+    g = torch.Generator().manual_seed(n + E)
+    ids = torch.randint(-1, E + 1, (n,), generator=g)
+    ids[::3] = int(torch.randint(0, E, (1,), generator=g))          # one expert with a third of the slots
+    order, dst, seg = (t.cpu() for t in G.run_moe_ep_preproess(ids.cuda(), E))
+    ok = (ids >= 0) & (ids < E)
+    slots = ok.nonzero().view(-1)
+    rows = slots[torch.sort(ids[slots], stable=True)[1]]
+    want = torch.full((n,), -1, dtype=torch.int32)
+    want[rows] = torch.arange(len(rows), dtype=torch.int32)
+    assert torch.equal(dst, want) and torch.equal(order[:len(rows)], ids[rows])
+    assert torch.equal(seg, torch.cat([torch.zeros(1, dtype=torch.int64), torch.bincount(ids[slots], minlength=E).cumsum(0)]))
+
+
+# registers per lane 1, 8 and 32; groups that do and do not divide the 32 lanes; more splits than loads in flight
+@pytest.mark.parametrize("T", [1, 8, 9])
+@pytest.mark.parametrize("E,groups,kept,k,splits", [(8, 1, 1, 2, 1), (32, 4, 2, 4, 9), (48, 3, 2, 5, 3), (256, 8, 4, 8, 16),
+                                                    (257, 1, 1, 8, 2), (1024, 32, 7, 32, 1)])
+@pytest.mark.parametrize("scoring", [0, 1])
+def test_selection_from_partial_sums(T, E, groups, kept, k, splits, scoring):
+    from llm_kernels_b200 import _native as N
+    g = torch.Generator().manual_seed(E + T)
+    stride = E + 3
+    part = torch.randn(splits, T, stride, generator=g) * 0.01
+    bias = torch.randint(-40, 40, (E,), generator=g) / 4.0
+    idx = torch.empty(T, k, dtype=torch.int64, device="cuda")
+    w = torch.empty(T, k, device="cuda")
+    pc, bc = part.cuda(), bias.cuda()
+    N.check(N.lib().b200moe_router_select(pc.data_ptr(), splits, stride, bc.data_ptr(), T, E, k, groups, kept, scoring, 1, 1.5,
+                                          idx.data_ptr(), w.data_ptr(), N.stream()))
+    logits = part[..., :E].double().sum(0)
+    score = logits.sigmoid() if scoring == 0 else logits.softmax(-1)
+    choice = score + bias.double()
+    sure = torch.ones(T, dtype=torch.bool)
+    if groups > 1:
+        gs = choice.view(T, groups, -1).topk(2, dim=-1)[0].sum(-1)
+        best, order = torch.sort(gs, dim=-1, descending=True, stable=True)
+        sure = best[:, kept - 1] - best[:, kept] > 1e-5             # f32 could keep either group otherwise
+        keep = torch.zeros_like(gs, dtype=torch.bool).scatter_(1, order[:, :kept], True)
+        choice = torch.where(keep.repeat_interleave(E // groups, 1), choice, 0.0)
+    gap, want = torch.sort(choice, dim=-1, descending=True, stable=True)
+    for t in range(T):
+        # picks are compared up to the first pair that f32 could order either way
+        close = ((gap[t, :k] - gap[t, 1:k + 1]) < 1e-5).nonzero().view(-1) if k < E else torch.tensor([], dtype=torch.int64)
+        n = (int(close[0]) if len(close) else k) if sure[t] else 0
+        got = idx[t].cpu()
+        assert torch.equal(got[:n], want[t, :n])
+        ref = score[t, got] / (score[t, got].sum() + 1e-20) * 1.5
+        # a few f32 roundings of the scores and of their sum of up to 32 terms
+        assert float(((w[t].cpu().double() - ref) / ref).abs().max()) < 40 * 2 ** -23
+
+
+@pytest.mark.parametrize("T", [1, 2])
+@pytest.mark.parametrize("H,E", [(64, 128), (1088, 128), (7168, 256)])
+def test_router_logits_of_few_tokens(T, H, E):
+    """Against 64 bits.  The f32 weight is exactly the sum of its parts; a lane adds H / 128 products, then 8 sums follow: as many
+    roundings of partial sums at most, each below the sum of the products' sizes."""
+    from llm_kernels_b200 import _native as N
+    g = torch.Generator().manual_seed(T)
+    x = torch.randn(T, H, generator=g).to(torch.bfloat16)
+    w = torch.randn(E, H, generator=g) * 0.02
+    hi = w.to(torch.bfloat16)
+    mid = (w - hi.float()).to(torch.bfloat16)
+    lo = (w - hi.float() - mid.float()).to(torch.bfloat16)
+    w3 = torch.cat([hi, mid, lo], 1).cuda()
+    assert N.lib().b200moe_router_ksplits(T, H, E) == 1
+    part = torch.full((T, E), float("nan"), device="cuda")
+    xc = x.cuda()
+    N.check(N.lib().b200moe_router_logits_bf16x3(xc.data_ptr(), w3.data_ptr(), part.data_ptr(), T, H, E, 1, N.stream()))
+    exact = x.double() @ w.double().t()
+    size = x.double().abs() @ w.double().abs().t()
+    assert float(((part.cpu().double() - exact).abs() / size).max()) < (H / 128 + 9) * 2 ** -24
+
+
+# a block per round of columns below 512 tokens, one block per token from there on; rows that end inside a warp
+@pytest.mark.parametrize("T", [1, 3, 511, 512])
+@pytest.mark.parametrize("H", [128, 2176, 7168])
+@pytest.mark.parametrize("topk", [1, 5, 8])
+def test_permute_and_unpermute(T, H, topk):
+    from llm_kernels_b200 import _native as N
+    from llm_kernels_b200.quantization import fp8_kernel, int8_kernel
+    g = torch.Generator(device="cuda").manual_seed(H)
+    E, S = 16, T * topk
+    x = torch.randn(T, H, generator=g, device="cuda").to(torch.bfloat16)
+    ids = torch.rand(T, E, generator=g, device="cuda").topk(topk, dim=1)[1]
+    dst = torch.randperm(S, generator=g, device="cuda").to(torch.int32).view(T, topk)
+    lo, hi = 2, 13                                                   # some slots belong to other ranks
+    here = (ids >= lo) & (ids <= hi)
+    rows = dst[here].long()
+    src = torch.arange(T, device="cuda").view(T, 1).expand(T, topk)[here]
+    for name, quant, stride in (("fp8", fp8_kernel.act_quant, H + 8), ("fp8", fp8_kernel.act_quant, H + 16),
+                                ("int8", lambda v: int8_kernel.act_quant(v, rounding="floor_half"), H + 8)):
+        out = torch.zeros(S, stride, dtype=torch.uint8, device="cuda")
+        s = torch.zeros(S, H // 128 + 1, device="cuda")
+        fn = getattr(N.lib(), f"b200moe_permute_quant_{name}")
+        tail = (1,) if name == "int8" else ()
+        N.check(fn(x.data_ptr(), N.BF16, dst.data_ptr(), ids.data_ptr(), lo, hi, T, topk, H, out.data_ptr(), stride, s.data_ptr(),
+                   H // 128 + 1, *tail, N.stream()))
+        q, qs = quant(x)
+        want = torch.zeros_like(out)
+        want[rows, :H] = _bits(q)[src]
+        want_s = torch.zeros_like(s)
+        want_s[rows, :H // 128] = qs.float()[src]
+        assert torch.equal(out, want) and torch.equal(s, want_s)
+    down = torch.randn(S, H, generator=g, device="cuda").to(torch.bfloat16)
+    w = torch.rand(T, topk, generator=g, device="cuda")
+    y = torch.empty(T, H, dtype=torch.bfloat16, device="cuda")
+    N.check(N.lib().b200moe_post_reorder(down.data_ptr(), N.BF16, y.data_ptr(), dst.data_ptr(), ids.data_ptr(), w.data_ptr(), lo, hi,
+                                         T, topk, H, N.stream()))
+    acc = torch.zeros(T, H, dtype=torch.float64, device="cuda")
+    for j in range(topk):                                            # the kernel's f32 multiply-adds, in 64 bits and rounded
+        acc = torch.where(here[:, j:j + 1], (acc + down[dst[:, j].long()].double() * w[:, j:j + 1].double()).float().double(), acc)
+    assert torch.equal(y, acc.float().to(torch.bfloat16))
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 128), (3, 384), (129, 2176)])
+@pytest.mark.parametrize("pad", [0, 8, 16])
+def test_fp8_quantizer_rows_of_any_stride(rows, cols, pad):
+    from llm_kernels_b200 import _native as N
+    from oracle import restate as R
+    x = torch.randn(rows, cols, generator=torch.Generator().manual_seed(cols)).to(torch.bfloat16)
+    xc = x.cuda()
+    y = torch.zeros(rows, cols + pad, dtype=torch.uint8, device="cuda")
+    s = torch.zeros(rows, cols // 128 + (pad > 0), device="cuda")
+    N.check(N.lib().b200moe_act_quant_fp8(xc.data_ptr(), N.BF16, rows, cols, y.data_ptr(), cols + pad, s.data_ptr(), s.shape[1], N.stream()))
+    q, qs = R.act_quant_fp8(x)
+    assert torch.equal(y[:, :cols].cpu(), _bits(q)) and torch.equal(s[:, :cols // 128].cpu(), qs)
+    assert not y[:, cols:].any() and not s[:, cols // 128:].any()
