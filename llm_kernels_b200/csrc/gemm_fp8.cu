@@ -247,6 +247,8 @@ gemm_block_kernel(const __grid_constant__ RowMaps tmap_a,
     ptx::tmem_alloc<CG>(&sh->tmem_base, kTmemCols);
     ptx::tmem_relinquish<CG>();
   }
+  // the setup above overlaps the tail of the kernel before; from here on its results are read
+  wait_for_predecessors();
   // group row offsets
   for (int g = threadIdx.x; g <= p.num_groups; g += kThreads)
     sh->seg[g] = p.seg ? static_cast<int32_t>(p.seg[g]) : (g == 0 ? 0 : static_cast<int32_t>(p.M_total));
@@ -663,6 +665,9 @@ gemm_block_kernel(const __grid_constant__ RowMaps tmap_a,
 template <int KIND, bool PAIR>
 static int launch_gemm_as(const RowMaps& ma, const CUtensorMap& mb, const GemmParams& p, int grid, cudaStream_t st) {
   if (int rc = set_dynamic_smem(reinterpret_cast<const void*>(gemm_block_kernel<KIND, PAIR>), kSmemBytes)) return rc;
+  if constexpr (!PAIR)
+    return launch_dependent("gemm_block_kernel", gemm_block_kernel<KIND, PAIR>, dim3(static_cast<unsigned>(grid)), kThreads, kSmemBytes,
+                            st, ma, mb, p);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(grid));
   cfg.blockDim = dim3(kThreads);
@@ -670,10 +675,10 @@ static int launch_gemm_as(const RowMaps& ma, const CUtensorMap& mb, const GemmPa
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = PAIR ? 2 : 1;
+  attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
+  cfg.attrs = attr;                   // pairs serve large products: no dependent launch, whose gain is a few microseconds
   cfg.numAttrs = 1;
   cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_block_kernel<KIND, PAIR>, ma, mb, p);
   if (e != cudaSuccess) return fail(B200MOE_LAUNCH_FAILED, "gemm_block_kernel launch: %s", cudaGetErrorString(e));
@@ -764,6 +769,8 @@ namespace b200moe {
 template <typename T>
 __global__ void __launch_bounds__(256) sum_splits_kernel(const float* __restrict__ partials, int ksplits,
                                                          int64_t n, T* __restrict__ out) {
+  wait_for_predecessors();
+  allow_dependents();
   for (int64_t i = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) * 4; i < n;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x * 4) {
     float4 acc = *reinterpret_cast<const float4*>(partials + i);
@@ -785,10 +792,11 @@ __global__ void __launch_bounds__(256) sum_splits_kernel(const float* __restrict
 
 static int sum_splits(const float* partials, int ksplits, int64_t n, void* c, int c_dtype, cudaStream_t st) {
   const unsigned grid = static_cast<unsigned>(std::min<int64_t>((n / 4 + 255) / 256, 148 * 8));
-  if (c_dtype == B200MOE_F32) sum_splits_kernel<float><<<grid, 256, 0, st>>>(partials, ksplits, n, static_cast<float*>(c));
-  else if (c_dtype == B200MOE_BF16) sum_splits_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(partials, ksplits, n, static_cast<__nv_bfloat16*>(c));
-  else sum_splits_kernel<__half><<<grid, 256, 0, st>>>(partials, ksplits, n, static_cast<__half*>(c));
-  return check_launch("sum_splits");
+  auto go = [&](auto* out) {
+    return launch_dependent("sum_splits", sum_splits_kernel<std::remove_pointer_t<decltype(out)>>, dim3(grid), 256, 0, st, partials, ksplits, n, out);
+  };
+  if (c_dtype == B200MOE_F32) return go(static_cast<float*>(c));
+  return c_dtype == B200MOE_BF16 ? go(static_cast<__nv_bfloat16*>(c)) : go(static_cast<__half*>(c));
 }
 
 template <int KIND>

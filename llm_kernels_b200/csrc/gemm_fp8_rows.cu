@@ -173,6 +173,8 @@ gemm_fp8_rows_kernel(const __grid_constant__ w4::RowMaps tmap_a, const __grid_co
     ptx::tmem_alloc<1>(&sh->tmem_base, w4::kTmemCols);
     ptx::tmem_relinquish<1>();
   }
+  // the setup above overlaps the tail of the kernel before; from here on its results are read
+  wait_for_predecessors();
   for (int g = threadIdx.x; g <= p.num_groups; g += kThreads)
     sh->seg[g] = p.seg ? static_cast<int32_t>(p.seg[g]) : (g == 0 ? 0 : static_cast<int32_t>(p.M_total));
   ptx::tc_fence_before_sync();
@@ -409,8 +411,7 @@ int launch_fp8(const void* a, int64_t a_stride, const float* a_s, int64_t a_s_st
   Params p{a_s, a_s_stride, b_s, c, c_stride, c_s, c_s_stride, seg, widx, M_total, static_cast<int>(N), static_cast<int>(K),
            num_groups, c_dtype, fused, act, status};
   if (int rc = set_dynamic_smem(reinterpret_cast<const void*>(gemm_fp8_rows_kernel), kSmem)) return rc;
-  gemm_fp8_rows_kernel<<<sms, kThreads, kSmem, st>>>(ma, mb, p);
-  return check_launch("gemm_fp8_rows_kernel");
+  return launch_dependent("gemm_fp8_rows_kernel", gemm_fp8_rows_kernel, dim3(static_cast<unsigned>(sms)), kThreads, kSmem, st, ma, mb, p);
 }
 
 }  // namespace rows

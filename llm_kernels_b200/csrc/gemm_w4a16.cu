@@ -177,6 +177,8 @@ gemm_w4a16_kernel(const __grid_constant__ w4::RowMaps tmap_a, const __grid_const
     ptx::tmem_alloc<1>(&sh->tmem_base, w4::kTmemCols);
     ptx::tmem_relinquish<1>();
   }
+  // the setup above overlaps the tail of the kernel before; from here on its results are read
+  wait_for_predecessors();
   for (int g = threadIdx.x; g <= p.num_groups; g += kThreads) sh->seg[g] = static_cast<int32_t>(p.seg[g]);
   ptx::tc_fence_before_sync();
   __syncthreads();
@@ -405,8 +407,7 @@ constexpr int kWideChunkRows = 48;
 template <int CHUNK>
 static int launch_chunk(const w4::RowMaps& ma, const CUtensorMap& mp, const Params& p, int sms, cudaStream_t st) {
   if (int rc = set_dynamic_smem(reinterpret_cast<const void*>(gemm_w4a16_kernel<CHUNK>), kSmem)) return rc;
-  gemm_w4a16_kernel<CHUNK><<<sms, kThreads, kSmem, st>>>(ma, mp, p);
-  return check_launch("gemm_w4a16_kernel");
+  return launch_dependent("gemm_w4a16_kernel", gemm_w4a16_kernel<CHUNK>, dim3(static_cast<unsigned>(sms)), kThreads, kSmem, st, ma, mp, p);
 }
 
 static int launch(const void* a, int64_t a_stride, const void* b_packed, const void* scale_zero_t, void* c, int c_dtype,

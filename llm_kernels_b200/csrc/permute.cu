@@ -45,6 +45,8 @@ __global__ void __launch_bounds__(256) pre_reorder_kernel(
     int topk, int64_t H) {
   __shared__ int32_t s_dst[kMaxK], s_exp[kMaxK];
   const int64_t t = blockIdx.x;
+  wait_for_predecessors();
+  allow_dependents();
   const int n = load_slots(src2dst, topk_ids, t, topk, lo, hi, s_dst, s_exp);
   if (n == 0) return;
   for (int64_t c = first_chunk() * 8; c < H; c += chunk_step() * 8) {
@@ -73,6 +75,8 @@ __global__ void __launch_bounds__(256) permute_quant_fp8_kernel(
     uint8_t* __restrict__ out_q, int64_t q_stride, float* __restrict__ out_s, int64_t s_stride, bool wide) {
   __shared__ int32_t s_dst[kMaxK], s_exp[kMaxK];
   const int64_t t = blockIdx.x;
+  wait_for_predecessors();
+  allow_dependents();
   const int n = load_slots(src2dst, topk_ids, t, topk, lo, hi, s_dst, s_exp);
   if (n == 0) return;
   const int64_t chunks = H / 16;                        // multiple of 8
@@ -118,6 +122,8 @@ __global__ void __launch_bounds__(256) permute_quant_int8_kernel(
     int rounding) {
   __shared__ int32_t s_dst[kMaxK], s_exp[kMaxK];
   const int64_t t = blockIdx.x;
+  wait_for_predecessors();
+  allow_dependents();
   const int n = load_slots(src2dst, topk_ids, t, topk, lo, hi, s_dst, s_exp);
   if (n == 0) return;
   const int64_t chunks = H / 8;
@@ -199,6 +205,8 @@ __global__ void __launch_bounds__(256) post_reorder_kernel(
   __shared__ int32_t s_dst[kMaxK], s_exp[kMaxK];
   __shared__ float s_w[kMaxK];
   const int64_t t = blockIdx.x;
+  wait_for_predecessors();
+  allow_dependents();
   const int n = load_slots(src2dst, topk_ids, t, topk, lo, hi, s_dst, s_exp);
   if (threadIdx.x < n) s_w[threadIdx.x] = w[t * topk + (s_exp[threadIdx.x] >> 16)];
   __syncthreads();
@@ -279,12 +287,12 @@ extern "C" int b200moe_pre_reorder(const void* x, int x_dtype, void* out, int ou
   const RowGrid g = row_grid(T, H / 8);
 #define LAUNCH_PRE(TI)                                                                            \
   if (out_dtype == B200MOE_FP8_E4M3)                                                              \
-    pre_reorder_kernel<TI, uint8_t><<<g.grid, g.threads, 0, st>>>(static_cast<const TI*>(x), static_cast<uint8_t*>(out), src2dst, topk_ids, a1_scales, start_expert_id, end_expert_id, topk, H); \
+    return launch_dependent("pre_reorder", pre_reorder_kernel<TI, uint8_t>, g.grid, g.threads, 0, st, static_cast<const TI*>(x), static_cast<uint8_t*>(out), src2dst, topk_ids, a1_scales, start_expert_id, end_expert_id, topk, H); \
   else                                                                                            \
-    pre_reorder_kernel<TI, TI><<<g.grid, g.threads, 0, st>>>(static_cast<const TI*>(x), static_cast<TI*>(out), src2dst, topk_ids, a1_scales, start_expert_id, end_expert_id, topk, H)
+    return launch_dependent("pre_reorder", pre_reorder_kernel<TI, TI>, g.grid, g.threads, 0, st, static_cast<const TI*>(x), static_cast<TI*>(out), src2dst, topk_ids, a1_scales, start_expert_id, end_expert_id, topk, H)
   DISPATCH_16BIT_OR_F32(x_dtype, LAUNCH_PRE)
 #undef LAUNCH_PRE
-  return check_launch("pre_reorder");
+  return B200MOE_OK;
 }
 
 extern "C" int b200moe_permute_quant_fp8(const void* x, int x_dtype, const int32_t* src2dst,
@@ -305,12 +313,12 @@ extern "C" int b200moe_permute_quant_fp8(const void* x, int x_dtype, const int32
   cudaStream_t st = as_stream(stream);
   const RowGrid g = row_grid(T, H / 16);
 #define LAUNCH_PQ(TI)                                                                           \
-  permute_quant_fp8_kernel<TI><<<g.grid, g.threads, 0, st>>>(static_cast<const TI*>(x), src2dst, topk_ids, \
+  return launch_dependent("permute_quant_fp8", permute_quant_fp8_kernel<TI>, g.grid, g.threads, 0, st, static_cast<const TI*>(x), src2dst, topk_ids, \
       start_expert_id, end_expert_id, topk, H, static_cast<uint8_t*>(out_q),                     \
       out_q_row_stride_bytes, out_s, out_s_row_stride, aligned(out_q, 16) && out_q_row_stride_bytes % 16 == 0)
   DISPATCH_16BIT_OR_F32(x_dtype, LAUNCH_PQ)
 #undef LAUNCH_PQ
-  return check_launch("permute_quant_fp8");
+  return B200MOE_OK;
 }
 
 extern "C" int b200moe_permute_quant_int8(const void* x, int x_dtype, const int32_t* src2dst,
@@ -332,12 +340,12 @@ extern "C" int b200moe_permute_quant_int8(const void* x, int x_dtype, const int3
   cudaStream_t st = as_stream(stream);
   const RowGrid g = row_grid(T, H / 8);
 #define LAUNCH_PQ8(TI)                                                                           \
-  permute_quant_int8_kernel<TI><<<g.grid, g.threads, 0, st>>>(static_cast<const TI*>(x), src2dst, topk_ids, \
+  return launch_dependent("permute_quant_int8", permute_quant_int8_kernel<TI>, g.grid, g.threads, 0, st, static_cast<const TI*>(x), src2dst, topk_ids, \
       start_expert_id, end_expert_id, topk, H, static_cast<int8_t*>(out_q),                       \
       out_q_row_stride_bytes, out_s, out_s_row_stride, rounding)
   DISPATCH_16BIT_OR_F32(x_dtype, LAUNCH_PQ8)
 #undef LAUNCH_PQ8
-  return check_launch("permute_quant_int8");
+  return B200MOE_OK;
 }
 
 extern "C" int b200moe_gather_rows(const void* src, void* dst, const int32_t* row_map, int64_t n,
@@ -389,9 +397,9 @@ extern "C" int b200moe_post_reorder(const void* down_output, int dtype, void* ou
   cudaStream_t st = as_stream(stream);
   const RowGrid g = row_grid(T, H / 8);
 #define LAUNCH_POST(TT)                                                                      \
-  (T < kFewTokens ? post_reorder_kernel<TT, 4> : post_reorder_kernel<TT, 1>)<<<g.grid, g.threads, 0, st>>>( \
+  return launch_dependent("post_reorder", T < kFewTokens ? post_reorder_kernel<TT, 4> : post_reorder_kernel<TT, 1>, g.grid, g.threads, 0, st, \
       static_cast<const TT*>(down_output), static_cast<TT*>(out), src2dst, topk_ids, topk_weights, start_expert_id, end_expert_id, topk, H)
   DISPATCH_16BIT_OR_F32(dtype, LAUNCH_POST)
 #undef LAUNCH_POST
-  return check_launch("post_reorder");
+  return B200MOE_OK;
 }

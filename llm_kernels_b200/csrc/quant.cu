@@ -17,6 +17,8 @@ __global__ void __launch_bounds__(256) act_quant_fp8_kernel(
     int64_t y_stride, float* __restrict__ s, int64_t s_stride, bool dense, bool wide) {
   // total is a multiple of 8, the grid is sized so whole groups of eight lanes are in or out
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  wait_for_predecessors();
+  allow_dependents();
   const bool live = i < total;
   float v[16];
   if (live) { load8(x + i * 16, *reinterpret_cast<float(*)[8]>(v)); load8(x + i * 16 + 8, *reinterpret_cast<float(*)[8]>(v + 8)); }
@@ -98,6 +100,8 @@ __global__ void __launch_bounds__(256) act_quant_int8_kernel(
     const T* __restrict__ x, int64_t total_chunks, int8_t* __restrict__ y,
     __half* __restrict__ s, int rounding) {
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  wait_for_predecessors();
+  allow_dependents();
   const bool live = i < total_chunks;
   float v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   if (live) load8(x + i * 8, v);
@@ -202,14 +206,11 @@ extern "C" int b200moe_act_quant_fp8(const void* x, int x_dtype, int64_t rows, i
   cudaStream_t st = as_stream(stream);
   switch (x_dtype) {
     case B200MOE_F32:
-      act_quant_fp8_kernel<float><<<grid, 256, 0, st>>>(static_cast<const float*>(x), total, chunks, y8, y_row_stride_bytes, s, s_row_stride, dense, wide);
-      break;
+      return launch_dependent("act_quant_fp8", act_quant_fp8_kernel<float>, dim3(grid), 256, 0, st, static_cast<const float*>(x), total, chunks, y8, y_row_stride_bytes, s, s_row_stride, dense, wide);
     case B200MOE_F16:
-      act_quant_fp8_kernel<__half><<<grid, 256, 0, st>>>(static_cast<const __half*>(x), total, chunks, y8, y_row_stride_bytes, s, s_row_stride, dense, wide);
-      break;
+      return launch_dependent("act_quant_fp8", act_quant_fp8_kernel<__half>, dim3(grid), 256, 0, st, static_cast<const __half*>(x), total, chunks, y8, y_row_stride_bytes, s, s_row_stride, dense, wide);
     case B200MOE_BF16:
-      act_quant_fp8_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(x), total, chunks, y8, y_row_stride_bytes, s, s_row_stride, dense, wide);
-      break;
+      return launch_dependent("act_quant_fp8", act_quant_fp8_kernel<__nv_bfloat16>, dim3(grid), 256, 0, st, static_cast<const __nv_bfloat16*>(x), total, chunks, y8, y_row_stride_bytes, s, s_row_stride, dense, wide);
     default:
       return fail(B200MOE_BAD_DTYPE, "act_quant_fp8: x dtype %d", x_dtype);
   }
@@ -267,9 +268,9 @@ extern "C" int b200moe_act_quant_int8(const void* x, int x_dtype, int64_t rows, 
   int8_t* y8 = static_cast<int8_t*>(y);
   __half* sh = static_cast<__half*>(s_f16);
   switch (x_dtype) {
-    case B200MOE_F32: act_quant_int8_kernel<float><<<grid, 256, 0, st>>>(static_cast<const float*>(x), total, y8, sh, rounding); break;
-    case B200MOE_F16: act_quant_int8_kernel<__half><<<grid, 256, 0, st>>>(static_cast<const __half*>(x), total, y8, sh, rounding); break;
-    case B200MOE_BF16: act_quant_int8_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(x), total, y8, sh, rounding); break;
+    case B200MOE_F32: return launch_dependent("act_quant_int8", act_quant_int8_kernel<float>, dim3(grid), 256, 0, st, static_cast<const float*>(x), total, y8, sh, rounding);
+    case B200MOE_F16: return launch_dependent("act_quant_int8", act_quant_int8_kernel<__half>, dim3(grid), 256, 0, st, static_cast<const __half*>(x), total, y8, sh, rounding);
+    case B200MOE_BF16: return launch_dependent("act_quant_int8", act_quant_int8_kernel<__nv_bfloat16>, dim3(grid), 256, 0, st, static_cast<const __nv_bfloat16*>(x), total, y8, sh, rounding);
     default: return fail(B200MOE_BAD_DTYPE, "act_quant_int8: x dtype %d", x_dtype);
   }
   return check_launch("act_quant_int8");

@@ -133,6 +133,8 @@ __global__ void __launch_bounds__(kChunk) route_one_kernel(const int64_t* __rest
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   for (int i = tid; i < 2 * E; i += kChunk) s_one[i] = 0;
   for (int i = tid; i < kOneWarps * E / 2; i += kChunk) reinterpret_cast<uint32_t*>(cnt)[i] = 0u;
+  wait_for_predecessors();
+  allow_dependents();
   __syncthreads();
   const int64_t base = static_cast<int64_t>(blockIdx.x) * kChunk, own = base + tid;
   const int64_t e64 = own < n ? ids[own] : -1;
@@ -198,8 +200,8 @@ static int route_one(const int64_t* ids, int64_t n, int E, int64_t* reorder_ids,
   const size_t smem = one_smem(E);                          // 72 KB at 1024 experts
   if (smem > 48 * 1024)
     if (int rc = set_dynamic_smem(reinterpret_cast<const void*>(route_one_kernel), one_smem(kMaxExperts))) return rc;
-  route_one_kernel<<<static_cast<unsigned>((n + kChunk - 1) / kChunk), kChunk, smem, st>>>(ids, n, E, reorder_ids, src2dst, seg);
-  return check_launch("route_metadata");
+  return launch_dependent("route_metadata", route_one_kernel, dim3(static_cast<unsigned>((n + kChunk - 1) / kChunk)), kChunk, smem,
+                          st, ids, n, E, reorder_ids, src2dst, seg);
 }
 
 }  // namespace b200moe

@@ -280,6 +280,8 @@ __global__ void __launch_bounds__(256) router_few_kernel(const __nv_bfloat16* __
   float acc[kFewTokens];
 #pragma unroll
   for (int k = 0; k < kFewTokens; ++k) acc[k] = 0.f;
+  wait_for_predecessors();
+  allow_dependents();
 #pragma unroll 2
   for (int64_t h = ((warp & 3) * 32 + lane) * 8; h < H; h += 1024) {  // H is a multiple of 64
     float hi[8], mid[8], lo[8];
@@ -315,8 +317,8 @@ __global__ void __launch_bounds__(256) router_few_kernel(const __nv_bfloat16* __
 
 int router_logits_few(const void* x_bf16, const void* w3_bf16, float* logits, int64_t T, int64_t H, int E, cudaStream_t st) {
   const dim3 grid(static_cast<unsigned>(E / 2), static_cast<unsigned>((T + kFewTokens - 1) / kFewTokens));
-  router_few_kernel<<<grid, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(x_bf16), static_cast<const __nv_bfloat16*>(w3_bf16), logits, T, H, E);
-  return check_launch("router_logits");
+  return launch_dependent("router_logits", router_few_kernel, grid, 256, 0, st, static_cast<const __nv_bfloat16*>(x_bf16),
+                          static_cast<const __nv_bfloat16*>(w3_bf16), logits, T, H, E);
 }
 
 // ---- selection from precomputed logits (tensor-core path) ----------------------------------
@@ -330,6 +332,8 @@ __global__ void __launch_bounds__(256) router_select_kernel(const float* __restr
   extern __shared__ __align__(16) float smem[];   // [8 tokens][2][E]
   const int warp = threadIdx.x >> 5;
   const int64_t t0 = static_cast<int64_t>(blockIdx.x) * kSelectTokens;
+  wait_for_predecessors();
+  allow_dependents();
   const int tokens = static_cast<int>(min(p.T - t0, static_cast<int64_t>(kSelectTokens)));
   const int64_t step = p.T * row_stride;
 #pragma unroll 1
@@ -424,9 +428,6 @@ extern "C" int b200moe_router_select(const float* partials, int nsplit, int64_t 
   const size_t smem = sizeof(float) * kSelectTokens * 2 * E;
   if (E > 256)
     if (int rc = set_dynamic_smem(reinterpret_cast<const void*>(router_select_kernel<32>), sizeof(float) * kSelectTokens * 2 * 1024)) return rc;
-  auto launch = [&](auto kernel) { kernel<<<grid, 256, smem, as_stream(stream)>>>(partials, nsplit, partials_row_stride, p); };
-  if (E <= 32) launch(router_select_kernel<1>);
-  else if (E <= 256) launch(router_select_kernel<8>);
-  else launch(router_select_kernel<32>);
-  return check_launch("router_select");
+  return launch_dependent("router_select", E <= 32 ? router_select_kernel<1> : E <= 256 ? router_select_kernel<8> : router_select_kernel<32>,
+                          dim3(grid), 256, smem, as_stream(stream), partials, nsplit, partials_row_stride, p);
 }
