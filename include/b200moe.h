@@ -328,6 +328,11 @@ B200MOE_API int b200moe_grouped_gemm_fp8(const void* a, int64_t a_row_stride_byt
  * N % 8 == 0, K % 128 == 0. */
 B200MOE_API int b200moe_w4a8_expand_int8(const void* packed, const int8_t* s4, const int8_t* z4, void* out,
                              int64_t W, int64_t N, int64_t K, void* stream);
+/* The operands of one w4a8_gemm in one launch: b200moe_w4a8_expand_int8 of one weight, and the f16 scales of the
+ * activations (a_s_count values) and of the 128x128 blocks (b_s_count) as f32.  A count of 0 leaves that part out. */
+B200MOE_API int b200moe_w4a8_gemm_operands(const void* packed, const int8_t* s4, const int8_t* z4, void* out,
+                                           int64_t N, int64_t K, const void* a_s_f16, float* a_s, int64_t a_s_count,
+                                           const void* b_s_f16, float* b_s, int64_t b_s_count, void* stream);
 
 /* Writes 0 to *ok (device, the caller sets it to 1) if (q - z4) * s4 leaves int8 for a nibble that a weight of the stack
  * holds: such a weight cannot go through b200moe_grouped_gemm_w4a8.  Layouts as for b200moe_w4a8_expand_int8. */

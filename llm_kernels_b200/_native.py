@@ -55,6 +55,7 @@ SIGNATURES = {
     "b200moe_permute_quant_fp8_push": (_i, [_p, _i, _p, _p, _p, _p, _i, _i64, _i, _i64, _i64, _p, _i64, _p]),
     "b200moe_gather_rows": (_i, [_p, _p, _p, _i64, _i64, _p]),
     "b200moe_w4a8_expand_int8": (_i, [_p, _p, _p, _p, _i64, _i64, _i64, _p]),
+    "b200moe_w4a8_gemm_operands": (_i, [_p, _p, _p, _p, _i64, _i64, _p, _p, _i64, _p, _p, _i64, _p]),
     "b200moe_w4a8_range_check": (_i, [_p, _p, _p, _i64, _i64, _i64, _p, _p]),
     "b200moe_w4a16_expand_bf16": (_i, [_p, _p, _p, _p, _i64, _i64, _p]),
     "b200moe_grouped_gemm_i8": (_i, [_p, _i64, _p, _i64, _p, _p, _p, _i, _i64, _i64, _i64, _i64, _i, _i,

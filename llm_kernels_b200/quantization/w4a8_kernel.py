@@ -76,23 +76,44 @@ def w4a8_gemm(a: torch.Tensor, a_s: torch.Tensor, b: torch.Tensor, b_s: torch.Te
     assert pack_direction == "row" and GROUP_SIZE_INT4 == 128 and elements_per_sample == 8
     K = a.size(-1)
     M = a.numel() // K
+    a_s = a_s.reshape(M, -1)
+    # The dense launches take their sizes and strides from M, N and K alone, so they serve operands that agree on them; any
+    # others go to the grouped launch, which checks them and reads the scales by their own stride.
+    if _opts() is None and b.dim() == 2 and b.size(1) == K and a_s.size(1) * 128 == K and M > 0:
+        return _gemm_dense(a, a_s, b, b_s, b_s4, b_z4, M, K, out_dtype)
     w8 = expand_int8(b, b_s4, b_z4)
     Nn = w8.shape[0]
     c = a.new_empty(*a.size()[:-1], Nn, dtype=out_dtype or torch.get_default_dtype())
-    ks = _split_k(M, Nn, K)
-    a_s, b_s = a_s.reshape(M, -1).float(), b_s.float()
-    # The dense launches take their sizes and strides from M, N and K alone, so they serve operands that agree on them; any
-    # others go to the grouped launch, which checks them and reads the scales by their own stride.
-    if _opts() is None and tuple(w8.shape) == (Nn, K) and a_s.shape[1] * 128 == K:
-        N.require_cuda(a, a_s, b_s)
-        assert a.dtype == torch.int8
-        args = (N.ptr(a), N.ptr(a_s), N.ptr(w8), N.ptr(b_s), N.ptr(c), N.dtype_code(c.dtype), M, Nn, K)
-        if ks > 1:
-            part = a_s.new_empty(ks * M * Nn)          # the call's own, as in fp8_gemm
-            N.check(N.lib().b200moe_gemm_i8_block_splitk(*args, ks, N.ptr(part), part.numel() * 4, N.stream()))
-        else:
-            N.check(N.lib().b200moe_gemm_i8_block(*args, N.stream()))
-        return c
+    a_s, b_s = a_s.float(), b_s.float()
     seg = torch.tensor([0, M], dtype=torch.int64, device=a.device)
     grouped_gemm_i8(a.view(M, K), a_s, w8.unsqueeze(0), b_s.unsqueeze(0), seg, None, c.view(M, Nn))
+    return c
+
+
+def _gemm_dense(a, a_s, b, b_s, b_s4, b_z4, M, K, out_dtype):
+    """w4a8_gemm of operands that agree on M, N and K: one launch expands the weight and turns f16 scales into f32, the GEMM
+    follows.  Everything in between is one allocation of the call's own: memory of the caching allocator is ordered by stream,
+    belongs to a graph that captures the call, and calls of two threads on one stream do not meet in it."""
+    N.require_cuda(a, a_s, b, b_s, b_s4, b_z4)
+    assert a.dtype == torch.int8
+    Nn = b.size(0) * 8
+    c = a.new_empty(*a.size()[:-1], Nn, dtype=out_dtype or torch.get_default_dtype())
+    ks = _split_k(M, Nn, K)
+    casts = [(t, t.numel()) if t.dtype == torch.float16 else (t if t.dtype == torch.float32 else t.float(), 0) for t in (a_s, b_s)]
+    sizes = [Nn * K, casts[0][1] * 4, casts[1][1] * 4, ks * M * Nn * 4 if ks > 1 else 0]
+    offsets, total = [], 0
+    for size in sizes:
+        offsets.append(total)
+        total += (size + 255) & ~255
+    scratch = torch.empty(total, dtype=torch.uint8, device=a.device)
+    w8, fa, fb, part = (scratch.data_ptr() + o for o in offsets)
+    lib, stream = N.lib(), N.stream()
+    N.check(lib.b200moe_w4a8_gemm_operands(N.ptr(b), N.ptr(b_s4), N.ptr(b_z4), w8, Nn, K, N.ptr(casts[0][0]), fa, casts[0][1],
+                                           N.ptr(casts[1][0]), fb, casts[1][1], stream))
+    pa, pb = fa if casts[0][1] else N.ptr(casts[0][0]), fb if casts[1][1] else N.ptr(casts[1][0])
+    args = (N.ptr(a), pa, w8, pb, N.ptr(c), N.dtype_code(c.dtype), M, Nn, K)
+    if ks > 1:
+        N.check(lib.b200moe_gemm_i8_block_splitk(*args, ks, part, sizes[3], stream))
+    else:
+        N.check(lib.b200moe_gemm_i8_block(*args, stream))
     return c

@@ -1,4 +1,5 @@
-"""The launches around the GEMMs at the sizes where their routes and tiles change (csrc/router.cu, route.cu, permute.cu, quant.cu)."""
+"""The launches around the GEMMs at the sizes where their routes and tiles change (csrc/router.cu, route.cu, permute.cu, quant.cu,
+w4.cu)."""
 import pytest
 import torch
 
@@ -141,3 +142,21 @@ def test_fp8_quantizer_rows_of_any_stride(rows, cols, pad):
     q, qs = R.act_quant_fp8(x)
     assert torch.equal(y[:, :cols].cpu(), _bits(q)) and torch.equal(s[:, :cols // 128].cpu(), qs)
     assert not y[:, cols:].any() and not s[:, cols // 128:].any()
+
+
+@pytest.mark.parametrize("N_,K", [(8, 128), (40, 384), (264, 2176)])
+def test_int4_expansions_for_every_scale(N_, K):
+    """All int8 scales and zero points (the products wrap), and the asymmetric format with zero points that are no whole numbers."""
+    from llm_kernels_b200.quantization import w4a8_kernel, w4a16_kernel
+    g = torch.Generator().manual_seed(K)
+    q = torch.randint(0, 16, (N_, K), generator=g)
+    s4, z4 = (torch.randint(-128, 128, (N_, K // 128), dtype=torch.int8, generator=g) for _ in range(2))
+    packed = sum(q.view(N_ // 8, 8, K)[:, c] << (4 * c) for c in range(8)).to(torch.int32)
+    want = ((q - z4.long().repeat_interleave(128, 1)) * s4.long().repeat_interleave(128, 1)).to(torch.int8)
+    assert torch.equal(w4a8_kernel.expand_int8(packed.cuda(), s4.cuda(), z4.cuda()).cpu(), want)
+    words = sum(q.view(N_, K // 8, 8)[..., j] << (4 * j) for j in range(8)).to(torch.int32)
+    sc, zp = (torch.rand(N_, K // 128, generator=g) * m for m in (0.1, 15.0))
+    sc, zp = sc.to(torch.bfloat16), zp.to(torch.bfloat16)
+    wide = lambda t: t.float().repeat_interleave(128, 1)
+    want = ((q.float() - wide(zp)) * wide(sc)).to(torch.bfloat16)
+    assert torch.equal(w4a16_kernel.expand_bf16(words.cuda(), sc.cuda(), zp.cuda()).cpu(), want)
