@@ -125,6 +125,20 @@ def lib() -> C.CDLL:
     return _lib
 
 
+_calls_module = None
+
+
+def calls():
+    """The compiled call paths (csrc/calls.cpp); raises if they have not been built."""
+    global _calls_module
+    if _calls_module is None:
+        if not os.path.exists(os.path.join(_HERE, "_calls.so")):
+            raise RuntimeError(f"{_HERE}/_calls.so is missing: build it with `python -m llm_kernels_b200.build`")
+        from . import _calls
+        _calls_module = _calls
+    return _calls_module
+
+
 def check(status: int) -> None:
     """Maps a non-zero status to an exception.  Shape/argument problems raise
     AssertionError (the reference's wrappers use bare asserts for those), the

@@ -15,6 +15,7 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libb200moe.so")
+CALLS = os.path.join(HERE, "_calls.so")          # Python module over the library and torch's C++ API (csrc/calls.cpp)
 SOURCES = ["api.cu", "quant.cu", "router.cu", "route.cu", "permute.cu", "gemm_fp8.cu", "gemm_fp8_rows.cu", "gemm_w4a8.cu", "gemm_w4a16.cu", "bitpack.cu", "w4.cu", "wquant.cu", "ep_fused.cu", "layer.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-lineinfo",
@@ -30,12 +31,25 @@ def _nvcc() -> str:
 
 
 def needs_build() -> bool:
-    if not os.path.exists(LIB):
+    if not os.path.exists(LIB) or not os.path.exists(CALLS):
         return True
-    t = os.path.getmtime(LIB)
+    t = min(os.path.getmtime(LIB), os.path.getmtime(CALLS))
     deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)] + [
         os.path.join(HERE, "..", "include", "b200moe.h"), os.path.abspath(__file__)]
     return any(os.path.getmtime(d) > t for d in deps)
+
+
+def _build_calls() -> None:
+    import sysconfig
+    import torch
+    base = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    includes = [os.path.join(base, "include"), os.path.join(base, "include", "torch", "csrc", "api", "include"),
+                sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
+    subprocess.check_call([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+                           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *[f"-I{d}" for d in includes],
+                           os.path.join(CSRC, "calls.cpp"), "-o", CALLS, LIB, f"-L{os.path.join(base, 'lib')}", "-lc10", "-lc10_cuda",
+                           "-ltorch_cpu", "-ltorch_python", "-Wl,-rpath,$ORIGIN"])
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -61,7 +75,8 @@ def build(force: bool = False, verbose: bool = False) -> str:
         failed |= p.returncode != 0
     if failed:
         raise RuntimeError("nvcc failed")
-    subprocess.check_call([nvcc, "-arch=sm_100a", "-shared", "-o", LIB, *objs])
+    subprocess.check_call([nvcc, "-arch=sm_100a", "-shared", "-Xlinker", "-soname=libb200moe.so", "-o", LIB, *objs])
+    _build_calls()
     return LIB
 
 

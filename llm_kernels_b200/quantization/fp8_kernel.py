@@ -13,6 +13,10 @@ from .. import _native as N
 
 def act_quant(x: torch.Tensor, block_size: int = 128) -> Tuple[torch.Tensor, torch.Tensor]:
     """Per-(1 x block_size) quantization: returns (y e4m3 same shape, s f32 [..., D/block_size])."""
+    if block_size == 128:
+        out = N.calls().act_quant(x, 0)             # None: not taken as it is, the checks below say why
+        if out is not None:
+            return out if type(out) is tuple else N.check(out)
     N.require_cuda(x)
     assert x.is_contiguous(), 'Input tensor must be contiguous'
     assert block_size == 128, 'block_size must be 128'
@@ -70,16 +74,19 @@ def fp8_gemm(a: torch.Tensor, a_s: torch.Tensor, b: torch.Tensor, b_s: torch.Ten
     default dtype unless out_dtype is given (tcgen05 kernel).  ksplits (None = chosen from the shape):
     M <= 128 splits the K loop over several sets of tiles whose f32 partial products are added in
     split order by a second kernel, so that the weights stream on all SMs."""
+    K = a.size(-1)
+    ks = _split_k(a.numel() // K if K else 0, b.size(0), K) if ksplits is None else int(ksplits)
+    out = N.calls().fp8_gemm(a, a_s, b, b_s, out_dtype or torch.get_default_dtype(), ks)
+    if out is not None:
+        return N.check(out) if type(out) is int else out
     N.require_cuda(a, a_s, b, b_s)
     assert a.is_contiguous() and b.is_contiguous(), 'Input tensors must be contiguous'
     assert a_s.is_contiguous() and b_s.is_contiguous(), 'Scaling factor tensors must be contiguous'
     assert a.dtype == torch.float8_e4m3fn and b.dtype == torch.float8_e4m3fn, 'operands must be float8_e4m3fn'
     assert a_s.dtype == torch.float32 and b_s.dtype == torch.float32, 'scales must be float32'
-    K = a.size(-1)
     M = a.numel() // K
     Nn = b.size(0)
     c = a.new_empty(*a.size()[:-1], Nn, dtype=out_dtype or torch.get_default_dtype())
-    ks = _split_k(M, Nn, K) if ksplits is None else int(ksplits)
     if ks > 1 and M > 0:
         # The splits' scratch belongs to the call: the caching allocator orders its memory by stream and gives a captured call
         # memory of its graph, and calls of two threads on one stream must not meet in one buffer.

@@ -62,6 +62,10 @@ def weight_dequant(y: torch.Tensor, s: torch.Tensor, s4: torch.Tensor, z4: torch
 
 def act_quant(x: torch.Tensor, block_size: int = 128) -> Tuple[torch.Tensor, torch.Tensor]:
     """int8 per 1x128 group, floor(v + 0.5) rounding, f16 scales (reference :171-193)."""
+    if block_size == 128:
+        out = N.calls().act_quant(x, 1)             # None: not taken as it is, the checks of int8_kernel say why
+        if out is not None:
+            return out if type(out) is tuple else N.check(out)
     return int8_kernel.act_quant(x, block_size, rounding="floor_half")
 
 
@@ -70,6 +74,12 @@ def w4a8_gemm(a: torch.Tensor, a_s: torch.Tensor, b: torch.Tensor, b_s: torch.Te
               pack_direction: str = "row", out_dtype: torch.dtype = None) -> torch.Tensor:
     """c[..., N] = a[..., K] (int8) . dequant(b)^T with per-K-block scales (reference :406-448).  Few rows (M <= 128) split
     the K loop over all SMs as fp8_gemm does: one m-tile alone kept N / 256 of them busy (M = 24, N = 4096, K = 7168)."""
+    if _opts() is None and pack_direction == "row" and GROUP_SIZE_INT4 == 128 and elements_per_sample == 8 and a.numel():
+        K = a.size(-1)
+        ks = _split_k(a.numel() // K, b.size(0) * 8, K) if b.numel() else 1
+        out = N.calls().w4a8_gemm(a, a_s, b, b_s, b_s4, b_z4, out_dtype or torch.get_default_dtype(), ks)
+        if out is not None:                         # None: not taken as they are, the checks below say why
+            return N.check(out) if type(out) is int else out
     assert a.is_contiguous() and b.is_contiguous(), 'Input tensors must be contiguous'
     assert a_s.is_contiguous() and b_s.is_contiguous(), 'Scaling factor tensors must be contiguous'
     assert b_s4.is_contiguous() and b_z4.is_contiguous(), 'Scaling factor and zero point tensors must be contiguous'

@@ -1,5 +1,5 @@
 """The launches around the GEMMs at the sizes where their routes and tiles change (csrc/router.cu, route.cu, permute.cu, quant.cu,
-w4.cu)."""
+w4.cu), and the compiled call paths (csrc/calls.cpp) against the Python functions."""
 import pytest
 import torch
 
@@ -160,3 +160,47 @@ def test_int4_expansions_for_every_scale(N_, K):
     wide = lambda t: t.float().repeat_interleave(128, 1)
     want = ((q.float() - wide(zp)) * wide(sc)).to(torch.bfloat16)
     assert torch.equal(w4a16_kernel.expand_bf16(words.cuda(), sc.cuda(), zp.cuda()).cpu(), want)
+
+
+@pytest.mark.parametrize("M", [1, 24, 128, 129])
+@pytest.mark.parametrize("N_,K", [(256, 128), (384, 1152)])
+def test_compiled_calls_give_what_the_python_functions_give(M, N_, K, monkeypatch):
+    from llm_kernels_b200 import _native as N
+    from llm_kernels_b200.quantization import fp8_kernel, w4a8_kernel
+
+    class NotTaken:
+        def __getattr__(self, name):
+            return lambda *args: None
+
+    def run():
+        out = []
+        g = torch.Generator(device="cuda").manual_seed(3)
+        x = torch.randn(2, M, K, generator=g, device="cuda").to(torch.bfloat16)
+        w = torch.randn(N_, K, generator=g, device="cuda") * 0.02
+        for mod, gemm in ((fp8_kernel, fp8_kernel.fp8_gemm), (w4a8_kernel, w4a8_kernel.w4a8_gemm)):
+            q, s = mod.act_quant(x)
+            weight = mod.weight_quant(w)
+            out += [q, s, gemm(q, s, *weight, out_dtype=torch.bfloat16), gemm(q[:1].contiguous(), s[:1].contiguous(), *weight)]
+            if mod is w4a8_kernel:
+                out.append(gemm(q, s.float(), weight[0], weight[1].float(), *weight[2:], out_dtype=torch.float16))
+        return out
+    fast = run()
+    monkeypatch.setattr(N, "_calls_module", NotTaken())
+    for a, b in zip(fast, run()):
+        assert a.dtype == b.dtype and a.shape == b.shape and torch.equal(_bits(a), _bits(b))
+
+
+def test_compiled_calls_leave_what_they_do_not_take():
+    from llm_kernels_b200 import _native as N
+    f8 = torch.float8_e4m3fn
+    x = torch.zeros(4, 256, device="cuda", dtype=torch.bfloat16)
+    a, s, b, bs = x.to(f8), torch.ones(4, 2, device="cuda"), torch.zeros(256, 256, device="cuda").to(f8), torch.ones(2, 2, device="cuda")
+    c = N.calls()
+    assert c.act_quant(x, 0) is not None and c.fp8_gemm(a, s, b, bs, torch.bfloat16, 1) is not None
+    for bad in (x.cpu(), x.t(), x[:, ::2], x.double(), x[:, :100].contiguous(), None, x[0, 0]):
+        assert c.act_quant(bad, 0) is None
+    for i, bad in ((0, a.t()), (0, x), (1, s.double()), (2, b.t()), (3, bs.cpu()), (4, torch.int8), (4, None), (0, a[:0])):
+        args = [a, s, b, bs, torch.bfloat16, 1]
+        args[i] = bad
+        assert c.fp8_gemm(*args) is None
+    assert type(c.fp8_gemm(a, s, b, bs, torch.bfloat16, 3)) is int          # an empty split: the library's status
