@@ -153,7 +153,8 @@ B200MOE_API int b200moe_router_topk(const void* x, int x_dtype, const float* w, 
                         int scoring, int norm_topk_prob, float routed_scaling_factor,
                         int64_t* topk_idx, float* topk_weight, void* stream);
 
-/* K splits with which b200moe_router_logits_bf16x3 should run for T tokens and E padded expert rows. */
+/* K splits with which b200moe_router_logits_bf16x3 should run for T tokens and E padded expert rows.  1 for one or two
+ * tokens, whose logits the CUDA cores then form in f32. */
 B200MOE_API int b200moe_router_ksplits(int64_t T, int64_t H, int E);
 
 /* Tensor-core form of the same router for large expert counts, in two launches.
