@@ -198,7 +198,8 @@ __global__ void __launch_bounds__(kChunk) route_one_kernel(const int64_t* __rest
 
 static int route_one(const int64_t* ids, int64_t n, int E, int64_t* reorder_ids, int32_t* src2dst, int64_t* seg, cudaStream_t st) {
   const size_t smem = one_smem(E);                          // 72 KB at 1024 experts
-  if (smem > 48 * 1024)
+  // the 48 KB that need no opt-in hold static shared memory too: reached at 681 experts, asked for well before
+  if (E > 512)
     if (int rc = set_dynamic_smem(reinterpret_cast<const void*>(route_one_kernel), one_smem(kMaxExperts))) return rc;
   return launch_dependent("route_metadata", route_one_kernel, dim3(static_cast<unsigned>((n + kChunk - 1) / kChunk)), kChunk, smem,
                           st, ids, n, E, reorder_ids, src2dst, seg);

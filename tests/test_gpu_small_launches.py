@@ -28,6 +28,24 @@ def test_sort_is_stable_at_its_chunk_edges(n, E):
     assert torch.equal(seg, torch.cat([torch.zeros(1, dtype=torch.int64), torch.bincount(ids[slots], minlength=E).cumsum(0)]))
 
 
+def test_sort_opts_in_to_shared_memory_in_time():
+    """Static and dynamic shared memory together leave the default limit at 681 experts.  A process of its own: once a kernel has
+    been opted in, the limit stays raised."""
+    import os
+    import subprocess
+    import sys
+    code = ("import torch\n"
+            "from llm_kernels_b200.moe import group_gemm_kernel as G\n"
+            "for E in (680, 681, 682, 683):\n"
+            "    ids = torch.arange(64).mul(37) % E\n"
+            "    order, dst, seg = (t.cpu() for t in G.run_moe_ep_preproess(ids.cuda(), E))\n"
+            "    want, rows = torch.sort(ids, stable=True)\n"
+            "    assert torch.equal(order, want) and torch.equal(dst[rows], torch.arange(64, dtype=torch.int32)), E\n")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    done = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True)
+    assert done.returncode == 0, done.stderr
+
+
 # registers per lane 1, 8 and 32; groups that do and do not divide the 32 lanes; more splits than loads in flight
 @pytest.mark.parametrize("T", [1, 8, 9])
 @pytest.mark.parametrize("E,groups,kept,k,splits", [(8, 1, 1, 2, 1), (32, 4, 2, 4, 9), (48, 3, 2, 5, 3), (256, 8, 4, 8, 16),
