@@ -33,7 +33,7 @@ int set_dynamic_smem(const void* kernel, size_t bytes) {
   for (int i = 0; i < count; ++i)
     if (done[i].kernel == kernel && done[i].dev == dev && done[i].bytes >= bytes) return B200MOE_OK;
   const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
-  if (e != cudaSuccess) return fail(B200MOE_LAUNCH_FAILED, "%zu bytes of shared memory: %s", bytes, cudaGetErrorString(e));
+  if (e != cudaSuccess) return refused("opt-in to shared memory", e);
   if (count < 128) done[count++] = {kernel, dev, bytes};
   return B200MOE_OK;
 }

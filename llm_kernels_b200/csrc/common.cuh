@@ -22,6 +22,12 @@ inline cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s
 // Returns B200MOE_OK or records the CUDA launch error.
 int check_launch(const char* what);
 
+// The error of a refused call, taken from the runtime too: what it keeps would be reported by the next launch.
+inline int refused(const char* what, cudaError_t e) {
+  cudaGetLastError();
+  return fail(B200MOE_LAUNCH_FAILED, "%s: %s", what, cudaGetErrorString(e));
+}
+
 // Opts a kernel in to `bytes` of dynamic shared memory on the current device, once per kernel and device.
 int set_dynamic_smem(const void* kernel, size_t bytes);
 
@@ -53,7 +59,7 @@ int launch_dependent(const char* what, void (*kernel)(P...), dim3 grid, int thre
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
-  return e == cudaSuccess ? check_launch(what) : fail(B200MOE_LAUNCH_FAILED, "%s launch: %s", what, cudaGetErrorString(e));
+  return e == cudaSuccess ? check_launch(what) : refused(what, e);
 }
 
 // Router logits of few tokens on the CUDA cores (router.cu), from the operands of b200moe_router_logits_bf16x3 (gemm_fp8.cu).

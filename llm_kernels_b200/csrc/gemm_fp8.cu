@@ -681,7 +681,7 @@ static int launch_gemm_as(const RowMaps& ma, const CUtensorMap& mb, const GemmPa
   cfg.attrs = attr;                   // pairs serve large products: no dependent launch, whose gain is a few microseconds
   cfg.numAttrs = 1;
   cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_block_kernel<KIND, PAIR>, ma, mb, p);
-  if (e != cudaSuccess) return fail(B200MOE_LAUNCH_FAILED, "gemm_block_kernel launch: %s", cudaGetErrorString(e));
+  if (e != cudaSuccess) return refused("gemm_block_kernel", e);
   return check_launch("gemm_block_kernel");
 }
 

@@ -46,6 +46,18 @@ def test_sort_opts_in_to_shared_memory_in_time():
     assert done.returncode == 0, done.stderr
 
 
+def test_a_refused_launch_is_not_reported_by_the_next():
+    from llm_kernels_b200 import _native as N
+    lib = N.lib()
+    x = torch.randn(2, 2048, device="cuda").to(torch.bfloat16)
+    y, s = torch.zeros(2, 2048, dtype=torch.uint8, device="cuda"), torch.zeros(2, 16, device="cuda")
+
+    def quant(rows):
+        return lib.b200moe_act_quant_fp8(x.data_ptr(), N.BF16, rows, 2048, y.data_ptr(), 2048, s.data_ptr(), 16, N.stream())
+    assert quant(1 << 33) == 6              # 2^32 blocks, which a 32-bit count holds as none: the runtime launches nothing
+    assert not y.any() and quant(2) == 0 and y.any()
+
+
 # registers per lane 1, 8 and 32; groups that do and do not divide the 32 lanes; more splits than loads in flight
 @pytest.mark.parametrize("T", [1, 8, 9])
 @pytest.mark.parametrize("E,groups,kept,k,splits", [(8, 1, 1, 2, 1), (32, 4, 2, 4, 9), (48, 3, 2, 5, 3), (256, 8, 4, 8, 16),
