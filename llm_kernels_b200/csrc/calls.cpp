@@ -8,6 +8,9 @@
 // Every function returns None for operands that are not what the launches take as they are (other types, shapes, strides or
 // devices, tensor subclasses, CPU tensors); the Python functions then go through their own checks and messages.  A non-zero
 // status of the library is returned as a number and raised by the caller.
+//
+// The interpreter is released around allocations and launches: an allocation can wait for the device, a launch for room in the
+// launch queue, and other threads, also those that the queued work itself waits for, go on meanwhile.
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/DynamicTypes.h>
@@ -23,14 +26,25 @@
 
 namespace {
 
-// The operand as a tensor that a launch can take: a plain contiguous tensor on the current device.
-const at::Tensor* plain(PyObject* o) {
-  if (!THPVariable_CheckExact(o)) return nullptr;
+// The operand as a tensor that a launch can take: a plain contiguous tensor on the current device; undefined otherwise.  A
+// reference of the call's own, since other threads run meanwhile.
+at::Tensor plain(PyObject* o) {
+  if (!THPVariable_CheckExact(o)) return {};
   const at::Tensor& t = THPVariable_Unpack(o);
   return t.is_cuda() && t.get_device() == c10::cuda::current_device() && t.layout() == at::kStrided && t.is_contiguous() &&
                  !t.is_neg() && t.dim() > 0
-             ? &t : nullptr;
+             ? t : at::Tensor();
 }
+
+class ReleasedInterpreter {
+ public:
+  ReleasedInterpreter() : state_(PyEval_SaveThread()) {}
+  ~ReleasedInterpreter() { PyEval_RestoreThread(state_); }
+  ReleasedInterpreter(const ReleasedInterpreter&) = delete;
+
+ private:
+  PyThreadState* state_;
+};
 
 int dtype_code(at::ScalarType t) {
   switch (t) {
@@ -55,18 +69,22 @@ PyObject* none() { Py_RETURN_NONE; }
 PyObject* act_quant(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   if (n != 2) return none();
-  const at::Tensor* x = plain(args[0]);
+  const at::Tensor x = plain(args[0]);
   const long kind = PyLong_AsLong(args[1]);
-  if (!x || dtype_code(x->scalar_type()) < 0) return none();
-  const int64_t cols = x->size(-1);
+  if (!x.defined() || dtype_code(x.scalar_type()) < 0) return none();
+  const int64_t cols = x.size(-1);
   if (cols == 0 || cols % 128 != 0) return none();
-  const int64_t rows = x->numel() / cols;
-  at::Tensor y = at::empty(x->sizes(), x->options().dtype(kind == 0 ? at::kFloat8_e4m3fn : at::kChar));
-  at::Tensor s = at::empty(with_last(*x, cols / 128), x->options().dtype(kind == 0 ? at::kFloat : at::kHalf));
-  const int rc = kind == 0 ? b200moe_act_quant_fp8(x->data_ptr(), dtype_code(x->scalar_type()), rows, cols, y.data_ptr(), cols,
-                                                   static_cast<float*>(s.data_ptr()), cols / 128, stream())
-                           : b200moe_act_quant_int8(x->data_ptr(), dtype_code(x->scalar_type()), rows, cols, y.data_ptr(), s.data_ptr(),
-                                                    1, stream());
+  const int64_t rows = x.numel() / cols;
+  at::Tensor y, s;
+  int rc;
+  {
+    ReleasedInterpreter released;
+    y = at::empty(x.sizes(), x.options().dtype(kind == 0 ? at::kFloat8_e4m3fn : at::kChar));
+    s = at::empty(with_last(x, cols / 128), x.options().dtype(kind == 0 ? at::kFloat : at::kHalf));
+    rc = kind == 0 ? b200moe_act_quant_fp8(x.data_ptr(), dtype_code(x.scalar_type()), rows, cols, y.data_ptr(), cols,
+                                           static_cast<float*>(s.data_ptr()), cols / 128, stream())
+                   : b200moe_act_quant_int8(x.data_ptr(), dtype_code(x.scalar_type()), rows, cols, y.data_ptr(), s.data_ptr(), 1, stream());
+  }
   if (rc) return PyLong_FromLong(rc);
   PyObject* out = PyTuple_New(2);
   PyTuple_SET_ITEM(out, 0, THPVariable_Wrap(std::move(y)));
@@ -79,26 +97,29 @@ PyObject* act_quant(PyObject*, PyObject* const* args, Py_ssize_t n) {
 PyObject* fp8_gemm(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   if (n != 6 || !THPDtype_Check(args[4])) return none();
-  const at::Tensor *a = plain(args[0]), *a_s = plain(args[1]), *b = plain(args[2]), *b_s = plain(args[3]);
-  if (!a || !a_s || !b || !b_s || a->scalar_type() != at::kFloat8_e4m3fn || b->scalar_type() != at::kFloat8_e4m3fn ||
-      a_s->scalar_type() != at::kFloat || b_s->scalar_type() != at::kFloat) return none();
+  const at::Tensor a = plain(args[0]), a_s = plain(args[1]), b = plain(args[2]), b_s = plain(args[3]);
+  if (!a.defined() || !a_s.defined() || !b.defined() || !b_s.defined() || a.scalar_type() != at::kFloat8_e4m3fn ||
+      b.scalar_type() != at::kFloat8_e4m3fn || a_s.scalar_type() != at::kFloat || b_s.scalar_type() != at::kFloat) return none();
   const at::ScalarType out_t = reinterpret_cast<THPDtype*>(args[4])->scalar_type;
   const int code = dtype_code(out_t);
-  const int64_t K = a->size(-1), N = b->size(0);
-  if (code < 0 || K == 0 || a->numel() == 0) return none();
-  const int64_t M = a->numel() / K;
+  const int64_t K = a.size(-1), N = b.size(0);
+  if (code < 0 || K == 0 || a.numel() == 0) return none();
+  const int64_t M = a.numel() / K;
   const long ks = PyLong_AsLong(args[5]);
-  at::Tensor c = at::empty(with_last(*a, N), a->options().dtype(out_t));
+  at::Tensor c;
   int rc;
-  if (ks > 1) {
-    // the call's own, as in the Python function
-    at::Tensor part = at::empty({ks * M * N}, a_s->options());
-    rc = b200moe_gemm_fp8_block_splitk(a->data_ptr(), static_cast<const float*>(a_s->data_ptr()), b->data_ptr(),
-                                       static_cast<const float*>(b_s->data_ptr()), c.data_ptr(), code, M, N, K, static_cast<int>(ks),
-                                       static_cast<float*>(part.data_ptr()), part.numel() * 4, stream());
-  } else {
-    rc = b200moe_gemm_fp8_block(a->data_ptr(), static_cast<const float*>(a_s->data_ptr()), b->data_ptr(),
-                                static_cast<const float*>(b_s->data_ptr()), c.data_ptr(), code, M, N, K, stream());
+  {
+    ReleasedInterpreter released;
+    c = at::empty(with_last(a, N), a.options().dtype(out_t));
+    const auto *as = static_cast<const float*>(a_s.data_ptr()), *bs = static_cast<const float*>(b_s.data_ptr());
+    if (ks > 1) {
+      // the call's own, as in the Python function
+      at::Tensor part = at::empty({ks * M * N}, a_s.options());
+      rc = b200moe_gemm_fp8_block_splitk(a.data_ptr(), as, b.data_ptr(), bs, c.data_ptr(), code, M, N, K, static_cast<int>(ks),
+                                         static_cast<float*>(part.data_ptr()), part.numel() * 4, stream());
+    } else {
+      rc = b200moe_gemm_fp8_block(a.data_ptr(), as, b.data_ptr(), bs, c.data_ptr(), code, M, N, K, stream());
+    }
   }
   return rc ? PyLong_FromLong(rc) : THPVariable_Wrap(std::move(c));
   END_HANDLE_TH_ERRORS
@@ -108,9 +129,9 @@ PyObject* fp8_gemm(PyObject*, PyObject* const* args, Py_ssize_t n) {
 PyObject* w4a8_gemm(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   if (n != 8 || !THPDtype_Check(args[6])) return none();
-  const at::Tensor* t[6];
-  for (int i = 0; i < 6; ++i) if (!(t[i] = plain(args[i]))) return none();
-  const at::Tensor &a = *t[0], &a_s = *t[1], &b = *t[2], &b_s = *t[3], &s4 = *t[4], &z4 = *t[5];
+  at::Tensor t[6];
+  for (int i = 0; i < 6; ++i) if (!(t[i] = plain(args[i])).defined()) return none();
+  const at::Tensor &a = t[0], &a_s = t[1], &b = t[2], &b_s = t[3], &s4 = t[4], &z4 = t[5];
   auto scales = [](const at::Tensor& s) { return s.scalar_type() == at::kHalf || s.scalar_type() == at::kFloat; };
   if (a.scalar_type() != at::kChar || b.scalar_type() != at::kInt || s4.scalar_type() != at::kChar || z4.scalar_type() != at::kChar ||
       !scales(a_s) || !scales(b_s) || b.dim() != 2) return none();
@@ -124,18 +145,23 @@ PyObject* w4a8_gemm(PyObject*, PyObject* const* args, Py_ssize_t n) {
   const int64_t na = a_s.scalar_type() == at::kHalf ? a_s.numel() : 0, nb = b_s.scalar_type() == at::kHalf ? b_s.numel() : 0;
   auto up = [](int64_t v) { return (v + 255) / 256 * 256; };
   const int64_t w8 = up(N * K), fa = up(na * 4), fb = up(nb * 4), part = ks > 1 ? ks * M * N * 4 : 0;
-  at::Tensor c = at::empty(with_last(a, N), a.options().dtype(out_t));
-  at::Tensor scratch = at::empty({w8 + fa + fb + part}, a.options().dtype(at::kByte));
-  char* base = static_cast<char*>(scratch.data_ptr());
-  float *pa = reinterpret_cast<float*>(base + w8), *pb = reinterpret_cast<float*>(base + w8 + fa);
-  int rc = b200moe_w4a8_gemm_operands(b.data_ptr(), static_cast<const int8_t*>(s4.data_ptr()), static_cast<const int8_t*>(z4.data_ptr()),
-                                      base, N, K, a_s.data_ptr(), pa, na, b_s.data_ptr(), pb, nb, stream());
-  if (rc) return PyLong_FromLong(rc);
-  const float* as = na ? pa : static_cast<const float*>(a_s.data_ptr());
-  const float* bs = nb ? pb : static_cast<const float*>(b_s.data_ptr());
-  rc = ks > 1 ? b200moe_gemm_i8_block_splitk(a.data_ptr(), as, base, bs, c.data_ptr(), code, M, N, K, static_cast<int>(ks),
-                                             reinterpret_cast<float*>(base + w8 + fa + fb), part, stream())
-              : b200moe_gemm_i8_block(a.data_ptr(), as, base, bs, c.data_ptr(), code, M, N, K, stream());
+  at::Tensor c;
+  int rc;
+  {
+    ReleasedInterpreter released;
+    c = at::empty(with_last(a, N), a.options().dtype(out_t));
+    at::Tensor scratch = at::empty({w8 + fa + fb + part}, a.options().dtype(at::kByte));
+    char* base = static_cast<char*>(scratch.data_ptr());
+    float *pa = reinterpret_cast<float*>(base + w8), *pb = reinterpret_cast<float*>(base + w8 + fa);
+    rc = b200moe_w4a8_gemm_operands(b.data_ptr(), static_cast<const int8_t*>(s4.data_ptr()), static_cast<const int8_t*>(z4.data_ptr()),
+                                    base, N, K, a_s.data_ptr(), pa, na, b_s.data_ptr(), pb, nb, stream());
+    const float* as = na ? pa : static_cast<const float*>(a_s.data_ptr());
+    const float* bs = nb ? pb : static_cast<const float*>(b_s.data_ptr());
+    if (!rc)
+      rc = ks > 1 ? b200moe_gemm_i8_block_splitk(a.data_ptr(), as, base, bs, c.data_ptr(), code, M, N, K, static_cast<int>(ks),
+                                                 reinterpret_cast<float*>(base + w8 + fa + fb), part, stream())
+                  : b200moe_gemm_i8_block(a.data_ptr(), as, base, bs, c.data_ptr(), code, M, N, K, stream());
+  }
   return rc ? PyLong_FromLong(rc) : THPVariable_Wrap(std::move(c));
   END_HANDLE_TH_ERRORS
 }

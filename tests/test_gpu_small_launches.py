@@ -234,3 +234,42 @@ def test_compiled_calls_leave_what_they_do_not_take():
         args[i] = bad
         assert c.fp8_gemm(*args) is None
     assert type(c.fp8_gemm(a, s, b, bs, torch.bfloat16, 3)) is int          # an empty split: the library's status
+
+
+@pytest.mark.parametrize("kind", ["act_quant", "fp8_gemm", "w4a8_gemm"])
+def test_compiled_calls_let_other_threads_run(kind):
+    """A launch that waits for room in the queue does so without the interpreter.  The queue is held by a sleep of about 0.8 s; a
+    second thread notes the longest time that it could not run."""
+    import threading
+    import time
+    from llm_kernels_b200.quantization import fp8_kernel, w4a8_kernel
+    x = torch.randn(16, 256, device="cuda").to(torch.bfloat16)
+    w = torch.randn(256, 256, device="cuda")
+    mod = w4a8_kernel if kind == "w4a8_gemm" else fp8_kernel
+    q, s = mod.act_quant(x)
+    weight = mod.weight_quant(w)
+    call = {"act_quant": lambda: mod.act_quant(x), "fp8_gemm": lambda: fp8_kernel.fp8_gemm(q, s, *weight),
+            "w4a8_gemm": lambda: w4a8_kernel.w4a8_gemm(q, s, *weight)}[kind]
+    call()
+    torch.cuda.synchronize()
+    done, longest_gap = threading.Event(), [0.0]
+
+    def ticker():
+        last = time.perf_counter()
+        while not done.is_set():
+            time.sleep(0.002)
+            now = time.perf_counter()
+            longest_gap[0], last = max(longest_gap[0], now - last), now
+    thread = threading.Thread(target=ticker)
+    thread.start()
+    torch.cuda._sleep(1_500_000_000)
+    waited, began = 0.0, time.perf_counter()
+    while waited < 0.1 and time.perf_counter() - began < 3:       # until one call has waited for the queue
+        t = time.perf_counter()
+        call()
+        waited = time.perf_counter() - t
+    done.set()
+    thread.join()
+    torch.cuda.synchronize()
+    assert waited >= 0.1, "no call met a full queue"
+    assert longest_gap[0] < waited / 2
