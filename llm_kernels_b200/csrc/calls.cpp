@@ -65,13 +65,21 @@ std::vector<int64_t> with_last(const at::Tensor& t, int64_t last) {
 
 PyObject* none() { Py_RETURN_NONE; }
 
+// A Python integer that fits the library's int.
+bool to_int(PyObject* o, int* out) {
+  const long v = PyLong_AsLong(o);
+  if (v == -1 && PyErr_Occurred()) { PyErr_Clear(); return false; }
+  *out = static_cast<int>(v);
+  return *out == v;
+}
+
 // act_quant(x, kind): kind 0 fp8, 1 int8 with f16 scales and floor(v + 0.5)
 PyObject* act_quant(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   if (n != 2) return none();
   const at::Tensor x = plain(args[0]);
-  const long kind = PyLong_AsLong(args[1]);
-  if (!x.defined() || dtype_code(x.scalar_type()) < 0) return none();
+  int kind;
+  if (!to_int(args[1], &kind) || !x.defined() || dtype_code(x.scalar_type()) < 0) return none();
   const int64_t cols = x.size(-1);
   if (cols == 0 || cols % 128 != 0) return none();
   const int64_t rows = x.numel() / cols;
@@ -105,7 +113,8 @@ PyObject* fp8_gemm(PyObject*, PyObject* const* args, Py_ssize_t n) {
   const int64_t K = a.size(-1), N = b.size(0);
   if (code < 0 || K == 0 || a.numel() == 0) return none();
   const int64_t M = a.numel() / K;
-  const long ks = PyLong_AsLong(args[5]);
+  int ks;
+  if (!to_int(args[5], &ks)) return none();
   at::Tensor c;
   int rc;
   {
@@ -114,8 +123,8 @@ PyObject* fp8_gemm(PyObject*, PyObject* const* args, Py_ssize_t n) {
     const auto *as = static_cast<const float*>(a_s.data_ptr()), *bs = static_cast<const float*>(b_s.data_ptr());
     if (ks > 1) {
       // the call's own, as in the Python function
-      at::Tensor part = at::empty({ks * M * N}, a_s.options());
-      rc = b200moe_gemm_fp8_block_splitk(a.data_ptr(), as, b.data_ptr(), bs, c.data_ptr(), code, M, N, K, static_cast<int>(ks),
+      at::Tensor part = at::empty({M * N * ks}, a_s.options());
+      rc = b200moe_gemm_fp8_block_splitk(a.data_ptr(), as, b.data_ptr(), bs, c.data_ptr(), code, M, N, K, ks,
                                          static_cast<float*>(part.data_ptr()), part.numel() * 4, stream());
     } else {
       rc = b200moe_gemm_fp8_block(a.data_ptr(), as, b.data_ptr(), bs, c.data_ptr(), code, M, N, K, stream());
@@ -141,10 +150,11 @@ PyObject* w4a8_gemm(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (code < 0 || K == 0 || a.numel() == 0 || b.size(1) != K) return none();
   const int64_t M = a.numel() / K;
   if (a_s.numel() * 128 != M * K) return none();
-  const long ks = PyLong_AsLong(args[7]);
+  int ks;
+  if (!to_int(args[7], &ks)) return none();
   const int64_t na = a_s.scalar_type() == at::kHalf ? a_s.numel() : 0, nb = b_s.scalar_type() == at::kHalf ? b_s.numel() : 0;
   auto up = [](int64_t v) { return (v + 255) / 256 * 256; };
-  const int64_t w8 = up(N * K), fa = up(na * 4), fb = up(nb * 4), part = ks > 1 ? ks * M * N * 4 : 0;
+  const int64_t w8 = up(N * K), fa = up(na * 4), fb = up(nb * 4), part = ks > 1 ? M * N * ks * 4 : 0;
   at::Tensor c;
   int rc;
   {
@@ -158,7 +168,7 @@ PyObject* w4a8_gemm(PyObject*, PyObject* const* args, Py_ssize_t n) {
     const float* as = na ? pa : static_cast<const float*>(a_s.data_ptr());
     const float* bs = nb ? pb : static_cast<const float*>(b_s.data_ptr());
     if (!rc)
-      rc = ks > 1 ? b200moe_gemm_i8_block_splitk(a.data_ptr(), as, base, bs, c.data_ptr(), code, M, N, K, static_cast<int>(ks),
+      rc = ks > 1 ? b200moe_gemm_i8_block_splitk(a.data_ptr(), as, base, bs, c.data_ptr(), code, M, N, K, ks,
                                                  reinterpret_cast<float*>(base + w8 + fa + fb), part, stream())
                   : b200moe_gemm_i8_block(a.data_ptr(), as, base, bs, c.data_ptr(), code, M, N, K, stream());
   }

@@ -234,6 +234,8 @@ def test_compiled_calls_leave_what_they_do_not_take():
         args[i] = bad
         assert c.fp8_gemm(*args) is None
     assert type(c.fp8_gemm(a, s, b, bs, torch.bfloat16, 3)) is int          # an empty split: the library's status
+    for ks in (2 ** 31, 2 ** 70, -2 ** 70, 2.0, None):                      # no C int
+        assert c.fp8_gemm(a, s, b, bs, torch.bfloat16, ks) is None
 
 
 @pytest.mark.parametrize("kind", ["act_quant", "fp8_gemm", "w4a8_gemm"])
