@@ -9,6 +9,7 @@ from __future__ import annotations
 import ctypes as C
 import os
 import threading
+import warnings
 
 import torch
 
@@ -125,17 +126,27 @@ def lib() -> C.CDLL:
     return _lib
 
 
+class _NoCalls:
+    """Stands in for the compiled calls: takes no operands, so that the Python functions serve them."""
+    act_quant = fp8_gemm = w4a8_gemm = staticmethod(lambda *args: None)
+
+
 _calls_module = None
 
 
 def calls():
-    """The compiled call paths (csrc/calls.cpp); raises if they have not been built."""
+    """The compiled call paths (csrc/calls.cpp).  They belong to one torch and one Python; where they are missing or were built for
+    others, the Python functions launch the same kernels, with more time between them."""
     global _calls_module
     if _calls_module is None:
-        if not os.path.exists(os.path.join(_HERE, "_calls.so")):
-            raise RuntimeError(f"{_HERE}/_calls.so is missing: build it with `python -m llm_kernels_b200.build`")
-        from . import _calls
-        _calls_module = _calls
+        from . import build
+        if build.calls_fit():
+            from . import _calls
+            _calls_module = _calls
+        else:
+            warnings.warn(f"{build.CALLS} is missing or not {build.calls_stamp()}: calls of few rows take longer.  Build it with "
+                          "`python -m llm_kernels_b200.build`", RuntimeWarning, stacklevel=3)
+            _calls_module = _NoCalls
     return _calls_module
 
 

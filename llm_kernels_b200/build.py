@@ -15,7 +15,8 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libb200moe.so")
-CALLS = os.path.join(HERE, "_calls.so")          # Python module over the library and torch's C++ API (csrc/calls.cpp)
+# Python module over the library and torch's C++ API (csrc/calls.cpp); belongs to one build of torch and one Python, which it names
+CALLS = os.path.join(HERE, "_calls.so")
 SOURCES = ["api.cu", "quant.cu", "router.cu", "route.cu", "permute.cu", "gemm_fp8.cu", "gemm_fp8_rows.cu", "gemm_w4a8.cu", "gemm_w4a16.cu", "bitpack.cu", "w4.cu", "wquant.cu", "ep_fused.cu", "layer.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-lineinfo",
@@ -30,31 +31,80 @@ def _nvcc() -> str:
     raise RuntimeError("nvcc not found; set NVCC or put it on PATH")
 
 
-def needs_build() -> bool:
-    if not os.path.exists(LIB) or not os.path.exists(CALLS):
+def _older(target: str, names) -> bool:
+    """target is missing or older than a source, the header or this file."""
+    if not os.path.exists(target):
         return True
-    t = min(os.path.getmtime(LIB), os.path.getmtime(CALLS))
-    deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)] + [
-        os.path.join(HERE, "..", "include", "b200moe.h"), os.path.abspath(__file__)]
-    return any(os.path.getmtime(d) > t for d in deps)
+    deps = [os.path.join(CSRC, f) for f in names] + [os.path.join(HERE, "..", "include", "b200moe.h"), os.path.abspath(__file__)]
+    return any(os.path.getmtime(d) > os.path.getmtime(target) for d in deps)
+
+
+def _library_sources():
+    return [f for f in os.listdir(CSRC) if f != "calls.cpp"]
+
+
+def calls_stamp() -> str:
+    """The torch and the Python that the compiled calls must have been built for."""
+    import torch
+    return f"built for torch {torch.__version__}, {sys.implementation.cache_tag}"
+
+
+def calls_fit() -> bool:
+    """Whether the compiled calls are there and belong to this torch and this Python.  Looked up in the file: a module of another
+    torch may not even load."""
+    if not os.path.exists(CALLS):
+        return False
+    with open(CALLS, "rb") as f:
+        return calls_stamp().encode() + b"\0" in f.read()
+
+
+def _calls_possible() -> bool:
+    """Whether there is a torch with CUDA and its headers to build the compiled calls against.  The library needs neither."""
+    try:
+        import torch
+    except ImportError:
+        return False
+    return torch.version.cuda is not None and os.path.exists(os.path.join(_torch_include(torch), "torch", "csrc", "Exceptions.h"))
+
+
+def _torch_include(torch) -> str:
+    return os.path.join(os.path.dirname(torch.__file__), "include")
+
+
+def _calls_due() -> bool:
+    return _calls_possible() and (_older(CALLS, ["calls.cpp"]) or not calls_fit())
+
+
+def needs_build() -> bool:
+    return _older(LIB, _library_sources()) or _calls_due()
 
 
 def _build_calls() -> None:
     import sysconfig
     import torch
-    base = os.path.dirname(torch.__file__)
     cuda = os.path.dirname(os.path.dirname(_nvcc()))
-    includes = [os.path.join(base, "include"), os.path.join(base, "include", "torch", "csrc", "api", "include"),
-                sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
+    include = _torch_include(torch)
+    includes = [include, os.path.join(include, "torch", "csrc", "api", "include"), sysconfig.get_paths()["include"],
+                os.path.join(cuda, "include")]
     subprocess.check_call([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
-                           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *[f"-I{d}" for d in includes],
-                           os.path.join(CSRC, "calls.cpp"), "-o", CALLS, LIB, f"-L{os.path.join(base, 'lib')}", "-lc10", "-lc10_cuda",
-                           "-ltorch_cpu", "-ltorch_python", "-Wl,-rpath,$ORIGIN"])
+                           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f'-DCALLS_STAMP="{calls_stamp()}"',
+                           *[f"-I{d}" for d in includes], os.path.join(CSRC, "calls.cpp"), "-o", CALLS, LIB,
+                           f"-L{os.path.join(os.path.dirname(include), 'lib')}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python",
+                           "-Wl,-rpath,$ORIGIN"])
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
-    if not force and not needs_build():
-        return LIB
+    if force or _older(LIB, _library_sources()):
+        _build_library(verbose)
+        force = True
+    if force and not _calls_possible():
+        sys.stderr.write("no torch with CUDA and its headers: the library is built, the compiled calls are left out\n")
+    elif force or _calls_due():
+        _build_calls()
+    return LIB
+
+
+def _build_library(verbose: bool) -> None:
     nvcc = _nvcc()
     objs = []
     procs = []
@@ -76,8 +126,6 @@ def build(force: bool = False, verbose: bool = False) -> str:
     if failed:
         raise RuntimeError("nvcc failed")
     subprocess.check_call([nvcc, "-arch=sm_100a", "-shared", "-Xlinker", "-soname=libb200moe.so", "-o", LIB, *objs])
-    _build_calls()
-    return LIB
 
 
 if __name__ == "__main__":

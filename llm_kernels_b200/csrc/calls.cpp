@@ -185,4 +185,8 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_calls", nullptr, -1, methods, nul
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__calls() { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit__calls() {
+  PyObject* m = PyModule_Create(&module);
+  if (m && PyModule_AddStringConstant(m, "stamp", CALLS_STAMP) < 0) { Py_DECREF(m); return nullptr; }   // looked up by build.py
+  return m;
+}

@@ -374,3 +374,35 @@ def test_layer_moved_to_another_device_is_refused(layer_host, host, monkeypatch)
     monkeypatch.setattr(host, "require_cuda", require_cuda)
     with pytest.raises(RuntimeError, match="current device"):
         layer(x)
+
+
+def test_quantized_calls_do_without_their_compiled_module(host, monkeypatch, tmp_path):
+    """It is missing, or belongs to another torch: the Python functions serve the call and make their own checks."""
+    from llm_kernels_b200 import build
+    from llm_kernels_b200.quantization import fp8_kernel, w4a8_kernel
+    assert build.calls_fit() and not build.needs_build()
+    for patch in (lambda m: m.setattr(build, "CALLS", str(tmp_path / "_calls.so")),
+                  lambda m: m.setattr(build, "calls_stamp", lambda: "built for another torch")):
+        with monkeypatch.context() as m:
+            lib = Recorder()
+            m.setattr(host, "_lib", lib)
+            m.setattr(host, "_calls_module", None)
+            patch(m)
+            with pytest.warns(RuntimeWarning, match="take longer"):
+                fp8_kernel.act_quant(torch.zeros(2, 128))
+            w4a8_kernel.act_quant(torch.zeros(2, 128))
+            fp8_kernel.fp8_gemm(torch.zeros(200, 256, dtype=torch.float8_e4m3fn), torch.ones(200, 2),
+                                torch.zeros(256, 256, dtype=torch.float8_e4m3fn), torch.ones(2, 2))
+            w4a8_kernel.w4a8_gemm(*_w4a8_operands(200, 256, 256, 2))
+            assert lib.names() == ["b200moe_act_quant_fp8", "b200moe_act_quant_int8", "b200moe_gemm_fp8_block",
+                                   "b200moe_w4a8_gemm_operands", "b200moe_gemm_i8_block"]
+            assert build.needs_build()
+
+
+def test_library_is_built_without_the_compiled_calls(monkeypatch, tmp_path):
+    """Other hosts need the library alone: no torch with CUDA, or none with headers."""
+    from llm_kernels_b200 import build
+    build.build()
+    monkeypatch.setattr(build, "CALLS", str(tmp_path / "_calls.so"))
+    monkeypatch.setattr(build, "_calls_possible", lambda: False)
+    assert not build.needs_build() and build.build() == build.LIB and not (tmp_path / "_calls.so").exists()
