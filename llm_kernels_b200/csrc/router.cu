@@ -60,14 +60,11 @@ template <int J>
 __device__ void select_token(const RouterParams& p, int64_t t, const float* score, float* sfc) {
   const int lane = threadIdx.x & 31;
   const int E = p.E;
-  float v[J];
-#pragma unroll
-  for (int j = 0; j < J; ++j) v[j] = lane + 32 * j < E ? score[lane + 32 * j] : 0.f;
   float s[J];                                            // selection scores
 #pragma unroll
   for (int j = 0; j < J; ++j) {
     const int e = lane + 32 * j;
-    s[j] = e < E ? v[j] + (p.bias ? p.bias[e] : 0.f) : -INFINITY;
+    s[j] = e < E ? score[e] + (p.bias ? p.bias[e] : 0.f) : -INFINITY;
   }
 
   if (p.n_group > 1) {
@@ -125,10 +122,9 @@ __device__ void select_token(const RouterParams& p, int64_t t, const float* scor
 #pragma unroll
     for (int j = J - 1; j >= 0; --j) if (key[j] == best) cand = static_cast<uint32_t>(lane + 32 * j);
     const int i = best == 0u ? 0 : static_cast<int>(__reduce_min_sync(0xffffffffu, cand));   // ties: the lower id
-    float mine = v[0];
 #pragma unroll
-    for (int j = 0; j < J; ++j) if ((i >> 5) == j) { mine = v[j]; if (lane == (i & 31)) key[j] = 0u; }
-    const float sc = __shfl_sync(0xffffffffu, mine, i & 31);
+    for (int j = 0; j < J; ++j) if (i == lane + 32 * j) key[j] = 0u;
+    const float sc = score[i];
     if (lane == r) { my_w = sc; my_i = i; }
     wsum += sc;
   }
@@ -322,38 +318,77 @@ int router_logits_few(const void* x_bf16, const void* w3_bf16, float* logits, in
 }
 
 // ---- selection from precomputed logits (tensor-core path) ----------------------------------
-// Eight tokens per block.  All threads add the partial sums, an expert each (in index order, eight loads in flight), then a warp
-// selects for one token.  A thread per expert keeps the code short: with a warp per token all the way, eight experts per lane
-// unrolled, a single token waited longer for instructions than for data (decode of one token, with the logits above: 117 -> 108 us).
+// Eight tokens per block, a warp selects for one; J registers per lane cover E experts.  What bounds it: the latency of the loads
+// of the partial sums, so many of them are in flight, and for a token or two the fetch of the code.
+//
+// Few tokens (they fit side by side in the block's threads; with more than 256 experts, one or two): a thread per expert, short
+// code with eight splits in flight.  More tokens: each warp adds its own, J experts a lane, 32 (J 8, 32) or 64 (J 16) loads in
+// flight; with the first form for all, 16 splits took eight rounds of 16 loads one after another.  us, 16 splits, first form -> a
+// warp each: 256 experts, top-8 of 8 groups: one token 6.1 -> 6.9, two 8.3 -> 6.7, 77 tokens 18 -> 7.6, 4096 35 -> 17, 8192
+// 83 -> 36; 384 experts, one token 5.7 -> 6.9, two 7.6 -> 6.8, 4096 72 -> 25; 1024 experts, one token 16 -> 19, three 21 -> 19,
+// 4096 132 -> 70.
+//
+// Registers: 80 for 256 experts, where the compiler takes 64 by itself (one token 6.9 -> 6.1 us, 4096 tokens 15.4 -> 17.2); 48 up to
+// 32 experts (eight experts, 4096 tokens: 4.5 us, 5.2 with 80).
 constexpr int kSelectTokens = 8;
 template <int J>
-__global__ void __launch_bounds__(256) router_select_kernel(const float* __restrict__ partials,
+__global__ void __launch_bounds__(256, J == 1 ? 5 : 1) router_select_kernel(const float* __restrict__ partials,
                                                             int nsplit, int64_t row_stride, RouterParams p) {
   extern __shared__ __align__(16) float smem[];   // [8 tokens][2][E]
-  const int warp = threadIdx.x >> 5;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t t0 = static_cast<int64_t>(blockIdx.x) * kSelectTokens;
   wait_for_predecessors();
   allow_dependents();
   const int tokens = static_cast<int>(min(p.T - t0, static_cast<int64_t>(kSelectTokens)));
   const int64_t step = p.T * row_stride;
-#pragma unroll 1
-  for (int i = threadIdx.x; i < tokens * p.E; i += 256) {
-    const int k = i / p.E, e = i - k * p.E;
-    const float* src = partials + (t0 + k) * row_stride + e;
-    float v = 0.f;
-#pragma unroll 1
-    for (int s0 = 0; s0 < nsplit; s0 += 8) {
-      float x[8];
-#pragma unroll
-      for (int s = 0; s < 8; ++s) x[s] = s0 + s < nsplit ? src[(s0 + s) * step] : 0.f;
-#pragma unroll
-      for (int s = 0; s < 8; ++s) v += x[s];             // past the last split: + 0, which changes nothing
-    }
-    smem[k * 2 * p.E + e] = p.scoring == 1 ? v : sigmoid_score(v);
-  }
-  __syncthreads();
-  if (warp >= tokens) return;
+  const int side = p.E < 256 ? 256 / p.E : 1;               // tokens side by side
   float* score = smem + warp * 2 * p.E;
+  if (J == 1 || tokens <= (J >= 16 ? 2 : 1) * side) {       // J == 1: eight tokens always fit
+    const int k0 = p.E < 256 ? static_cast<int>(threadIdx.x) / p.E : 0;
+    if (k0 < side) {
+#pragma unroll 1
+      for (int e = threadIdx.x - k0 * p.E; e < p.E; e += 256) {
+#pragma unroll 1
+        for (int k = k0; k < tokens; k += side) {
+          const float* src = partials + (t0 + k) * row_stride + e;
+          float v = 0.f;
+#pragma unroll 1
+          for (int s0 = 0; s0 < nsplit; s0 += 8, src += 8 * step) {
+            float x[8];
+#pragma unroll
+            for (int s = 0; s < 8; ++s) x[s] = s0 + s < nsplit ? src[s * step] : 0.f;
+#pragma unroll
+            for (int s = 0; s < 8; ++s) v += x[s];           // past the last split: + 0, which changes nothing
+          }
+          smem[k * 2 * p.E + e] = p.scoring == 1 ? v : sigmoid_score(v);
+        }
+      }
+    }
+    __syncthreads();
+    if (warp >= tokens) return;
+  } else {
+    if (warp >= tokens) return;
+    constexpr int S = J == 32 ? 1 : 4;                      // splits in flight (32 experts a lane, 4096 tokens: 70 us, 97 with two)
+    const float* src = partials + (t0 + warp) * row_stride + lane;
+    float v[J];
+#pragma unroll
+    for (int j = 0; j < J; ++j) v[j] = 0.f;
+#pragma unroll 1
+    for (int s0 = 0; s0 < nsplit; s0 += S, src += S * step) {
+      float x[S][J];
+#pragma unroll
+      for (int s = 0; s < S; ++s)
+#pragma unroll
+        for (int j = 0; j < J; ++j) x[s][j] = s0 + s < nsplit && lane + 32 * j < p.E ? src[s * step + 32 * j] : 0.f;
+#pragma unroll
+      for (int s = 0; s < S; ++s)
+#pragma unroll
+        for (int j = 0; j < J; ++j) v[j] += x[s][j];
+    }
+#pragma unroll
+    for (int j = 0; j < J; ++j) if (lane + 32 * j < p.E) score[lane + 32 * j] = p.scoring == 1 ? v[j] : sigmoid_score(v[j]);
+    __syncwarp();
+  }
   if (p.scoring == 1) { softmax_scores(score, p.E); __syncwarp(); }
   select_token<J>(p, t0 + warp, score, score + p.E);
 }
@@ -426,8 +461,9 @@ extern "C" int b200moe_router_select(const float* partials, int nsplit, int64_t 
                  routed_scaling_factor, topk_idx, topk_weight};
   const unsigned grid = static_cast<unsigned>((T + 7) / 8);
   const size_t smem = sizeof(float) * kSelectTokens * 2 * E;
-  if (E > 256)
+  if (E > 512)
     if (int rc = set_dynamic_smem(reinterpret_cast<const void*>(router_select_kernel<32>), sizeof(float) * kSelectTokens * 2 * 1024)) return rc;
-  return launch_dependent("router_select", E <= 32 ? router_select_kernel<1> : E <= 256 ? router_select_kernel<8> : router_select_kernel<32>,
-                          dim3(grid), 256, smem, as_stream(stream), partials, nsplit, partials_row_stride, p);
+  const auto kernel = E <= 32 ? router_select_kernel<1> : E <= 256 ? router_select_kernel<8>
+                    : E <= 512 ? router_select_kernel<16> : router_select_kernel<32>;
+  return launch_dependent("router_select", kernel, dim3(grid), 256, smem, as_stream(stream), partials, nsplit, partials_row_stride, p);
 }

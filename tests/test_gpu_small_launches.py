@@ -96,6 +96,32 @@ def test_selection_from_partial_sums(T, E, groups, kept, k, splits, scoring):
         assert float(((w[t].cpu().double() - ref) / ref).abs().max()) < 40 * 2 ** -23
 
 
+# a thread per expert for one token (or what fits beside it), a warp per token otherwise; 1, 8, 16 and 32 experts a lane
+@pytest.mark.parametrize("E,groups,kept", [(8, 1, 1), (33, 1, 1), (64, 4, 2), (128, 1, 1), (255, 5, 2), (256, 8, 4), (257, 1, 1), (384, 1, 1),
+                                           (512, 8, 4), (513, 1, 1), (1024, 32, 7)])
+@pytest.mark.parametrize("splits", [1, 3, 16])
+@pytest.mark.parametrize("scoring", [0, 1])
+def test_selection_does_not_depend_on_the_batch(E, groups, kept, splits, scoring):
+    """The sums run in the order of the splits in either form: the same bits."""
+    from llm_kernels_b200 import _native as N
+    g = torch.Generator(device="cuda").manual_seed(E)
+    T, k, stride = 13, min(8, E), E + 3
+    part = torch.randn(splits, T, stride, generator=g, device="cuda")
+    bias = torch.randn(E, generator=g, device="cuda")
+
+    def select(part):
+        n = part.shape[1]
+        idx, w = torch.full((n, k), -1, dtype=torch.int64, device="cuda"), torch.full((n, k), -1.0, device="cuda")
+        N.check(N.lib().b200moe_router_select(part.data_ptr(), splits, stride, bias.data_ptr(), n, E, k, groups, kept, scoring, 1, 2.5,
+                                              idx.data_ptr(), w.data_ptr(), N.stream()))
+        return idx, w
+    whole = select(part)
+    for n in (1, 2, 3, 5):
+        for t in range(0, T - n + 1, n):
+            for a, b in zip(whole, select(part[:, t:t + n].contiguous())):
+                assert torch.equal(_bits(a[t:t + n]), _bits(b))
+
+
 @pytest.mark.parametrize("T", [1, 2])
 @pytest.mark.parametrize("H,E", [(64, 128), (1088, 128), (7168, 256)])
 def test_router_logits_of_few_tokens(T, H, E):
