@@ -6,12 +6,13 @@
 //   act_and_mul        moe/group_gemm_kernel.py:120-168 (silu), :176-235 (gelu)
 //   post_reorder       moe/group_gemm_kernel.py:238-288 with the f32 accumulation
 //                      of moe/all2all_moe.py:270-278
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace b200moe {
 
 constexpr int kMaxK = 32;
-constexpr int64_t kFewTokens = 512;         // see row_grid
 
 // Destination rows of the token's local slots, shared by the CTA.
 __device__ __forceinline__ int load_slots(const int32_t* src2dst, const int64_t* topk_ids,
@@ -195,9 +196,9 @@ __global__ void __launch_bounds__(256) act_and_mul_kernel(
   }
 }
 
-// AHEAD rows of a token are loaded before the first is added: 4 for few tokens, whose blocks wait for memory with nothing else
-// on the SM (one token 9.4 -> 5.0 us); 1 otherwise, where more resident blocks hide more (4096 tokens: 103 us, 151 with 4).
-template <typename T, int AHEAD>
+// One row of the token at a time: four loaded ahead were slower throughout (hidden size 7168, top-8: one token 2.8 -> 3.3 us, 256
+// tokens 8.0 -> 12.9, 4096 91 -> 151).
+template <typename T>
 __global__ void __launch_bounds__(256) post_reorder_kernel(
     const T* __restrict__ down, T* __restrict__ out, const int32_t* __restrict__ src2dst,
     const int64_t* __restrict__ topk_ids, const float* __restrict__ w, int lo, int hi, int topk,
@@ -212,17 +213,12 @@ __global__ void __launch_bounds__(256) post_reorder_kernel(
   __syncthreads();
   for (int64_t c = first_chunk() * 8; c < H; c += chunk_step() * 8) {
     float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (int j0 = 0; j0 < n; j0 += AHEAD) {        // added in slot order
-      float v[AHEAD][8];
+    for (int j = 0; j < n; ++j) {                  // added in slot order
+      float v[8];
+      load8(down + static_cast<int64_t>(s_dst[j]) * H + c, v);
+      const float wj = s_w[j];
 #pragma unroll
-      for (int u = 0; u < AHEAD; ++u) if (j0 + u < n) load8(down + static_cast<int64_t>(s_dst[j0 + u]) * H + c, v[u]);
-#pragma unroll
-      for (int u = 0; u < AHEAD; ++u) {
-        if (j0 + u >= n) break;
-        const float wj = s_w[j0 + u];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) acc[k] = fmaf(v[u][k], wj, acc[k]);
-      }
+      for (int k = 0; k < 8; ++k) acc[k] = fmaf(v[k], wj, acc[k]);
     }
     store8(out + t * H + c, acc);
   }
@@ -241,15 +237,23 @@ __global__ void __launch_bounds__(256) gather_rows_kernel(const uint8_t* __restr
   for (int64_t c = threadIdx.x; c < row_bytes / 16; c += blockDim.x) out[c] = in[c];
 }
 
-// Launch of a kernel whose block x works on token x: as many threads as divide the row's chunks into equal rounds, and for few
-// tokens a block per round, since a round waits for the loads of the one before (un-permute of one token, hidden size 7168,
-// top-8: 9.4 us with one block).
+// Launch of a kernel whose block x works on token x: as many threads as divide the row's chunks into equal rounds.  `side`: a block
+// per round, since a round waits for the loads of the one before; otherwise one block takes the rounds in turn.
+//
+// us, one block -> a block per round.  Hidden size 7168, top-8: pre_reorder 512 tokens 14.2 -> 12.0, 1024 30.2 -> 23.5, 4096 94.3 ->
+// 90.5, 8192 183 -> 179; post_reorder one token 6.6 -> 2.8, 512 19.2 -> 14.1, 1024 25.1 -> 25.6, 1536 42.6 -> 34.9, 4096 92.2 -> 90.5,
+// 8192 169 -> 176.  Hidden size 4096, top-2: 1024 5.6 -> 5.6 and 5.4 -> 5.9, 4096 18.9 -> 18.9 and 19.8 -> 19.5, 8192 35.1 -> 38.2 and
+// 35.9 -> 41.1.  Up to kSideTokens.
+// The quantizers write half the bytes and repeat the look-up of the token's slots (7168, top-8): fp8 512 tokens 10.2 -> 9.3, 1024
+// 17.7 -> 15.7, 2048 30.2 -> 29.6, 4096 55.8 -> 59.0; int8 512 15.2 -> 11.2, 1024 21.8 -> 19.4, 1536 28.1 -> 28.6, 4096 64.7 -> 77.2.
+// Up to kQuantSideTokens.
+constexpr int64_t kSideTokens = 4096, kQuantSideTokens = 1024;
 struct RowGrid { dim3 grid; int threads; };
-static RowGrid row_grid(int64_t tokens, int64_t chunks) {
+static RowGrid row_grid(int64_t tokens, int64_t chunks, bool side) {
   const int64_t rounds = (chunks + 255) / 256;
   RowGrid g;
   g.threads = static_cast<int>(((chunks + rounds - 1) / rounds + 31) / 32 * 32);
-  g.grid = dim3(static_cast<unsigned>(tokens), tokens < kFewTokens ? static_cast<unsigned>(rounds) : 1u);
+  g.grid = dim3(static_cast<unsigned>(tokens), side ? static_cast<unsigned>(std::min<int64_t>(rounds, 65535)) : 1u);
   return g;
 }
 
@@ -284,7 +288,7 @@ extern "C" int b200moe_pre_reorder(const void* x, int x_dtype, void* out, int ou
                   "pre_reorder: out dtype %d must equal the input dtype or be e4m3", out_dtype);
   if (T == 0) return B200MOE_OK;
   cudaStream_t st = as_stream(stream);
-  const RowGrid g = row_grid(T, H / 8);
+  const RowGrid g = row_grid(T, H / 8, T <= kSideTokens);
 #define LAUNCH_PRE(TI)                                                                            \
   if (out_dtype == B200MOE_FP8_E4M3)                                                              \
     return launch_dependent("pre_reorder", pre_reorder_kernel<TI, uint8_t>, g.grid, g.threads, 0, st, static_cast<const TI*>(x), static_cast<uint8_t*>(out), src2dst, topk_ids, a1_scales, start_expert_id, end_expert_id, topk, H); \
@@ -311,7 +315,7 @@ extern "C" int b200moe_permute_quant_fp8(const void* x, int x_dtype, const int32
                   "permute_quant_fp8: output strides smaller than a row");
   if (T == 0) return B200MOE_OK;
   cudaStream_t st = as_stream(stream);
-  const RowGrid g = row_grid(T, H / 16);
+  const RowGrid g = row_grid(T, H / 16, T <= kQuantSideTokens);
 #define LAUNCH_PQ(TI)                                                                           \
   return launch_dependent("permute_quant_fp8", permute_quant_fp8_kernel<TI>, g.grid, g.threads, 0, st, static_cast<const TI*>(x), src2dst, topk_ids, \
       start_expert_id, end_expert_id, topk, H, static_cast<uint8_t*>(out_q),                     \
@@ -338,7 +342,7 @@ extern "C" int b200moe_permute_quant_int8(const void* x, int x_dtype, const int3
                   "permute_quant_int8: output strides smaller than a row");
   if (T == 0) return B200MOE_OK;
   cudaStream_t st = as_stream(stream);
-  const RowGrid g = row_grid(T, H / 8);
+  const RowGrid g = row_grid(T, H / 8, T <= kQuantSideTokens);
 #define LAUNCH_PQ8(TI)                                                                           \
   return launch_dependent("permute_quant_int8", permute_quant_int8_kernel<TI>, g.grid, g.threads, 0, st, static_cast<const TI*>(x), src2dst, topk_ids, \
       start_expert_id, end_expert_id, topk, H, static_cast<int8_t*>(out_q),                       \
@@ -395,9 +399,9 @@ extern "C" int b200moe_post_reorder(const void* down_output, int dtype, void* ou
   B200MOE_REQUIRE(aligned(down_output, 16) && aligned(out, 16), B200MOE_BAD_ALIGN, "post_reorder: alignment");
   if (T == 0) return B200MOE_OK;
   cudaStream_t st = as_stream(stream);
-  const RowGrid g = row_grid(T, H / 8);
+  const RowGrid g = row_grid(T, H / 8, T <= kSideTokens);
 #define LAUNCH_POST(TT)                                                                      \
-  return launch_dependent("post_reorder", T < kFewTokens ? post_reorder_kernel<TT, 4> : post_reorder_kernel<TT, 1>, g.grid, g.threads, 0, st, \
+  return launch_dependent("post_reorder", post_reorder_kernel<TT>, g.grid, g.threads, 0, st, \
       static_cast<const TT*>(down_output), static_cast<TT*>(out), src2dst, topk_ids, topk_weights, start_expert_id, end_expert_id, topk, H)
   DISPATCH_16BIT_OR_F32(dtype, LAUNCH_POST)
 #undef LAUNCH_POST

@@ -144,8 +144,8 @@ def test_router_logits_of_few_tokens(T, H, E):
     assert float(((part.cpu().double() - exact).abs() / size).max()) < (H / 128 + 9) * 2 ** -24
 
 
-# a block per round of columns below 512 tokens, one block per token from there on; rows that end inside a warp
-@pytest.mark.parametrize("T", [1, 3, 511, 512])
+# a block per round of columns, one block per token from 1025 (quantizers) or 4097 tokens on; rows that end inside a warp
+@pytest.mark.parametrize("T", [1, 3, 511, 512, 1024, 1025, 4096, 4097])
 @pytest.mark.parametrize("H", [128, 2176, 7168])
 @pytest.mark.parametrize("topk", [1, 5, 8])
 def test_permute_and_unpermute(T, H, topk):
