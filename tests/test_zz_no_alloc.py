@@ -40,9 +40,10 @@ def test_noalloc_matches_workspace_entry_point_twice():
     import llm_kernels_b200._native as N
     dev = torch.device("cuda:0")
     g = torch.Generator().manual_seed(77)
-    # first call: a large table (all 32 chunks x 256 experts written); second call: a smaller,
-    # differently shaped problem that reuses the same array with the first call's contents in it
-    for T, k, E in ((4096, 8, 256), (777, 3, 40)):
+    # first call: a large table (all 128 chunks x 256 experts written); second call: a smaller,
+    # differently shaped problem that reuses the same array with the first call's contents in it;
+    # third: few enough slots (65536 at most) for the one launch that needs no table
+    for T, k, E in ((16384, 8, 256), (23500, 3, 40), (777, 3, 40)):
         ids = torch.rand(T, E, generator=g).topk(k, dim=-1)[1].to(dev).contiguous().view(-1)
         want, got = _both(N, ids, E)
         for a, b in zip(want, got):
