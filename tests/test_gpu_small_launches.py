@@ -10,6 +10,17 @@ def _bits(t):
     return t.contiguous().view({1: torch.uint8, 2: torch.int16, 4: torch.int32, 8: torch.int64}[t.element_size()])
 
 
+def _select(part, bias, E, k, groups, kept, scoring):
+    """b200moe_router_select on partial sums [splits, T, stride] -> (idx, weights) on the host."""
+    from llm_kernels_b200 import _native as N
+    splits, T, stride = part.shape
+    pc, bc = part.cuda(), bias.cuda()
+    idx, w = torch.full((T, k), -1, dtype=torch.int64, device="cuda"), torch.full((T, k), -1.0, device="cuda")
+    N.check(N.lib().b200moe_router_select(pc.data_ptr(), splits, stride, bc.data_ptr(), T, E, k, groups, kept, scoring, 1, 1.5,
+                                          idx.data_ptr(), w.data_ptr(), N.stream()))
+    return idx.cpu(), w.cpu()
+
+
 # one launch up to 65536 slots, chunks of 1024; three launches beyond.  Some ids lie outside [0, E).
 @pytest.mark.parametrize("n", [1, 31, 33, 1023, 1024, 1025, 5000, 65535, 65536, 65537])
 @pytest.mark.parametrize("E", [1, 7, 256, 1024])
@@ -64,16 +75,12 @@ def test_a_refused_launch_is_not_reported_by_the_next():
                                                     (257, 1, 1, 8, 2), (1024, 32, 7, 32, 1)])
 @pytest.mark.parametrize("scoring", [0, 1])
 def test_selection_from_partial_sums(T, E, groups, kept, k, splits, scoring):
-    from llm_kernels_b200 import _native as N
+    """The biases are spread far wider than f32 rounds, and positive, so that masked experts (0) are out of the question."""
     g = torch.Generator().manual_seed(E + T)
     stride = E + 3
-    part = torch.randn(splits, T, stride, generator=g) * 0.01
-    bias = torch.randint(-40, 40, (E,), generator=g) / 4.0
-    idx = torch.empty(T, k, dtype=torch.int64, device="cuda")
-    w = torch.empty(T, k, device="cuda")
-    pc, bc = part.cuda(), bias.cuda()
-    N.check(N.lib().b200moe_router_select(pc.data_ptr(), splits, stride, bc.data_ptr(), T, E, k, groups, kept, scoring, 1, 1.5,
-                                          idx.data_ptr(), w.data_ptr(), N.stream()))
+    part = torch.randn(splits, T, stride, generator=g)
+    bias = torch.linspace(0.5, 4.5, E)[torch.randperm(E, generator=g)]
+    idx, w = _select(part, bias, E, k, groups, kept, scoring)
     logits = part[..., :E].double().sum(0)
     score = logits.sigmoid() if scoring == 0 else logits.softmax(-1)
     choice = score + bias.double()
@@ -85,15 +92,39 @@ def test_selection_from_partial_sums(T, E, groups, kept, k, splits, scoring):
         keep = torch.zeros_like(gs, dtype=torch.bool).scatter_(1, order[:, :kept], True)
         choice = torch.where(keep.repeat_interleave(E // groups, 1), choice, 0.0)
     gap, want = torch.sort(choice, dim=-1, descending=True, stable=True)
+    compared = 0
     for t in range(T):
-        # picks are compared up to the first pair that f32 could order either way
-        close = ((gap[t, :k] - gap[t, 1:k + 1]) < 1e-5).nonzero().view(-1) if k < E else torch.tensor([], dtype=torch.int64)
-        n = (int(close[0]) if len(close) else k) if sure[t] else 0
-        got = idx[t].cpu()
-        assert torch.equal(got[:n], want[t, :n])
-        ref = score[t, got] / (score[t, got].sum() + 1e-20) * 1.5
+        assert len(set(idx[t].tolist())) == k
         # a few f32 roundings of the scores and of their sum of up to 32 terms
-        assert float(((w[t].cpu().double() - ref) / ref).abs().max()) < 40 * 2 ** -23
+        ref = score[t, idx[t]] / (score[t, idx[t]].sum() + 1e-20) * 1.5
+        assert float(((w[t].double() - ref) / ref).abs().max()) < 40 * 2 ** -23
+        if not sure[t]:
+            continue
+        assert bool((choice[t, idx[t]] > 0).all())                  # of the groups that were kept
+        # picks are compared up to the first pair that f32 could order either way
+        close = (gap[t, :k] - gap[t, 1:k + 1] < 1e-5).nonzero().view(-1)
+        n = int(close[0]) if len(close) else k
+        assert torch.equal(idx[t, :n], want[t, :n])
+        compared += n == k
+    assert compared >= max(1, T - 1)
+
+
+@pytest.mark.parametrize("T", [1, 9])
+@pytest.mark.parametrize("E,groups,kept,k", [(8, 1, 1, 4), (32, 4, 2, 8), (255, 5, 2, 8), (384, 1, 1, 32), (1024, 32, 7, 32)])
+@pytest.mark.parametrize("scoring", [0, 1])
+def test_selection_takes_the_lower_id_of_equals(T, E, groups, kept, k, scoring):
+    """Three different logits over all experts: almost every comparison, of experts and of groups, is a tie."""
+    g = torch.Generator().manual_seed(E)
+    level = torch.tensor([-1.0, 0.0, 2.0])
+    which = torch.randint(0, 3, (1, T, E + 3), generator=g)
+    idx, _ = _select(level[which], torch.zeros(E), E, k, groups, kept, scoring)
+    choice = (level.sigmoid() if scoring == 0 else level.exp())[which[0, :, :E]]     # orders as the scores do
+    if groups > 1:
+        gs = choice.view(T, groups, -1).topk(2, dim=-1)[0].sum(-1)
+        order = torch.sort(gs, dim=-1, descending=True, stable=True)[1][:, :kept]
+        keep = torch.zeros(T, groups, dtype=torch.bool).scatter_(1, order, True)
+        choice = torch.where(keep.repeat_interleave(E // groups, 1), choice, 0.0)
+    assert torch.equal(idx, torch.sort(choice, dim=-1, descending=True, stable=True)[1][:, :k])
 
 
 # a thread per expert for one token (or what fits beside it), a warp per token otherwise; 1, 8, 16 and 32 experts a lane
@@ -103,22 +134,14 @@ def test_selection_from_partial_sums(T, E, groups, kept, k, splits, scoring):
 @pytest.mark.parametrize("scoring", [0, 1])
 def test_selection_does_not_depend_on_the_batch(E, groups, kept, splits, scoring):
     """The sums run in the order of the splits in either form: the same bits."""
-    from llm_kernels_b200 import _native as N
-    g = torch.Generator(device="cuda").manual_seed(E)
-    T, k, stride = 13, min(8, E), E + 3
-    part = torch.randn(splits, T, stride, generator=g, device="cuda")
-    bias = torch.randn(E, generator=g, device="cuda")
-
-    def select(part):
-        n = part.shape[1]
-        idx, w = torch.full((n, k), -1, dtype=torch.int64, device="cuda"), torch.full((n, k), -1.0, device="cuda")
-        N.check(N.lib().b200moe_router_select(part.data_ptr(), splits, stride, bias.data_ptr(), n, E, k, groups, kept, scoring, 1, 2.5,
-                                              idx.data_ptr(), w.data_ptr(), N.stream()))
-        return idx, w
-    whole = select(part)
+    g = torch.Generator().manual_seed(E)
+    T, k = 13, min(8, E)
+    part = torch.randn(splits, T, E + 3, generator=g)
+    bias = torch.randn(E, generator=g)
+    whole = _select(part, bias, E, k, groups, kept, scoring)
     for n in (1, 2, 3, 5):
         for t in range(0, T - n + 1, n):
-            for a, b in zip(whole, select(part[:, t:t + n].contiguous())):
+            for a, b in zip(whole, _select(part[:, t:t + n].contiguous(), bias, E, k, groups, kept, scoring)):
                 assert torch.equal(_bits(a[t:t + n]), _bits(b))
 
 
@@ -301,3 +324,84 @@ def test_compiled_calls_let_other_threads_run(kind):
     torch.cuda.synchronize()
     assert waited >= 0.1, "no call met a full queue"
     assert longest_gap[0] < waited / 2
+
+
+def _split_calls(seed):
+    """Quantizers and split GEMMs of a linear layer, their scratch freed as they return: -> a function that gives the outputs."""
+    from llm_kernels_b200.quantization import fp8_kernel, w4a8_kernel
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    x = torch.randn(24, 1152, generator=g, device="cuda").to(torch.bfloat16)
+    w = torch.randn(384, 1152, generator=g, device="cuda") * 0.02
+    up = torch.randn(1152, 384, generator=g, device="cuda") * 0.02
+    weights = [(fp8_kernel.weight_quant(w), fp8_kernel.weight_quant(up)), (w4a8_kernel.weight_quant(w), w4a8_kernel.weight_quant(up))]
+
+    def run():
+        out = []
+        for mod, gemm, pair in ((fp8_kernel, fp8_kernel.fp8_gemm, weights[0]), (w4a8_kernel, w4a8_kernel.w4a8_gemm, weights[1])):
+            y = gemm(*mod.act_quant(x), *pair[0], out_dtype=torch.bfloat16)
+            out.append(gemm(*mod.act_quant(y), *pair[1], out_dtype=torch.bfloat16))
+        return out
+    return run
+
+
+def _alone(run):
+    """The same with the device idle between any two launches' calls."""
+    from llm_kernels_b200 import _native as N
+    calls = N.calls()
+
+    class Waiting:
+        def __getattr__(self, name):
+            def call(*args):
+                out = getattr(calls, name)(*args)
+                torch.cuda.synchronize()
+                return out
+            return call
+    N._calls_module = Waiting()
+    try:
+        return run()
+    finally:
+        N._calls_module = calls
+
+
+def test_dependent_launches_keep_the_order_of_the_stream():
+    """Short launches one after another, whose scratch and intermediate results are freed and taken again at once: a kernel that
+    started before its predecessor was through would read or overwrite what that one still uses.  Eager and captured."""
+    run = _split_calls(5)
+    want = _alone(run)
+    got = [run() for _ in range(50)]
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        outs = [run() for _ in range(5)]
+    for _ in range(10):
+        graph.replay()
+        got += [[t.clone() for t in out] for out in outs]
+    torch.cuda.synchronize()
+    for out in got:
+        for a, b in zip(out, want):
+            assert torch.equal(_bits(a), _bits(b))
+
+
+@pytest.mark.parametrize("own_streams", [False, True])
+def test_split_gemms_of_two_threads_have_scratch_of_their_own(own_streams):
+    """Compiled calls of two threads, on one stream or two, with other inputs each: the launches of the two come in any order."""
+    import threading
+    runs = [_split_calls(seed) for seed in (7, 8)]
+    want = [_alone(run) for run in runs]
+    got, start = [[], []], threading.Barrier(2)
+    torch.cuda.synchronize()
+
+    def work(i):
+        with torch.cuda.stream(torch.cuda.Stream() if own_streams else torch.cuda.default_stream()):
+            start.wait()
+            got[i] = [runs[i]() for _ in range(100)]
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    for i in range(2):
+        assert len(got[i]) == 100
+        for out in got[i]:
+            for a, b in zip(out, want[i]):
+                assert torch.equal(_bits(a), _bits(b))
