@@ -63,8 +63,9 @@ int launch_dependent(const char* what, void (*kernel)(P...), dim3 grid, int thre
 }
 
 // Router logits of few tokens on the CUDA cores (router.cu), from the operands of b200moe_router_logits_bf16x3 (gemm_fp8.cu).
-// us, tensor cores with 16 splits -> here: hidden size 7168, 256 experts 18.6 -> 14.7 for one token, 18.8 -> 22.5 for four; 4096
-// and 128 rows 14.4 -> 10.3 and 14.4 -> 16.4.
+// us without the selection, weight out of memory, tensor cores with 16 splits -> here: hidden size 7168, 256 experts 18.6 -> 14.4 for
+// one token, 18.5 -> 14.3 for two, 18.8 -> 22.5 for four; 4096 and 128 rows 14.3 -> 10.3, 14.3 -> 10.2, 14.4 -> 16.4; 1024 and 128 rows
+// 11.1 -> 6.3 for one, 10.4 -> 8.2 for two.
 constexpr int64_t kRouterFewTokens = 2;
 int router_logits_few(const void* x_bf16, const void* w3_bf16, float* logits, int64_t T, int64_t H, int E, cudaStream_t st);
 

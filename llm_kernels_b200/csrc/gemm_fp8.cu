@@ -171,8 +171,9 @@ __device__ __forceinline__ float tmem_value(uint32_t r) {
   else return __uint_as_float(r);
 }
 
-// acc[0..32) += value(r[0..32)) * s.  The promotion is bound by FMA issue slots (8 warps x 128
-// accumulators per K block), so f32 products go through the packed two-wide FMA.
+// acc[0..32) += value(r[0..32)) * s.  f32 products go through the packed two-wide FMA, half the issue slots of the scalar one.
+// The FMAs of a K block (8 warps x 128 accumulators) take 259 cycles by themselves and the tensor-memory loads 168, of the 1 040
+// to 1 060 that the promotion warps spend on it; what the rest goes to has not been taken apart.
 template <int KIND>
 __device__ __forceinline__ void promote32(float* acc, const uint32_t (&r)[32], float s) {
   if constexpr (KIND == kI8) {
@@ -501,9 +502,10 @@ gemm_block_kernel(const __grid_constant__ RowMaps tmap_a,
           if (col0 >= p.N) continue;                       // warp-uniform
           if constexpr (!kPromote) {
             // f32 rows of a launch with several tiles per CTA (the router's partial sums) go through shared memory as the
-            // 16-bit rows below, 32 columns at a time: 4096 tokens 88 -> 58 us.  With one tile per CTA this code is fetched
-            // for one use, which costs more than the direct stores (one token 13.7 us direct, 18.8 us this way); in the
-            // block-scaled kinds its registers slow every tile down (4096 x 7168 x 7168: 248 -> 259 us).
+            // 16-bit rows below, 32 columns at a time: 7168 x 256 experts, 4096 tokens 68 -> 51 us.  With one tile per CTA the
+            // direct stores are the better form for few rows (16 tokens 12.2 us, 14.0 this way) but not for full tiles (128
+            // tokens 17.9 and 14.9).  In the block-scaled kinds its registers slow every tile down (4096 x 7168 x 7168: 248 ->
+            // 259 us).
             if (p.c_dtype == B200MOE_F32 && !one_tile) {
               uint8_t* stg = sh->out_stage[e];
 #pragma unroll

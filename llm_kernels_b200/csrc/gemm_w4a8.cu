@@ -598,8 +598,8 @@ extern "C" int b200moe_grouped_gemm_w4a8(const void* a, int64_t a_row_stride_byt
                 seg_indptr, weight_indices, M_total, static_cast<int>(N), static_cast<int>(K), num_groups, c_dtype,
                 epilogue != 0 ? 1 : 0, epilogue == 4 ? 1 : 0, status_word};
   if (int rc = set_dynamic_smem(reinterpret_cast<const void*>(w4::gemm_w4a8_kernel), w4::kSmem8)) return rc;
-  // a plain launch: two of 0.4 ms or more follow each other here, and as dependent launches they gained nothing (3000 tokens of a
-  // DeepSeek-V3 layer 4616 us plain, 4624 dependent; 64 tokens 1238 and 1251)
+  // a plain launch: as dependent launches these long kernels gained nothing (DeepSeek-V3 layer of 64 tokens 1273 us either way, of
+  // 3000 tokens 4585 us plain, 4637 dependent; two runs of one side differ by 0.5 %)
   w4::gemm_w4a8_kernel<<<sms, w4::kThreads8, w4::kSmem8, as_stream(stream)>>>(ma, mp, p);
   return check_launch("gemm_w4a8_kernel");
 }

@@ -117,6 +117,8 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) route_rank_kernel(
 // The whole sort in one launch, a block of 1024 threads per chunk of 1024 slots.  Each block reads all ids and counts those
 // before, in and after its chunk, which costs n * 8 bytes from L2 per block instead of two more launches; the slots of the
 // chunk are ranked by 32 warps side by side instead of by one warp in 32 steps.
+// us, three launches -> one: 1024 slots over 256 experts 22.7 -> 4.2, 32768 25.6 -> 8.0, 65536 28.7 -> 11.9; 65536 slots all of one
+// expert 22.7 -> 11.0, over 1024 experts 30.9 -> 13.2.  The cost of every block grows with the slots; more were not tried.
 constexpr int64_t kOneLaunchSlots = 65536;
 constexpr int kOneWarps = kChunk / 32;
 

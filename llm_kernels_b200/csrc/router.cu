@@ -264,7 +264,8 @@ __global__ void __launch_bounds__(256) router_tiled_kernel(const T* __restrict__
 // logits[t, e] = x[t] . w[e] in f32, w given as its three bf16 parts side by side (hi + mid + lo = w exactly).  Bound by the
 // 6 E H bytes of the parts.  A block takes two experts and up to two tokens, four warps an expert, each a quarter of the columns;
 // their sums are added in order.
-constexpr int kFewTokens = 2;
+constexpr int kFewTokens = static_cast<int>(kRouterFewTokens);
+static_assert((kFewTokens & (kFewTokens - 1)) == 0, "tokens of a block are told apart by a mask");
 __global__ void __launch_bounds__(256) router_few_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w3,
                                                          float* __restrict__ logits, int64_t T, int64_t H, int E) {
   __shared__ float part[8][kFewTokens];

@@ -101,9 +101,11 @@ def w4a8_gemm(a: torch.Tensor, a_s: torch.Tensor, b: torch.Tensor, b_s: torch.Te
 
 
 def _gemm_dense(a, a_s, b, b_s, b_s4, b_z4, M, K, out_dtype):
-    """w4a8_gemm of operands that agree on M, N and K: one launch expands the weight and turns f16 scales into f32, the GEMM
-    follows.  Everything in between is one allocation of the call's own: memory of the caching allocator is ordered by stream,
-    belongs to a graph that captures the call, and calls of two threads on one stream do not meet in it."""
+    """w4a8_gemm of operands that agree on M, N and K, where the compiled call does not take them (tensor subclasses, scales of other
+    types, no module for this torch); the launches are the same as there (csrc/calls.cpp).  One launch expands the weight and turns
+    f16 scales into f32, the GEMM follows.  Everything in between is one allocation of the call's own: memory of the caching
+    allocator is ordered by stream, belongs to a graph that captures the call, and calls of two threads on one stream do not meet
+    in it."""
     N.require_cuda(a, a_s, b, b_s, b_s4, b_z4)
     assert a.dtype == torch.int8
     Nn = b.size(0) * 8
